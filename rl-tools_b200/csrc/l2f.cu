@@ -304,12 +304,13 @@ __device__ __forceinline__ float l2f_reward(const L2fArgs& a, const float (&mdp)
     return (reward > 0 || mdp[0] == 0.0f) ? reward : 0.0f;
 }
 
-// One CTA of 14 warps per SM: 448 quadrotors, so 65536 of them (443 per SM) are resident at once. A lane owns one quadrotor for the
+// One CTA of up to 14 warps per SM: 448 quadrotors, so 65536 of them (443 per SM) are resident at once; fewer quadrotors take CTAs of as many
+// warps as spread them over all SMs (launch_l2f_rollout). A lane owns one quadrotor for the
 // environment part (reset, observe, step, reward) and, for the two hidden layers, a register tile of 8 quadrotors x H/8 units of its warp's
 // 32 x H product: operands come from shared memory as 16-byte loads that each feed 32 multiply-adds (one broadcast weight per multiply-add,
 // as a thread-per-quadrotor layer would load it, leaves the kernel bound by shared-memory wavefronts). Every unit still accumulates
 // bias + sum over k in ascending k with fused multiply-adds, so the actor's values are those of a plain per-sample loop.
-constexpr int L2F_ROLLOUT_WARPS = 14, L2F_ROLLOUT_THREADS = 32 * L2F_ROLLOUT_WARPS;
+constexpr int L2F_ROLLOUT_WARPS = 14, L2F_ROLLOUT_THREADS = 32 * L2F_ROLLOUT_WARPS;      // the most of a CTA
 template <int H>
 struct L2fRolloutLayout {
     static constexpr int O = 18, A = 4;
@@ -319,7 +320,7 @@ struct L2fRolloutLayout {
     // floats from the start of shared memory; the first two layers transposed ([k][slot]), the last as [unit][4]
     static constexpr int W1T = 0, B1 = W1T + O * H, W2T = B1 + H, B2 = W2T + H * H, W3T = B2 + H, B3 = W3T + A * H, WARP0 = B3 + A;
     static constexpr int OBS_TILE = O * 32, HID_TILE = H * PITCH, PER_WARP = OBS_TILE + HID_TILE;
-    static constexpr size_t BYTES = sizeof(float) * (WARP0 + L2F_ROLLOUT_WARPS * PER_WARP);
+    static constexpr size_t bytes(int warps){ return sizeof(float) * (WARP0 + (size_t)warps * PER_WARP); }
     __host__ __device__ static constexpr int slot(int j){ return ((j / 8) / VW) * (8 * VW) + (j % 8) * VW + (j / 8) % VW; }
 };
 
@@ -483,9 +484,14 @@ __global__ void __launch_bounds__(L2F_ROLLOUT_THREADS, 1) l2f_rollout_kernel(L2f
 
 template <int H>
 static int launch_l2f_rollout(const L2fRolloutArgs& a, cudaStream_t s){
-    constexpr size_t SMEM = L2fRolloutLayout<H>::BYTES;
-    B200RL_CUDA_TRY(cudaFuncSetAttribute(l2f_rollout_kernel<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM));
-    l2f_rollout_kernel<H><<<(a.n_envs + L2F_ROLLOUT_THREADS - 1) / L2F_ROLLOUT_THREADS, L2F_ROLLOUT_THREADS, SMEM, s>>>(a);
+    int sms = 0;
+    int rc = sm_count(&sms);
+    if(rc) return rc;
+    const int total = (a.n_envs + 31) / 32;
+    int warps = (total + sms - 1) / sms;
+    if(warps > L2F_ROLLOUT_WARPS) warps = L2F_ROLLOUT_WARPS;
+    B200RL_CUDA_TRY(cudaFuncSetAttribute(l2f_rollout_kernel<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L2fRolloutLayout<H>::bytes(L2F_ROLLOUT_WARPS)));
+    l2f_rollout_kernel<H><<<(total + warps - 1) / warps, 32 * warps, L2fRolloutLayout<H>::bytes(warps), s>>>(a);
     B200RL_LAUNCH_CHECK("l2f_rollout");
     return B200RL_OK;
 }

@@ -207,6 +207,18 @@ int b200rl_adam_advance_dev(const float* hyper9, uint32_t* age, float* c1, float
 int b200rl_adam_update_dev(float* params, const float* grads, float* m, float* v, size_t n, const float* hyper9, const float* c1,
                            const float* c2, b200rl_stream_t stream);
 
+/* One whole training step of a network on `rows` rows in chunks of `chunk_rows` (a divisor of rows): gradients zeroed, then per chunk
+ * forward, mean-squared-error gradient with `loss_weight` (b200rl_mse_gradient on the chunk) and backward, gradients accumulating over the
+ * chunks; with optimize != 0 one Adam step over the n parameters of the arena (n may exceed the network's own parameters, which the
+ * optimizer then steps with zero gradients). The sequence nn_models::mlp callers run as zero_gradient / forward / mse::gradient / backward /
+ * step, as one call, so that small batches can be one launch instead of a chain of them. pre / out hold the LAST chunk's activations
+ * afterwards (as b200rl_mlp_forward leaves them); d_out, tick, tock, scratch and workspace are work areas, sized for chunk_rows rows as for
+ * the separate calls (scratch: b200rl_mlp_backward_scratch_bytes, 16-byte aligned). */
+int b200rl_mlp_train_step(const b200rl_mlp_shape* shape, float* params, float* grads, float* m, float* v, size_t n, b200rl_adam_hyper hyper, uint32_t* state,
+                          const float* x, int ldx, const float* target, int ldt, int rows, int chunk_rows, float loss_weight, float* pre, float* out, float* d_out,
+                          float* tick, float* tock, void* scratch, size_t scratch_bytes, void* workspace, size_t workspace_bytes, int optimize,
+                          b200rl_stream_t stream);
+
 /* ---------------------------------------------------------------------------------------------------------
  * PPO update pieces (host scalar loops in the reference, which therefore cannot run on its CUDA device).
  * All column arguments carry an element pitch (ld_*): pass the dataset matrix's row pitch to work on column views of the

@@ -12,7 +12,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB_PATH = os.path.join(HERE, "libb200rl.so")
-SOURCES = ["dense.cu", "dense_tc.cu", "dense_skinny.cu", "mlp_fused.cu", "mlp_coop.cu", "adam.cu", "rollout.cu", "rollout_tc.cu", "ppo.cu", "host_api.cu", "sac.cu", "normalize.cu", "rollout_env.cu", "l2f.cu"]
+SOURCES = ["dense.cu", "dense_tc.cu", "dense_skinny.cu", "mlp_fused.cu", "mlp_coop.cu", "mlp_team.cu", "adam.cu", "rollout.cu", "rollout_tc.cu", "ppo.cu", "host_api.cu", "sac.cu", "normalize.cu", "rollout_env.cu", "l2f.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-shared"]
 # per-source flags: the quadrotor dynamics keep the reference's association of every expression (bit-for-bit parity with its CPU step)
 SOURCE_FLAGS = {"l2f.cu": ["-fmad=false"]}
@@ -152,6 +152,7 @@ def lib():
         L.b200rl_mlp_backward_scratch_bytes.argtypes = [shape_p, i]
         L.b200rl_mlp_backward_scratch_bytes.restype = sz
         L.b200rl_mlp_backward.argtypes = [shape_p, vp, vp, vp, i, vp, vp, vp, vp, vp, vp, i, vp, sz, vp]
+        L.b200rl_mlp_train_step.argtypes = [shape_p, vp, vp, vp, vp, sz, AdamHyper, vp, vp, i, vp, i, i, i, f, vp, vp, vp, vp, vp, vp, sz, vp, sz, i, vp]
         L.b200rl_adam_reset.argtypes = [vp, vp]
         L.b200rl_adam_step.argtypes = [vp, vp, vp, vp, sz, AdamHyper, vp, vp]
         L.b200rl_pendulum_rollout.argtypes = [shape_p, vp, vp, vp, vp, vp, vp, i, i, i, i, vp, vp, vp, vp, vp]
@@ -221,13 +222,15 @@ def check(status: int, what: str = ""):
         raise B200RLError(f"{what} failed with status {status} ({msg})")
 
 
+# What a call costs on the host decides the small calls (a policy inference is 5 us on the GPU): addresses travel as plain integers (the
+# argument types turn them into pointers), and the current stream is looked up without building a Stream object.
 def _ptr(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _stream():
-    import torch
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    from torch import _C
+    return _C._cuda_getCurrentRawStream(_C._cuda_getDevice())
 
 
 def _act(a):
@@ -455,6 +458,14 @@ class Mlp:
         check(lib().b200rl_mlp_backward(C.byref(self.shape), _ptr(self.params), _ptr(self.grads) if accumulate_gradients else None, _ptr(x), x.stride(0), _ptr(self.pre), _ptr(self.out),
                                         _ptr(d_out), _ptr(d_input), _ptr(self.tick), _ptr(self.tock), self.batch, _ptr(self.scratch), self.scratch_bytes,
                                         _stream()), "b200rl_mlp_backward")
+
+    def train_step(self, x, target, loss_weight=1.0, optimize=True):
+        """zero_gradient, then forward / mse_gradient / backward over chunks of `batch` rows of x and target, then (optimize) step: one native call."""
+        check(lib().b200rl_mlp_train_step(C.byref(self.shape), self.params.data_ptr(), self.grads.data_ptr(), self.m.data_ptr(), self.v.data_ptr(), self.params.numel(),
+                                          self.hyper, self.adam_state.data_ptr(), x.data_ptr(), x.stride(0), target.data_ptr(), target.stride(0), x.shape[0], self.batch,
+                                          loss_weight, self.pre.data_ptr(), self.out.data_ptr(), self.d_out_buffer().data_ptr(), self.tick.data_ptr(), self.tock.data_ptr(),
+                                          self.scratch.data_ptr(), self.scratch_bytes, self.workspace.data_ptr(), self.workspace_bytes, optimize, _stream()),
+              "b200rl_mlp_train_step")
 
     def zero_gradient(self):
         fill(self.grads, 0.0)

@@ -513,6 +513,13 @@ int mlp_fused_forward(const b200rl_mlp_shape* sh, const float* params, const flo
 int mlp_fused_backward(const b200rl_mlp_shape* sh, const float* params, float* grads, const float* x, int ldx, const float* pre, const float* out, float* d_out,
                        float* d_input, int batch, void* scratch, size_t scratch_bytes, cudaStream_t s);
 
+// whole training step in one cooperative launch (mlp_team.cu)
+bool mlp_team_eligible(const b200rl_mlp_shape* sh, int rows);
+size_t mlp_team_scratch_bytes(const b200rl_mlp_shape* sh, int rows);
+int mlp_team_step(const b200rl_mlp_shape* sh, float* params, float* grads, float* m, float* v, size_t n_total, const b200rl_adam_hyper& hyper, uint32_t* adam_state,
+                  const float* x, int ldx, const float* target, int ldt, int rows, int chunk_rows, float loss_weight, float* pre, float* out, void* scratch, size_t scratch_bytes,
+                  int optimize, cudaStream_t s);
+
 // whole-pass cooperative kernel for wide networks at small batches (mlp_coop.cu)
 bool mlp_coop_eligible(const b200rl_mlp_shape* sh, int batch, bool forward);
 int mlp_coop_forward(const b200rl_mlp_shape* sh, const float* params, const float* x, int ldx, float* pre, float* out, float* y, int ldy,
@@ -524,6 +531,12 @@ static bool valid_shape(const b200rl_mlp_shape* sh){
     if(!sh || sh->n_layers < 1 || sh->n_layers > B200RL_MAX_LAYERS || sh->input_dim < 1) return false;
     for(int l = 0; l < sh->n_layers; l++) if(sh->dims[l] < 1 || !valid_activation(sh->acts[l])) return false;
     return true;
+}
+
+static size_t outputs_before_last(const b200rl_mlp_shape* sh){
+    size_t n = 0;
+    for(int l = 0; l + 1 < sh->n_layers; l++) n += (size_t)sh->dims[l];
+    return n;
 }
 
 }  // namespace b200rl
@@ -671,8 +684,9 @@ size_t b200rl_mlp_backward_scratch_bytes(const b200rl_mlp_shape* sh, int batch){
     if(!valid_shape(sh) || batch < 1) return 0;
     size_t m = 0; int I = sh->input_dim;
     for(int l = 0; l < sh->n_layers; l++){ const size_t b = backward_scratch_total(batch, I, sh->dims[l]); if(b > m) m = b; I = sh->dims[l]; }
-    const size_t fused = mlp_fused_backward_scratch_bytes(sh, batch);
-    return fused > m ? fused : m;
+    const size_t fused = mlp_fused_backward_scratch_bytes(sh, batch), team = mlp_team_scratch_bytes(sh, batch);
+    if(fused > m) m = fused;
+    return team > m ? team : m;
 }
 
 int b200rl_mlp_backward(const b200rl_mlp_shape* sh, const float* params, float* grads, const float* x, int ldx, const float* pre,
@@ -703,6 +717,31 @@ int b200rl_mlp_backward(const b200rl_mlp_shape* sh, const float* params, float* 
         d_cur = d_in; ldd = I;
     }
     return B200RL_OK;
+}
+
+int b200rl_mlp_train_step(const b200rl_mlp_shape* sh, float* params, float* grads, float* m, float* v, size_t n, b200rl_adam_hyper hyper, uint32_t* state,
+                          const float* x, int ldx, const float* target, int ldt, int rows, int chunk_rows, float loss_weight, float* pre, float* out, float* d_out,
+                          float* tick, float* tock, void* scratch, size_t scratch_bytes, void* workspace, size_t workspace_bytes, int optimize, b200rl_stream_t stream){
+    if(!valid_shape(sh) || !params || !grads || !x || !target || !pre || !out || !d_out || rows < 1 || chunk_rows < 1 || rows % chunk_rows != 0 || ldx < sh->input_dim ||
+       ldt < sh->dims[sh->n_layers - 1] || n < b200rl_mlp_num_params(sh) || (optimize && (!m || !v || !state)))
+        return B200RL_ERR_INVALID_ARGUMENT;
+    const int L = sh->n_layers, O = sh->dims[L - 1];
+    if(L > 1 && (!tick || (L > 2 && !tock))) return B200RL_ERR_INVALID_ARGUMENT;
+    if(mlp_team_eligible(sh, rows)){
+        const int rc = mlp_team_step(sh, params, grads, m, v, n, hyper, state, x, ldx, target, ldt, rows, chunk_rows, loss_weight, pre, out, scratch, scratch_bytes, optimize,
+                                     (cudaStream_t)stream);
+        if(rc != B200RL_ERR_UNSUPPORTED) return rc;
+    }
+    int rc = b200rl_fill(grads, n, 0.0f, stream);
+    if(rc) return rc;
+    const float* last = out + outputs_before_last(sh) * (size_t)chunk_rows;
+    for(int r = 0; r < rows; r += chunk_rows){
+        const float* xc = x + (size_t)r * ldx;
+        if((rc = b200rl_mlp_forward_ws(sh, params, xc, ldx, pre, out, chunk_rows, workspace, workspace_bytes, stream))) return rc;
+        if((rc = b200rl_mse_gradient(last, O, target + (size_t)r * ldt, ldt, d_out, O, chunk_rows, O, loss_weight, stream))) return rc;
+        if((rc = b200rl_mlp_backward(sh, params, grads, xc, ldx, pre, out, d_out, nullptr, tick, tock, chunk_rows, scratch, scratch_bytes, stream))) return rc;
+    }
+    return optimize ? b200rl_adam_step(params, grads, m, v, n, hyper, state, stream) : B200RL_OK;
 }
 
 }  // extern "C"

@@ -15,6 +15,7 @@
 // The barrier counts arrivals in a device word and spins with a limit; a launch that runs into the limit sets a sticky status word and
 // all of its CTAs return. The launch is cooperative, so all CTAs are resident together whatever else the device runs.
 #include "common.cuh"
+#include "grid_barrier.cuh"
 #include <cstdlib>
 #include <mutex>
 #include <vector>
@@ -23,7 +24,6 @@ namespace b200rl {
 
 constexpr int CO_T = 32, CO_KC = 256, CO_PITCH = 36, CO_THREADS = 256, CO_WARPS = 8;
 constexpr size_t CO_SMEM = sizeof(float) * 2 * CO_KC * CO_PITCH;          // both operand tiles; the eight partial tiles (32 KB) reuse the space
-constexpr unsigned CO_SPIN_LIMIT = 1000000u;                              // polls of the barrier words (two L2 round trips each): about a second
 // Barrier words per device, handed out round-robin per launch (a captured launch keeps the slot it got at capture time). Two launches may
 // share a slot as long as they never run at the same time: launches on one stream never do, and the parallel branches of one captured graph
 // get consecutive slots. What is not supported: two launches whose slots coincide after a wrap of the ring (4,096 launches apart) running
@@ -48,25 +48,11 @@ static_assert(sizeof(CoopArgs) <= 4000, "kernel arguments");
 
 static __device__ unsigned g_coop_barriers[CO_SLOTS * 4];                 // per slot: arrivals, exits, status (sticky), unused
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p){
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 // false: the wait ran into its limit (or another CTA's did)
 __device__ bool coop_barrier(unsigned* bar, unsigned target){
     __shared__ int ok_s;
     __syncthreads();
-    if(threadIdx.x == 0){
-        __threadfence();
-        atomicAdd(bar, 1u);
-        int ok = 1;
-        unsigned spins = 0;
-        while(ld_acquire_u32(bar) < target){
-            if(++spins > CO_SPIN_LIMIT || ld_acquire_u32(bar + 2) != 0u){ atomicExch(bar + 2, 1u); ok = 0; break; }
-        }
-        ok_s = ok;
-    }
+    if(threadIdx.x == 0){ grid_barrier_arrive(bar); ok_s = grid_barrier_wait(bar, target); }
     __syncthreads();
     return ok_s != 0;
 }
@@ -257,10 +243,7 @@ __global__ void __launch_bounds__(CO_THREADS, 1) mlp_coop_kernel(CoopArgs a){
         }
     }
     // the last CTA out clears the slot for its next launch (every CTA has left the last barrier before it counts itself out)
-    if(threadIdx.x == 0 && a.n_phases > 1){
-        const unsigned old = atomicAdd(a.barrier + 1, 1u);
-        if(old == gridDim.x - 1){ a.barrier[0] = 0u; a.barrier[1] = 0u; __threadfence(); }
-    }
+    if(threadIdx.x == 0 && a.n_phases > 1) grid_barrier_leave(a.barrier, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------------------------
@@ -282,7 +265,7 @@ bool mlp_coop_eligible(const b200rl_mlp_shape* sh, int batch, bool forward){
     return true;
 }
 
-static int coop_slot(unsigned** out){
+int grid_barrier_slots(int count, unsigned** out){
     static unsigned* base[MAX_DEVICES] = {};
     static unsigned next[MAX_DEVICES] = {};
     static std::mutex mutex;
@@ -295,7 +278,9 @@ static int coop_slot(unsigned** out){
         B200RL_CUDA_TRY(cudaGetSymbolAddress(&p, g_coop_barriers));
         base[dev] = static_cast<unsigned*>(p);
     }
-    *out = base[dev] + 4 * (next[dev]++ % CO_SLOTS);
+    if(next[dev] + (unsigned)count > (unsigned)CO_SLOTS) next[dev] = 0;
+    *out = base[dev] + 4 * next[dev];
+    next[dev] += (unsigned)count;
     return B200RL_OK;
 }
 
@@ -313,7 +298,7 @@ static int coop_launch(CoopArgs& a, cudaStream_t s){
         if(items > most) most = items;
     }
     const int grid = most < sms ? most : sms;
-    rc = coop_slot(&a.barrier);
+    rc = grid_barrier_slots(1, &a.barrier);
     if(rc) return rc;
     B200RL_CUDA_TRY(cudaFuncSetAttribute(mlp_coop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CO_SMEM));
     void* params[] = { &a };

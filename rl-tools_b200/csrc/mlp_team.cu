@@ -1,0 +1,257 @@
+// One training step of a network in ONE cooperative launch: gradients zeroed, forward, mean-squared-error gradient, backward, gradient sums over
+// the whole batch, optimizer step -- for batches that leave the tensor-core kernels without enough row tiles (the replay batches of the off-policy
+// algorithms, the minibatches of the on-policy ones). Built on the team walk of mlp_team.cuh: a team of C CTAs takes tiles of R rows through the
+// network, the teams' gradient sums meet in scratch memory behind one grid-wide barrier.
+// Same operations as zero_gradient, forward, mse::gradient, backward, step (nn_models/mlp/operations_generic.h:77-217,
+// nn/loss_functions/mse/operations_generic.h:43-58, nn/optimizers/adam/operations_generic.h:49-64) run one after the other.
+#include "common.cuh"
+#include "grid_barrier.cuh"
+#include "mlp_team.cuh"
+#include <atomic>
+#include <mutex>
+
+namespace b200rl {
+using namespace team;
+
+struct TeamStepArgs {
+    Net net;
+    float* params; float* grads; float* m; float* v; uint32_t* adam_state;
+    b200rl_adam_hyper hyper;
+    const float* x; const float* target; int ldx, ldt;
+    float* pre; float* out;
+    float4* partial; unsigned* barrier;
+    int rows, chunk_rows, n_total, optimize, row_tiles, teams, lanes;
+    float constant;                          // 2 / (rows of a chunk x columns) x loss weight, evaluated like the reference does
+    int stage_x, stage_y, y_off, out_off;    // shared-memory offsets: next tile's rows as they come, this tile's targets and outputs
+};
+
+template <int C, int L, int TPT>
+__global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_constant__ TeamStepArgs a){
+    extern __shared__ __align__(16) float smem[];
+    __shared__ float s_scalars[2];
+    __shared__ int s_ok;
+    const Net& n = a.net;
+    const int tid = threadIdx.x, rank = C == 1 ? 0 : (int)cluster_rank(), t = blockIdx.x / C;
+    const Layer& last = n.layer[L - 1];
+    const int I0 = n.layer[0].I, R = n.R;
+    auto stage = [&](int tile){              // the tile's input rows and this CTA's target columns, zero beyond the batch
+        const int row0 = tile * R;
+        for(int i = tid; i < R * I0; i += THREADS){
+            const int r = quotient(i, n.by_I0), k = i - r * I0;
+            if(row0 + r < a.rows) copy4_async(smem + a.stage_x + i, a.x + (size_t)(row0 + r) * a.ldx + k);
+            else smem[a.stage_x + i] = 0.0f;
+        }
+        for(int i = tid; i < R * last.S; i += THREADS){
+            const int r = quotient(i, last.by_S), unit = rank * last.S + i - r * last.S;
+            if(row0 + r < a.rows && unit < last.O) copy4_async(smem + a.stage_y + i, a.target + (size_t)(row0 + r) * a.ldt + unit);
+        }
+    };
+    stage(t);
+    clear_rows<L>(n, smem);
+    load_weights<L>(n, smem, a.params, rank);
+    Patch patches[TPT];
+    float2 acc[TPT][4][2];
+#pragma unroll
+    for(int k = 0; k < TPT; k++){
+        patches[k] = patch<L>(n, k * THREADS + tid);
+#pragma unroll
+        for(int i = 0; i < 4; i++){ acc[k][i][0] = make_float2(0.0f, 0.0f); acc[k][i][1] = make_float2(0.0f, 0.0f); }
+    }
+    const int keep_from = a.rows - a.chunk_rows;          // the activations of the last chunk stay behind in pre / out
+    for(int tile = t; tile < a.row_tiles; tile += a.teams){
+        copies_wait();
+        __syncthreads();
+        for(int i = tid; i < R * I0; i += THREADS){ const int r = quotient(i, n.by_I0), k = i - r * I0; smem[n.layer[0].a + r * n.layer[0].P + k] = smem[a.stage_x + i]; }
+        for(int i = tid; i < R * last.S; i += THREADS) smem[a.y_off + i] = smem[a.stage_y + i];
+        sync_team<C>();                                   // also: every CTA of the team has set its buffers up before the first remote store
+        if(tile + a.teams < a.row_tiles) stage(tile + a.teams);
+        const int row0 = tile * R;
+#pragma unroll
+        for(int l = 0; l < L; l++){
+            const Layer& y = n.layer[l];
+            forward_layer<C, L>(n, l, smem, rank, [&](int r, int unit, int idx, float value, float derivative){
+                if(l == L - 1){
+                    smem[y.d + idx] = row0 + r < a.rows ? __fmul_rn(__fsub_rn(value, smem[a.y_off + idx]), a.constant) * derivative : 0.0f;
+                    smem[a.out_off + idx] = value;
+                }
+            });
+            if(l == L - 1) __syncthreads();
+            else sync_team<C>();
+        }
+#pragma unroll
+        for(int l = L - 1; l > 0; l--) backward_layer<C>(n, l, smem, rank, (L - l) & 1);
+        store_activations<L>(n, smem, smem + a.out_off, rank, row0, a.rows, keep_from, a.chunk_rows, a.pre, a.out);
+        accumulate_gradients<TPT>(n, smem, patches, acc);
+        sync_team<C>();
+    }
+    store_gradients<C, TPT>(n, a.partial + (size_t)t * C * n.n_tiles * 4, rank, acc);
+    __syncthreads();
+    const uint32_t age = a.optimize ? *reinterpret_cast<volatile uint32_t*>(a.adam_state) : 1u;
+    if(tid == 0){ grid_barrier_arrive(a.barrier); s_ok = grid_barrier_wait(a.barrier, gridDim.x); }
+    else if(a.optimize && (tid == 32 || tid == 33)) s_scalars[tid - 32] = adam_bias_correction(tid == 32 ? a.hyper.beta_1 : a.hyper.beta_2, age);
+    __syncthreads();
+    if(!s_ok) return;
+    const float c1 = s_scalars[0], c2 = s_scalars[1];
+    struct Moments { float p, m, v; };
+    auto prefetch = [&](int i){ return a.optimize && i >= 0 ? Moments{a.params[i], a.m[i], a.v[i]} : Moments{0.0f, 0.0f, 0.0f}; };
+    auto sink = [&](int i, float g, Moments s){
+        a.grads[i] = g;
+        if(a.optimize){
+            a.params[i] = adam_update(s.p, g, s.m, s.v, a.hyper, c1, c2);
+            a.m[i] = s.m; a.v[i] = s.v;
+        }
+    };
+    reduce_gradients<C, L>(n, a.partial, a.teams, blockIdx.x, gridDim.x, a.lanes, prefetch, sink);
+    if(blockIdx.x == 0){
+        for(int i = n.n_params + tid; i < a.n_total; i += THREADS) sink(i, 0.0f, prefetch(i));      // parameters outside the layers: no gradient from this loss
+        if(tid == 0 && a.optimize){ a.adam_state[0] = age + 1u; a.adam_state[1] = 0u; a.adam_state[2] = __float_as_uint(c1); a.adam_state[3] = __float_as_uint(c2); }
+    }
+    if(tid == 0) grid_barrier_leave(a.barrier, gridDim.x);
+}
+
+// ---- host side ---------------------------------------------------------------------------------------------------------------------------
+struct TeamChoice { Net net; int C, teams, row_tiles, stage_x, stage_y, y_off, out_off; size_t smem; };
+
+constexpr size_t TEAM_SMEM = 220 * 1024;
+constexpr int TEAM_MAX_ROWS = 8192;          // beyond, the per-layer kernels' larger tiles are the better use of the SMs
+
+// teams of C CTAs that are resident at once on the current device (clusters do not tile every GPC completely); 0: unknown
+static int team_capacity(int C);
+
+// Team size and rows per tile by an estimate of the launch in clock cycles, with constants from timelines of the kernel (64- and 256-wide networks,
+// batches of 256 ... 5,003): a layer of a tile costs its latencies (about 2,000 cycles over both directions, twice that where the team exchanges
+// through cluster barriers) plus its products at a third of the multiply-add peak; loading the weights and adding the teams' sums cost per float.
+static bool choose_team(const b200rl_mlp_shape* sh, int rows, TeamChoice* out){
+    for(int l = 0, I = sh->input_dim; l < sh->n_layers; I = sh->dims[l], l++) if(sh->dims[l] > 512 || I > 512) return false;
+    double best = 0.0;
+    for(int C = 1; C <= 8; C *= 2){
+        const int max_teams = team_capacity(C);
+        if(max_teams < 1) continue;
+        for(int R = 4; R <= 32; R += 4){
+            TeamChoice c{};
+            if(!plan(sh, C, R, 0, &c.net)) continue;
+            c.C = C;
+            const Layer& last = c.net.layer[c.net.n_layers - 1];
+            int off = (c.net.end + 3) / 4 * 4;
+            c.stage_x = off; off += (R * sh->input_dim + 3) / 4 * 4;
+            c.stage_y = off; off += R * last.S;
+            c.y_off = off; off += R * last.S;
+            c.out_off = off; off += R * last.S;
+            c.smem = sizeof(float) * (size_t)off;
+            if(c.smem > TEAM_SMEM) continue;
+            c.row_tiles = (rows + R - 1) / R;
+            c.teams = c.row_tiles < max_teams ? c.row_tiles : max_teams;
+            double weights = 0.0, tile = 0.0;
+            for(int l = 0; l < c.net.n_layers; l++){
+                const Layer& y = c.net.layer[l];
+                weights += (double)y.S * y.P;
+                tile += (C == 1 ? 2000.0 : 4000.0) + 3.0 * R * y.S * y.P / 42.0;
+            }
+            const double cost = 0.15 * weights + tile * ((c.row_tiles + c.teams - 1) / c.teams) + 64.0 * C * c.net.n_tiles * c.teams / (12.0 * c.teams * C);
+            if(best == 0.0 || cost < best){ best = cost; *out = c; }
+        }
+    }
+    return best > 0.0;
+}
+
+bool mlp_team_eligible(const b200rl_mlp_shape* sh, int rows){
+    TeamChoice c;
+    return rows >= 1 && rows <= TEAM_MAX_ROWS && choose_team(sh, rows, &c);
+}
+// for any number of rows up to the limit (a training step may run over several chunks of the batch the scratch was asked for)
+size_t mlp_team_scratch_bytes(const b200rl_mlp_shape* sh, int rows){
+    TeamChoice c;
+    if(rows < 1 || !choose_team(sh, rows, &c)) return 0;
+    return sizeof(float4) * (size_t)team_capacity(c.C) * c.C * c.net.n_tiles * 4;
+}
+
+static void team_attributes(cudaLaunchAttribute (&attr)[2], int C){
+    attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = C; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeCooperative; attr[1].val.cooperative = 1;
+}
+template <int C>
+static int query_capacity(){
+    int n = 0;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    team_attributes(attr, C);
+    cfg.gridDim = dim3(NUM_SMS / C * C); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = TEAM_SMEM; cfg.attrs = attr; cfg.numAttrs = 1;
+    if(cudaFuncSetAttribute(mlp_team_step_kernel<C, 3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TEAM_SMEM) != cudaSuccess ||
+       cudaOccupancyMaxActiveClusters(&n, mlp_team_step_kernel<C, 3, 1>, &cfg) != cudaSuccess){ cudaGetLastError(); return 0; }
+    return n;
+}
+static int team_capacity(int C){
+    static std::atomic<int> cached[MAX_DEVICES][4];                      // capacity + 1
+    const int k = C == 1 ? 0 : C == 2 ? 1 : C == 4 ? 2 : 3;
+    int dev = 0;
+    if(cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES){ cudaGetLastError(); return 0; }
+    int n = cached[dev][k].load(std::memory_order_relaxed);
+    if(n == 0){
+        n = 1 + (k == 0 ? query_capacity<1>() : k == 1 ? query_capacity<2>() : k == 2 ? query_capacity<4>() : query_capacity<8>());
+        cached[dev][k].store(n, std::memory_order_relaxed);
+    }
+    return n - 1;
+}
+
+template <int C, int L, int TPT>
+static int launch_team_step(const TeamStepArgs& a, size_t smem, cudaStream_t s){
+    static std::atomic<bool> configured[MAX_DEVICES];
+    int dev = 0;
+    int rc = current_device(&dev);
+    if(rc) return rc;
+    if(!configured[dev].load(std::memory_order_acquire)){
+        B200RL_CUDA_TRY(cudaFuncSetAttribute(mlp_team_step_kernel<C, L, TPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TEAM_SMEM));
+        configured[dev].store(true, std::memory_order_release);
+    }
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    team_attributes(attr, C);
+    cfg.gridDim = dim3(a.teams * C); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = s; cfg.attrs = attr; cfg.numAttrs = 2;
+    B200RL_CUDA_TRY(cudaLaunchKernelEx(&cfg, mlp_team_step_kernel<C, L, TPT>, a));
+    return B200RL_OK;
+}
+template <int C, int L>
+static int launch_team_step_l(const TeamStepArgs& a, size_t smem, cudaStream_t s){
+    const int per_thread = (a.net.n_tiles + THREADS - 1) / THREADS;
+    if(per_thread <= 1) return launch_team_step<C, L, 1>(a, smem, s);
+    if(per_thread <= 2) return launch_team_step<C, L, 2>(a, smem, s);
+    if(per_thread <= 4) return launch_team_step<C, L, 4>(a, smem, s);
+    return launch_team_step<C, L, 8>(a, smem, s);
+}
+template <int C>
+static int launch_team_step_c(const TeamStepArgs& a, size_t smem, cudaStream_t s){
+    switch(a.net.n_layers){
+        case 1: return launch_team_step_l<C, 1>(a, smem, s);
+        case 2: return launch_team_step_l<C, 2>(a, smem, s);
+        case 3: return launch_team_step_l<C, 3>(a, smem, s);
+        default: return launch_team_step_l<C, 4>(a, smem, s);
+    }
+}
+
+int mlp_team_step(const b200rl_mlp_shape* sh, float* params, float* grads, float* m, float* v, size_t n_total, const b200rl_adam_hyper& hyper, uint32_t* adam_state,
+                  const float* x, int ldx, const float* target, int ldt, int rows, int chunk_rows, float loss_weight, float* pre, float* out, void* scratch, size_t scratch_bytes,
+                  int optimize, cudaStream_t s){
+    TeamChoice c;
+    if(!choose_team(sh, rows, &c) || !scratch || (reinterpret_cast<uintptr_t>(scratch) & 15u) || scratch_bytes < sizeof(float4) * (size_t)c.teams * c.C * c.net.n_tiles * 4)
+        return B200RL_ERR_UNSUPPORTED;
+    TeamStepArgs a{};
+    a.net = c.net;
+    a.params = params; a.grads = grads; a.m = m; a.v = v; a.adam_state = adam_state; a.hyper = hyper;
+    a.x = x; a.ldx = ldx; a.target = target; a.ldt = ldt; a.pre = pre; a.out = out;
+    a.partial = static_cast<float4*>(scratch);
+    a.rows = rows; a.chunk_rows = chunk_rows; a.n_total = (int)n_total; a.optimize = optimize; a.row_tiles = c.row_tiles; a.teams = c.teams;
+    a.constant = 2.0f / ((float)chunk_rows * (float)sh->dims[sh->n_layers - 1]) * loss_weight;
+    a.stage_x = c.stage_x; a.stage_y = c.stage_y; a.y_off = c.y_off; a.out_off = c.out_off;
+    // threads per quad of the reduction: as many as let the grid take all quads in one pass, no more than there are sums to add
+    const int quads = c.C * c.net.n_tiles * 4, threads = c.teams * c.C * THREADS;
+    a.lanes = 4;
+    while(a.lanes < 32 && 2 * a.lanes <= c.teams && (long long)quads * 2 * a.lanes <= threads) a.lanes *= 2;
+    int rc = grid_barrier_slots(1, &a.barrier);
+    if(rc) return rc;
+    if(c.C == 1) return launch_team_step_c<1>(a, c.smem, s);
+    if(c.C == 2) return launch_team_step_c<2>(a, c.smem, s);
+    if(c.C == 4) return launch_team_step_c<4>(a, c.smem, s);
+    return launch_team_step_c<8>(a, c.smem, s);
+}
+
+}  // namespace b200rl

@@ -34,13 +34,11 @@ def sharded_train_step(pkg, net, x_shard, y_shard, total_rows: int, dist=None, g
     on the current stream right before and right after the all-reduce, so that the exchange can be timed on its own."""
     rows = x_shard.shape[0]
     assert rows % net.batch == 0, "shard rows must be a multiple of the chunk size"
-    net.zero_gradient()
-    w = chunk_loss_weight(net.batch, total_rows)
-    for c in range(0, rows, net.batch):
-        x, y = x_shard[c:c + net.batch], y_shard[c:c + net.batch]
-        out = net.forward(x)
-        d_out = pkg.mse_gradient(out, y, w, d_a=net.d_out_buffer())
-        net.backward(x, d_out)
+    alone = dist is None or not dist.is_initialized() or dist.get_world_size(group) == 1
+    # one native call (small batches: one launch); the optimizer step is part of it where no exchange comes between
+    net.train_step(x_shard, y_shard, chunk_loss_weight(net.batch, total_rows), optimize=alone and exchange_events is None)
+    if alone and exchange_events is None:
+        return
     if exchange_events is not None:
         exchange_events[0].record()
     allreduce_sum_(net.grads, dist, group)

@@ -244,6 +244,25 @@ int b200rl_ppo_policy_gradient(const float* current_actions, int ld_current, con
                                float* d_log_std, int batch, int action_dim, float epsilon_clip, float entropy_coefficient, float advantage_epsilon,
                                int normalize_advantage, int learn_action_std, void* scratch, size_t scratch_bytes, b200rl_stream_t stream);
 
+/* All minibatch updates of one epoch in order: minibatch k are the rows [k batch, (k + 1) batch) of the column views (row pitch ld in elements for
+ * all of them). Per minibatch what the pieces above do one after the other for actor (with the log_std parameters behind its layers in the
+ * arena) and critic: gradients zeroed, forward, clipped-surrogate gradient / 0.5-weighted MSE gradient against the target values, backward, one
+ * Adam step each. Two launches (the advantages' statistics, then everything else) instead of about 24 per minibatch. Networks that do not fit
+ * the kernel (more than three layers, about 18,000 parameters) give B200RL_ERR_UNSUPPORTED; scratch: b200rl_ppo_train_epoch_scratch_bytes
+ * (0 for such networks), 16-byte aligned.
+ * Replaces the minibatch loop of train (rl/algorithms/ppo/operations_generic.h:159-336). */
+typedef struct {
+    float* params; float* grads; float* m; float* v;     /* arenas of n floats */
+    size_t n;
+    uint32_t* adam_state;                                /* as for b200rl_adam_step */
+    b200rl_adam_hyper hyper;
+} b200rl_mlp_arenas;
+size_t b200rl_ppo_train_epoch_scratch_bytes(const b200rl_mlp_shape* actor, const b200rl_mlp_shape* critic, int batch, int n_minibatches);
+int b200rl_ppo_train_epoch(const b200rl_mlp_shape* actor, const b200rl_mlp_arenas* actor_arenas, const b200rl_mlp_shape* critic, const b200rl_mlp_arenas* critic_arenas,
+                           const float* observations, const float* actions, const float* log_probs, const float* advantages, const float* target_values, int ld,
+                           int batch, int n_minibatches, float epsilon_clip, float entropy_coefficient, float advantage_epsilon, int normalize_advantage,
+                           int learn_action_std, void* scratch, size_t scratch_bytes, b200rl_stream_t stream);
+
 /* ---------------------------------------------------------------------------------------------------------
  * Device memory and copies for hosts compiled without the CUDA toolkit (the header-only adapter needs nothing but
  * this header). Replace cudaMalloc / cudaFree / cudaMemcpyAsync + synchronise in containers/matrix/operations_cuda.h

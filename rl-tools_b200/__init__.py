@@ -12,7 +12,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB_PATH = os.path.join(HERE, "libb200rl.so")
-SOURCES = ["dense.cu", "dense_tc.cu", "dense_skinny.cu", "mlp_fused.cu", "mlp_coop.cu", "mlp_team.cu", "adam.cu", "rollout.cu", "rollout_tc.cu", "ppo.cu", "host_api.cu", "sac.cu", "normalize.cu", "rollout_env.cu", "l2f.cu"]
+SOURCES = ["dense.cu", "dense_tc.cu", "dense_skinny.cu", "mlp_fused.cu", "mlp_coop.cu", "mlp_team.cu", "ppo_team.cu", "adam.cu", "rollout.cu", "rollout_tc.cu", "ppo.cu", "host_api.cu", "sac.cu", "normalize.cu", "rollout_env.cu", "l2f.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-shared"]
 # per-source flags: the quadrotor dynamics keep the reference's association of every expression (bit-for-bit parity with its CPU step)
 SOURCE_FLAGS = {"l2f.cu": ["-fmad=false"]}
@@ -114,6 +114,11 @@ class AdamHyper(C.Structure):
         super().__init__(alpha, beta_1, beta_2, epsilon, epsilon_sqrt)
 
 
+class MlpArenas(C.Structure):
+    """Mirror of b200rl_mlp_arenas."""
+    _fields_ = [("params", C.c_void_p), ("grads", C.c_void_p), ("m", C.c_void_p), ("v", C.c_void_p), ("n", C.c_size_t), ("adam_state", C.c_void_p), ("hyper", AdamHyper)]
+
+
 def lib():
     """The loaded C-ABI library (ctypes). Raises if it has not been built: there is no fallback path."""
     global _lib
@@ -136,6 +141,9 @@ def lib():
         L.b200rl_ppo_scratch_bytes.argtypes = [i, i]
         L.b200rl_ppo_scratch_bytes.restype = sz
         L.b200rl_ppo_policy_gradient.argtypes = [vp, i, vp, i, vp, vp, i, vp, i, vp, i, vp, i, i, f, f, f, i, i, vp, sz, vp]
+        L.b200rl_ppo_train_epoch_scratch_bytes.argtypes = [shape_p, shape_p, i, i]
+        L.b200rl_ppo_train_epoch_scratch_bytes.restype = sz
+        L.b200rl_ppo_train_epoch.argtypes = [shape_p, C.POINTER(MlpArenas), shape_p, C.POINTER(MlpArenas), vp, vp, vp, vp, vp, i, i, i, f, f, f, i, i, vp, sz, vp]
         L.b200rl_mse_gradient.argtypes = [vp, i, vp, i, vp, i, i, i, f, vp]
         L.b200rl_fill.argtypes = [vp, sz, f, vp]
         L.b200rl_mlp_num_params.argtypes = [shape_p]
@@ -417,6 +425,9 @@ class Mlp:
     def extra(self, arena="params"):
         """View of the extra parameters (or their gradient / moments) behind the layers."""
         return getattr(self, arena)[self.n_mlp:]
+
+    def arenas(self):
+        return MlpArenas(self.params.data_ptr(), self.grads.data_ptr(), self.m.data_ptr(), self.v.data_ptr(), self.params.numel(), self.adam_state.data_ptr(), self.hyper)
 
     def save_code(self, name, batch=1):
         """The network as C++ source in the reference's export format (what its `save_code` writes for a forward-only MLP and its

@@ -1,0 +1,377 @@
+// One epoch of the PPO update -- all of its minibatches, actor and critic -- in ONE cooperative launch.
+//
+// A minibatch update is about 24 dependent launches of two to thirteen microseconds each (65 us per update even when they are replayed as a CUDA
+// graph), for arithmetic of a microsecond. Here half of the CTAs keep the actor and half the critic; the two never wait for each other. A CTA
+// takes its rows of a minibatch through the network (mlp_team.cuh, teams of one CTA), the row-wise loss gradient of the clipped surrogate or of
+// the value regression in between, writes its gradient sums, and behind a barrier over the network's CTAs every thread adds the sums of the one
+// parameter it owns and steps the optimizer for it, with the moments in registers for the whole epoch. A second barrier publishes the new
+// parameters. Replaces the per-minibatch body of train (rl/algorithms/ppo/operations_generic.h:159-336), per sample :214-296; Gaussian head
+// random/operations_generic.h:87-121.
+#include "common.cuh"
+#include "grid_barrier.cuh"
+#include "mlp_team.cuh"
+#include <atomic>
+#include <math.h>
+
+namespace b200rl {
+using namespace team;
+
+struct PpoNetArgs {
+    Net net;
+    float* params; float* grads; float* m; float* v; uint32_t* adam_state;
+    b200rl_adam_hyper hyper;
+    float4* partial; float* partial_std; unsigned* barrier;
+    int ctas, teams, lanes, row_tiles;
+    int stage_x, stage_aux, aux, out;        // shared memory: next rows and columns as they come, this tile's columns ([4][R] behind actions [R][S]), outputs [R][S]
+};
+struct PpoEpochArgs {
+    PpoNetArgs actor, critic;
+    const float* observations; const float* actions; const float* log_probs; const float* advantages; const float* targets;
+    const float* stats;                      // [minibatch][2]: mean and standard deviation of its advantages
+    int ld, batch, minibatches, action_dim;
+    float epsilon_clip, entropy_coefficient, advantage_epsilon, neg_log_sqrt_pi;
+    int normalize_advantage, learn_action_std;
+};
+
+constexpr int PPO_TEAM_MAX_ACTIONS = 64;
+
+// mean and standard deviation of every minibatch's advantages (:173-184), one CTA each
+__global__ void __launch_bounds__(1024) ppo_epoch_stats_kernel(const float* __restrict__ advantages, int ld, int batch, float* __restrict__ stats){
+    __shared__ float s_sum[32], s_sq[32];
+    const float* adv = advantages + (size_t)blockIdx.x * batch * ld;
+    float sum = 0.0f, sq = 0.0f;
+    for(int b = threadIdx.x; b < batch; b += blockDim.x){ const float a = adv[(size_t)b * ld]; sum += a; sq = fmaf(a, a, sq); }
+    for(int o = 16; o > 0; o >>= 1){ sum += __shfl_xor_sync(0xffffffffu, sum, o); sq += __shfl_xor_sync(0xffffffffu, sq, o); }
+    if((threadIdx.x & 31) == 0){ s_sum[threadIdx.x >> 5] = sum; s_sq[threadIdx.x >> 5] = sq; }
+    __syncthreads();
+    if(threadIdx.x == 0){
+        float ts = 0.0f, tq = 0.0f;
+        for(int w = 0; w < 32; w++){ ts += s_sum[w]; tq += s_sq[w]; }
+        const float mean = ts / batch, msq = tq / batch;
+        stats[2 * blockIdx.x] = mean; stats[2 * blockIdx.x + 1] = sqrtf(fmaxf(0.0f, msq - mean * mean));
+    }
+}
+
+template <bool ACTOR, int L, int TPT>
+__device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArgs& w, int cta, float* smem){
+    __shared__ float s_scalars[2][64];       // bias corrections of the next minibatches
+    __shared__ float s_log_std[PPO_TEAM_MAX_ACTIONS], s_std[PPO_TEAM_MAX_ACTIONS];
+    __shared__ int s_ok;
+    const Net& n = w.net;
+    const Layer& last = n.layer[L - 1];
+    const int tid = threadIdx.x, R = n.R, I0 = n.layer[0].I, A = a.action_dim, S = last.S;
+    const bool has_rows = cta < w.row_tiles;
+    auto stage = [&](int minibatch, int tile){
+        const int row0 = tile * R;
+        const size_t base = (size_t)minibatch * a.batch + row0;
+        const int rows = min(R, a.batch - row0);
+        for(int i = tid; i < R * I0; i += THREADS){
+            const int r = quotient(i, n.by_I0), k = i - r * I0;
+            if(r < rows) copy4_async(smem + w.stage_x + i, a.observations + (base + r) * a.ld + k);
+            else smem[w.stage_x + i] = 0.0f;
+        }
+        if constexpr(ACTOR){
+            for(int i = tid; i < R * S; i += THREADS){
+                const int r = quotient(i, last.by_S), k = i - r * S;
+                if(r < rows && k < A) copy4_async(smem + w.stage_aux + i, a.actions + (base + r) * a.ld + k);
+            }
+            if(tid < rows){
+                copy4_async(smem + w.stage_aux + R * S + tid, a.log_probs + (base + tid) * a.ld);
+                copy4_async(smem + w.stage_aux + R * S + R + tid, a.advantages + (base + tid) * a.ld);
+            }
+        }
+        else if(tid < rows) copy4_async(smem + w.stage_aux + tid, a.targets + (base + tid) * a.ld);
+    };
+    if(has_rows) stage(0, cta);
+    clear_rows<L>(n, smem);
+    load_weights<L>(n, smem, w.params, 0);
+    auto load_std = [&](){
+        if(ACTOR && tid < A){ const float ls = __ldcg(w.params + n.n_params + tid); s_log_std[tid] = ls; s_std[tid] = expf(ls); }
+    };
+    load_std();
+    // the parameter this thread owns: `lanes` threads per quad, one pass over all quads (guaranteed by the host's choice of lanes)
+    const int quads = n.n_tiles * 4, lane = tid & (w.lanes - 1), lane_bits = __popc(w.lanes - 1), u = cta * (THREADS >> lane_bits) + (tid >> lane_bits);
+    const int index = u < quads && lane < 4 ? arena_index<L>(n, u, lane) : -1;
+    float my_p = 0.0f, my_m = 0.0f, my_v = 0.0f, my_g = 0.0f;
+    if(index >= 0){ my_p = w.params[index]; my_m = w.m[index]; my_v = w.v[index]; }
+    const uint32_t age0 = *reinterpret_cast<volatile uint32_t*>(w.adam_state);
+    Patch patches[TPT];
+#pragma unroll
+    for(int k = 0; k < TPT; k++) patches[k] = patch<L>(n, k * THREADS + tid);
+    const float value_constant = 2.0f / ((float)a.batch * 1.0f) * 0.5f;
+    unsigned target = 0;
+    for(int mb = 0; mb < a.minibatches; mb++){
+        if((mb & 63) == 0 && tid < 128) s_scalars[tid & 1][tid >> 1] = adam_bias_correction(tid & 1 ? w.hyper.beta_2 : w.hyper.beta_1, age0 + (uint32_t)(mb + (tid >> 1)));
+        float2 acc[TPT][4][2];
+        float std_gradient = 0.0f;
+#pragma unroll
+        for(int k = 0; k < TPT; k++)
+#pragma unroll
+            for(int i = 0; i < 4; i++){ acc[k][i][0] = make_float2(0.0f, 0.0f); acc[k][i][1] = make_float2(0.0f, 0.0f); }
+        float mean = 0.0f, deviation = 1.0f;
+        if(ACTOR && a.normalize_advantage){ mean = __ldg(a.stats + 2 * mb); deviation = __fadd_rn(__ldg(a.stats + 2 * mb + 1), a.advantage_epsilon); }
+        for(int tile = cta; tile < w.row_tiles; tile += w.teams){
+            const int rows = min(R, a.batch - tile * R);
+            copies_wait();
+            __syncthreads();
+            for(int i = tid; i < R * I0; i += THREADS){ const int r = quotient(i, n.by_I0), k = i - r * I0; smem[n.layer[0].a + r * n.layer[0].P + k] = smem[w.stage_x + i]; }
+            if constexpr(ACTOR){ for(int i = tid; i < R * S + 2 * R; i += THREADS) smem[w.aux + i] = smem[w.stage_aux + i]; }
+            else if(tid < R) smem[w.aux + tid] = smem[w.stage_aux + tid];
+            __syncthreads();
+            {
+                const bool more = tile + w.teams < w.row_tiles;
+                if(more) stage(mb, tile + w.teams);
+                else if(mb + 1 < a.minibatches) stage(mb + 1, cta);
+            }
+#pragma unroll
+            for(int l = 0; l < L; l++){
+                forward_layer<1, L>(n, l, smem, 0, [&](int r, int unit, int idx, float value, float derivative){
+                    if(l == L - 1){
+                        if constexpr(ACTOR) smem[w.out + idx] = value;
+                        else smem[last.d + idx] = r < rows ? __fmul_rn(__fsub_rn(value, smem[w.aux + r]), value_constant) * derivative : 0.0f;
+                    }
+                });
+                __syncthreads();
+            }
+            if constexpr(ACTOR){
+                float* lp = smem + n.rb[1];                      // [R][S] log-probability terms, then [R][S] (action - mean) / std, then [R] dL / d log-probability
+                float* ps = lp + R * S;
+                float* dl = ps + R * S;
+                for(int i = tid; i < R * S; i += THREADS){
+                    const int r = quotient(i, last.by_S), k = i - r * S;
+                    if(k < A){
+                        const float p = __fdiv_rn(__fsub_rn(smem[w.aux + i], smem[w.out + i]), s_std[k]);
+                        // (constant - log_std) - 0.5 p^2 rounded once: p^2 as an exact float pair (see ppo.cu)
+                        const float h = __fmul_rn(p, p), lo = __fmaf_rn(p, p, -h);
+                        const float c = __fsub_rn(a.neg_log_sqrt_pi, s_log_std[k]), hh = __fmul_rn(0.5f, h);
+                        const float d = __fsub_rn(c, hh), db = __fsub_rn(d, c);
+                        const float de = __fsub_rn(__fsub_rn(c, __fsub_rn(d, db)), __fadd_rn(hh, db));
+                        lp[i] = __fadd_rn(d, __fmaf_rn(-0.5f, lo, de));
+                        ps[i] = p;
+                    }
+                }
+                __syncthreads();
+                if(tid < R){
+                    float d = 0.0f;
+                    if(tid < rows){
+                        float log_prob = 0.0f;
+                        for(int k = 0; k < A; k++) log_prob = __fadd_rn(log_prob, lp[tid * S + k]);
+                        float advantage = smem[w.aux + R * S + R + tid];
+                        if(a.normalize_advantage) advantage = __fdiv_rn(__fsub_rn(advantage, mean), deviation);
+                        const float ratio = expf(__fsub_rn(log_prob, smem[w.aux + R * S + tid]));
+                        const float lo = 1.0f - a.epsilon_clip, hi = 1.0f + a.epsilon_clip;
+                        const float clipped_ratio = ratio < lo ? lo : (ratio > hi ? hi : ratio);
+                        const bool clipped = ratio != clipped_ratio;
+                        const bool unclipped_is_smaller = __fsub_rn(__fmul_rn(ratio, advantage), __fmul_rn(clipped_ratio, advantage)) <= 0.0f;
+                        const float d_ratio = unclipped_is_smaller ? advantage : (clipped ? 0.0f : advantage);
+                        d = __fmul_rn(__fmul_rn(-1.0f / (float)a.batch, d_ratio), ratio);
+                    }
+                    dl[tid] = d;
+                }
+                __syncthreads();
+                for(int i = tid; i < R * S; i += THREADS){
+                    const int r = quotient(i, last.by_S), k = i - r * S;
+                    if(k < A) smem[last.d + i] = r < rows ? __fmul_rn(__fdiv_rn(ps[i], s_std[k]), dl[r]) * smem[last.g + i] : 0.0f;
+                }
+                if(tid >= 128 && tid < 128 + A){                 // the log_std gradient of the CTA's rows, in row order
+                    const int k = tid - 128;
+                    for(int r = 0; r < rows; r++) std_gradient += __fmul_rn(dl[r], __fadd_rn(-1.0f, __fmul_rn(ps[r * S + k], ps[r * S + k])));
+                }
+                __syncthreads();
+            }
+#pragma unroll
+            for(int l = L - 1; l > 0; l--) backward_layer<1>(n, l, smem, 0, (L - 1 - l) & 1);
+            accumulate_gradients<TPT>(n, smem, patches, acc);
+            if(tile + w.teams < w.row_tiles) __syncthreads();
+        }
+        if(has_rows){
+            store_gradients<1, TPT>(n, w.partial + (size_t)cta * quads, 0, acc);
+            if(ACTOR && a.learn_action_std && tid >= 128 && tid < 128 + A) __stcg(w.partial_std + (size_t)cta * A + tid - 128, std_gradient);
+        }
+        __syncthreads();
+        target += (unsigned)w.ctas;
+        if(tid == 0){ grid_barrier_arrive(w.barrier); s_ok = grid_barrier_wait(w.barrier, target); }
+        __syncthreads();
+        if(!s_ok) return;
+        const float c1 = s_scalars[0][mb & 63], c2 = s_scalars[1][mb & 63];
+        {
+            float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if(u < quads){
+                const float4* src = w.partial + u;
+                for(int t = lane; t < w.teams; t += 8 * w.lanes){
+                    float4 v[8];
+#pragma unroll
+                    for(int k = 0; k < 8; k++) v[k] = t + k * w.lanes < w.teams ? __ldcg(src + (size_t)(t + k * w.lanes) * quads) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+                    for(int k = 0; k < 8; k++){ s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
+                }
+            }
+            for(int o = w.lanes >> 1; o > 0; o >>= 1){
+                s.x += __shfl_xor_sync(0xffffffffu, s.x, o); s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+                s.z += __shfl_xor_sync(0xffffffffu, s.z, o); s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
+            }
+            if(index >= 0){
+                my_g = lane == 0 ? s.x : lane == 1 ? s.y : lane == 2 ? s.z : s.w;
+                my_p = adam_update(my_p, my_g, my_m, my_v, w.hyper, c1, c2);
+                __stcg(w.params + index, my_p);
+            }
+            if(ACTOR && cta == w.ctas - 1){                      // log_std: a warp per action, teams over the lanes
+                for(int k = tid >> 5; k < A; k += THREADS / 32){
+                    float g = 0.0f;
+                    if(a.learn_action_std){
+                        for(int t = tid & 31; t < w.teams; t += 32) g += __ldcg(w.partial_std + (size_t)t * A + k);
+#pragma unroll
+                        for(int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+                        g += (float)a.batch * (-1.0f / (float)a.batch * a.entropy_coefficient);      // the entropy bonus of every sample (:262-266)
+                    }
+                    if((tid & 31) == 0){
+                        const int i = n.n_params + k;
+                        float mm = w.m[i], vv = w.v[i];
+                        __stcg(w.params + i, adam_update(__ldcg(w.params + i), g, mm, vv, w.hyper, c1, c2));
+                        w.m[i] = mm; w.v[i] = vv; w.grads[i] = g;
+                    }
+                }
+            }
+        }
+        if(mb + 1 == a.minibatches) break;
+        __syncthreads();
+        target += (unsigned)w.ctas;
+        if(tid == 0){ grid_barrier_arrive(w.barrier); s_ok = grid_barrier_wait(w.barrier, target); }
+        __syncthreads();
+        if(!s_ok) return;
+        if(has_rows){ load_weights<L>(n, smem, w.params, 0); load_std(); }
+    }
+    copies_wait();
+    if(index >= 0){ w.m[index] = my_m; w.v[index] = my_v; w.grads[index] = my_g; }
+    if(cta == 0 && tid == 0){
+        const int last_mb = (a.minibatches - 1) & 63;
+        w.adam_state[0] = age0 + (uint32_t)a.minibatches; w.adam_state[1] = 0u;
+        w.adam_state[2] = __float_as_uint(s_scalars[0][last_mb]); w.adam_state[3] = __float_as_uint(s_scalars[1][last_mb]);
+    }
+    if(tid == 0) grid_barrier_leave(w.barrier, (unsigned)w.ctas);
+}
+
+template <int L, int TPT>
+__global__ void __launch_bounds__(THREADS, 1) ppo_epoch_kernel(const __grid_constant__ PpoEpochArgs a){
+    extern __shared__ __align__(16) float smem[];
+    if((int)blockIdx.x < a.actor.ctas) ppo_epoch<true, L, TPT>(a, a.actor, blockIdx.x, smem);
+    else ppo_epoch<false, L, TPT>(a, a.critic, blockIdx.x - a.actor.ctas, smem);
+}
+
+// ---- host side ---------------------------------------------------------------------------------------------------------------------------
+constexpr size_t PPO_TEAM_SMEM = 200 * 1024;
+
+// rows per tile: one tile per CTA where the batch allows it
+static bool plan_ppo_net(const b200rl_mlp_shape* sh, int batch, int ctas, bool actor, PpoNetArgs* w, size_t* smem){
+    const int want = (batch + ctas - 1) / ctas, A = sh->dims[sh->n_layers - 1];
+    for(int R = want >= 32 ? 32 : (want + 3) / 4 * 4; R >= 4; R -= 4){
+        Net n;
+        if(!team::plan(sh, 1, R, 0, &n)) continue;
+        const int S = n.layer[n.n_layers - 1].S;
+        // the surrogate's work area lies in the second exchange buffer
+        if(actor && n.end - n.rb[1] < 2 * R * S + R) n.end = n.rb[1] + 2 * R * S + R;
+        int off = (n.end + 3) / 4 * 4;
+        w->stage_x = off; off += (R * sh->input_dim + 3) / 4 * 4;
+        w->stage_aux = off; off += R * S + 2 * R;
+        w->aux = off; off += R * S + 2 * R;
+        w->out = off; off += R * S;
+        if(sizeof(float) * (size_t)off > PPO_TEAM_SMEM) continue;
+        w->net = n; w->ctas = ctas; w->row_tiles = (batch + R - 1) / R; w->teams = w->row_tiles < ctas ? w->row_tiles : ctas;
+        // one parameter per thread, one pass: lanes x quads within the threads of the network's CTAs
+        const int quads = n.n_tiles * 4, threads = ctas * THREADS;
+        if(4ll * quads > threads || A > PPO_TEAM_MAX_ACTIONS) return false;
+        w->lanes = 4;
+        while(w->lanes < 32 && 2 * w->lanes <= w->teams && 2ll * w->lanes * quads <= threads) w->lanes *= 2;
+        *smem = sizeof(float) * (size_t)off;
+        return true;
+    }
+    return false;
+}
+struct PpoChoice { PpoNetArgs actor, critic; size_t smem, bytes; };
+static bool choose_ppo(const b200rl_mlp_shape* actor, const b200rl_mlp_shape* critic, int batch, int minibatches, PpoChoice* out){
+    int sms = 0;
+    if(!actor || !critic || actor->n_layers != critic->n_layers || actor->n_layers < 1 || actor->n_layers > 3 || batch < 1 || sm_count(&sms) != B200RL_OK) return false;
+    PpoChoice c{};
+    size_t sa = 0, sc = 0;
+    if(!plan_ppo_net(actor, batch, sms / 2, true, &c.actor, &sa) || !plan_ppo_net(critic, batch, sms / 2, false, &c.critic, &sc)) return false;
+    if(c.actor.net.n_tiles > 4 * THREADS || c.critic.net.n_tiles > 4 * THREADS) return false;
+    c.smem = sa > sc ? sa : sc;
+    c.bytes = sizeof(float4) * 4 * ((size_t)c.actor.teams * c.actor.net.n_tiles + (size_t)c.critic.teams * c.critic.net.n_tiles) +
+              sizeof(float) * ((size_t)c.actor.teams * actor->dims[actor->n_layers - 1] + 2 * (size_t)minibatches);
+    *out = c;
+    return true;
+}
+
+template <int L, int TPT>
+static int launch_ppo_epoch(const PpoEpochArgs& a, size_t smem, cudaStream_t s){
+    static std::atomic<bool> configured[MAX_DEVICES];
+    int dev = 0;
+    int rc = current_device(&dev);
+    if(rc) return rc;
+    if(!configured[dev].load(std::memory_order_acquire)){
+        B200RL_CUDA_TRY(cudaFuncSetAttribute(ppo_epoch_kernel<L, TPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PPO_TEAM_SMEM));
+        configured[dev].store(true, std::memory_order_release);
+    }
+    PpoEpochArgs copy = a;
+    void* params[] = { &copy };
+    B200RL_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(ppo_epoch_kernel<L, TPT>), dim3(a.actor.ctas + a.critic.ctas), dim3(THREADS), params, smem, s));
+    return B200RL_OK;
+}
+template <int L>
+static int launch_ppo_epoch_l(const PpoEpochArgs& a, size_t smem, cudaStream_t s){
+    const int tiles = a.actor.net.n_tiles > a.critic.net.n_tiles ? a.actor.net.n_tiles : a.critic.net.n_tiles;
+    return tiles <= 2 * THREADS ? launch_ppo_epoch<L, 2>(a, smem, s) : launch_ppo_epoch<L, 4>(a, smem, s);
+}
+
+}  // namespace b200rl
+using namespace b200rl;
+
+extern "C" size_t b200rl_ppo_train_epoch_scratch_bytes(const b200rl_mlp_shape* actor, const b200rl_mlp_shape* critic, int batch, int n_minibatches){
+    PpoChoice c;
+    return choose_ppo(actor, critic, batch, n_minibatches, &c) ? c.bytes : 0;
+}
+
+extern "C" int b200rl_ppo_train_epoch(const b200rl_mlp_shape* actor, const b200rl_mlp_arenas* actor_arenas, const b200rl_mlp_shape* critic, const b200rl_mlp_arenas* critic_arenas,
+                                      const float* observations, const float* actions, const float* log_probs, const float* advantages, const float* target_values, int ld,
+                                      int batch, int n_minibatches, float epsilon_clip, float entropy_coefficient, float advantage_epsilon, int normalize_advantage,
+                                      int learn_action_std, void* scratch, size_t scratch_bytes, b200rl_stream_t stream){
+    if(!actor || !critic || !actor_arenas || !critic_arenas || !observations || !actions || !log_probs || !advantages || !target_values || batch < 1 || n_minibatches < 0 || ld < 1)
+        return B200RL_ERR_INVALID_ARGUMENT;
+    const size_t na = b200rl_mlp_num_params(actor), nc = b200rl_mlp_num_params(critic);
+    if(na == 0 || nc == 0) return B200RL_ERR_INVALID_ARGUMENT;
+    const int A = actor->dims[actor->n_layers - 1];
+    for(const b200rl_mlp_arenas* r : {actor_arenas, critic_arenas}) if(!r->params || !r->grads || !r->m || !r->v || !r->adam_state) return B200RL_ERR_INVALID_ARGUMENT;
+    if(actor_arenas->n != na + (size_t)A || critic_arenas->n != nc) return B200RL_ERR_UNSUPPORTED;
+    PpoChoice c;
+    if(critic->dims[critic->n_layers - 1] != 1 || actor->input_dim != critic->input_dim || !choose_ppo(actor, critic, batch, n_minibatches, &c)) return B200RL_ERR_UNSUPPORTED;
+    if(n_minibatches == 0) return B200RL_OK;
+    if(!scratch || scratch_bytes < c.bytes || (reinterpret_cast<uintptr_t>(scratch) & 15u)) return B200RL_ERR_INVALID_ARGUMENT;
+    PpoEpochArgs a{};
+    a.actor = c.actor; a.critic = c.critic;
+    float4* p = static_cast<float4*>(scratch);
+    auto arenas = [](PpoNetArgs& w, const b200rl_mlp_arenas* r){ w.params = r->params; w.grads = r->grads; w.m = r->m; w.v = r->v; w.adam_state = r->adam_state; w.hyper = r->hyper; };
+    arenas(a.actor, actor_arenas); arenas(a.critic, critic_arenas);
+    a.actor.partial = p; p += (size_t)c.actor.teams * c.actor.net.n_tiles * 4;
+    a.critic.partial = p; p += (size_t)c.critic.teams * c.critic.net.n_tiles * 4;
+    a.actor.partial_std = reinterpret_cast<float*>(p);
+    float* stats = a.actor.partial_std + (size_t)c.actor.teams * A;
+    a.observations = observations; a.actions = actions; a.log_probs = log_probs; a.advantages = advantages; a.targets = target_values; a.stats = stats;
+    a.ld = ld; a.batch = batch; a.minibatches = n_minibatches; a.action_dim = A;
+    a.epsilon_clip = epsilon_clip; a.entropy_coefficient = entropy_coefficient; a.advantage_epsilon = advantage_epsilon;
+    a.neg_log_sqrt_pi = (float)(-0.5 * (double)logf(2.0f * 3.14159265358979323846f));
+    a.normalize_advantage = normalize_advantage; a.learn_action_std = learn_action_std;
+    unsigned* bars = nullptr;
+    int rc = grid_barrier_slots(2, &bars);
+    if(rc) return rc;
+    a.actor.barrier = bars; a.critic.barrier = bars + 4;
+    cudaStream_t s = (cudaStream_t)stream;
+    if(normalize_advantage){
+        ppo_epoch_stats_kernel<<<n_minibatches, 1024, 0, s>>>(advantages, ld, batch, stats);
+        B200RL_LAUNCH_CHECK("ppo_epoch_stats");
+    }
+    switch(actor->n_layers){
+        case 1: return launch_ppo_epoch_l<1>(a, c.smem, s);
+        case 2: return launch_ppo_epoch_l<2>(a, c.smem, s);
+        default: return launch_ppo_epoch_l<3>(a, c.smem, s);
+    }
+}

@@ -4,7 +4,9 @@
 `estimate_generalized_advantages` and `train` follow rl/algorithms/ppo/operations_generic.h:59-95 and :96-336 with the default
 parameters of rl/algorithms/ppo/ppo.h:13-38. Everything runs on the GPU on torch CUDA tensors; there is no CPU path.
 """
-from . import gae as _gae, mse_gradient as _mse_gradient, ppo_policy_gradient as _ppo_policy_gradient, permute_rows as _permute_rows, shuffle_permutation_host as _shuffle_permutation_host
+import ctypes as C
+
+from . import lib, check, _stream, gae as _gae, mse_gradient as _mse_gradient, ppo_policy_gradient as _ppo_policy_gradient, permute_rows as _permute_rows, shuffle_permutation_host as _shuffle_permutation_host
 
 
 class DatasetLayout:
@@ -91,6 +93,28 @@ class MinibatchGraphs:
             t.copy_(s)                                                                          # the warm-up update is undone
 
 
+def _train_epoch(actor, critic, dataset, layout, n_minibatches, batch_size, epsilon_clip, entropy_coefficient, advantage_epsilon, normalize_advantage, learn_action_std):
+    """All minibatch updates of one epoch as one native call; False for networks that its kernel does not take."""
+    import torch
+    work = actor.__dict__.setdefault("_epoch_scratch", {})
+    key = (n_minibatches, batch_size, bytes(actor.shape), bytes(critic.shape))
+    if work.get("key") != key:
+        n = lib().b200rl_ppo_train_epoch_scratch_bytes(C.byref(actor.shape), C.byref(critic.shape), batch_size, n_minibatches)
+        work["key"], work["bytes"], work["buffer"] = key, n, torch.empty(n, device=dataset.device, dtype=torch.uint8) if n else None
+    if not work["bytes"]:
+        return False
+    base, ld = dataset.data_ptr(), dataset.stride(0)
+    at = lambda column: base + 4 * column
+    rc = lib().b200rl_ppo_train_epoch(C.byref(actor.shape), C.byref(actor.arenas()), C.byref(critic.shape), C.byref(critic.arenas()), at(layout.observations.start),
+                                      at(layout.actions.start), at(layout.action_log_probs), at(layout.advantages), at(layout.target_values), ld, batch_size, n_minibatches,
+                                      epsilon_clip, entropy_coefficient, advantage_epsilon, normalize_advantage, learn_action_std, work["buffer"].data_ptr(), work["bytes"],
+                                      _stream())
+    if rc == 2:                                                         # B200RL_ERR_UNSUPPORTED
+        return False
+    check(rc, "b200rl_ppo_train_epoch")
+    return True
+
+
 def train(actor, critic, dataset, layout, n_rows, batch_size, n_epochs=10, epsilon_clip=0.2, entropy_coefficient=0.01, advantage_epsilon=1e-8,
           normalize_advantage=True, learn_action_std=True, shuffle_rng_state=None, graphs=None):
     """n_epochs x (n_rows // batch_size) minibatch updates. shuffle_rng_state (from rng_init_host) switches the reference's SHUFFLE_EPOCH
@@ -98,8 +122,9 @@ def train(actor, critic, dataset, layout, n_rows, batch_size, n_epochs=10, epsil
     place with the permutation the reference's engine would produce (:127-158); None keeps dataset order. Per minibatch: zero_gradient,
     actor forward, clipped-surrogate gradient (+ log_std gradient), actor backward, critic forward, 0.5-weighted MSE gradient against
     the target values, critic backward, one Adam step each. `actor` is an Mlp with extra_params = action_dim (the log_std behind the
-    layers), `critic` an Mlp with one output; both built for batch_size rows. graphs = a MinibatchGraphs built for these arguments
-    replays each minibatch update as one CUDA graph launch instead of ~24 kernel launches (same kernels, same results)."""
+    layers), `critic` an Mlp with one output; both built for batch_size rows. An epoch is one native call where its kernel takes the networks
+    (small ones: up to three layers and about 18,000 parameters); otherwise graphs = a MinibatchGraphs built for these arguments replays each
+    minibatch update as one CUDA graph launch instead of ~24 kernel launches (same kernels, same results)."""
     import torch
     assert actor.batch == batch_size and critic.batch == batch_size and actor.n_extra == layout.action_dim
     hyper = dict(epsilon_clip=epsilon_clip, entropy_coefficient=entropy_coefficient, advantage_epsilon=advantage_epsilon,
@@ -112,6 +137,8 @@ def train(actor, critic, dataset, layout, n_rows, batch_size, n_epochs=10, epsil
         if shuffle_rng_state is not None:
             perm = torch.from_numpy(_shuffle_permutation_host(shuffle_rng_state, n_rows)).to(dataset.device)
             _permute_rows(dataset, n_rows, perm, shuffled)
+        if _train_epoch(actor, critic, dataset, layout, n_rows // batch_size, batch_size, **hyper):
+            continue
         for b in range(n_rows // batch_size):
             if graphs is not None:
                 graphs.graphs[b].replay()

@@ -1,4 +1,5 @@
-"""The one-call training step (b200rl_mlp_train_step) against the sequence of separate calls it stands for, at the sizes where their kernels can go wrong: rows that fill no tile, one row, widths that are no multiple of four, every team
+"""The one-call training step (b200rl_mlp_train_step) and the one-call PPO epoch (b200rl_ppo_train_epoch) against the sequences of separate calls
+they stand for, at the sizes where their kernels can go wrong: rows that fill no tile, one row, widths that are no multiple of four, every team
 size, several chunks, parameters outside the layers."""
 import numpy as np
 import pytest
@@ -55,3 +56,29 @@ def test_train_step_equals_the_separate_calls(lib, batch, chunks, I, dims, acts)
         for name in ("grads", "params", "m", "v", "pre", "out"):
             _close(getattr(a, name), getattr(b, name))
         assert int(a.adam_state[0]) == int(b.adam_state[0]) == 41
+
+
+@pytest.mark.parametrize("batch,minibatches,obs,actions,hidden,act,options", [
+    (512, 3, 3, 1, 64, "relu", {}), (2048, 2, 27, 8, 64, "tanh", {}), (97, 4, 5, 3, 32, "tanh", {}), (1000, 2, 18, 5, 100, "relu", dict(normalize_advantage=False)),
+    (30, 70, 4, 2, 16, "tanh", dict(learn_action_std=False))])
+def test_ppo_epoch_equals_the_separate_calls(lib, batch, minibatches, obs, actions, hidden, act, options):
+    import torch
+    from rl_tools_b200 import ppo
+    layout = ppo.DatasetLayout(obs, actions)
+    rows = batch * minibatches
+    data = mg.det_normal(3, rows * layout.data_dim).reshape(rows, layout.data_dim).astype(np.float32)
+    data[:, layout.action_log_probs] = data[:, layout.action_log_probs] * 0.5 - actions
+    dataset = torch.from_numpy(data).cuda()
+    acts = [act, act, "identity"]
+    nets = [[_net(lib, torch, batch, obs, [hidden, hidden, actions], acts, 20, extra=actions), _net(lib, torch, batch, obs, [hidden, hidden, 1], acts, 30)] for _ in range(2)]
+    for actor, _ in nets:
+        actor.extra("params").fill_(-0.5)
+    full = dict(epsilon_clip=0.2, entropy_coefficient=0.01, advantage_epsilon=1e-8, normalize_advantage=True, learn_action_std=True)
+    full.update(options)
+    assert ppo._train_epoch(*nets[0], dataset, layout, minibatches, batch, **full)
+    for k in range(minibatches):
+        ppo._minibatch_update(*nets[1], dataset[k * batch:(k + 1) * batch], layout, **full)
+    for got, want in zip(*nets):
+        for name in ("params", "v", "m", "grads"):
+            _close(getattr(got, name), getattr(want, name), 2e-6 if name in ("params", "v") else 2e-4)
+        assert torch.equal(got.adam_state, want.adam_state)

@@ -513,6 +513,12 @@ int mlp_fused_forward(const b200rl_mlp_shape* sh, const float* params, const flo
 int mlp_fused_backward(const b200rl_mlp_shape* sh, const float* params, float* grads, const float* x, int ldx, const float* pre, const float* out, float* d_out,
                        float* d_input, int batch, void* scratch, size_t scratch_bytes, cudaStream_t s);
 
+// all layers of a pass in one tensor-core kernel (mlp_chain.cu)
+bool mlp_chain_eligible(const b200rl_mlp_shape* sh, int batch);
+size_t mlp_chain_workspace_bytes(const b200rl_mlp_shape* sh);
+int mlp_chain_forward(const b200rl_mlp_shape* sh, const float* params, const float* x, int ldx, float* pre, float* out, float* y, int ldy, int batch, void* workspace,
+                      size_t workspace_bytes, cudaStream_t s);
+
 // whole training step in one cooperative launch (mlp_team.cu)
 bool mlp_team_eligible(const b200rl_mlp_shape* sh, int rows);
 size_t mlp_team_scratch_bytes(const b200rl_mlp_shape* sh, int rows);
@@ -633,6 +639,7 @@ size_t b200rl_mlp_forward_workspace_bytes(const b200rl_mlp_shape* sh, int batch)
     if(!valid_shape(sh) || batch < 1) return 0;
     size_t m = 0; int I = sh->input_dim;
     for(int l = 0; l < sh->n_layers; l++){ const size_t b = forward_workspace_bytes(batch, I, sh->dims[l]); if(b > m) m = b; I = sh->dims[l]; }
+    if(mlp_chain_eligible(sh, batch)){ const size_t b = mlp_chain_workspace_bytes(sh); if(b > m) m = b; }
     return m;
 }
 
@@ -645,6 +652,10 @@ int b200rl_mlp_evaluate_ws(const b200rl_mlp_shape* sh, const float* params, cons
     if(!valid_shape(sh) || !params || !x || !y || batch < 0 || ldx < sh->input_dim || ldy < sh->dims[sh->n_layers - 1]) return B200RL_ERR_INVALID_ARGUMENT;
     if(sh->n_layers > 1 && (!tick || (sh->n_layers > 2 && !tock))) return B200RL_ERR_INVALID_ARGUMENT;
     if(batch == 0) return B200RL_OK;
+    if(mlp_chain_eligible(sh, batch)){
+        const int rc = mlp_chain_forward(sh, params, x, ldx, nullptr, nullptr, y, ldy, batch, workspace, workspace_bytes, (cudaStream_t)stream);
+        if(rc != B200RL_ERR_UNSUPPORTED) return rc;
+    }
     if(mlp_fused_eligible(sh, batch)) return mlp_fused_forward(sh, params, x, ldx, nullptr, nullptr, y, ldy, batch, (cudaStream_t)stream);
     if(mlp_coop_eligible(sh, batch, true)) return mlp_coop_forward(sh, params, x, ldx, nullptr, nullptr, y, ldy, tick, tock, batch, (cudaStream_t)stream);
     const float* in = x; int ldin = ldx, I = sh->input_dim; const float* p = params;
@@ -667,6 +678,10 @@ int b200rl_mlp_forward_ws(const b200rl_mlp_shape* sh, const float* params, const
                           int batch, void* workspace, size_t workspace_bytes, b200rl_stream_t stream){
     if(!valid_shape(sh) || !params || !x || !pre || !out || batch < 0 || ldx < sh->input_dim) return B200RL_ERR_INVALID_ARGUMENT;
     if(batch == 0) return B200RL_OK;
+    if(mlp_chain_eligible(sh, batch)){
+        const int rc = mlp_chain_forward(sh, params, x, ldx, pre, out, nullptr, 0, batch, workspace, workspace_bytes, (cudaStream_t)stream);
+        if(rc != B200RL_ERR_UNSUPPORTED) return rc;
+    }
     if(mlp_fused_eligible(sh, batch)) return mlp_fused_forward(sh, params, x, ldx, pre, out, nullptr, 0, batch, (cudaStream_t)stream);
     if(mlp_coop_eligible(sh, batch, true)) return mlp_coop_forward(sh, params, x, ldx, pre, out, nullptr, 0, nullptr, nullptr, batch, (cudaStream_t)stream);
     const float* in = x; int ldin = ldx, I = sh->input_dim; const float* p = params;

@@ -1,0 +1,567 @@
+// A whole network over large batches on the tensor cores (sm_100a, tcgen05 + TMEM), one kernel for all layers of a pass: 128 batch rows stay on the
+// SM from the first layer to the last, and only what the pass owes its caller crosses HBM -- the inputs and the outputs of an evaluation, the
+// pre-activations and outputs of a training forward pass. Serves
+//   evaluate                 y = mlp(x)                                                        (nn_models/mlp/operations_generic.h:77-102)
+//   forward                  the same, keeping pre-activations and outputs of every layer       (:103-120)
+//
+// Arithmetic: fp32 operands as two fp16 parts, x = lead + rest (11 + 11 significant bits), three passes rest * lead, lead * rest, lead * lead with
+// fp32 accumulation -- the precision of three tf32 passes at twice their rate and half their shared memory. fp16's range is met by powers of two
+// that divide out exactly: a layer's weights are scaled by their largest magnitude, every 64-column piece of an activation row by that piece's, so a
+// remainder is subnormal only for values below 2^-17 of those maxima (and then off by at most 2^-39 of them). The tensor core truncates when it accumulates, so a chain of MMAs is kept
+// to 64 summed columns (12 MMAs); the pieces are added, unscaled, to fp32 registers with fused multiply-adds.
+//
+// Roles: 16 warps (112 registers) move accumulators to registers and do everything element-wise; one thread each of two further warps issues MMAs, one
+// of a third brings the weights in. A unit of work is one 64-column piece of the summed index into all outputs of a layer. An MMA of 128 rows takes about
+// 128 cycles however narrow it is (the rows of A pass through the tensor core once per instruction), so that only N = 256 runs it at its rate:
+//   - layers of more than 128 outputs: 12 MMAs M128 N256 K16 per unit (lead * rest, rest * lead, lead * lead);
+//   - up to 128 outputs: the weights' two parts are stacked into one operand of twice the columns, 8 MMAs (rest * both, lead * both), and the two
+//     column ranges are added when the accumulator is read.
+// Two 256-column accumulators in turn. A thread that issues is held up until the tensor core has room, so two threads take the units in turn: one gets
+// its barriers out of the way while the other's MMAs run.
+// Element-wise work is a third of the MMAs' time per layer and cannot hide behind this tile's own MMAs as long as a layer needs all of its input; so
+// every warp owns 16 columns of EVERY piece of its 32 rows, and the pieces are finished one after the other: the next layer's MMAs start on the first
+// piece while the second is being split. A row's scale is the largest exponent among the four warps that share the row (a byte each, exchanged
+// through shared memory at a barrier of those four warps).
+// The activations of the 128 rows fill 128 KB of shared memory (both parts, up to 256 columns); the weights, split once per call into an image of
+// exactly the shared-memory tiles, stream through three 32 KB slots by bulk copies (every CTA reads all weights from L2 for each of its row tiles: 592
+// KB per tile of 64-256-256-256-16).
+//
+// Bound by the tensor core and, between layers, by what the 16 warps do to a row tile before the next layer can start (about a third of the time), in
+// the forward pass by the stores. Measured, 64-256-256-256-16 at 1,048,576 rows: evaluate 3,236 -> 1,450 us (0.58 ms at the rate of three fp16
+// passes), forward 3,366 -> 2,850 us (6.8 GB, 1.0 ms at the copy bandwidth); 27-64-64-8 at 524,288 rows: evaluate 336 -> 218 us, forward 367 -> 369.
+#include "common.cuh"
+#include "tcgen05.cuh"
+#include <atomic>
+#include <cuda_fp16.h>
+
+namespace b200rl {
+
+namespace {
+constexpr int CH_ROWS = 128, CH_WARPS = 16, CH_THREADS = 32 * (CH_WARPS + 4), CH_MAX_STEPS = 8, CH_STAGES = 3;
+constexpr uint32_t CH_TILE = 128 * 128;                           // one fp16 operand tile: 128 rows x 64 columns
+constexpr uint32_t CH_STAGE = 2 * CH_TILE;                        // a slot of the weights; a piece of the activations: both parts
+constexpr uint32_t CH_A = 4 * CH_STAGE;                           // both parts of four 64-column pieces of the activations
+constexpr uint32_t CH_EXP = 4 * CH_ROWS + 2 * 4 * CH_ROWS;        // exponents of the pieces' scales; two buffers of the four warps' exponents per row
+constexpr uint32_t CH_SMEM = CH_A + CH_STAGES * CH_STAGE + CH_EXP + 256 + 1024;
+static_assert(CH_SMEM <= 227 * 1024, "shared memory");
+constexpr size_t CH_TAIL = 2048;                                  // behind an image: see ChainStep::tail
+constexpr long long CH_WAIT_LIMIT = 2000000000LL;
+enum { CH_EVALUATE = 0, CH_FORWARD = 1 };
+}
+
+struct ChainStep {
+    int N, K, pieces, n, act;                         // n: N rounded up to 16
+    const uint8_t* image; const float* tail;          // tail: 256 biases (zeros beyond N), then the inverse of the weights' scale
+    float* pre; float* out; long long ld;             // forward: this layer's arenas [rows, N]; evaluate: the last layer's outputs with their row pitch
+};
+struct ChainArgs {
+    int n_steps, rows, tiles;
+    ChainStep step[CH_MAX_STEPS];
+    const float* in; long long ld_in; int in_cols;
+};
+
+__device__ int g_chain_error = 0;
+
+namespace {
+__device__ __forceinline__ uint32_t pack_f16(float lo, float hi){
+    uint32_t r;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+__device__ __forceinline__ void split_pair(float2 v, uint32_t& lead, uint32_t& rest){
+    lead = pack_f16(v.x, v.y);
+    const float2 back = __half22float2(*reinterpret_cast<const __half2*>(&lead));
+    const float2 d = __ffma2_rn(back, make_float2(-1.0f, -1.0f), v);
+    rest = pack_f16(d.x, d.y);
+}
+// biased exponent of the piece's largest magnitude, clamped so that the scale 2^(14 - e) and its inverse are normal numbers
+__device__ __forceinline__ uint32_t scale_exponent(float largest){
+    const uint32_t e = (__float_as_uint(largest) >> 23) & 0xFFu;
+    return e < 15u ? 15u : e > 254u ? 254u : e;
+}
+__device__ __forceinline__ float scale_of(uint32_t e){ return __uint_as_float((268u - e) << 23); }
+__device__ __forceinline__ float inverse_scale_of(uint32_t e){ return __uint_as_float((e - 14u) << 23); }
+
+// Where the 16 values (8 pairs of neighbouring columns) of a thread lie in its warp's 16 columns of a piece.
+//   ROWS:  one row, 16 columns (tcgen05.ld 32x32b): no exchange within the warp, 16-byte shared-memory stores; pair i = columns 2 i, 2 i + 1 of row `lane`
+//   !ROWS: four rows 8 apart, 4 columns each (16x256b): a global store instruction writes whole 32-byte sectors; pair 2 s + j = columns 8 j + 2 (lane & 3),
+//          + 1 of row 8 s + (lane >> 2)
+template <bool ROWS> struct Spread {
+    static __device__ __forceinline__ int row(int lane, int i){ return ROWS ? lane : 8 * (i >> 1) + (lane >> 2); }
+    static __device__ __forceinline__ int column(int lane, int i){ return ROWS ? 2 * i : 8 * (i & 1) + 2 * (lane & 3); }
+};
+typedef float2 Slice[8];
+template <int ACT>
+__device__ __forceinline__ void activate_slice(Slice& v){
+#pragma unroll
+    for(int i = 0; i < 8; i++){ v[i].x = activation<ACT>(v[i].x); v[i].y = activation<ACT>(v[i].y); }
+}
+__device__ __forceinline__ void activate_slice_rt(Slice& v, int act){
+    switch(act){
+        case B200RL_ACT_IDENTITY: break;
+        case B200RL_ACT_RELU: activate_slice<B200RL_ACT_RELU>(v); break;
+        case B200RL_ACT_TANH: activate_slice<B200RL_ACT_TANH>(v); break;
+        case B200RL_ACT_FAST_TANH: activate_slice<B200RL_ACT_FAST_TANH>(v); break;
+        default: activate_slice<B200RL_ACT_SIGMOID>(v); break;
+    }
+}
+// a slice at (row0, col0) of a [rows, N] matrix with row pitch ld
+struct Place { int row0, col0, rows, N; long long ld; };
+__device__ __forceinline__ bool aligned_pairs(const float* p, long long ld){ return (ld & 1) == 0 && (reinterpret_cast<uintptr_t>(p) & 7u) == 0; }
+__device__ __forceinline__ bool aligned_quads(const float* p, long long ld){ return (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+template <bool ROWS>
+__device__ __forceinline__ void store_slice(const Place& p, float* dst, int lane, const Slice& v){
+    const bool whole = p.col0 + 16 <= p.N && aligned_pairs(dst, p.ld), quads = ROWS && aligned_quads(dst, p.ld);
+#pragma unroll
+    for(int i = 0; i < 8; i++){
+        const int row = p.row0 + Spread<ROWS>::row(lane, i), col = p.col0 + Spread<ROWS>::column(lane, i);
+        if(row >= p.rows) continue;
+        float* at = dst + (long long)row * p.ld + col;
+        if(whole && quads){ if((i & 1) == 0) *reinterpret_cast<float4*>(at) = make_float4(v[i].x, v[i].y, v[i | 1].x, v[i | 1].y); }
+        else if(whole) *reinterpret_cast<float2*>(at) = v[i];
+        else{
+            if(col < p.N) at[0] = v[i].x;
+            if(col + 1 < p.N) at[1] = v[i].y;
+        }
+    }
+}
+template <bool ROWS>
+__device__ __forceinline__ void load_slice(const Place& p, const float* src, int lane, Slice& v){
+    const bool whole = p.col0 + 16 <= p.N && aligned_pairs(src, p.ld), quads = ROWS && aligned_quads(src, p.ld);
+#pragma unroll
+    for(int i = 0; i < 8; i++){
+        const int row = p.row0 + Spread<ROWS>::row(lane, i), col = p.col0 + Spread<ROWS>::column(lane, i);
+        const float* at = src + (long long)row * p.ld + col;
+        if(whole && quads){
+            if((i & 1) == 0){
+                const float4 t = row < p.rows ? *reinterpret_cast<const float4*>(at) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                v[i] = make_float2(t.x, t.y); v[i | 1] = make_float2(t.z, t.w);
+            }
+        }
+        else if(whole) v[i] = row < p.rows ? *reinterpret_cast<const float2*>(at) : make_float2(0.0f, 0.0f);
+        else v[i] = make_float2(row < p.rows && col < p.N ? at[0] : 0.0f, row < p.rows && col + 1 < p.N ? at[1] : 0.0f);
+    }
+}
+// columns of the slice beyond the layer (whatever lay in tensor memory, or an activation of zero that is not zero) become zeros
+template <bool ROWS>
+__device__ __forceinline__ void clear_beyond(int col0, int N, int lane, Slice& v){
+    if(col0 + 16 <= N) return;
+#pragma unroll
+    for(int i = 0; i < 8; i++){
+        const int col = col0 + Spread<ROWS>::column(lane, i);
+        if(col >= N) v[i].x = 0.0f;
+        if(col + 1 >= N) v[i].y = 0.0f;
+    }
+}
+__device__ __forceinline__ void ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]){
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
+// 16 rows (lanes of the address on) x 16 columns: r[4 j + 2 s], r[4 j + 2 s + 1] = columns 8 j + 2 (lane & 3), + 1 of row 8 s + (lane >> 2)
+__device__ __forceinline__ void ld_16x256b_x2(uint32_t taddr, uint32_t* r){
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+}  // namespace
+
+template <int MODE>
+__global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_constant__ ChainArgs a){
+    constexpr bool ROWS = MODE == CH_EVALUATE;                          // only the last outputs go to memory
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* base = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint8_t* stages = base + CH_A;
+    uint8_t* exps = stages + CH_STAGES * CH_STAGE;                      // [piece][row], then two exchange buffers [row][warp of the row]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(exps + CH_EXP);
+    uint64_t* w_full = bars; uint64_t* w_empty = bars + CH_STAGES; uint64_t* acc_full = bars + 2 * CH_STAGES; uint64_t* acc_empty = acc_full + 2;
+    uint64_t* turn = acc_empty + 2;                                     // whose unit's MMAs may be issued next
+    uint64_t* a_full = turn + 2;                                        // [piece]: every warp has stored its columns of it
+    uint32_t* slot = reinterpret_cast<uint32_t*>(a_full + 4);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(slot + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if(tid == 0){
+        for(int i = 0; i < CH_STAGES; i++){ tc::mbar_init(w_full + i, 1); tc::mbar_init(w_empty + i, 1); }
+        for(int i = 0; i < 2; i++){ tc::mbar_init(acc_full + i, 1); tc::mbar_init(acc_empty + i, CH_WARPS); tc::mbar_init(turn + i, 1); }
+        for(int i = 0; i < 4; i++) tc::mbar_init(a_full + i, CH_WARPS);
+        tc::fence_mbar_init(); *abort_flag = 0;
+    }
+    if(warp == CH_WARPS){ tc::tmem_alloc(slot, 512); tc::tmem_relinquish(); }
+    tc::fence_before_thread_sync();
+    __syncthreads();
+    tc::fence_after_thread_sync();
+    const uint32_t tmem = *slot;
+    auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+        if(tc::mbar_try_wait(bar, parity)) return true;
+        const long long t0 = clock64();
+        while(!tc::mbar_try_wait(bar, parity)){
+            if(*abort_flag || clock64() - t0 > CH_WAIT_LIMIT){ *abort_flag = 1; g_chain_error = 1; return false; }
+        }
+        return true;
+    };
+    if(warp >= CH_WARPS){
+        tc::setmaxnreg_dec<32>();
+        if(lane == 0 && (warp == CH_WARPS || warp == CH_WARPS + 2)){
+            // ---- the issuing threads: units 0, 2, ... and 1, 3, ...; both follow every fill of the activation pieces ----
+            const uint32_t mine = warp == CH_WARPS ? 0u : 1u;
+            uint32_t u = 0, w = 0, ready = 0;                           // running unit and slot; bit c: parity of piece c's next fill
+            bool ok = true;
+            for(int tile = blockIdx.x; tile < a.tiles && ok; tile += gridDim.x){
+                for(int st = 0; st < a.n_steps && ok; st++){
+                    const ChainStep& y = a.step[st];
+                    const int pieces = y.pieces, K = y.K, n = y.n;
+                    const bool stacked = n <= 128;
+                    const uint32_t idesc = tc::make_idesc_f16(CH_ROWS, stacked ? 2 * n : n);
+                    for(int c = 0; c < pieces; c++, u++, w += stacked ? 1u : 2u){
+                        if(!(ok = wait(a_full + c, (ready >> c) & 1u))) break;
+                        ready ^= 1u << c;
+                        if((u & 1u) != mine) continue;
+                        const int ksteps = min(4, (K - 64 * c + 15) / 16);
+                        const uint64_t lead = tc::make_desc_kmajor_sw128(tc::smem_u32(base + c * CH_STAGE)), rest = lead + (CH_TILE >> 4);
+                        const uint32_t d = tmem + (u & 1u) * 256, s0 = w % CH_STAGES;
+                        if(!(ok = wait(acc_empty + (u & 1u), ((u >> 1) & 1u) ^ 1u))) break;
+                        if(!(ok = wait(w_full + s0, (w / CH_STAGES) & 1u))) break;
+                        const uint32_t s1 = (w + 1) % CH_STAGES;
+                        if(!stacked && !(ok = wait(w_full + s1, ((w + 1) / CH_STAGES) & 1u))) break;
+                        // units in order: interleaved, both would finish late and their accumulators be read late
+                        if(u > 0 && !(ok = wait(turn + (u & 1u), ((u - 1) >> 1) & 1u))) break;
+                        tc::fence_after_thread_sync();
+                        const uint64_t w0 = tc::make_desc_kmajor_sw128(tc::smem_u32(stages + s0 * CH_STAGE));
+                        // the small products first
+                        const uint64_t first = stacked ? rest : lead;
+                        for(int k = 0; k < ksteps; k++) tc::mma_f16_ss(d, first + (uint64_t)(2 * k), w0 + (uint64_t)(2 * k), idesc, k ? 1u : 0u);
+                        if(stacked){
+                            tc::mbar_arrive(turn + ((u + 1) & 1u));
+                            for(int k = 0; k < ksteps; k++) tc::mma_f16_ss(d, lead + (uint64_t)(2 * k), w0 + (uint64_t)(2 * k), idesc, 1u);
+                            tc::commit(acc_full + (u & 1u));
+                            tc::commit(w_empty + s0);
+                        }
+                        else{
+                            tc::commit(w_empty + s0);
+                            const uint64_t w1 = tc::make_desc_kmajor_sw128(tc::smem_u32(stages + s1 * CH_STAGE));
+                            for(int k = 0; k < ksteps; k++) tc::mma_f16_ss(d, rest + (uint64_t)(2 * k), w1 + (uint64_t)(2 * k), idesc, 1u);
+                            tc::mbar_arrive(turn + ((u + 1) & 1u));      // a few MMAs early: the other thread needs about as long to get going
+                            for(int k = 0; k < ksteps; k++) tc::mma_f16_ss(d, lead + (uint64_t)(2 * k), w1 + (uint64_t)(2 * k), idesc, 1u);
+                            tc::commit(acc_full + (u & 1u));
+                            tc::commit(w_empty + s1);
+                        }
+                    }
+                }
+            }
+        }
+        else if(lane == 0 && warp == CH_WARPS + 1){
+            // ---- the weights: per unit a slot with the remainder tile and one with the leading tile, or one slot with both (up to 128 outputs) ----
+            uint32_t w = 0;                                             // running slot
+            bool ok = true;
+            for(int tile = blockIdx.x; tile < a.tiles && ok; tile += gridDim.x){
+                for(int st = 0; st < a.n_steps && ok; st++){
+                    const ChainStep& y = a.step[st];
+                    const uint32_t part = (uint32_t)y.n * 128;
+                    const bool stacked = y.n <= 128;
+                    const uint8_t* unit = y.image;
+                    for(int c = 0; c < y.pieces && ok; c++, unit += 2 * part){
+                        for(int k = stacked ? 0 : 1; k >= 0; k--, w++){
+                            const uint32_t s = w % CH_STAGES, bytes = stacked ? 2 * part : part;
+                            if(!(ok = wait(w_empty + s, ((w / CH_STAGES) & 1u) ^ 1u))) break;
+                            tc::mbar_expect_tx(w_full + s, bytes);
+                            tc::bulk_load(stages + s * CH_STAGE, unit + k * part, bytes, w_full + s);
+                            tc::mbar_arrive(w_full + s);
+                        }
+                    }
+                }
+            }
+            // every copy that was started must have landed before the CTA may leave
+            for(uint32_t k = w < CH_STAGES ? 0 : w - CH_STAGES; k < w; k++) tc::mbar_wait_bounded(w_full + k % CH_STAGES, (k / CH_STAGES) & 1u, CH_WAIT_LIMIT);
+        }
+    }
+    else{
+        tc::setmaxnreg_inc<112>();
+        const int q = warp & 3, g = warp >> 2;                          // rows (TMEM lanes) 32 q ... + 31; columns 16 g ... + 15 of every piece
+        const uint32_t tmem_lane = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(16 * g);
+        uint32_t u = 0, exchange = 0;                                   // running unit; running exchange of exponents
+        bool ok = true;
+        // this warp's slice of a piece of the next operand: scaled by the largest magnitude of each row in the piece, split, stored
+        auto store_operand = [&](int piece, const Slice& v){
+            uint8_t* buffer = exps + 4 * CH_ROWS + (exchange & 1u) * 4 * CH_ROWS + 4 * q * 32;
+            exchange++;
+            constexpr int SLOTS = ROWS ? 1 : 4, PER = 8 / SLOTS;
+#pragma unroll
+            for(int s = 0; s < SLOTS; s++){
+                float m0 = 0.0f, m1 = 0.0f;
+#pragma unroll
+                for(int j = 0; j < PER; j++){ m0 = fmaxf(m0, fabsf(v[s * PER + j].x)); m1 = fmaxf(m1, fabsf(v[s * PER + j].y)); }
+                float m = fmaxf(m0, m1);
+                if constexpr(!ROWS){
+                    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+                    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+                }
+                if(ROWS || (lane & 3) == 0) buffer[4 * Spread<ROWS>::row(lane, s * PER) + g] = (uint8_t)scale_exponent(m);
+            }
+            tc::named_barrier_sync(1 + q, 128);                          // the four warps of these rows; all of them have read the previous layer's sums
+            uint8_t* tile_lead = base + piece * CH_STAGE;
+            const float2 zero = make_float2(0.0f, 0.0f);
+#pragma unroll
+            for(int s = 0; s < SLOTS; s++){
+                const int r = Spread<ROWS>::row(lane, s * PER);
+                const uint32_t four = *reinterpret_cast<const uint32_t*>(buffer + 4 * r);
+                const uint32_t e = max(max(four & 0xFFu, (four >> 8) & 0xFFu), max((four >> 16) & 0xFFu, four >> 24));
+                if(g == 0 && (ROWS || (lane & 3) == 0)) exps[piece * CH_ROWS + q * 32 + r] = (uint8_t)e;
+                const float2 f = make_float2(scale_of(e), scale_of(e));
+                const uint32_t row = (uint32_t)(q * 32 + r), x = row & 7u;
+                uint32_t lead[PER], rest[PER];
+#pragma unroll
+                for(int j = 0; j < PER; j++) split_pair(__ffma2_rn(v[s * PER + j], f, zero), lead[j], rest[j]);
+                if constexpr(ROWS){
+#pragma unroll
+                    for(int j = 0; j < 2; j++){
+                        const uint32_t off = row * 128 + (((uint32_t)(2 * g + j) ^ x) << 4);
+                        *reinterpret_cast<uint4*>(tile_lead + off) = make_uint4(lead[4 * j], lead[4 * j + 1], lead[4 * j + 2], lead[4 * j + 3]);
+                        *reinterpret_cast<uint4*>(tile_lead + CH_TILE + off) = make_uint4(rest[4 * j], rest[4 * j + 1], rest[4 * j + 2], rest[4 * j + 3]);
+                    }
+                }
+                else{
+#pragma unroll
+                    for(int j = 0; j < 2; j++){
+                        const uint32_t off = row * 128 + (((uint32_t)(2 * g + j) ^ x) << 4) + (uint32_t)(lane & 3) * 4;
+                        *reinterpret_cast<uint32_t*>(tile_lead + off) = lead[j];
+                        *reinterpret_cast<uint32_t*>(tile_lead + CH_TILE + off) = rest[j];
+                    }
+                }
+            }
+            tc::fence_proxy_async_smem();
+            __syncwarp();
+            if(lane == 0) tc::mbar_arrive(a_full + piece);
+        };
+        // this warp's slice of a piece of a tile's inputs
+        auto load_input = [&](int tile, int piece, Slice& v){
+            load_slice<ROWS>(Place{tile * CH_ROWS + q * 32, 64 * piece + 16 * g, a.rows, a.in_cols, a.ld_in}, a.in, lane, v);
+        };
+        Slice acc[4];                                                   // this layer's sums, a slice per piece
+        bool loaded = false;                                            // acc[2], acc[3]: the tile's first two input pieces
+        for(int tile = blockIdx.x; tile < a.tiles && ok; tile += gridDim.x){
+            const int row0 = tile * CH_ROWS + q * 32;
+            // ---- the first layer's input (every MMA of the previous tile has completed: its last unit was drained) ----
+#pragma unroll
+            for(int p = 0; p < 4; p++){
+                if(p >= a.step[0].pieces) break;
+                if(p < 2){ if(!loaded) load_input(tile, p, acc[2 + p]); store_operand(p, acc[2 + p]); }
+                else{ load_input(tile, p, acc[p - 2]); store_operand(p, acc[p - 2]); }
+            }
+            loaded = false;
+            for(int st = 0; st < a.n_steps && ok; st++){
+                const ChainStep& y = a.step[st];
+                const bool last = st + 1 == a.n_steps, stacked = y.n <= 128;
+                const int outs = (y.N + 63) / 64;                       // pieces of the output
+#pragma unroll
+                for(int p = 0; p < 4; p++){                              // the sums start with the bias
+                    if(p >= outs) break;
+                    const float* at = y.tail + 64 * p + 16 * g;
+                    if constexpr(ROWS){
+#pragma unroll
+                        for(int j = 0; j < 4; j++){
+                            const float4 b = __ldg(reinterpret_cast<const float4*>(at) + j);
+                            acc[p][2 * j] = make_float2(b.x, b.y); acc[p][2 * j + 1] = make_float2(b.z, b.w);
+                        }
+                    }
+                    else{
+#pragma unroll
+                        for(int j = 0; j < 2; j++){
+                            const float2 b = __ldg(reinterpret_cast<const float2*>(at + Spread<ROWS>::column(lane, j)));
+#pragma unroll
+                            for(int s = 0; s < 4; s++) acc[p][2 * s + j] = b;
+                        }
+                    }
+                }
+                if(last && stacked && tile + (int)gridDim.x < a.tiles){  // a narrow last layer leaves room for the next tile's inputs
+                    load_input(tile + gridDim.x, 0, acc[2]);
+                    if(a.step[0].pieces > 1) load_input(tile + gridDim.x, 1, acc[3]);
+                    loaded = true;
+                }
+                const float weights = __ldg(y.tail + 256);              // inverse of the weights' scale
+                for(int c = 0; c < y.pieces; c++, u++){
+                    if(!(ok = wait(acc_full + (u & 1u), (u >> 1) & 1u))) break;
+                    tc::fence_after_thread_sync();
+                    const uint8_t* e = exps + c * CH_ROWS + q * 32;
+                    float inv[ROWS ? 1 : 4];
+#pragma unroll
+                    for(int s = 0; s < (ROWS ? 1 : 4); s++) inv[s] = weights * inverse_scale_of(e[Spread<ROWS>::row(lane, 2 * s)]);
+                    const uint32_t from = tmem_lane + (u & 1u) * 256;
+#pragma unroll
+                    for(int p = 0; p < 4; p++){
+                        if(p >= outs) break;
+                        uint32_t d[16], d2[16];
+                        auto read = [&](uint32_t column, uint32_t (&r)[16]){
+                            if constexpr(ROWS) ld_32x32b_x16(from + column, r);
+                            else{ ld_16x256b_x2(from + column, r); ld_16x256b_x2(from + column + (16u << 16), r + 8); }
+                        };
+                        read((uint32_t)(64 * p), d);
+                        if(p < 2 && stacked) read((uint32_t)(64 * p + y.n), d2);       // stacked parts: both column ranges
+                        tc::tmem_wait_ld();
+#pragma unroll
+                        for(int i = 0; i < 8; i++){
+                            // ROWS: register pair i = pair i; else register pair 4 x + 2 j + s = pair 2 (2 x + s) + j
+                            const int at = ROWS ? i : 2 * (2 * (i >> 2) + (i & 1)) + ((i >> 1) & 1);
+                            const float f = inv[ROWS ? 0 : at >> 1];
+                            acc[p][at] = __ffma2_rn(make_float2(__uint_as_float(d[2 * i]), __uint_as_float(d[2 * i + 1])), make_float2(f, f), acc[p][at]);
+                            if(p < 2 && stacked)
+                                acc[p][at] = __ffma2_rn(make_float2(__uint_as_float(d2[2 * i]), __uint_as_float(d2[2 * i + 1])), make_float2(f, f), acc[p][at]);
+                        }
+                    }
+                    tc::fence_before_thread_sync();
+                    __syncwarp();
+                    if(lane == 0) tc::mbar_arrive(acc_empty + (u & 1u));
+                }
+                if(!ok) break;
+                // every MMA of this layer has completed: its input may be overwritten
+#pragma unroll
+                for(int p = 0; p < 4; p++){
+                    if(p >= outs) break;
+                    const Place at{row0, 64 * p + 16 * g, a.rows, y.N, y.ld};
+                    if constexpr(MODE == CH_FORWARD) store_slice<ROWS>(at, y.pre, lane, acc[p]);
+                    activate_slice_rt(acc[p], y.act);
+                    clear_beyond<ROWS>(at.col0, y.N, lane, acc[p]);
+                    if(!last) store_operand(p, acc[p]);
+                    else store_slice<ROWS>(at, y.out, lane, acc[p]);
+                }
+                if(MODE == CH_FORWARD && !last){
+#pragma unroll
+                    for(int p = 0; p < 4; p++){
+                        if(p >= outs) break;
+                        store_slice<ROWS>(Place{row0, 64 * p + 16 * g, a.rows, y.N, y.ld}, y.out, lane, acc[p]);
+                    }
+                }
+            }
+        }
+    }
+    tc::fence_before_thread_sync();
+    __syncthreads();
+    if(warp == CH_WARPS) tc::tmem_dealloc(tmem, 512);
+}
+
+// ---- weight images: a CTA per 32 output rows of a product, a warp per row. Every CTA finds the
+// largest magnitude of its layer's weights for itself (at most 256 KB from L2), which saves a launch in front ----------------------------------
+struct ChainImage { const float* W; const float* bias; uint8_t* image; float* tail; int N, K, block_begin; };
+struct ChainImages { int n; ChainImage y[CH_MAX_STEPS]; int blocks; };
+__global__ void __launch_bounds__(1024) chain_image_kernel(const __grid_constant__ ChainImages a){
+    __shared__ float largest[32];
+    int l = 0;
+    while(l + 1 < a.n && (int)blockIdx.x >= a.y[l + 1].block_begin) l++;
+    const ChainImage& y = a.y[l];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = (blockIdx.x - y.block_begin) * 32 + warp, rows = (y.N + 15) / 16 * 16, pieces = (y.K + 63) / 64;
+    float m = 0.0f;
+    const int count = y.N * y.K;
+    if((reinterpret_cast<uintptr_t>(y.W) & 15u) == 0 && (count & 3) == 0){
+#pragma unroll 8
+        for(int i = threadIdx.x; i < count / 4; i += 1024){ const float4 t = __ldg(reinterpret_cast<const float4*>(y.W) + i); m = fmaxf(m, fmaxf(fmaxf(fabsf(t.x), fabsf(t.y)), fmaxf(fabsf(t.z), fabsf(t.w)))); }
+    }
+    else{
+#pragma unroll 8
+        for(int i = threadIdx.x; i < count; i += 1024) m = fmaxf(m, fabsf(__ldg(y.W + i)));
+    }
+#pragma unroll
+    for(int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if(lane == 0) largest[warp] = m;
+    __syncthreads();
+    m = largest[lane];
+#pragma unroll
+    for(int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const uint32_t e = scale_exponent(m);
+    const float f = scale_of(e);
+    if((int)blockIdx.x == y.block_begin){
+        for(int i = threadIdx.x; i < 256; i += 1024) y.tail[i] = y.bias && i < y.N ? __ldg(y.bias + i) : 0.0f;
+        if(threadIdx.x == 0) y.tail[256] = inverse_scale_of(e);
+    }
+    if(n >= rows) return;
+    const uint32_t off = (uint32_t)n * 128 + ((((uint32_t)lane >> 2) ^ ((uint32_t)n & 7u)) << 4) + ((uint32_t)lane & 3u) * 4;
+    for(int c = 0; c < pieces; c++){
+        float v[2];
+#pragma unroll
+        for(int k = 0; k < 2; k++){
+            const int i = 64 * c + 2 * lane + k;
+            v[k] = n < y.N && i < y.K ? __ldg(y.W + (size_t)n * y.K + i) : 0.0f;
+        }
+        uint32_t lead, rest;
+        split_pair(make_float2(v[0] * f, v[1] * f), lead, rest);
+        uint8_t* unit = y.image + (size_t)c * rows * 256;
+        *reinterpret_cast<uint32_t*>(unit + off) = lead;
+        *reinterpret_cast<uint32_t*>(unit + (size_t)rows * 128 + off) = rest;
+    }
+}
+
+// ---- host side ---------------------------------------------------------------------------------------------------------------------------
+// Networks of up to eight layers, no wider than 256. A CTA takes 128 rows through all layers in the same time however few CTAs there are (37 us for
+// 64-256-256-256-16, 56 us when everything is kept; 17 and 21 us for 27-64-64-8), while the kernel per layer gains from a smaller batch: for wide
+// networks the lines cross between 1,024 and 2,048 rows (36 vs 70 us and 56 vs 73 us at 2,048, 36 vs 35 and 57 vs 35 at 512), for networks of up to
+// 128 columns near 8,192 (17 vs 24 and 21 vs 23 us).
+bool mlp_chain_eligible(const b200rl_mlp_shape* sh, int batch){
+    if(sh->n_layers > CH_MAX_STEPS) return false;
+    int widest = sh->input_dim;
+    for(int l = 0; l < sh->n_layers; l++) if(sh->dims[l] > widest) widest = sh->dims[l];
+    return widest <= 256 && batch >= (widest > 128 ? 2048 : 8192);
+}
+static size_t chain_image_bytes(int N, int K){
+    const size_t rows = (N + 15) / 16 * 16;
+    return rows * ((K + 63) / 64) * 256 + CH_TAIL;
+}
+size_t mlp_chain_workspace_bytes(const b200rl_mlp_shape* sh){
+    size_t n = 0; int I = sh->input_dim;
+    for(int l = 0; l < sh->n_layers; l++){ n += chain_image_bytes(sh->dims[l], I); I = sh->dims[l]; }
+    return n;
+}
+// the word that a kernel's expired wait sets, and its reset (b200rl_device_error_state, b200rl_device_error_clear)
+int mlp_chain_error_get(int* word){ B200RL_CUDA_TRY(cudaMemcpyFromSymbol(word, g_chain_error, sizeof(int))); return B200RL_OK; }
+int mlp_chain_error_clear(){ const int zero = 0; B200RL_CUDA_TRY(cudaMemcpyToSymbol(g_chain_error, &zero, sizeof(int))); return B200RL_OK; }
+
+static void chain_step(ChainStep& y, ChainImages& images, const float* W, const float* bias, int N, int K, uint8_t*& ws){
+    y.N = N; y.K = K; y.pieces = (K + 63) / 64; y.n = (N + 15) / 16 * 16;
+    ChainImage& m = images.y[images.n++];
+    m.W = W; m.N = N; m.K = K; m.block_begin = images.blocks;
+    m.bias = bias; m.image = ws; m.tail = reinterpret_cast<float*>(ws + chain_image_bytes(N, K) - CH_TAIL);
+    images.blocks += (y.n + 31) / 32;
+    y.image = m.image; y.tail = m.tail;
+    ws += chain_image_bytes(N, K);
+}
+template <int MODE>
+static int launch_chain(ChainArgs& a, const ChainImages& images, cudaStream_t s){
+    static std::atomic<bool> configured[MAX_DEVICES];
+    int dev = 0, sms = 0;
+    int rc = current_device(&dev);
+    if(rc) return rc;
+    if((rc = sm_count(&sms))) return rc;
+    if(!configured[dev].load(std::memory_order_acquire)){
+        B200RL_CUDA_TRY(cudaFuncSetAttribute(mlp_chain_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_SMEM));
+        configured[dev].store(true, std::memory_order_release);
+    }
+    chain_image_kernel<<<images.blocks, 1024, 0, s>>>(images);
+    B200RL_LAUNCH_CHECK("chain_image");
+    a.tiles = (a.rows + CH_ROWS - 1) / CH_ROWS;
+    mlp_chain_kernel<MODE><<<a.tiles < sms ? a.tiles : sms, CH_THREADS, CH_SMEM, s>>>(a);
+    B200RL_LAUNCH_CHECK("mlp_chain");
+    return B200RL_OK;
+}
+
+// pre == NULL: evaluate into y; otherwise forward into the arenas
+int mlp_chain_forward(const b200rl_mlp_shape* sh, const float* params, const float* x, int ldx, float* pre, float* out, float* y, int ldy, int batch, void* workspace,
+                      size_t workspace_bytes, cudaStream_t s){
+    if(!workspace || workspace_bytes < mlp_chain_workspace_bytes(sh) || (reinterpret_cast<uintptr_t>(workspace) & 15u)) return B200RL_ERR_UNSUPPORTED;
+    // a CTA reads inputs while another one writes outputs: outputs over the inputs take the kernels per layer
+    if(y && y < x + (size_t)batch * ldx && x < y + (size_t)batch * ldy) return B200RL_ERR_UNSUPPORTED;
+    ChainArgs a{};
+    ChainImages images{};
+    uint8_t* ws = static_cast<uint8_t*>(workspace);
+    a.rows = batch; a.in = x; a.ld_in = ldx; a.in_cols = sh->input_dim;
+    int I = sh->input_dim;
+    const float* p = params;
+    for(int l = 0; l < sh->n_layers; l++){
+        const int O = sh->dims[l];
+        ChainStep& t = a.step[a.n_steps++];
+        chain_step(t, images, p, p + (size_t)O * I, O, I, ws);
+        t.act = sh->acts[l]; t.ld = O;
+        if(pre){ t.pre = pre; t.out = out; pre += (size_t)batch * O; out += (size_t)batch * O; }
+        else if(l + 1 == sh->n_layers){ t.out = y; t.ld = ldy; }
+        p += (size_t)O * I + O; I = O;
+    }
+    return pre ? launch_chain<CH_FORWARD>(a, images, s) : launch_chain<CH_EVALUATE>(a, images, s);
+}
+
+}  // namespace b200rl

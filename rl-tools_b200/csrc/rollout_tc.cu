@@ -1,5 +1,5 @@
 // Tensor-core rollout for the OBS -> 64 -> 64 -> 1 actor (sm_100a, tcgen05 + TMEM). The environment is a compile-time policy (envs.cuh):
-// the Pendulum (the headline workload; also the on-policy collect and the device-side random numbers) and the two Acrobot variants
+// the Pendulum (the headline workload; also the on-policy collect and the device-side random numbers) and, from some 9,000 environments on, the two Acrobot variants
 // (trajectories from reset tables, with the terminated flag of every transition on request).
 //
 // One persistent CTA per SM, 512 threads = 4 independent groups of 128 threads. A group owns a tile of up to 128
@@ -121,7 +121,11 @@ __device__ __forceinline__ float act_or_rt(float x, int rt){
 // one step later, at the barrier it already has before its MMA batch. Three buffers rotate: the buffer of step t is read by the copy issued
 // after barrier t+1, the leader waits for that read before barrier t+2, and the buffer is written again in step t+3. Requires 16-byte aligned
 // row starts (n_envs and the slab origin multiples of 4, aligned output pointers); the host selects the plain-store instantiation otherwise.
-template <typename ENV, int A1, int A2, bool COLLECT, bool BULK>
+// PART: tiles of at most three warps of environments. A warp without an environment takes no part in a step but for the barriers, and group g's tile starts at
+// warp g, so that the four groups' environments share out the SM's four schedulers. (A kernel of its own: in the full one the test of
+// it costs 2 %.) With tiles dealt out over the SMs first, a step of 500 environments takes 1.95 us (2.91 with four tiles to a CTA), of 10,007 1.94
+// (2.73), of 20,000 2.44 (3.06).
+template <typename ENV, int A1, int A2, bool COLLECT, bool BULK, bool PART>
 __global__ void __launch_bounds__(THREADS, 1) rollout_tc_kernel(RolloutArgs a, int n_tiles, int envs_per_tile){
     static_assert(!(COLLECT && BULK), "dataset rows are strided: plain stores");
     constexpr bool IS_PENDULUM = std::is_same<ENV, PendulumEnv>::value;
@@ -214,9 +218,11 @@ __global__ void __launch_bounds__(THREADS, 1) rollout_tc_kernel(RolloutArgs a, i
     if constexpr(COLLECT) head.init(a.log_std);
     uint8_t* stage_base = base + OFF_STAGE + (uint32_t)g * STAGE_GROUP_BYTES;
 
+    const int vr = PART ? (r + TILE - 32 * g) & (TILE - 1) : r;              // row of the tile
+    const bool active = !PART || (vr & ~31) < envs_per_tile;
     const int rounds = (n_tiles + (int)gridDim.x * GROUPS - 1) / ((int)gridDim.x * GROUPS);
     for(int round = 0; round < rounds && !failed; round++){
-        const int tile = (round * (int)gridDim.x + (int)blockIdx.x) * GROUPS + g;
+        const int tile = (round * GROUPS + g) * (int)gridDim.x + (int)blockIdx.x;             // over the SMs first
         if(tile >= n_tiles){
             // no environments for this group in this round: it still hands the tensor token on, once per step
             if(r == 0){
@@ -228,8 +234,8 @@ __global__ void __launch_bounds__(THREADS, 1) rollout_tc_kernel(RolloutArgs a, i
             }
             continue;
         }
-        const int local = tile * envs_per_tile + r;
-        const bool valid = r < envs_per_tile && local < a.env_count;
+        const int local = tile * envs_per_tile + vr;
+        const bool valid = vr < envs_per_tile && local < a.env_count;
         const int e = a.env_begin + (valid ? local : 0);
         float state[S], er = 0.0f; int es = 0, resets = 0; bool trunc = false;
 #pragma unroll
@@ -257,66 +263,68 @@ __global__ void __launch_bounds__(THREADS, 1) rollout_tc_kernel(RolloutArgs a, i
             float* st_act = st_obs + TILE * O;
             float* st_rew = st_act + TILE;
             StepDraws draws{};             // the trajectory-only kernels need the draws at a reset only: nothing per step on their hot path
-            if constexpr(IS_PENDULUM){ if(a.device_rng && (COLLECT || trunc)) draws = step_draws(a.rng_seed, a.rng_step0 + (unsigned long long)t, (uint32_t)e); }
-            if(trunc && valid){
-                bool drawn = false;
-                if constexpr(IS_PENDULUM){
-                    if(a.device_rng){    // theta ~ U(-pi, pi), theta_dot ~ U(-1, 1) (rl/environments/pendulum/operations_generic.h:57-61)
-                        state[0] = fmaf(draws.u_theta, 2.0f * pendulum::PI_F, -pendulum::PI_F); state[1] = fmaf(draws.u_theta_dot, 2.0f, -1.0f);
-                        drawn = true;
-                    }
-                }
-                if(!drawn){
-                    if(a.reset_states != nullptr && resets < a.n_reset_rounds){
-                        const float* rs = a.reset_states + ((size_t)resets * a.n_envs + e) * RD;      // scalar loads: the table may be a view at any 4-byte offset
-                        float u[RD];
-#pragma unroll
-                        for(int k = 0; k < RD; k++) u[k] = __ldg(rs + k);
-                        ENV::reset(state, u);
-                    }
-                    else if(a.error_flag) *a.error_flag = 1;
-                }
-                resets++; es = 0; er = 0.0f;
-            }
             float o[O];
-            ENV::observe(state, o);
             const size_t row = (size_t)t * a.n_envs + e;
             float* drow = COLLECT ? a.dataset + row * ld : nullptr;
-            if(valid){
-#pragma unroll
-                for(int k = 0; k < O; k++){
-                    if constexpr(COLLECT) drow[COL_OBS + k] = o[k];
-                    else if constexpr(BULK) st_obs[r * O + k] = o[k];
-                    else a.obs[row * O + k] = o[k];
-                }
-            }
-
-            // ---- layer 1 (CUDA cores, weights as constant-bank operands); leading fp16 parts -> TMEM, remainder parts -> swizzled smem tile ----
-            uint32_t lead_all[32];
-            float2 o2[O];
-#pragma unroll
-            for(int k = 0; k < O; k++) o2[k] = make_float2(o[k], o[k]);
-#pragma unroll
-            for(int c = 0; c < 8; c++){                  // 16-byte chunk c of the row: units 8c .. 8c+7
-                uint32_t rest[4];
-#pragma unroll
-                for(int q = 0; q < 4; q++){
-                    float h[2];
-                    {
-                        const int pair = c * 4 + q;                                          // units 2 pair, 2 pair + 1
-                        float2 acc = *reinterpret_cast<const float2*>(&c_actor[C_B1 + 2 * pair]);            // bias first, inputs ascending: the reference's order
-#pragma unroll
-                        for(int k = 0; k < O; k++) acc = __ffma2_rn(c_w1_pairs[pair * O + k], o2[k], acc);
-                        if constexpr(A1 == B200RL_ACT_RELU){ h[0] = acc.x; h[1] = acc.y; }       // the ReLU rides on the conversions below
-                        else { h[0] = act_or_rt<A1>(acc.x, act1); h[1] = act_or_rt<A1>(acc.y, act1); }
+            if(active){
+                if constexpr(IS_PENDULUM){ if(a.device_rng && (COLLECT || trunc)) draws = step_draws(a.rng_seed, a.rng_step0 + (unsigned long long)t, (uint32_t)e); }
+                if(trunc && valid){
+                    bool drawn = false;
+                    if constexpr(IS_PENDULUM){
+                        if(a.device_rng){    // theta ~ U(-pi, pi), theta_dot ~ U(-1, 1) (rl/environments/pendulum/operations_generic.h:57-61)
+                            state[0] = fmaf(draws.u_theta, 2.0f * pendulum::PI_F, -pendulum::PI_F); state[1] = fmaf(draws.u_theta_dot, 2.0f, -1.0f);
+                            drawn = true;
+                        }
                     }
-                    if constexpr(A1 == B200RL_ACT_RELU) split_f16_pair_relu(h[0], h[1], lead_all[c * 4 + q], rest[q]);
-                    else split_f16_pair(h[0], h[1], lead_all[c * 4 + q], rest[q]);
+                    if(!drawn){
+                        if(a.reset_states != nullptr && resets < a.n_reset_rounds){
+                            const float* rs = a.reset_states + ((size_t)resets * a.n_envs + e) * RD;      // scalar loads: the table may be a view at any 4-byte offset
+                            float u[RD];
+#pragma unroll
+                            for(int k = 0; k < RD; k++) u[k] = __ldg(rs + k);
+                            ENV::reset(state, u);
+                        }
+                        else if(a.error_flag) *a.error_flag = 1;
+                    }
+                    resets++; es = 0; er = 0.0f;
                 }
-                *reinterpret_cast<uint4*>(my_row_rest + (((uint32_t)c ^ swz) << 4)) = make_uint4(rest[0], rest[1], rest[2], rest[3]);
+                ENV::observe(state, o);
+                if(valid){
+#pragma unroll
+                    for(int k = 0; k < O; k++){
+                        if constexpr(COLLECT) drow[COL_OBS + k] = o[k];
+                        else if constexpr(BULK) st_obs[vr * O + k] = o[k];
+                        else a.obs[row * O + k] = o[k];
+                    }
+                }
+
+                // ---- layer 1 (CUDA cores, weights as constant-bank operands); leading fp16 parts -> TMEM, remainder parts -> swizzled smem tile ----
+                uint32_t lead_all[32];
+                float2 o2[O];
+#pragma unroll
+                for(int k = 0; k < O; k++) o2[k] = make_float2(o[k], o[k]);
+#pragma unroll
+                for(int c = 0; c < 8; c++){                  // 16-byte chunk c of the row: units 8c .. 8c+7
+                    uint32_t rest[4];
+#pragma unroll
+                    for(int q = 0; q < 4; q++){
+                        float h[2];
+                        {
+                            const int pair = c * 4 + q;                                          // units 2 pair, 2 pair + 1
+                            float2 acc = *reinterpret_cast<const float2*>(&c_actor[C_B1 + 2 * pair]);            // bias first, inputs ascending: the reference's order
+#pragma unroll
+                            for(int k = 0; k < O; k++) acc = __ffma2_rn(c_w1_pairs[pair * O + k], o2[k], acc);
+                            if constexpr(A1 == B200RL_ACT_RELU){ h[0] = acc.x; h[1] = acc.y; }       // the ReLU rides on the conversions below
+                            else { h[0] = act_or_rt<A1>(acc.x, act1); h[1] = act_or_rt<A1>(acc.y, act1); }
+                        }
+                        if constexpr(A1 == B200RL_ACT_RELU) split_f16_pair_relu(h[0], h[1], lead_all[c * 4 + q], rest[q]);
+                        else split_f16_pair(h[0], h[1], lead_all[c * 4 + q], rest[q]);
+                    }
+                    *reinterpret_cast<uint4*>(my_row_rest + (((uint32_t)c ^ swz) << 4)) = make_uint4(rest[0], rest[1], rest[2], rest[3]);
+                }
+                tc::tmem_st_32x32(tmem_a + lane_off, lead_all);
+                tc::tmem_wait_st();
             }
-            tc::tmem_st_32x32(tmem_a + lane_off, lead_all);
-            tc::tmem_wait_st();
             tc::fence_proxy_async_smem();
             tc::fence_before_thread_sync();
             if constexpr(BULK){ if(r == 0) tc::bulk_wait_read<0>(); }      // the copy of step t-2 has read its buffer (re-used from step t+1 on)
@@ -345,6 +353,7 @@ __global__ void __launch_bounds__(THREADS, 1) rollout_tc_kernel(RolloutArgs a, i
                 if constexpr(BULK){ if(t > 0) bulk_flush(t - 1); }          // every thread of the group finished step t-1 before this step's barrier
             }
             __syncwarp();                                     // the leader's lanes rejoin before the warp-wide TMEM loads
+            if(!active){ phase ^= 1; continue; }
             if(!tc::mbar_wait_bounded(mbar, phase, WAIT_LIMIT_CYCLES)){
                 *abort_flag = 1;                              // seen by the whole group after its next barrier
                 if(a.error_flag) *a.error_flag = 2;
@@ -392,7 +401,7 @@ __global__ void __launch_bounds__(THREADS, 1) rollout_tc_kernel(RolloutArgs a, i
             }
             else{
                 if(valid){
-                    if constexpr(BULK){ st_act[r] = action; st_rew[r] = rwd; }
+                    if constexpr(BULK){ st_act[vr] = action; st_rew[vr] = rwd; }
                     else{ a.act[row] = action; a.rew[row] = rwd; }
                 }
                 bool term = false;
@@ -440,7 +449,7 @@ __global__ void __launch_bounds__(THREADS, 1) rollout_tc_kernel(RolloutArgs a, i
 // The kernel fills every SM, so this ordering costs no concurrency. The event, like the kernel's shared-memory attribute, belongs
 // to a device: both are kept per device ordinal.
 namespace {
-struct TcDeviceState { cudaEvent_t order = nullptr; bool configured[3][16] = {}; float2* w1_pairs = nullptr; };
+struct TcDeviceState { cudaEvent_t order = nullptr; bool configured[3][16][2] = {}; float2* w1_pairs = nullptr; };
 TcDeviceState g_tc_state[MAX_DEVICES];
 std::mutex g_tc_mutex;
 }
@@ -466,35 +475,40 @@ static int upload_small_layers(TcDeviceState& st, const float* params, int obs_d
 
 template <typename ENV> struct EnvIndex { static constexpr int value = std::is_same<ENV, PendulumEnv>::value ? 0 : std::is_same<ENV, AcrobotSwingupEnv>::value ? 1 : 2; };
 
-template <typename ENV, int A1, int A2, bool COLLECT, bool BULK>
-static int launch_tc_variant(const RolloutArgs& a, cudaStream_t s, int variant){
+template <typename ENV, int A1, int A2, bool COLLECT, bool BULK, bool PART>
+static int launch_tc_part(const RolloutArgs& a, cudaStream_t s, int variant, int sms, int ept){
     constexpr uint32_t SMEM_BYTES = smem_bytes(ENV::OBS_DIM);
-    int dev = 0, sms = 0;
+    int dev = 0;
     int rc = current_device(&dev);
-    if(rc) return rc;
-    rc = sm_count(&sms);
     if(rc) return rc;
     std::lock_guard<std::mutex> lock(g_tc_mutex);
     TcDeviceState& st = g_tc_state[dev];
-    if(!st.configured[EnvIndex<ENV>::value][variant]){
-        B200RL_CUDA_TRY(cudaFuncSetAttribute(rollout_tc_kernel<ENV, A1, A2, COLLECT, BULK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
-        st.configured[EnvIndex<ENV>::value][variant] = true;
+    if(!st.configured[EnvIndex<ENV>::value][variant][PART]){
+        B200RL_CUDA_TRY(cudaFuncSetAttribute(rollout_tc_kernel<ENV, A1, A2, COLLECT, BULK, PART>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
+        st.configured[EnvIndex<ENV>::value][variant][PART] = true;
     }
     cudaEvent_t order_event = nullptr;
     rc = upload_small_layers(st, a.params, ENV::OBS_DIM, s, &order_event);
+    if(rc) return rc;
+    const int n_tiles = (a.env_count + ept - 1) / ept;
+    const int grid = n_tiles < sms ? n_tiles : sms;
+    rollout_tc_kernel<ENV, A1, A2, COLLECT, BULK, PART><<<grid, THREADS, SMEM_BYTES, s>>>(a, n_tiles, ept);
+    B200RL_LAUNCH_CHECK("rollout_tc");
+    if(order_event) B200RL_CUDA_TRY(cudaEventRecord(order_event, s));
+    return B200RL_OK;
+}
+
+template <typename ENV, int A1, int A2, bool COLLECT, bool BULK>
+static int launch_tc_variant(const RolloutArgs& a, cudaStream_t s, int variant){
+    int sms = 0;
+    const int rc = sm_count(&sms);
     if(rc) return rc;
     // spread the environments evenly over every group of every SM: tiles of <= 128 environments (a multiple of 4)
     const int groups_total = sms * GROUPS;
     int ept = ((a.env_count + groups_total - 1) / groups_total + 3) / 4 * 4;
     if(ept < 32) ept = 32;
     if(ept > TILE) ept = TILE;
-    const int n_tiles = (a.env_count + ept - 1) / ept;
-    int grid = (n_tiles + GROUPS - 1) / GROUPS;
-    if(grid > sms) grid = sms;
-    rollout_tc_kernel<ENV, A1, A2, COLLECT, BULK><<<grid, THREADS, SMEM_BYTES, s>>>(a, n_tiles, ept);
-    B200RL_LAUNCH_CHECK("rollout_tc");
-    if(order_event) B200RL_CUDA_TRY(cudaEventRecord(order_event, s));
-    return B200RL_OK;
+    return ept <= TILE - 32 ? launch_tc_part<ENV, A1, A2, COLLECT, BULK, true>(a, s, variant, sms, ept) : launch_tc_part<ENV, A1, A2, COLLECT, BULK, false>(a, s, variant, sms, ept);
 }
 
 // Bulk stores need 16-byte aligned row starts in all three outputs; per-thread stores otherwise (and always for the strided dataset rows)

@@ -247,3 +247,28 @@ def test_unsupported_actor_width_is_refused(lib, torch):
     st, es, tr, er = runner(torch, np.zeros((4, 2), np.float32))
     with pytest.raises(lib.B200RLError):
         lib.pendulum_rollout(shape, torch.zeros(48 * 3 + 48 + 48 * 48 + 48 + 48 + 1, device="cuda"), st, es, tr, er, None, 1, 200)
+
+
+@pytest.mark.parametrize("env,hidden,n", [("acrobot", 64, 1), ("acrobot", 64, 3553), ("acrobot", 32, 9473), ("acrobot_swingup", 128, 3552), ("acrobot_swingup", 16, 9472),
+                                          ("pendulum", 128, 37), ("pendulum", 128, 3553), ("pendulum", 128, 9473), ("pendulum", 32, 9473)])
+def test_lanes_per_environment(lib, torch, env, hidden, n):
+    """16, 4 and 1 threads per environment on both sides of the numbers of environments where the launch changes from one to the next: the first environments'
+    trajectories are the same bits as in a launch of their own, and one step agrees with the oracle."""
+    envs = {"pendulum": (lib.ENV_PENDULUM, 3, 2, 2), "acrobot_swingup": (lib.ENV_ACROBOT_SWINGUP, 6, 4, 2), "acrobot": (lib.ENV_ACROBOT, 6, 4, 4)}
+    index, O, S, R = envs[env]
+    rs = np.random.RandomState(n)
+    T, acts = 7, ["relu", "tanh", "tanh"]
+    shape, oshape = lib.MlpShape.make(O, [hidden, hidden, 1], acts), oracle.MlpShape.make(O, [hidden, hidden, 1], acts)
+    params = (rs.uniform(-1, 1, shape.num_params()) * (1.5 / np.sqrt(hidden))).astype(np.float32)
+    states, table = rs.uniform(-1, 1, (n, S)).astype(np.float32), rs.uniform(-1, 1, (3, n, R)).astype(np.float32)
+
+    def rollout(count, steps):
+        st, es, tr, er = runner(torch, states[:count])
+        obs, act, rew = lib.env_rollout(index, shape, dev(torch, params), st, es, tr, er, dev(torch, np.ascontiguousarray(table[:, :count])), steps, 3)
+        return [t.cpu().numpy().reshape(steps, count, -1) for t in (obs, act, rew)] + [t.cpu().numpy() for t in (st, es, tr, er)]
+    whole, few = rollout(n, T), rollout(min(n, 33), T)
+    for a, b in zip(whole, few):
+        a = a[:, :b.shape[1]] if a.ndim == 3 else a[:len(b)]
+        assert np.array_equal(a, b)
+    want_act = oracle.Oracle().mlp_evaluate(oshape, params, whole[0].reshape(T * n, O)).reshape(-1)
+    close(whole[1].reshape(-1), want_act, what="actions on the kernel's observations")

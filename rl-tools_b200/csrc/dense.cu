@@ -506,6 +506,13 @@ static int dense_backward_impl(const float* W, const float* x, int ldx, const fl
     return B200RL_OK;
 }
 
+// dst[i] += the sum of `segments` partial sums `stride` apart, in a fixed order
+int reduce_partials_into(float* dst, const float* partial, int n, long long stride, int segments, cudaStream_t s){
+    reduce_strided_partials_kernel<<<(n + 31) / 32, dim3(32, 8), 0, s>>>(dst, partial, n, stride, segments);
+    B200RL_LAUNCH_CHECK("reduce_partials");
+    return B200RL_OK;
+}
+
 // whole-network kernels for small batches (mlp_fused.cu)
 bool mlp_fused_eligible(const b200rl_mlp_shape* sh, int batch);
 size_t mlp_fused_backward_scratch_bytes(const b200rl_mlp_shape* sh, int batch);
@@ -518,6 +525,10 @@ bool mlp_chain_eligible(const b200rl_mlp_shape* sh, int batch);
 size_t mlp_chain_workspace_bytes(const b200rl_mlp_shape* sh);
 int mlp_chain_forward(const b200rl_mlp_shape* sh, const float* params, const float* x, int ldx, float* pre, float* out, float* y, int ldy, int batch, void* workspace,
                       size_t workspace_bytes, cudaStream_t s);
+bool mlp_chain_backward_eligible(const b200rl_mlp_shape* sh, int batch);
+size_t mlp_chain_backward_scratch_bytes(const b200rl_mlp_shape* sh, int batch);
+int mlp_chain_backward(const b200rl_mlp_shape* sh, const float* params, float* grads, const float* x, int ldx, const float* pre, const float* out, const float* d_out,
+                       float* d_input, int batch, void* scratch, size_t scratch_bytes, cudaStream_t s);
 
 // whole training step in one cooperative launch (mlp_team.cu)
 bool mlp_team_eligible(const b200rl_mlp_shape* sh, int rows);
@@ -700,7 +711,9 @@ size_t b200rl_mlp_backward_scratch_bytes(const b200rl_mlp_shape* sh, int batch){
     size_t m = 0; int I = sh->input_dim;
     for(int l = 0; l < sh->n_layers; l++){ const size_t b = backward_scratch_total(batch, I, sh->dims[l]); if(b > m) m = b; I = sh->dims[l]; }
     const size_t fused = mlp_fused_backward_scratch_bytes(sh, batch), team = mlp_team_scratch_bytes(sh, batch);
+    const size_t chain = mlp_chain_backward_scratch_bytes(sh, batch);
     if(fused > m) m = fused;
+    if(chain > m) m = chain;
     return team > m ? team : m;
 }
 
@@ -712,6 +725,10 @@ int b200rl_mlp_backward(const b200rl_mlp_shape* sh, const float* params, float* 
     int L = sh->n_layers;
     if(L > 1 && (!tick || (L > 2 && !tock))) return B200RL_ERR_INVALID_ARGUMENT;
     if(batch == 0) return B200RL_OK;
+    if(mlp_chain_backward_eligible(sh, batch)){
+        const int rc = mlp_chain_backward(sh, params, grads, x, ldx, pre, out, d_out, d_input, batch, scratch, scratch_bytes, (cudaStream_t)stream);
+        if(rc != B200RL_ERR_UNSUPPORTED) return rc;
+    }
     // small batches: the whole pass in two launches, when the caller's scratch has room for the gradients of all layers
     if(mlp_fused_eligible(sh, batch) && scratch && scratch_bytes >= mlp_fused_backward_scratch_bytes(sh, batch))
         return mlp_fused_backward(sh, params, grads, x, ldx, pre, out, d_out, d_input, batch, scratch, scratch_bytes, (cudaStream_t)stream);

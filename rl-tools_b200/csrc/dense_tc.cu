@@ -541,19 +541,20 @@ int launch_gemm_tc(const GemmArgs& a, int epilogue, int activation, bool a_kcont
 
 }  // namespace b200rl
 
-namespace b200rl { int mlp_chain_error_get(int* word); int mlp_chain_error_clear(); }                // mlp_chain.cu
+namespace b200rl { int mlp_chain_error_get(int* word); int mlp_chain_error_clear(); int mlp_grad_error_get(int* word); int mlp_grad_error_clear(); }     // mlp_chain.cu, mlp_grad.cu
 
 extern "C" int b200rl_device_error_state(int* state_host){
     if(!state_host) return B200RL_ERR_INVALID_ARGUMENT;
     B200RL_CUDA_TRY(cudaMemcpyFromSymbol(state_host, b200rl::g_dense_tc_error, sizeof(int)));
-    int chain = 0;
-    const int rc = b200rl::mlp_chain_error_get(&chain);
-    if(rc) return rc;
-    *state_host |= chain;
+    int chain = 0, grad = 0;
+    int rc = b200rl::mlp_chain_error_get(&chain);
+    if(rc || (rc = b200rl::mlp_grad_error_get(&grad))) return rc;
+    *state_host |= chain | grad;
     return B200RL_OK;
 }
 extern "C" int b200rl_device_error_clear(void){
     const int zero = 0;
     B200RL_CUDA_TRY(cudaMemcpyToSymbol(b200rl::g_dense_tc_error, &zero, sizeof(int)));
-    return b200rl::mlp_chain_error_clear();
+    const int rc = b200rl::mlp_chain_error_clear();
+    return rc ? rc : b200rl::mlp_grad_error_clear();
 }

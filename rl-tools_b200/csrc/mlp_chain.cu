@@ -3,6 +3,8 @@
 // pre-activations and outputs of a training forward pass. Serves
 //   evaluate                 y = mlp(x)                                                        (nn_models/mlp/operations_generic.h:77-102)
 //   forward                  the same, keeping pre-activations and outputs of every layer       (:103-120)
+//   backward                 the chain d_pre = act'(pre) * (W^T d_pre of the layer above), every d_pre kept for the parameter gradients (mlp_grad.cu), and
+//                            the input gradient (:152-173)
 //
 // Arithmetic: fp32 operands as two fp16 parts, x = lead + rest (11 + 11 significant bits), three passes rest * lead, lead * rest, lead * lead with
 // fp32 accumulation -- the precision of three tf32 passes at twice their rate and half their shared memory. fp16's range is met by powers of two
@@ -29,10 +31,11 @@
 // Bound by the tensor core and, between layers, by what the 16 warps do to a row tile before the next layer can start (about a third of the time), in
 // the forward pass by the stores. Measured, 64-256-256-256-16 at 1,048,576 rows: evaluate 3,236 -> 1,450 us (0.58 ms at the rate of three fp16
 // passes), forward 3,366 -> 2,850 us (6.8 GB, 1.0 ms at the copy bandwidth); 27-64-64-8 at 524,288 rows: evaluate 336 -> 218 us, forward 367 -> 369.
+// Backward, 64-256-256-256-16 at 1,048,576 rows: 3.04 ms for the chain of d_pre (6.5 GB; the products per layer and the passes over d_pre took 4.1 ms).
 #include "common.cuh"
 #include "tcgen05.cuh"
+#include "split_f16.cuh"
 #include <atomic>
-#include <cuda_fp16.h>
 
 namespace b200rl {
 
@@ -46,42 +49,29 @@ constexpr uint32_t CH_SMEM = CH_A + CH_STAGES * CH_STAGE + CH_EXP + 256 + 1024;
 static_assert(CH_SMEM <= 227 * 1024, "shared memory");
 constexpr size_t CH_TAIL = 2048;                                  // behind an image: see ChainStep::tail
 constexpr long long CH_WAIT_LIMIT = 2000000000LL;
-enum { CH_EVALUATE = 0, CH_FORWARD = 1 };
+enum { CH_EVALUATE = 0, CH_FORWARD = 1, CH_BACKWARD = 2 };
 }
 
 struct ChainStep {
     int N, K, pieces, n, act;                         // n: N rounded up to 16
     const uint8_t* image; const float* tail;          // tail: 256 biases (zeros beyond N), then the inverse of the weights' scale
     float* pre; float* out; long long ld;             // forward: this layer's arenas [rows, N]; evaluate: the last layer's outputs with their row pitch
+    // backward: pre_in = pre-activations [rows, N] of the layer below, act = its activation (identity where there is none), out = its d_pre with
+    // row pitch ld, or the network's input gradient, or NULL
+    const float* pre_in;
 };
 struct ChainArgs {
     int n_steps, rows, tiles;
     ChainStep step[CH_MAX_STEPS];
     const float* in; long long ld_in; int in_cols;
+    // backward: in = gradient of the outputs; the last layer's pre-activations [rows, in_cols] and activation; its d_pre, NULL when that is `in` or not wanted
+    const float* in_pre; int in_act;
+    float* in_out; long long ld_in_out;
 };
 
 __device__ int g_chain_error = 0;
 
 namespace {
-__device__ __forceinline__ uint32_t pack_f16(float lo, float hi){
-    uint32_t r;
-    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
-}
-__device__ __forceinline__ void split_pair(float2 v, uint32_t& lead, uint32_t& rest){
-    lead = pack_f16(v.x, v.y);
-    const float2 back = __half22float2(*reinterpret_cast<const __half2*>(&lead));
-    const float2 d = __ffma2_rn(back, make_float2(-1.0f, -1.0f), v);
-    rest = pack_f16(d.x, d.y);
-}
-// biased exponent of the piece's largest magnitude, clamped so that the scale 2^(14 - e) and its inverse are normal numbers
-__device__ __forceinline__ uint32_t scale_exponent(float largest){
-    const uint32_t e = (__float_as_uint(largest) >> 23) & 0xFFu;
-    return e < 15u ? 15u : e > 254u ? 254u : e;
-}
-__device__ __forceinline__ float scale_of(uint32_t e){ return __uint_as_float((268u - e) << 23); }
-__device__ __forceinline__ float inverse_scale_of(uint32_t e){ return __uint_as_float((e - 14u) << 23); }
-
 // Where the 16 values (8 pairs of neighbouring columns) of a thread lie in its warp's 16 columns of a piece.
 //   ROWS:  one row, 16 columns (tcgen05.ld 32x32b): no exchange within the warp, 16-byte shared-memory stores; pair i = columns 2 i, 2 i + 1 of row `lane`
 //   !ROWS: four rows 8 apart, 4 columns each (16x256b): a global store instruction writes whole 32-byte sectors; pair 2 s + j = columns 8 j + 2 (lane & 3),
@@ -103,6 +93,20 @@ __device__ __forceinline__ void activate_slice_rt(Slice& v, int act){
         case B200RL_ACT_TANH: activate_slice<B200RL_ACT_TANH>(v); break;
         case B200RL_ACT_FAST_TANH: activate_slice<B200RL_ACT_FAST_TANH>(v); break;
         default: activate_slice<B200RL_ACT_SIGMOID>(v); break;
+    }
+}
+template <int ACT>
+__device__ __forceinline__ void differentiate_slice(Slice& v, const Slice& pre){
+#pragma unroll
+    for(int i = 0; i < 8; i++){ v[i].x *= d_activation<ACT>(pre[i].x); v[i].y *= d_activation<ACT>(pre[i].y); }
+}
+__device__ __forceinline__ void differentiate_slice_rt(Slice& v, const Slice& pre, int act){
+    switch(act){
+        case B200RL_ACT_IDENTITY: break;
+        case B200RL_ACT_RELU: differentiate_slice<B200RL_ACT_RELU>(v, pre); break;
+        case B200RL_ACT_TANH: differentiate_slice<B200RL_ACT_TANH>(v, pre); break;
+        case B200RL_ACT_FAST_TANH: differentiate_slice<B200RL_ACT_FAST_TANH>(v, pre); break;
+        default: differentiate_slice<B200RL_ACT_SIGMOID>(v, pre); break;
     }
 }
 // a slice at (row0, col0) of a [rows, N] matrix with row pitch ld
@@ -163,6 +167,11 @@ __device__ __forceinline__ void ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16])
 __device__ __forceinline__ void ld_16x256b_x2(uint32_t taddr, uint32_t* r){
     asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+// a tile's rows of a matrix into L2
+__device__ __forceinline__ void prefetch_rows(const float* p, long long ld, int row0, int rows){
+    const uintptr_t from = (reinterpret_cast<uintptr_t>(p + row0 * ld) + 15) & ~(uintptr_t)15, to = reinterpret_cast<uintptr_t>(p + (long long)min(row0 + CH_ROWS, rows) * ld) & ~(uintptr_t)15;
+    if(to > from) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(from), "r"((uint32_t)(to - from)) : "memory");
 }
 }  // namespace
 
@@ -259,6 +268,13 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
                     const uint32_t part = (uint32_t)y.n * 128;
                     const bool stacked = y.n <= 128;
                     const uint8_t* unit = y.image;
+                    if constexpr(MODE == CH_BACKWARD){                  // what the element-wise part will read, into L2 about a layer's MMAs ahead of it
+                        if(y.act != B200RL_ACT_IDENTITY) prefetch_rows(y.pre_in, y.N, tile * CH_ROWS, a.rows);
+                        if(st == 0 && tile + (int)gridDim.x < a.tiles){
+                            prefetch_rows(a.in, a.ld_in, (tile + gridDim.x) * CH_ROWS, a.rows);
+                            if(a.in_act != B200RL_ACT_IDENTITY) prefetch_rows(a.in_pre, a.in_cols, (tile + gridDim.x) * CH_ROWS, a.rows);
+                        }
+                    }
                     for(int c = 0; c < y.pieces && ok; c++, unit += 2 * part){
                         for(int k = stacked ? 0 : 1; k >= 0; k--, w++){
                             const uint32_t s = w % CH_STAGES, bytes = stacked ? 2 * part : part;
@@ -344,7 +360,18 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
 #pragma unroll
             for(int p = 0; p < 4; p++){
                 if(p >= a.step[0].pieces) break;
-                if(p < 2){ if(!loaded) load_input(tile, p, acc[2 + p]); store_operand(p, acc[2 + p]); }
+                if constexpr(MODE == CH_BACKWARD){
+                    const Place at{row0, 64 * p + 16 * g, a.rows, a.in_cols, a.ld_in};
+                    load_slice<ROWS>(at, a.in, lane, acc[0]);
+                    if(a.in_act != B200RL_ACT_IDENTITY){
+                        load_slice<ROWS>(Place{at.row0, at.col0, a.rows, a.in_cols, a.in_cols}, a.in_pre, lane, acc[1]);
+                        differentiate_slice_rt(acc[0], acc[1], a.in_act);
+                        clear_beyond<ROWS>(at.col0, a.in_cols, lane, acc[0]);
+                    }
+                    store_operand(p, acc[0]);
+                    if(a.in_out) store_slice<ROWS>(Place{at.row0, at.col0, a.rows, a.in_cols, a.ld_in_out}, a.in_out, lane, acc[0]);
+                }
+                else if(p < 2){ if(!loaded) load_input(tile, p, acc[2 + p]); store_operand(p, acc[2 + p]); }
                 else{ load_input(tile, p, acc[p - 2]); store_operand(p, acc[p - 2]); }
             }
             loaded = false;
@@ -372,13 +399,17 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
                         }
                     }
                 }
-                if(last && stacked && tile + (int)gridDim.x < a.tiles){  // a narrow last layer leaves room for the next tile's inputs
+                if(MODE != CH_BACKWARD && last && stacked && tile + (int)gridDim.x < a.tiles){  // a narrow last layer leaves room for the next tile's inputs
                     load_input(tile + gridDim.x, 0, acc[2]);
                     if(a.step[0].pieces > 1) load_input(tile + gridDim.x, 1, acc[3]);
                     loaded = true;
                 }
                 const float weights = __ldg(y.tail + 256);              // inverse of the weights' scale
+                Slice below;                                             // backward: pre-activations of the next piece
                 for(int c = 0; c < y.pieces; c++, u++){
+                    if constexpr(MODE == CH_BACKWARD){
+                        if(c + 1 == y.pieces && y.act != B200RL_ACT_IDENTITY) load_slice<ROWS>(Place{row0, 16 * g, a.rows, y.N, y.N}, y.pre_in, lane, below);
+                    }
                     if(!(ok = wait(acc_full + (u & 1u), (u >> 1) & 1u))) break;
                     tc::fence_after_thread_sync();
                     const uint8_t* e = exps + c * CH_ROWS + q * 32;
@@ -418,12 +449,18 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
                     if(p >= outs) break;
                     const Place at{row0, 64 * p + 16 * g, a.rows, y.N, y.ld};
                     if constexpr(MODE == CH_FORWARD) store_slice<ROWS>(at, y.pre, lane, acc[p]);
-                    activate_slice_rt(acc[p], y.act);
+                    if constexpr(MODE == CH_BACKWARD){
+                        if(y.act != B200RL_ACT_IDENTITY){
+                            differentiate_slice_rt(acc[p], below, y.act);
+                            if(p + 1 < outs) load_slice<ROWS>(Place{row0, at.col0 + 64, a.rows, y.N, y.N}, y.pre_in, lane, below);
+                        }
+                    }
+                    else activate_slice_rt(acc[p], y.act);
                     clear_beyond<ROWS>(at.col0, y.N, lane, acc[p]);
                     if(!last) store_operand(p, acc[p]);
-                    else store_slice<ROWS>(at, y.out, lane, acc[p]);
+                    else if(MODE != CH_BACKWARD || y.out) store_slice<ROWS>(at, y.out, lane, acc[p]);
                 }
-                if(MODE == CH_FORWARD && !last){
+                if(MODE != CH_EVALUATE && !last && (MODE == CH_FORWARD || y.out)){
 #pragma unroll
                     for(int p = 0; p < 4; p++){
                         if(p >= outs) break;
@@ -440,7 +477,8 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
 
 // ---- weight images: a CTA per 32 output rows of a product, a warp per row. Every CTA finds the
 // largest magnitude of its layer's weights for itself (at most 256 KB from L2), which saves a launch in front ----------------------------------
-struct ChainImage { const float* W; const float* bias; uint8_t* image; float* tail; int N, K, block_begin; };
+// element (n, k) of the product's weights at W[n * stride_n + k * stride_k]
+struct ChainImage { const float* W; const float* bias; uint8_t* image; float* tail; int N, K, block_begin, stride_n, stride_k; };
 struct ChainImages { int n; ChainImage y[CH_MAX_STEPS]; int blocks; };
 __global__ void __launch_bounds__(1024) chain_image_kernel(const __grid_constant__ ChainImages a){
     __shared__ float largest[32];
@@ -478,7 +516,7 @@ __global__ void __launch_bounds__(1024) chain_image_kernel(const __grid_constant
 #pragma unroll
         for(int k = 0; k < 2; k++){
             const int i = 64 * c + 2 * lane + k;
-            v[k] = n < y.N && i < y.K ? __ldg(y.W + (size_t)n * y.K + i) : 0.0f;
+            v[k] = n < y.N && i < y.K ? __ldg(y.W + (size_t)n * y.stride_n + (size_t)i * y.stride_k) : 0.0f;
         }
         uint32_t lead, rest;
         split_pair(make_float2(v[0] * f, v[1] * f), lead, rest);
@@ -512,17 +550,17 @@ size_t mlp_chain_workspace_bytes(const b200rl_mlp_shape* sh){
 int mlp_chain_error_get(int* word){ B200RL_CUDA_TRY(cudaMemcpyFromSymbol(word, g_chain_error, sizeof(int))); return B200RL_OK; }
 int mlp_chain_error_clear(){ const int zero = 0; B200RL_CUDA_TRY(cudaMemcpyToSymbol(g_chain_error, &zero, sizeof(int))); return B200RL_OK; }
 
-static void chain_step(ChainStep& y, ChainImages& images, const float* W, const float* bias, int N, int K, uint8_t*& ws){
+static void chain_step(ChainStep& y, ChainImages& images, const float* W, const float* bias, int N, int K, uint8_t*& ws, bool transposed = false){
     y.N = N; y.K = K; y.pieces = (K + 63) / 64; y.n = (N + 15) / 16 * 16;
     ChainImage& m = images.y[images.n++];
-    m.W = W; m.N = N; m.K = K; m.block_begin = images.blocks;
+    m.W = W; m.N = N; m.K = K; m.stride_n = transposed ? 1 : K; m.stride_k = transposed ? N : 1; m.block_begin = images.blocks;
     m.bias = bias; m.image = ws; m.tail = reinterpret_cast<float*>(ws + chain_image_bytes(N, K) - CH_TAIL);
     images.blocks += (y.n + 31) / 32;
     y.image = m.image; y.tail = m.tail;
     ws += chain_image_bytes(N, K);
 }
 template <int MODE>
-static int launch_chain(ChainArgs& a, const ChainImages& images, cudaStream_t s){
+static int launch_chain(ChainArgs& a, const ChainImages& images, cudaStream_t s, bool with_images = true){
     static std::atomic<bool> configured[MAX_DEVICES];
     int dev = 0, sms = 0;
     int rc = current_device(&dev);
@@ -532,8 +570,10 @@ static int launch_chain(ChainArgs& a, const ChainImages& images, cudaStream_t s)
         B200RL_CUDA_TRY(cudaFuncSetAttribute(mlp_chain_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_SMEM));
         configured[dev].store(true, std::memory_order_release);
     }
-    chain_image_kernel<<<images.blocks, 1024, 0, s>>>(images);
-    B200RL_LAUNCH_CHECK("chain_image");
+    if(with_images){
+        chain_image_kernel<<<images.blocks, 1024, 0, s>>>(images);
+        B200RL_LAUNCH_CHECK("chain_image");
+    }
     a.tiles = (a.rows + CH_ROWS - 1) / CH_ROWS;
     mlp_chain_kernel<MODE><<<a.tiles < sms ? a.tiles : sms, CH_THREADS, CH_SMEM, s>>>(a);
     B200RL_LAUNCH_CHECK("mlp_chain");
@@ -562,6 +602,99 @@ int mlp_chain_forward(const b200rl_mlp_shape* sh, const float* params, const flo
         p += (size_t)O * I + O; I = O;
     }
     return pre ? launch_chain<CH_FORWARD>(a, images, s) : launch_chain<CH_EVALUATE>(a, images, s);
+}
+
+// ---- backward: d_pre of every layer in one chain of transposed products, then all parameter gradients (mlp_grad.cu) ----
+// Rows are taken in chunks of up to 2^18, so that the d_pre of all layers (784 columns of 64-256-256-256-16) take 0.8 GB, not a batch of them.
+constexpr int CHAIN_BACKWARD_ROWS = 1 << 18;
+int mlp_grad_splits(const b200rl_mlp_shape* sh);
+int mlp_grad_launch(const b200rl_mlp_shape* sh, const float* const* input, const long long* ld_input, const float* const* d_pre, const long long* ld_pre, int rows,
+                    float* partial, long long record, bool accumulate, cudaStream_t s);
+int pad_rows(const float* from, long long ld, int rows, int cols, float* to, cudaStream_t s);
+int reduce_partials_into(float* dst, const float* partial, int n, long long stride, int segments, cudaStream_t s);
+
+static int chain_backward_rows(int batch){
+    const int chunks = (batch + CHAIN_BACKWARD_ROWS - 1) / CHAIN_BACKWARD_ROWS;
+    return ((batch + chunks - 1) / chunks + CH_ROWS - 1) / CH_ROWS * CH_ROWS;
+}
+bool mlp_chain_backward_eligible(const b200rl_mlp_shape* sh, int batch){ return sh->n_layers > 1 && mlp_chain_eligible(sh, batch); }
+static size_t aligned256(size_t n){ return (n + 255) / 256 * 256; }
+static long long padded(int columns){ return (columns + 3) / 4 * 4; }           // row pitch for the gradient kernel: rows of whole 16 bytes
+static size_t transposed_images_bytes(const b200rl_mlp_shape* sh){
+    size_t n = 0; int I = sh->input_dim;
+    for(int l = 0; l < sh->n_layers; l++){ n += chain_image_bytes(I, sh->dims[l]); I = sh->dims[l]; }
+    return aligned256(n);
+}
+size_t mlp_chain_backward_scratch_bytes(const b200rl_mlp_shape* sh, int batch){
+    if(!mlp_chain_backward_eligible(sh, batch)) return 0;
+    size_t columns = padded(sh->input_dim);                                  // padded copies of inputs; whether x needs one depends on where it lies
+    bool copies = false;
+    for(int l = 0; l < sh->n_layers; l++){
+        copies = copies || sh->dims[l] % 4;                                  // a layer's outputs of such a width, or behind ones of such a width
+        columns += padded(sh->dims[l]) * (copies && l + 1 < sh->n_layers ? 2 : 1);
+    }
+    return transposed_images_bytes(sh) + aligned256(sizeof(float) * mlp_grad_splits(sh) * b200rl_mlp_num_params(sh)) + sizeof(float) * columns * (size_t)chain_backward_rows(batch);
+}
+int mlp_chain_backward(const b200rl_mlp_shape* sh, const float* params, float* grads, const float* x, int ldx, const float* pre, const float* out, const float* d_out,
+                       float* d_input, int batch, void* scratch, size_t scratch_bytes, cudaStream_t s){
+    if(!scratch || scratch_bytes < mlp_chain_backward_scratch_bytes(sh, batch) || (reinterpret_cast<uintptr_t>(scratch) & 15u)) return B200RL_ERR_UNSUPPORTED;
+    const int L = sh->n_layers, chunk = chain_backward_rows(batch);
+    const size_t n_params = b200rl_mlp_num_params(sh);
+    uint8_t* ws = static_cast<uint8_t*>(scratch);
+    float* partial = reinterpret_cast<float*>(ws + transposed_images_bytes(sh));
+    const float* input[CH_MAX_STEPS]; float* copy[CH_MAX_STEPS]; float* d_pre[CH_MAX_STEPS];
+    long long ld_input[CH_MAX_STEPS], ld[CH_MAX_STEPS]; size_t poff[CH_MAX_STEPS], aoff[CH_MAX_STEPS]; int Is[CH_MAX_STEPS];
+    {
+        float* p = partial + aligned256(sizeof(float) * mlp_grad_splits(sh) * n_params) / sizeof(float);
+        size_t po = 0, ao = 0; int I = sh->input_dim;
+        for(int l = 0; l < L; l++){
+            const int O = sh->dims[l];
+            poff[l] = po; aoff[l] = ao; Is[l] = I; ld[l] = padded(O); d_pre[l] = p;
+            p += (size_t)ld[l] * chunk;
+            const bool aligned = l > 0 ? I % 4 == 0 : ldx % 4 == 0;
+            const float* from = l > 0 ? out + aoff[l - 1] : x;
+            copy[l] = aligned && (reinterpret_cast<uintptr_t>(from) & 15u) == 0 ? nullptr : p;
+            ld_input[l] = copy[l] ? padded(I) : l > 0 ? I : ldx;
+            if(copy[l]) p += (size_t)padded(I) * chunk;
+            po += (size_t)O * I + O; ao += (size_t)batch * O; I = O;
+        }
+        if(reinterpret_cast<uint8_t*>(p) > ws + scratch_bytes) return B200RL_ERR_UNSUPPORTED;      // an output arena that is not aligned
+    }
+    const int O_last = sh->dims[L - 1], act_last = sh->acts[L - 1];
+    const bool copy_last = act_last != B200RL_ACT_IDENTITY || (O_last & 3) != 0 || (reinterpret_cast<uintptr_t>(d_out) & 15u) != 0;
+    if(!copy_last) ld[L - 1] = O_last;
+    for(int row0 = 0; row0 < batch; row0 += chunk){
+        ChainArgs a{};
+        ChainImages images{};
+        uint8_t* image = ws;
+        a.rows = batch - row0 < chunk ? batch - row0 : chunk;
+        a.in = d_out + (size_t)row0 * O_last; a.ld_in = O_last; a.in_cols = O_last;
+        a.in_pre = pre + aoff[L - 1] + (size_t)row0 * O_last; a.in_act = act_last;
+        a.in_out = grads && copy_last ? d_pre[L - 1] : nullptr; a.ld_in_out = ld[L - 1];
+        if(!copy_last) d_pre[L - 1] = const_cast<float*>(a.in);
+        for(int l = L - 1; l >= (d_input ? 0 : 1); l--){
+            ChainStep& t = a.step[a.n_steps++];
+            chain_step(t, images, params + poff[l], nullptr, Is[l], sh->dims[l], image, true);
+            if(l > 0){
+                t.act = sh->acts[l - 1]; t.pre_in = pre + aoff[l - 1] + (size_t)row0 * Is[l];
+                t.out = grads ? d_pre[l - 1] : nullptr; t.ld = ld[l - 1];
+            }
+            else{ t.act = B200RL_ACT_IDENTITY; t.out = d_input + (size_t)row0 * Is[0]; t.ld = Is[0]; }
+        }
+        int rc = launch_chain<CH_BACKWARD>(a, images, s, row0 == 0);
+        if(rc) return rc;
+        if(!grads) continue;
+        for(int l = 0; l < L; l++){
+            const long long pitch = l > 0 ? Is[l] : ldx;
+            input[l] = (l > 0 ? out + aoff[l - 1] : x) + row0 * pitch;
+            if(copy[l]){
+                if((rc = pad_rows(input[l], pitch, a.rows, Is[l], copy[l], s))) return rc;
+                input[l] = copy[l];
+            }
+        }
+        if((rc = mlp_grad_launch(sh, input, ld_input, d_pre, ld, a.rows, partial, (long long)n_params, row0 > 0, s))) return rc;
+    }
+    return grads ? reduce_partials_into(grads, partial, (int)n_params, (long long)n_params, mlp_grad_splits(sh), s) : B200RL_OK;
 }
 
 }  // namespace b200rl

@@ -123,7 +123,7 @@ __device__ __forceinline__ float act_or_rt(float x, int rt){
 // row starts (n_envs and the slab origin multiples of 4, aligned output pointers); the host selects the plain-store instantiation otherwise.
 // PART: tiles of at most three warps of environments. A warp without an environment takes no part in a step but for the barriers, and group g's tile starts at
 // warp g, so that the four groups' environments share out the SM's four schedulers. (A kernel of its own: in the full one the test of
-// it costs 2 %.) With tiles dealt out over the SMs first, a step of 500 environments takes 1.95 us (2.91 with four tiles to a CTA), of 10,007 1.94
+// it costs 2 %.) With the tiles dealt out over the SMs first instead of four to a CTA, a step of 500 environments takes 1.95 us (2.91 before), of 10,007 1.94
 // (2.73), of 20,000 2.44 (3.06).
 template <typename ENV, int A1, int A2, bool COLLECT, bool BULK, bool PART>
 __global__ void __launch_bounds__(THREADS, 1) rollout_tc_kernel(RolloutArgs a, int n_tiles, int envs_per_tile){
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(THREADS, 1) rollout_tc_kernel(RolloutArgs a, i
     const bool active = !PART || (vr & ~31) < envs_per_tile;
     const int rounds = (n_tiles + (int)gridDim.x * GROUPS - 1) / ((int)gridDim.x * GROUPS);
     for(int round = 0; round < rounds && !failed; round++){
-        const int tile = (round * GROUPS + g) * (int)gridDim.x + (int)blockIdx.x;             // over the SMs first
+        const int tile = PART ? (round * GROUPS + g) * (int)gridDim.x + (int)blockIdx.x : (round * (int)gridDim.x + (int)blockIdx.x) * GROUPS + g;
         if(tile >= n_tiles){
             // no environments for this group in this round: it still hands the tensor token on, once per step
             if(r == 0){
@@ -491,7 +491,7 @@ static int launch_tc_part(const RolloutArgs& a, cudaStream_t s, int variant, int
     rc = upload_small_layers(st, a.params, ENV::OBS_DIM, s, &order_event);
     if(rc) return rc;
     const int n_tiles = (a.env_count + ept - 1) / ept;
-    const int grid = n_tiles < sms ? n_tiles : sms;
+    const int ctas = PART ? n_tiles : (n_tiles + GROUPS - 1) / GROUPS, grid = ctas < sms ? ctas : sms;
     rollout_tc_kernel<ENV, A1, A2, COLLECT, BULK, PART><<<grid, THREADS, SMEM_BYTES, s>>>(a, n_tiles, ept);
     B200RL_LAUNCH_CHECK("rollout_tc");
     if(order_event) B200RL_CUDA_TRY(cudaEventRecord(order_event, s));

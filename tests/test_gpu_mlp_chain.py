@@ -52,3 +52,56 @@ def test_forward_and_evaluate_match_fp64(lib, rows, I, dims, acts, strided):
         close(net.pre[off:off + rows * d].view(rows, d), p); close(net.out[off:off + rows * d].view(rows, d), o)
         off += rows * d
     close(y, outs[-1])
+
+
+DERIVATIVE = {"identity": lambda v: v * 0 + 1, "relu": lambda v: (v > 0).to(v.dtype), "tanh": lambda v: 1 - v.tanh() ** 2, "sigmoid": lambda v: v.sigmoid() * (1 - v.sigmoid()),
+              "fast_tanh": lambda v: 1 - ACT["fast_tanh"](v) ** 2}
+
+
+@pytest.mark.parametrize("mode", ["gradients", "both", "input"])
+@pytest.mark.parametrize("rows,I,dims,acts", [n for n in NETS if len(n[2]) > 1] + [((1 << 18) + 131, 12, [40, 24, 4], ["relu", "tanh", "tanh"]), (9000, 140, [136, 3], ["relu", "identity"])])
+def test_backward_matches_fp64(lib, rows, I, dims, acts, mode):
+    """Backward in the same kernels: more than one chunk of 2^18 rows, both operands on either side of 128 and 256 columns, unaligned widths; gradients are
+    added to what is there, the input gradient alone leaves them untouched."""
+    import torch
+    net = lib.Mlp(I, dims, acts, rows)
+    off, fan_in = 0, I
+    for l, d in enumerate(dims):
+        n = d * fan_in + d
+        net.params[off:off + n] = torch.from_numpy(mg.det_uniform(7 + l, n) / np.float32(np.sqrt(fan_in))).cuda()
+        off += n; fan_in = d
+    x = torch.from_numpy(mg.det_normal(1, rows * I).reshape(rows, I)).cuda()
+    x[:, 0] *= 1e-3                                             # a column of small values, a row of zeros, a row of large values
+    x[1] = 0; x[2] *= 1e2
+    d_out = torch.from_numpy(mg.det_normal(2, rows * dims[-1]).reshape(rows, dims[-1])).cuda() / rows
+    d_out[:, 0] *= 1e-4
+    net.forward(x)
+    net.grads.copy_(torch.from_numpy(mg.det_normal(3, net.grads.numel())).cuda() * 1e-3)
+    before = net.grads.clone()
+    d_input = torch.zeros(rows, I, device="cuda") if mode != "gradients" else None
+    d, widths = d_out.double(), [I] + list(dims)
+    wants = [None] * len(dims)
+    poff = np.cumsum([0] + [o * i + o for i, o in zip(widths, dims)])
+    aoff = np.cumsum([0] + [rows * o for o in dims])
+    for l in range(len(dims) - 1, -1, -1):
+        i, o = widths[l], dims[l]
+        pre = net.pre[aoff[l]:aoff[l] + rows * o].view(rows, o).double()
+        inp = x.double() if l == 0 else net.out[aoff[l - 1]:aoff[l - 1] + rows * i].view(rows, i).double()
+        d = d * DERIVATIVE[acts[l]](pre)
+        wants[l] = (d.T @ inp, d.abs().T @ inp.abs(), d.sum(0), d.abs().sum(0))
+        d = d @ net.params[poff[l]:poff[l] + o * i].double().view(o, i)
+    net.backward(x, d_out.clone(), d_input=d_input, accumulate_gradients=mode != "input")
+    state = np.zeros(1, np.int32)
+    assert lib.lib().b200rl_device_error_state(state.ctypes.data) == 0 and state[0] == 0
+    if mode == "input":
+        assert torch.equal(net.grads, before)
+    else:
+        for l, (dW, size_W, db, size_b) in enumerate(wants):
+            i, o = widths[l], dims[l]
+            got = net.grads[poff[l]:poff[l + 1]].double() - before[poff[l]:poff[l + 1]].double()
+            # the sum of the terms' magnitudes, and the rounding of the sum with what was there
+            assert float(((got[:o * i].view(o, i) - dW).abs() - 2e-6 * size_W).max()) <= 1e-9, l
+            assert float(((got[o * i:] - db).abs() - 2e-6 * size_b).max()) <= 1e-9, l
+    if d_input is not None:
+        err, size = (d_input.double() - d).norm(dim=1), d.norm(dim=1)
+        assert float((err - 1e-5 * size).max()) <= 1e-6 / rows

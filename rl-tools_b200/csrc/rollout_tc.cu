@@ -264,8 +264,8 @@ __global__ void __launch_bounds__(THREADS, 1) rollout_tc_kernel(RolloutArgs a, i
             float* st_rew = st_act + TILE;
             StepDraws draws{};             // the trajectory-only kernels need the draws at a reset only: nothing per step on their hot path
             float o[O];
-            const size_t row = (size_t)t * a.n_envs + e;
-            float* drow = COLLECT ? a.dataset + row * ld : nullptr;
+            size_t row;
+            float* drow;
             if(active){
                 if constexpr(IS_PENDULUM){ if(a.device_rng && (COLLECT || trunc)) draws = step_draws(a.rng_seed, a.rng_step0 + (unsigned long long)t, (uint32_t)e); }
                 if(trunc && valid){
@@ -289,6 +289,8 @@ __global__ void __launch_bounds__(THREADS, 1) rollout_tc_kernel(RolloutArgs a, i
                     resets++; es = 0; er = 0.0f;
                 }
                 ENV::observe(state, o);
+                row = (size_t)t * a.n_envs + e;
+                drow = COLLECT ? a.dataset + row * ld : nullptr;
                 if(valid){
 #pragma unroll
                     for(int k = 0; k < O; k++){

@@ -584,8 +584,11 @@ static int launch_chain(ChainArgs& a, const ChainImages& images, cudaStream_t s,
 int mlp_chain_forward(const b200rl_mlp_shape* sh, const float* params, const float* x, int ldx, float* pre, float* out, float* y, int ldy, int batch, void* workspace,
                       size_t workspace_bytes, cudaStream_t s){
     if(!workspace || workspace_bytes < mlp_chain_workspace_bytes(sh) || (reinterpret_cast<uintptr_t>(workspace) & 15u)) return B200RL_ERR_UNSUPPORTED;
-    // a CTA reads inputs while another one writes outputs: outputs over the inputs take the kernels per layer
-    if(y && y < x + (size_t)batch * ldx && x < y + (size_t)batch * ldy) return B200RL_ERR_UNSUPPORTED;
+    // a CTA reads inputs while another one writes outputs: outputs over the inputs take the kernels per layer. Columns of one matrix do not overlap.
+    if(y && y < x + (size_t)batch * ldx && x < y + (size_t)batch * ldy){
+        const long long at = ldx == ldy ? ((y - x) % ldx + ldx) % ldx : 0;
+        if(at < sh->input_dim || at + sh->dims[sh->n_layers - 1] > ldx) return B200RL_ERR_UNSUPPORTED;
+    }
     ChainArgs a{};
     ChainImages images{};
     uint8_t* ws = static_cast<uint8_t*>(workspace);

@@ -128,6 +128,86 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_kernel(GemmArgs a){
         }
     }
 }
+// Forward product of a small problem (both operands contiguous along the summed index): 32 x 16 outputs per CTA, both operands of up to 256 summed indices
+// in one round trip to L2 by asynchronous copies. Bound by latency: so the eight warps share out the summed index, a lane takes 4 x 4 outputs with 16-byte reads along
+// it (32 packed multiply-adds to 8 reads; 16-byte pieces swizzled by the row: no bank conflicts), and the eight partial sums are added in warp
+// order. 256 x 256 x 256: 7.3 us with four k steps of 64 through transposing stores, 3.6 us this way; the update of the off-policy
+// loop with 256-wide networks, nine such passes one after the other: 280 -> 234 us.
+constexpr int SF_M = 32, SF_N = 16, SF_KC = 256, SF_PITCH = 20;
+__device__ __forceinline__ void small_copy(float* to, const float* from, int floats, bool vec){       // four floats, zeros behind the first `floats`
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(to);
+    if(vec) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(at), "l"(from), "r"(floats > 0 ? 16 : 0) : "memory");
+    else{
+#pragma unroll
+        for(int k = 0; k < 4; k++) asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" :: "r"(at + 4 * k), "l"(k < floats ? from + k : from), "r"(k < floats ? 4 : 0) : "memory");
+    }
+}
+template <int ACT>
+__global__ void __launch_bounds__(256) small_forward_kernel(GemmArgs a, int vec_a, int vec_b){
+    __shared__ __align__(16) float S[(SF_M + SF_N) * SF_KC];                      // [row][piece ^ (row & 7)][4]; later the partial sums [warp][32][20]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = lane >> 2, cg = lane & 3;
+    const int m0 = blockIdx.y * SF_M, n0 = blockIdx.x * SF_N;
+    float2 acc[4][4];                                                             // sums over even and odd k
+#pragma unroll
+    for(int i = 0; i < 4; i++)
+#pragma unroll
+        for(int j = 0; j < 4; j++) acc[i][j] = make_float2(0.0f, 0.0f);
+    for(int k0 = 0; k0 < a.K; k0 += SF_KC){
+        const int pieces = (min(SF_KC, a.K - k0) + 3) / 4;
+        if(k0) __syncthreads();
+        const int c = tid & 63, k = k0 + 4 * c;
+        if(c < pieces){
+#pragma unroll
+            for(int j = 0; j < (SF_M + SF_N) / 4; j++){
+                const int r = (tid >> 6) + 4 * j;
+                const bool of_a = r < SF_M;
+                const int row = of_a ? m0 + r : n0 + r - SF_M;
+                const bool in = row < (of_a ? a.M : a.N);
+                const float* from = of_a ? a.A + (long long)row * a.lda + k : a.B + (long long)row * a.ldb + k;
+                small_copy(S + r * SF_KC + 4 * (c ^ (r & 7)), in ? from : (of_a ? a.A : a.B), in ? a.K - k : 0, of_a ? vec_a : vec_b);
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        for(int p = warp; p < pieces; p += 8){
+            float4 x[4];
+#pragma unroll
+            for(int i = 0; i < 4; i++) x[i] = *reinterpret_cast<const float4*>(S + (rg + 8 * i) * SF_KC + 4 * (p ^ rg));
+#pragma unroll
+            for(int j = 0; j < 4; j++){
+                const float4 w = *reinterpret_cast<const float4*>(S + (SF_M + cg + 4 * j) * SF_KC + 4 * (p ^ (cg + 4 * (j & 1))));
+#pragma unroll
+                for(int i = 0; i < 4; i++){
+                    acc[i][j] = __ffma2_rn(make_float2(x[i].x, x[i].y), make_float2(w.x, w.y), acc[i][j]);
+                    acc[i][j] = __ffma2_rn(make_float2(x[i].z, x[i].w), make_float2(w.z, w.w), acc[i][j]);
+                }
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for(int i = 0; i < 4; i++)
+#pragma unroll
+        for(int j = 0; j < 4; j++) S[(warp * SF_M + rg + 8 * i) * SF_PITCH + cg + 4 * j] = acc[i][j].x + acc[i][j].y;
+    __syncthreads();
+    const int r = tid >> 3, c = 2 * (tid & 7), m = m0 + r;
+    float2 v = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for(int w = 0; w < 8; w++){
+        const float2 t = *reinterpret_cast<const float2*>(S + (w * SF_M + r) * SF_PITCH + c);
+        v.x += t.x; v.y += t.y;
+    }
+    if(m >= a.M) return;
+#pragma unroll
+    for(int j = 0; j < 2; j++){
+        const int n = n0 + c + j;
+        if(n >= a.N) continue;
+        const float s = (j ? v.y : v.x) + __ldg(a.bias + n);
+        if(a.pre) a.pre[(long long)m * a.ldpre + n] = s;
+        a.C[(long long)m * a.ldc + n] = activation<ACT>(s);
+    }
+}
+
 // 32-wide tiles when 64-wide ones would occupy less than half of the SMs
 static inline bool small_tiles(int M, int N, int splits){
     return (long long)((M + 63) / 64) * ((N + 63) / 64) * splits < NUM_SMS / 2;
@@ -352,7 +432,15 @@ static int dense_forward_impl(const float* W, const float* bias, const float* x,
         if(rc == B200RL_ERR_UNSUPPORTED) rc = launch_gemm_tc(a, EPI_FORWARD, act, true, true, 1, s);
         if(rc != B200RL_ERR_UNSUPPORTED) return rc;
     }
-    B200RL_DISPATCH_ACT(act, B200RL_LAUNCH_SIMT_GEMM(true, true, EPI_FORWARD, ACT, a, 1, s));
+    if(small_tiles(a.M, a.N, 1)){
+        auto vec = [&](const float* p, long long ld){ return a.K % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+        const dim3 grid((a.N + SF_N - 1) / SF_N, (a.M + SF_M - 1) / SF_M);
+        B200RL_DISPATCH_ACT(act, (small_forward_kernel<ACT><<<grid, 256, 0, s>>>(a, vec(a.A, a.lda), vec(a.B, a.ldb))));
+    }
+    else{
+        const dim3 grid((a.N + 63) / 64, (a.M + 63) / 64);
+        B200RL_DISPATCH_ACT(act, (gemm_kernel<64, true, true, EPI_FORWARD, ACT><<<grid, GEMM_THREADS, 0, s>>>(a)));
+    }
     B200RL_LAUNCH_CHECK("dense_forward");
     return B200RL_OK;
 }

@@ -216,7 +216,9 @@ __device__ void coop_bias_item(const CoopPhase& p, int item, float* smem){
     }
 }
 
-__global__ void __launch_bounds__(CO_THREADS, 1) mlp_coop_kernel(CoopArgs a){
+// Two CTAs per SM: the backward passes of two networks on two streams run side by side (one after the other they took 45 us of the off-policy update at 256-wide
+// networks, the grid of each being most of the SMs)
+__global__ void __launch_bounds__(CO_THREADS, 2) mlp_coop_kernel(CoopArgs a){
     extern __shared__ __align__(16) float smem[];
     unsigned target = 0;
     for(int ph = 0; ph < a.n_phases; ph++){
@@ -334,7 +336,7 @@ int mlp_coop_backward(const b200rl_mlp_shape* sh, const float* params, float* gr
     { size_t po = 0, ao = 0; int I = sh->input_dim;
       for(int l = 0; l < L; l++){ poff[l] = po; aoff[l] = ao; Is[l] = I; po += (size_t)sh->dims[l] * I + sh->dims[l]; ao += (size_t)batch * sh->dims[l]; I = sh->dims[l]; } }
     CoopArgs a{};
-    {
+    if(sh->acts[L - 1] != B200RL_ACT_IDENTITY){                   // otherwise d_out is d_pre
         CoopPhase& ph = a.phase[a.n_phases++];
         ph.type = CO_PHASE_DPRE; ph.d_out = d_out; ph.pre = pre + aoff[L - 1]; ph.ew_ldd = sh->dims[L - 1]; ph.ew_ldpre = sh->dims[L - 1];
         ph.ew_rows = batch; ph.ew_cols = sh->dims[L - 1]; ph.ew_act = sh->acts[L - 1];

@@ -46,8 +46,11 @@ class ActorCritic:
         # work of critic 1 (the two critics' chains are independent; captured in a CUDA graph they become parallel branches)
         self.next_input_2, self.q_next_2 = z(2 * batch, O + A), [z(2 * batch, 1), z(2 * batch, 1)]
         self.next_log_probs_2, self.target_2 = z(2 * batch), z(2 * batch, 1)
+        self.next_pre_squashing_2 = z(2 * batch, A)
         self.d_output_2 = [z(batch, 1), z(batch, 1)]
         self.side_stream = torch.cuda.Stream(device=device)
+        # update(): a third one for what depends on nothing but the batch -- the critics' passes and the actor's -- beside the target values
+        self.early_stream = torch.cuda.Stream(device=device)
 
     def copy_critics_to_targets(self):
         """init(): the target networks start as copies of the critics (:126-131)."""
@@ -76,17 +79,27 @@ class ActorCritic:
 
     def train_actor(self, batch, action_noise):
         """One actor update (and one log_alpha update) on `batch` with the external noise [B, A] of the action sample."""
+        self._actor_pass(batch, action_noise)
+        self._actor_update(batch, action_noise)
+
+    def _actor_pass(self, batch, action_noise):
+        """train_actor up to the sampled actions: needs neither the critics nor their targets."""
         O, A, B = self.observation_dim, self.action_dim, self.batch
+        observations = batch["oa_base"][0][:, :O]
+        self.actor_input.copy_(batch["oa_base"][0])
         self.actor.zero_gradient()
         fill(self.log_alpha_grad, 0.0)
-        self.actor_input.copy_(batch["oa_base"][0])
-        observations = self.actor_input[:, :O]
+        for c in range(2):
+            fill(self.d_output_2[c], self._minus_one_over_batch)                                 # the mean over the (all final) steps, negated (:424-431)
         head_input = self.actor.forward(observations)
         _head_forward(head_input, action_noise, output=self.actor_input[:, O:], pre_squashing=self.pre_squashing, log_probs=self.log_probs)
         self.actions.copy_(self.actor_input[:, O:])
+
+    def _actor_update(self, batch, action_noise):
+        O, A = self.observation_dim, self.action_dim
+        observations, head_input = batch["oa_base"][0][:, :O], self.actor.output()
         def through_critic(c):
             value = self.critics[c].forward(self.actor_input)
-            fill(self.d_output_2[c], self._minus_one_over_batch)                                 # the mean over the (all final) steps, negated (:424-431)
             self.critics[c].backward(self.actor_input, self.d_output_2[c], d_input=self.d_critic_input[c], accumulate_gradients=False)     # backward_input (:433-434)
             return value
         with self._fork():                                                                       # the two critics are independent: two streams
@@ -96,46 +109,63 @@ class ActorCritic:
         _min_value_d_output(q[0], q[1], self.d_critic_input[0], self.d_critic_input[1], A, d_actor_output=self.d_actor_output)
         _head_backward(head_input, action_noise, self.pre_squashing, self.actions, self.d_actor_output, self.log_alpha, log_alpha_gradient=self.log_alpha_grad,
                        target_entropy=self.target_entropy, d_input=self.d_head_input)
+        with self._fork():
+            check(lib().b200rl_adam_step(_ptr(self.log_alpha), _ptr(self.log_alpha_grad), _ptr(self.log_alpha_m), _ptr(self.log_alpha_v), 1, self.alpha_hyper,
+                                         _ptr(self.log_alpha_adam_state), _stream()), "b200rl_adam_step")
         self.actor.backward(observations, self.d_head_input)
         self.actor.step()
-        check(lib().b200rl_adam_step(_ptr(self.log_alpha), _ptr(self.log_alpha_grad), _ptr(self.log_alpha_m), _ptr(self.log_alpha_v), 1, self.alpha_hyper,
-                                     _ptr(self.log_alpha_adam_state), _stream()), "b200rl_adam_step")
+        self._join()
 
-    def _fork(self):
+    def _fork(self, stream=None):
         import torch
-        self.side_stream.wait_stream(torch.cuda.current_stream())
-        return torch.cuda.stream(self.side_stream)
+        stream = stream or self.side_stream
+        stream.wait_stream(torch.cuda.current_stream())
+        return torch.cuda.stream(stream)
 
-    def _join(self):
+    def _join(self, stream=None):
         import torch
-        torch.cuda.current_stream().wait_stream(self.side_stream)
+        torch.cuda.current_stream().wait_stream(stream or self.side_stream)
 
-    def train_critics(self, batch, noise_0, noise_1):
+    def train_critics(self, batch, noise_0, noise_1, early=None):
         """train_critic for both critics on one shared batch, with the same results as two train_critic calls: the actor's pass over the
         next observations is shared (it does not depend on the noise), each target network runs once over both critics' next inputs, and
-        the two critics' forward / backward / Adam chains run on two streams."""
+        the two critics' forward / backward / Adam chains run on two streams. The critics' forward passes, and `early` behind them (joined by the
+        caller), run on a third stream beside the target values."""
+        import torch
         O, B = self.observation_dim, self.batch
-        self.next_input_2[:B].copy_(batch["oa_base"][1]); self.next_input_2[B:].copy_(batch["oa_base"][1])
-        self.actor.evaluate(self.next_input_2[:B, :O], y=self.next_head_input)
-        for c, noise in enumerate((noise_0, noise_1)):
+        with self._fork(self.early_stream):
+            for critic in self.critics:
+                critic.zero_gradient()
+                critic.forward(batch["oa_base"][0])
+            critics_ready = torch.cuda.Event()
+            critics_ready.record()
+            if early is not None:
+                early()
+        with self._fork():
+            self.next_input_2[:B].copy_(batch["oa_base"][1]); self.next_input_2[B:].copy_(batch["oa_base"][1])
+        self.actor.evaluate(batch["oa_base"][1][:, :O], y=self.next_head_input)
+        self._join()
+        def next_action(c, noise):
             rows = slice(c * B, (c + 1) * B)
-            _head_forward(self.next_head_input, noise, output=self.next_input_2[rows, O:], pre_squashing=self.pre_squashing, log_probs=self.next_log_probs_2[rows])
+            _head_forward(self.next_head_input, noise, output=self.next_input_2[rows, O:], pre_squashing=self.next_pre_squashing_2[rows], log_probs=self.next_log_probs_2[rows])
+        with self._fork():
+            next_action(1, noise_1)
+        next_action(0, noise_0)
+        self._join()
         with self._fork():                                               # the two target networks are independent
             self.critics_target[1].evaluate(self.next_input_2, y=self.q_next_2[1])
         self.critics_target[0].evaluate(self.next_input_2, y=self.q_next_2[0])
         self._join()
-        for c in range(2):
-            rows = slice(c * B, (c + 1) * B)
-            _target_action_values(self.q_next_2[0][rows], self.q_next_2[1][rows], batch["rewards"], batch["terminated"], self.next_log_probs_2[rows], self.log_alpha,
-                                  gamma=self.gamma, target=self.target_2[rows])
         self.target_action_value = self.target_2[B:]                     # what the second train_critic call would have left behind
 
         def chain(c):
+            rows = slice(c * B, (c + 1) * B)
+            _target_action_values(self.q_next_2[0][rows], self.q_next_2[1][rows], batch["rewards"], batch["terminated"], self.next_log_probs_2[rows], self.log_alpha,
+                                  gamma=self.gamma, target=self.target_2[rows])
             critic = self.critics[c]
-            critic.zero_gradient()
-            values = critic.forward(batch["oa_base"][0])
-            critic.backward(batch["oa_base"][0], _mse_gradient(values, self.target_2[c * B:(c + 1) * B], 0.5, d_a=critic.d_out_buffer()))
+            critic.backward(batch["oa_base"][0], _mse_gradient(critic.output(), self.target_2[c * B:(c + 1) * B], 0.5, d_a=critic.d_out_buffer()))
             critic.step()
+        torch.cuda.current_stream().wait_event(critics_ready)
         with self._fork():
             chain(1)
         chain(0)
@@ -143,10 +173,15 @@ class ActorCritic:
 
     def update(self, batch, noise_critic_0, noise_critic_1, noise_actor):
         """One step of the reference's training loop on a shared batch (rl/algorithms/sac/loop/core/operations_generic.h:124-152)."""
-        self.train_critics(batch, noise_critic_0, noise_critic_1)
+        # the actor's own pass does not need the critics; beside its pass over the next observations unless the two would share a workspace
+        beside = self.actor.workspace_bytes == 0
+        self.train_critics(batch, noise_critic_0, noise_critic_1, early=(lambda: self._actor_pass(batch, noise_actor)) if beside else None)
+        self._join(self.early_stream)
+        if not beside:
+            self._actor_pass(batch, noise_actor)
         # the target update reads the critics and writes the targets; train_actor reads the critics only: independent of each other.
-        # (train_actor forks onto the same side stream itself, after this work in stream order.)
+        # (_actor_update forks onto the same side stream itself, after this work in stream order.)
         with self._fork():
             self.update_critic_targets()
-        self.train_actor(batch, noise_actor)
+        self._actor_update(batch, noise_actor)
         self._join()

@@ -140,11 +140,11 @@ __device__ void coop_gemm_tile(const CoopGemm& g, int tile, float* smem){
     float (*Bs)[CO_PITCH] = As + CO_KC;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rg = lane >> 2, cg = lane & 3;
     const int m0 = (tile / g.tiles_n) * CO_T, n0 = (tile % g.tiles_n) * CO_T;
-    float acc[4][8];
+    float2 acc[4][4];
 #pragma unroll
     for(int i = 0; i < 4; i++)
 #pragma unroll
-        for(int j = 0; j < 8; j++) acc[i][j] = 0.0f;
+        for(int j = 0; j < 4; j++) acc[i][j] = make_float2(0.0f, 0.0f);
     for(int k0 = 0; k0 < g.K; k0 += CO_KC){
         const int kc = min(CO_KC, g.K - k0);
         __syncthreads();                                   // whoever read this shared memory last (previous item, previous chunk) is done
@@ -154,11 +154,12 @@ __device__ void coop_gemm_tile(const CoopGemm& g, int tile, float* smem){
         for(int k = warp; k < kc; k += CO_WARPS){
             const float4 a = *reinterpret_cast<const float4*>(&As[k][4 * rg]);
             const float4 b0 = *reinterpret_cast<const float4*>(&Bs[k][8 * cg]), b1 = *reinterpret_cast<const float4*>(&Bs[k][8 * cg + 4]);
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+            const float av[4] = {a.x, a.y, a.z, a.w};
+            const float2 bv[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w), make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
 #pragma unroll
             for(int i = 0; i < 4; i++)
 #pragma unroll
-                for(int j = 0; j < 8; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+                for(int j = 0; j < 4; j++) acc[i][j] = __ffma2_rn(make_float2(av[i], av[i]), bv[j], acc[i][j]);
         }
     }
     __syncthreads();
@@ -166,8 +167,8 @@ __device__ void coop_gemm_tile(const CoopGemm& g, int tile, float* smem){
 #pragma unroll
     for(int i = 0; i < 4; i++){
         float* row = R + (warp * CO_T + 4 * rg + i) * CO_T + 8 * cg;
-        *reinterpret_cast<float4*>(row) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-        *reinterpret_cast<float4*>(row + 4) = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+        *reinterpret_cast<float4*>(row) = make_float4(acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y);
+        *reinterpret_cast<float4*>(row + 4) = make_float4(acc[i][2].x, acc[i][2].y, acc[i][3].x, acc[i][3].y);
     }
     __syncthreads();
     const int r = tid >> 3, c4 = (tid & 7) * 4, m = m0 + r;
@@ -216,36 +217,21 @@ __device__ void coop_bias_item(const CoopPhase& p, int item, float* smem){
     }
 }
 
-// Two CTAs per SM: the backward passes of two networks on two streams run side by side (one after the other they took 45 us of the off-policy update at 256-wide
-// networks, the grid of each being most of the SMs)
-__global__ void __launch_bounds__(CO_THREADS, 2) mlp_coop_kernel(CoopArgs a){
+__global__ void __launch_bounds__(CO_THREADS, 2) mlp_phase_kernel(const __grid_constant__ CoopPhase p){
     extern __shared__ __align__(16) float smem[];
-    unsigned target = 0;
-    for(int ph = 0; ph < a.n_phases; ph++){
-        const CoopPhase& p = a.phase[ph];
-        if(p.type == CO_PHASE_DPRE){
-            const int total = p.ew_rows * p.ew_cols;
-            for(int idx = blockIdx.x * CO_THREADS + threadIdx.x; idx < total; idx += gridDim.x * CO_THREADS){
-                const int r = idx / p.ew_cols, c = idx % p.ew_cols;
-                float* d = p.d_out + (size_t)r * p.ew_ldd + c;
-                *d = *d * d_activation_rt(p.pre[(size_t)r * p.ew_ldpre + c], p.ew_act);
-            }
-        }
-        else{
-            const int t0 = p.g[0].tiles, t1 = p.n_gemms > 1 ? p.g[1].tiles : 0, items = t0 + t1 + p.bias_items;
-            for(int item = blockIdx.x; item < items; item += gridDim.x){
-                if(item < t0) coop_gemm_tile(p.g[0], item, smem);
-                else if(item < t0 + t1) coop_gemm_tile(p.g[1], item - t0, smem);
-                else coop_bias_item(p, item - t0 - t1, smem);
-            }
-        }
-        if(ph + 1 < a.n_phases){
-            target += gridDim.x;
-            if(!coop_barrier(a.barrier, target)) return;
-        }
+    if(p.type == CO_PHASE_DPRE){
+        const int total = p.ew_rows * p.ew_cols, idx = blockIdx.x * CO_THREADS + threadIdx.x;
+        if(idx >= total) return;
+        const int r = idx / p.ew_cols, c = idx % p.ew_cols;
+        float* d = p.d_out + (size_t)r * p.ew_ldd + c;
+        *d = *d * d_activation_rt(p.pre[(size_t)r * p.ew_ldpre + c], p.ew_act);
     }
-    // the last CTA out clears the slot for its next launch (every CTA has left the last barrier before it counts itself out)
-    if(threadIdx.x == 0 && a.n_phases > 1) grid_barrier_leave(a.barrier, gridDim.x);
+    else{
+        const int item = blockIdx.x, t0 = p.g[0].tiles, t1 = p.n_gemms > 1 ? p.g[1].tiles : 0;
+        if(item < t0) coop_gemm_tile(p.g[0], item, smem);
+        else if(item < t0 + t1) coop_gemm_tile(p.g[1], item - t0, smem);
+        else coop_bias_item(p, item - t0 - t1, smem);
+    }
 }
 
 // ---------------------------------------------------------------------------------------------------------------------------------------
@@ -289,22 +275,14 @@ int grid_barrier_slots(int count, unsigned** out){
 static void set_tiles(CoopGemm& g){ g.tiles_n = (g.N + CO_T - 1) / CO_T; g.tiles = ((g.M + CO_T - 1) / CO_T) * g.tiles_n; }
 
 static int coop_launch(CoopArgs& a, cudaStream_t s){
-    int sms = 0;
-    int rc = sm_count(&sms);
-    if(rc) return rc;
-    int most = 1;
+    B200RL_CUDA_TRY(cudaFuncSetAttribute(mlp_phase_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CO_SMEM));
     for(int ph = 0; ph < a.n_phases; ph++){
         const CoopPhase& p = a.phase[ph];
         const int items = p.type == CO_PHASE_DPRE ? (p.ew_rows * p.ew_cols + CO_THREADS - 1) / CO_THREADS
                                                   : p.g[0].tiles + (p.n_gemms > 1 ? p.g[1].tiles : 0) + p.bias_items;
-        if(items > most) most = items;
+        mlp_phase_kernel<<<items, CO_THREADS, CO_SMEM, s>>>(p);
+        B200RL_LAUNCH_CHECK("mlp_phase");
     }
-    const int grid = most < sms ? most : sms;
-    rc = grid_barrier_slots(1, &a.barrier);
-    if(rc) return rc;
-    B200RL_CUDA_TRY(cudaFuncSetAttribute(mlp_coop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CO_SMEM));
-    void* params[] = { &a };
-    B200RL_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(mlp_coop_kernel), dim3(grid), dim3(CO_THREADS), params, CO_SMEM, s));
     return B200RL_OK;
 }
 

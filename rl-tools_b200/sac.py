@@ -180,8 +180,7 @@ class ActorCritic:
         if not beside:
             self._actor_pass(batch, noise_actor)
         # the target update reads the critics and writes the targets; train_actor reads the critics only: independent of each other.
-        # (_actor_update forks onto the same side stream itself, after this work in stream order.)
-        with self._fork():
+        with self._fork(self.early_stream):
             self.update_critic_targets()
         self._actor_update(batch, noise_actor)
-        self._join()
+        self._join(self.early_stream)

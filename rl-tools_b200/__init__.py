@@ -356,13 +356,13 @@ def randn_host_rng(rng_state, dst):
     return dst
 
 
-def gae(rewards, all_values, terminated, truncated, n_envs, steps, gamma=0.99, lam=0.95, ignore_termination=False):
+def gae(rewards, all_values, terminated, truncated, n_envs, steps, gamma=0.99, lam=0.95, ignore_termination=False, advantages=None, target_values=None):
     """Column tensors ([rows] or [rows, 1] views with any row stride) -> (advantages, target_values), both [steps * n_envs]."""
     import torch
-    adv = torch.empty(steps * n_envs, device=rewards.device, dtype=torch.float32)
-    tgt = torch.empty_like(adv)
+    adv = torch.empty(steps * n_envs, device=rewards.device, dtype=torch.float32) if advantages is None else advantages
+    tgt = torch.empty(steps * n_envs, device=rewards.device, dtype=torch.float32) if target_values is None else target_values
     check(lib().b200rl_gae(_ptr(rewards), rewards.stride(0), _ptr(all_values), all_values.stride(0), _ptr(terminated), terminated.stride(0),
-                           _ptr(truncated), truncated.stride(0), _ptr(adv), 1, _ptr(tgt), 1, n_envs, steps, gamma, lam, int(ignore_termination), _stream()), "b200rl_gae")
+                           _ptr(truncated), truncated.stride(0), _ptr(adv), adv.stride(0), _ptr(tgt), tgt.stride(0), n_envs, steps, gamma, lam, int(ignore_termination), _stream()), "b200rl_gae")
     return adv, tgt
 
 
@@ -603,22 +603,31 @@ def pendulum_rollout_device_rng(shape, params, states, episode_step, truncated, 
     return obs, act, rew
 
 
-def shuffle_permutation_host(rng_state, n_rows):
-    """The row permutation of one PPO epoch shuffle, drawn on the reference-compatible host engine (advanced in place): numpy int32[n_rows]."""
+def shuffle_permutation_host(rng_state, n_rows, out=None):
+    """The row permutation of one PPO epoch shuffle, drawn on the reference-compatible host engine (advanced in place): numpy int32[n_rows], or written to
+    the host address `out`."""
     import numpy as np
+    if out is not None:
+        check(lib().b200rl_shuffle_permutation_host(rng_state.ctypes.data, n_rows, out), "b200rl_shuffle_permutation_host")
+        return None
     perm = np.empty(n_rows, np.int32)
     check(lib().b200rl_shuffle_permutation_host(C.c_void_p(rng_state.ctypes.data), n_rows, C.c_void_p(perm.ctypes.data)), "b200rl_shuffle_permutation_host")
     return perm
 
 
-def permute_rows(data, n_rows, perm, columns):
-    """data[i, c] = old data[perm[i], c] for the given columns (in place on a 2-D CUDA tensor; perm = int32 CUDA tensor)."""
+def permute_rows_scratch(data, n_rows, columns):
+    """(column mask, scratch buffer, its bytes): what permute_rows needs besides its operands, for callers that shuffle more than once."""
     import torch
     mask = 0
     for c in columns:
         mask |= 1 << int(c)
     nbytes = lib().b200rl_permute_rows_scratch_bytes(n_rows, mask)
-    scratch = torch.empty(max(nbytes, 4), device=data.device, dtype=torch.uint8)
+    return mask, torch.empty(max(nbytes, 4), device=data.device, dtype=torch.uint8), nbytes
+
+
+def permute_rows(data, n_rows, perm, columns, scratch=None):
+    """data[i, c] = old data[perm[i], c] for the given columns (in place on a 2-D CUDA tensor; perm = int32 CUDA tensor)."""
+    mask, scratch, nbytes = permute_rows_scratch(data, n_rows, columns) if scratch is None else scratch
     check(lib().b200rl_permute_rows(_ptr(data), data.stride(0), n_rows, _ptr(perm), mask, _ptr(scratch), nbytes, _stream()), "b200rl_permute_rows")
 
 

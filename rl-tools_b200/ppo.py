@@ -6,7 +6,7 @@ parameters of rl/algorithms/ppo/ppo.h:13-38. Everything runs on the GPU on torch
 """
 import ctypes as C
 
-from . import lib, check, _ptr, _stream, gae as _gae, mse_gradient as _mse_gradient, ppo_policy_gradient as _ppo_policy_gradient, permute_rows as _permute_rows, shuffle_permutation_host as _shuffle_permutation_host
+from . import lib, check, _ptr, _stream, gae as _gae, mse_gradient as _mse_gradient, ppo_policy_gradient as _ppo_policy_gradient, permute_rows as _permute_rows, permute_rows_scratch as _permute_rows_scratch, shuffle_permutation_host as _shuffle_permutation_host
 
 
 class DatasetLayout:
@@ -33,10 +33,8 @@ def estimate_generalized_advantages(dataset, layout, n_envs, steps, gamma=0.99, 
     """Fills the advantage and target-value columns from rewards / values / flags, in place (one backward scan per environment).
     The value column must hold the critic's values of all (steps + 1) * n_envs observations."""
     rows = steps * n_envs
-    adv, tgt = _gae(dataset[:, layout.rewards], dataset[:, layout.values], dataset[:, layout.terminated], dataset[:, layout.truncated],
-                    n_envs, steps, gamma, lam, ignore_termination)
-    dataset[:rows, layout.advantages] = adv
-    dataset[:rows, layout.target_values] = tgt
+    _gae(dataset[:, layout.rewards], dataset[:, layout.values], dataset[:, layout.terminated], dataset[:, layout.truncated],
+         n_envs, steps, gamma, lam, ignore_termination, advantages=dataset[:rows, layout.advantages], target_values=dataset[:rows, layout.target_values])
     return dataset
 
 
@@ -105,8 +103,9 @@ class MinibatchGraphs:
             t.copy_(s)                                                                          # the warm-up update is undone
 
 
-def _train_epoch(actor, critic, dataset, layout, n_minibatches, batch_size, epsilon_clip, entropy_coefficient, advantage_epsilon, normalize_advantage, learn_action_std):
-    """All minibatch updates of one epoch as one native call; False for networks that its kernel does not take."""
+def _epoch_call(actor, critic, dataset, layout, n_minibatches, batch_size, epsilon_clip, entropy_coefficient, advantage_epsilon, normalize_advantage, learn_action_std):
+    """All minibatch updates of one epoch as one native call: a function that issues it, made once per train() (an epoch of small networks takes 100 us);
+    None for networks that its kernel does not take."""
     import torch
     work = actor.__dict__.setdefault("_epoch_scratch", {})
     key = (n_minibatches, batch_size, bytes(actor.shape), bytes(critic.shape))
@@ -114,17 +113,53 @@ def _train_epoch(actor, critic, dataset, layout, n_minibatches, batch_size, epsi
         n = lib().b200rl_ppo_train_epoch_scratch_bytes(C.byref(actor.shape), C.byref(critic.shape), batch_size, n_minibatches)
         work["key"], work["bytes"], work["buffer"] = key, n, torch.empty(n, device=dataset.device, dtype=torch.uint8) if n else None
     if not work["bytes"]:
-        return False
+        return None
     base, ld = dataset.data_ptr(), dataset.stride(0)
     at = lambda column: base + 4 * column
-    rc = lib().b200rl_ppo_train_epoch(C.byref(actor.shape), C.byref(actor.arenas()), C.byref(critic.shape), C.byref(critic.arenas()), at(layout.observations.start),
-                                      at(layout.actions.start), at(layout.action_log_probs), at(layout.advantages), at(layout.target_values), ld, batch_size, n_minibatches,
-                                      epsilon_clip, entropy_coefficient, advantage_epsilon, normalize_advantage, learn_action_std, work["buffer"].data_ptr(), work["bytes"],
-                                      _stream())
-    if rc == 2:                                                         # B200RL_ERR_UNSUPPORTED
-        return False
-    check(rc, "b200rl_ppo_train_epoch")
-    return True
+    args = (C.byref(actor.shape), C.byref(actor.arenas()), C.byref(critic.shape), C.byref(critic.arenas()), at(layout.observations.start), at(layout.actions.start),
+            at(layout.action_log_probs), at(layout.advantages), at(layout.target_values), ld, batch_size, n_minibatches, epsilon_clip, entropy_coefficient, advantage_epsilon,
+            normalize_advantage, learn_action_std, work["buffer"].data_ptr(), work["bytes"], _stream())
+    call = lib().b200rl_ppo_train_epoch
+
+    def epoch():
+        rc = call(*args)
+        if rc == 2:                                                     # B200RL_ERR_UNSUPPORTED
+            return False
+        check(rc, "b200rl_ppo_train_epoch")
+        return True
+    return epoch
+
+
+class _Shuffle:
+    """The epoch shuffle: the next epoch's permutation is drawn and sent, on a stream of its own and into the other of two buffers, while this one's kernels
+    run (a copy in the stream of the kernels held the epoch up by 25 to 40 us). Pinned memory comes from torch's pool, which waits for copies under way."""
+
+    def __init__(self, dataset, n_rows, columns):
+        import torch
+        self.n_rows, self.columns, self.epoch = n_rows, columns, 0
+        self.scratch = _permute_rows_scratch(dataset, n_rows, columns)
+        self.perm = torch.empty((2, n_rows), device=dataset.device, dtype=torch.int32)
+        self.used = [torch.cuda.current_stream().record_event()] * 2
+        self.stream = torch.cuda.Stream(device=dataset.device)
+
+    def __call__(self, dataset, rng_state):
+        import torch
+        main, k = torch.cuda.current_stream(), self.epoch & 1
+        host = torch.empty(self.n_rows, dtype=torch.int32, pin_memory=True)
+        _shuffle_permutation_host(rng_state, self.n_rows, host.data_ptr())
+        with torch.cuda.stream(self.stream):
+            self.stream.wait_event(self.used[k])
+            self.perm[k].copy_(host, non_blocking=True)
+            ready = self.stream.record_event()
+        main.wait_event(ready)
+        _permute_rows(dataset, self.n_rows, self.perm[k], self.columns, self.scratch)
+        self.used[k] = main.record_event()
+        self.epoch += 1
+
+
+def _train_epoch(*networks_and_sizes, **hyper):
+    epoch = _epoch_call(*networks_and_sizes, **hyper)
+    return epoch is not None and epoch()
 
 
 def train(actor, critic, dataset, layout, n_rows, batch_size, n_epochs=10, epsilon_clip=0.2, entropy_coefficient=0.01, advantage_epsilon=1e-8,
@@ -145,11 +180,17 @@ def train(actor, critic, dataset, layout, n_rows, batch_size, n_epochs=10, epsil
         assert graphs.key == (dataset.data_ptr(), n_rows, batch_size), "graphs were captured for another dataset matrix"
     shuffled = list(range(layout.observations.start, layout.observations.stop)) + list(range(layout.actions.start, layout.actions.stop)) + \
         [layout.action_log_probs, layout.advantages, layout.target_values]
+    epoch = _epoch_call(actor, critic, dataset, layout, n_rows // batch_size, batch_size, **hyper)
+    if shuffle_rng_state is not None:
+        key, work = (dataset.device, n_rows, tuple(shuffled)), actor.__dict__.setdefault("_shuffle", {})
+        if key not in work:
+            work.clear()
+            work[key] = _Shuffle(dataset, n_rows, shuffled)
+        shuffle = work[key]
     for _ in range(n_epochs):
         if shuffle_rng_state is not None:
-            perm = torch.from_numpy(_shuffle_permutation_host(shuffle_rng_state, n_rows)).to(dataset.device)
-            _permute_rows(dataset, n_rows, perm, shuffled)
-        if _train_epoch(actor, critic, dataset, layout, n_rows // batch_size, batch_size, **hyper):
+            shuffle(dataset, shuffle_rng_state)
+        if epoch is not None and epoch():
             continue
         for b in range(n_rows // batch_size):
             if graphs is not None:

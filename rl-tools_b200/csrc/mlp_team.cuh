@@ -16,6 +16,9 @@
 // the CTA has threads, the summed index is split over thread groups and the parts are added in group order.
 // Teams write their gradient sums to scratch memory; after a grid-wide barrier all CTAs share out the parameters, add the teams' sums in a fixed
 // order and apply the optimizer step.
+//
+// Loops over elements and layers stay rolled: a minibatch walks the whole code once, and what does not fit the instruction caches is fetched anew for every one of
+// them (PPO epoch kernel 220 -> 108 KB of code: 27-64-64-8, 2,048 rows 22.4 -> 20.3 us per minibatch).
 #pragma once
 #include "common.cuh"
 
@@ -155,7 +158,7 @@ __device__ __forceinline__ void clear_rows(const Net& n, float* smem){
 // this CTA's weight rows of every layer into shared memory by asynchronous copies; the caller waits for them
 template <int L>
 __device__ __forceinline__ void load_weights(const Net& n, float* smem, const float* params, int rank){
-#pragma unroll
+#pragma unroll 1
     for(int l = 0; l < L; l++){
         const Layer& y = n.layer[l];
         const float* W = params + y.poff + (size_t)rank * y.S * y.I;
@@ -163,11 +166,14 @@ __device__ __forceinline__ void load_weights(const Net& n, float* smem, const fl
         const int rows = min(y.S, y.O - rank * y.S);
         if((y.I & 3) == 0 && (reinterpret_cast<uintptr_t>(W) & 15u) == 0){
             const int q = y.I >> 2;
+#pragma unroll 2
             for(int i = threadIdx.x; i < rows * q; i += THREADS) copy16_async(sw + 4 * i + quotient(i, y.by_row) * (y.P - y.I), W + 4 * i);
         }
         else{
+#pragma unroll 2
             for(int i = threadIdx.x; i < rows * y.I; i += THREADS) copy4_async(sw + i + quotient(i, y.by_I) * (y.P - y.I), W + i);
         }
+#pragma unroll 1
         for(int o = threadIdx.x; o < rows; o += THREADS) copy4_async(sw + o * y.P + y.I, params + y.poff + (size_t)y.O * y.I + rank * y.S + o);
     }
 }
@@ -217,6 +223,7 @@ __device__ __forceinline__ void forward_layer(const Net& n, int l, float* smem, 
     forward_products(n, y, smem, rb);
     __syncthreads();
     const int count = n.R * y.S, next_a = l + 1 < L ? n.layer[l + 1].a : 0, next_p = l + 1 < L ? n.layer[l + 1].P : 0;
+#pragma unroll 1
     for(int idx = threadIdx.x; idx < count; idx += THREADS){
         const int r = quotient(idx, y.by_S), o = idx - r * y.S, unit = rank * y.S + o;
         float v = rb[idx], dv;
@@ -298,6 +305,7 @@ __device__ __forceinline__ void backward_layer(const Net& n, int l, float* smem,
     }
     sync_team<C>();
     const int count = n.R * z.S, parts = C * y.bwd_groups;
+#pragma unroll 1
     for(int idx = threadIdx.x; idx < count; idx += THREADS){
         const float dv = smem[z.g + idx];
         float v = 0.0f;
@@ -377,7 +385,7 @@ __device__ __forceinline__ int arena_index(const Net& n, int u, int comp){
     return index;
 }
 
-__device__ __forceinline__ float adam_bias_correction(float beta, uint32_t age){
+static __device__ __noinline__ float adam_bias_correction(float beta, uint32_t age){
     const float pw = (float)pow((double)beta, (double)(float)age);      // rounded to float once, as the per-arena kernel does
     return 1.0f / (1.0f - pw);
 }

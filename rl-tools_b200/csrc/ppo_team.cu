@@ -65,12 +65,14 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
         const int row0 = tile * R;
         const size_t base = (size_t)minibatch * a.batch + row0;
         const int rows = min(R, a.batch - row0);
+#pragma unroll 1
         for(int i = tid; i < R * I0; i += THREADS){
             const int r = quotient(i, n.by_I0), k = i - r * I0;
             if(r < rows) copy4_async(smem + w.stage_x + i, a.observations + (base + r) * a.ld + k);
             else smem[w.stage_x + i] = 0.0f;
         }
         if constexpr(ACTOR){
+#pragma unroll 1
             for(int i = tid; i < R * S; i += THREADS){
                 const int r = quotient(i, last.by_S), k = i - r * S;
                 if(r < rows && k < A) copy4_async(smem + w.stage_aux + i, a.actions + (base + r) * a.ld + k);
@@ -114,8 +116,12 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
             const int rows = min(R, a.batch - tile * R);
             copies_wait();
             __syncthreads();
+#pragma unroll 1
             for(int i = tid; i < R * I0; i += THREADS){ const int r = quotient(i, n.by_I0), k = i - r * I0; smem[n.layer[0].a + r * n.layer[0].P + k] = smem[w.stage_x + i]; }
-            if constexpr(ACTOR){ for(int i = tid; i < R * S + 2 * R; i += THREADS) smem[w.aux + i] = smem[w.stage_aux + i]; }
+            if constexpr(ACTOR){
+#pragma unroll 1
+                for(int i = tid; i < R * S + 2 * R; i += THREADS) smem[w.aux + i] = smem[w.stage_aux + i];
+            }
             else if(tid < R) smem[w.aux + tid] = smem[w.stage_aux + tid];
             __syncthreads();
             {
@@ -123,7 +129,7 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
                 if(more) stage(mb, tile + w.teams);
                 else if(mb + 1 < a.minibatches) stage(mb + 1, cta);
             }
-#pragma unroll
+#pragma unroll 1
             for(int l = 0; l < L; l++){
                 forward_layer<1, L>(n, l, smem, 0, [&](int r, int unit, int idx, float value, float derivative){
                     if(l == L - 1){
@@ -137,6 +143,7 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
                 float* lp = smem + n.rb[1];                      // [R][S] log-probability terms, then [R][S] (action - mean) / std, then [R] dL / d log-probability
                 float* ps = lp + R * S;
                 float* dl = ps + R * S;
+#pragma unroll 1
                 for(int i = tid; i < R * S; i += THREADS){
                     const int r = quotient(i, last.by_S), k = i - r * S;
                     if(k < A){
@@ -155,6 +162,7 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
                     float d = 0.0f;
                     if(tid < rows){
                         float log_prob = 0.0f;
+#pragma unroll 1
                         for(int k = 0; k < A; k++) log_prob = __fadd_rn(log_prob, lp[tid * S + k]);
                         float advantage = smem[w.aux + R * S + R + tid];
                         if(a.normalize_advantage) advantage = __fdiv_rn(__fsub_rn(advantage, mean), deviation);
@@ -169,17 +177,19 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
                     dl[tid] = d;
                 }
                 __syncthreads();
+#pragma unroll 1
                 for(int i = tid; i < R * S; i += THREADS){
                     const int r = quotient(i, last.by_S), k = i - r * S;
                     if(k < A) smem[last.d + i] = r < rows ? __fmul_rn(__fdiv_rn(ps[i], s_std[k]), dl[r]) * smem[last.g + i] : 0.0f;
                 }
                 if(tid >= 128 && tid < 128 + A){                 // the log_std gradient of the CTA's rows, in row order
                     const int k = tid - 128;
+#pragma unroll 4
                     for(int r = 0; r < rows; r++) std_gradient += __fmul_rn(dl[r], __fadd_rn(-1.0f, __fmul_rn(ps[r * S + k], ps[r * S + k])));
                 }
                 __syncthreads();
             }
-#pragma unroll
+#pragma unroll 1
             for(int l = L - 1; l > 0; l--) backward_layer<1>(n, l, smem, 0, (L - 1 - l) & 1);
             accumulate_gradients<TPT>(n, smem, patches, acc);
             if(tile + w.teams < w.row_tiles) __syncthreads();

@@ -105,3 +105,48 @@ def test_backward_matches_fp64(lib, rows, I, dims, acts, mode):
     if d_input is not None:
         err, size = (d_input.double() - d).norm(dim=1), d.norm(dim=1)
         assert float((err - 1e-5 * size).max()) <= 1e-6 / rows
+
+
+@pytest.mark.parametrize("rows,I,dims", [(2048, 64, [256, 256, 16]), (2100, 200, [130, 129]), (8192, 27, [64, 64, 8]), (8200, 100, [33, 128, 7])])
+def test_weights_far_below_the_largest_of_their_layer(lib, rows, I, dims):
+    """Every third output of a layer has weights 2^-24 of the layer's largest, and so has every third input (a column, which is an output of the
+    backward chain): each output column, input-gradient column and gradient row is as close to fp64 as its own size asks for. Two fp16 parts hold 22 bits
+    of an operand, so a product is off by 2^-21, and the truncating accumulation of a 64-column piece adds about as much: 1e-6 in all, for each product of a chain."""
+    import torch
+    net = lib.Mlp(I, dims, ["identity"] * len(dims), rows)
+    off, fan_in, weights = 0, I, []
+    for l, d in enumerate(dims):
+        W = torch.from_numpy(mg.det_uniform(7 + l, d * fan_in).reshape(d, fan_in) / np.float32(np.sqrt(fan_in))).cuda()
+        W[::3] *= 2.0 ** -24
+        W[:, 1::3] *= 2.0 ** -24
+        net.params[off:off + d * fan_in] = W.flatten()
+        weights.append(W.double())
+        off += d * fan_in + d; fan_in = d
+    x = torch.from_numpy(mg.det_normal(1, rows * I).reshape(rows, I)).cuda()
+
+    def close(got, want, products=1):
+        err, size = (got.double() - want).norm(dim=0), want.norm(dim=0)
+        assert float((err / size).max()) <= 1e-6 * products
+
+    y = net.evaluate(x)
+    net.forward(x)
+    inp, off = x.double(), 0
+    for W in weights:
+        got = net.out[off:off + rows * len(W)].view(rows, len(W))
+        off += rows * len(W)
+        close(got, inp @ W.T)
+        inp = got.double()
+    close(y, inp)
+    d_out = torch.from_numpy(mg.det_normal(2, rows * dims[-1]).reshape(rows, dims[-1])).cuda() / rows
+    d_input = torch.zeros(rows, I, device="cuda")
+    net.zero_gradient()
+    net.backward(x, d_out.clone(), d_input=d_input)
+    d, poff = d_out.double(), net.n_mlp
+    for l in range(len(dims) - 1, -1, -1):
+        o, i = weights[l].shape
+        poff -= o * i + o
+        if l == 0:
+            size = d.abs().T @ x.double().abs()                 # the sum over the rows cancels: its terms' magnitudes
+            assert float(((net.grads[poff:poff + o * i].view(o, i).double() - d.T @ x.double()).abs() / size).max()) <= 2e-6
+        d = d @ weights[l]
+    close(d_input, d, products=len(dims))

@@ -10,10 +10,11 @@
 // fp32 accumulation -- the precision of three tf32 passes at twice their rate and half their shared memory. fp16's range is met by powers of two
 // that divide out exactly: a layer's weights are scaled by their largest magnitude, every 64-column piece of an activation row by that piece's, so a
 // remainder is subnormal only for values below 2^-17 of those maxima (and then off by at most 2^-39 of them). An output whose weights all lie more than
-// 2^-12 below the layer's largest would lose bits by that (2.9e-5 of itself at 2^-24): it is scaled by its own largest, and the 16 columns of which it is
-// one multiply their sums by what they lack when the layer ends (all columns always: evaluate 1,447 -> 1,750 us, the loads stand between two layers). The
-// tensor core truncates when it accumulates, so a chain of MMAs is kept to 64 summed columns (12 MMAs); the pieces are added, unscaled, to fp32 registers
-// with fused multiply-adds.
+// 2^-12 below the layer's largest would lose bits by that (2.9e-5 of itself at 2^-24): it is scaled by its own largest, and a network that has such an
+// output multiplies every sum by what it lacks when the layer ends. For other networks that is one test per layer: what stands between two layers counts
+// (factors for all columns always: evaluate 1,447 -> 1,750 us at 1,048,576 rows; a test per piece: 1,551; two copies of the loop: the code to fetch costs 8 us
+// per launch once the activations have pushed it out of L2). The tensor core truncates when it accumulates, so a chain of MMAs is kept to 64 summed columns
+// (12 MMAs); the pieces are added, unscaled, to fp32 registers with fused multiply-adds.
 //
 // Roles: 16 warps (112 registers) move accumulators to registers and do everything element-wise; one thread each of two further warps issues MMAs, one
 // of a third brings the weights in. A unit of work is one 64-column piece of the summed index into all outputs of a layer. An MMA of 128 rows takes about
@@ -39,7 +40,6 @@
 #include "tcgen05.cuh"
 #include "split_f16.cuh"
 #include <atomic>
-#include <type_traits>
 
 namespace b200rl {
 
@@ -51,7 +51,7 @@ constexpr uint32_t CH_A = 4 * CH_STAGE;                           // both parts 
 constexpr uint32_t CH_EXP = 4 * CH_ROWS + 2 * 4 * CH_ROWS;        // exponents of the pieces' scales; two buffers of the four warps' exponents per row
 constexpr uint32_t CH_SMEM = CH_A + CH_STAGES * CH_STAGE + CH_EXP + 256 + 1024;
 static_assert(CH_SMEM <= 227 * 1024, "shared memory");
-constexpr size_t CH_TAIL = (2 * 256 + 8) * sizeof(float);         // behind an image: see ChainStep::tail
+constexpr size_t CH_TAIL = (3 * 256 + 4) * sizeof(float);        // behind an image: see ChainStep::tail
 constexpr uint32_t CH_OWN_SCALE = 12;                             // powers of two below the layer's largest weight from which on an output has its own scale
 constexpr long long CH_WAIT_LIMIT = 2000000000LL;
 enum { CH_EVALUATE = 0, CH_FORWARD = 1, CH_BACKWARD = 2 };
@@ -59,8 +59,8 @@ enum { CH_EVALUATE = 0, CH_FORWARD = 1, CH_BACKWARD = 2 };
 
 struct ChainStep {
     int N, K, pieces, n, act;                         // n: N rounded up to 16
-    const uint8_t* image; const float* tail;          // tail: 256 biases (zeros beyond N), the factors that 256 outputs' sums lack, the inverse of the weights' scale, behind three unused words four of bytes:
-    // [g][p] whether any of the columns 64 p + 16 g ... + 15 lacks one
+    const uint8_t* image; const float* tail;          // tail: 256 biases (zeros beyond N), the factors f that 256 outputs' sums lack, their biases x (1 - f), the inverse of the weights' scale, an
+    // unused word, eight flags of a byte: whether any of 32 outputs lacks a factor
     float* pre; float* out; long long ld;             // forward: this layer's arenas [rows, N]; evaluate: the last layer's outputs with their row pitch
     // backward: pre_in = pre-activations [rows, N] of the layer below, act = its activation (identity where there is none), out = its d_pre with
     // row pitch ld, or the network's input gradient, or NULL
@@ -163,13 +163,13 @@ __device__ __forceinline__ void clear_beyond(int col0, int N, int lane, Slice& v
         if(col + 1 >= N) v[i].y = 0.0f;
     }
 }
-// a slice's sums times their outputs' factors, plus their biases; tail points at the bias of the slice's first column
+// a slice's sums, which started with the bias, times their outputs' factors, plus what the bias lacks then: at[0 ... 15] and at[256 ... 271]
 template <bool ROWS>
-__device__ __forceinline__ void finish_sums(const float* tail, int lane, Slice& v){
+__device__ __forceinline__ void finish_sums(const float* at, int lane, Slice& v){
     if constexpr(ROWS){
 #pragma unroll
         for(int j = 0; j < 4; j++){
-            const float4 b = __ldg(reinterpret_cast<const float4*>(tail) + j), f = __ldg(reinterpret_cast<const float4*>(tail + 256) + j);
+            const float4 f = __ldg(reinterpret_cast<const float4*>(at) + j), b = __ldg(reinterpret_cast<const float4*>(at + 256) + j);
             v[2 * j] = __ffma2_rn(v[2 * j], make_float2(f.x, f.y), make_float2(b.x, b.y));
             v[2 * j + 1] = __ffma2_rn(v[2 * j + 1], make_float2(f.z, f.w), make_float2(b.z, b.w));
         }
@@ -177,7 +177,7 @@ __device__ __forceinline__ void finish_sums(const float* tail, int lane, Slice& 
     else{
 #pragma unroll
         for(int j = 0; j < 2; j++){
-            const float2 b = __ldg(reinterpret_cast<const float2*>(tail + Spread<ROWS>::column(lane, j))), f = __ldg(reinterpret_cast<const float2*>(tail + 256 + Spread<ROWS>::column(lane, j)));
+            const float2 f = __ldg(reinterpret_cast<const float2*>(at + Spread<ROWS>::column(lane, j))), b = __ldg(reinterpret_cast<const float2*>(at + 256 + Spread<ROWS>::column(lane, j)));
 #pragma unroll
             for(int s = 0; s < 4; s++) v[2 * s + j] = __ffma2_rn(v[2 * s + j], f, b);
         }
@@ -215,6 +215,8 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
     uint32_t* slot = reinterpret_cast<uint32_t*>(a_full + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(slot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // asked for here, needed once tensor memory is there
+    const uint2 own_flags = lane < a.n_steps ? __ldg(reinterpret_cast<const uint2*>(a.step[lane].tail + 770)) : make_uint2(0u, 0u);
     if(tid == 0){
         for(int i = 0; i < CH_STAGES; i++){ tc::mbar_init(w_full + i, 1); tc::mbar_init(w_empty + i, 1); }
         for(int i = 0; i < 2; i++){ tc::mbar_init(acc_full + i, 1); tc::mbar_init(acc_empty + i, CH_WARPS); tc::mbar_init(turn + i, 1); }
@@ -378,8 +380,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
         auto load_input = [&](int tile, int piece, Slice& v){
             load_slice<ROWS>(Place{tile * CH_ROWS + q * 32, 64 * piece + 16 * g, a.rows, a.in_cols, a.ld_in}, a.in, lane, v);
         };
-        auto tiles = [&](auto some_own){                                // some_own: whether any output of any layer has a scale of its own
-        constexpr bool OWN = decltype(some_own)::value;
+        const bool some_own = __any_sync(0xffffffffu, (own_flags.x | own_flags.y) != 0u);        // some output of the network has a scale of its own
         Slice acc[4];                                                   // this layer's sums, a slice per piece
         bool loaded = false;                                            // acc[2], acc[3]: the tile's first two input pieces
         for(int tile = blockIdx.x; tile < a.tiles && ok; tile += gridDim.x){
@@ -407,7 +408,6 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
                 const ChainStep& y = a.step[st];
                 const bool last = st + 1 == a.n_steps, stacked = y.n <= 128;
                 const int outs = (y.N + 63) / 64;                       // pieces of the output
-                const uint32_t own = !OWN ? 0u : __ldg(reinterpret_cast<const uint32_t*>(y.tail + 516) + g);       // byte p: this warp's slice of piece p has outputs with their own scale
 #pragma unroll
                 for(int p = 0; p < 4; p++){                              // the sums start with the bias
                     if(p >= outs) break;
@@ -427,17 +427,13 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
                             for(int s = 0; s < 4; s++) acc[p][2 * s + j] = b;
                         }
                     }
-                    if(OWN && ((own >> (8 * p)) & 0xFFu)){                // there it comes last
-#pragma unroll
-                        for(int i = 0; i < 8; i++) acc[p][i] = make_float2(0.0f, 0.0f);
-                    }
                 }
                 if(MODE != CH_BACKWARD && last && stacked && tile + (int)gridDim.x < a.tiles){  // a narrow last layer leaves room for the next tile's inputs
                     load_input(tile + gridDim.x, 0, acc[2]);
                     if(a.step[0].pieces > 1) load_input(tile + gridDim.x, 1, acc[3]);
                     loaded = true;
                 }
-                const float weights = __ldg(y.tail + 512);              // inverse of the weights' scale
+                const float weights = __ldg(y.tail + 768);              // inverse of the weights' scale
                 Slice below;                                             // backward: pre-activations of the next piece
                 for(int c = 0; c < y.pieces; c++, u++){
                     if constexpr(MODE == CH_BACKWARD){
@@ -476,12 +472,18 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
                     if(lane == 0) tc::mbar_arrive(acc_empty + (u & 1u));
                 }
                 if(!ok) break;
+                if(some_own){                                           // one test per layer: it stands between this layer's MMAs and the next one's
+#pragma unroll
+                    for(int p = 0; p < 4; p++){
+                        if(p >= outs) break;
+                        finish_sums<ROWS>(y.tail + 256 + 64 * p + 16 * g, lane, acc[p]);
+                    }
+                }
                 // every MMA of this layer has completed: its input may be overwritten
 #pragma unroll
                 for(int p = 0; p < 4; p++){
                     if(p >= outs) break;
                     const Place at{row0, 64 * p + 16 * g, a.rows, y.N, y.ld};
-                    if(OWN && ((own >> (8 * p)) & 0xFFu)) finish_sums<ROWS>(y.tail + at.col0, lane, acc[p]);
                     if constexpr(MODE == CH_FORWARD) store_slice<ROWS>(at, y.pre, lane, acc[p]);
                     if constexpr(MODE == CH_BACKWARD){
                         if(y.act != B200RL_ACT_IDENTITY){
@@ -503,15 +505,6 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
                 }
             }
         }
-        };
-        // two copies of the loop: the test for an own scale, small as it is, costs evaluate 7 % when it stands between the layers
-        uint32_t any = 0;
-        for(int st = 0; st < a.n_steps; st++){
-            const uint4 f = __ldg(reinterpret_cast<const uint4*>(a.step[st].tail + 516));
-            any |= f.x | f.y | f.z | f.w;
-        }
-        if(any) tiles(std::true_type{});
-        else tiles(std::false_type{});
     }
     tc::fence_before_thread_sync();
     __syncthreads();
@@ -525,12 +518,20 @@ struct ChainImage { const float* W; const float* bias; uint8_t* image; float* ta
 struct ChainImages { int n; ChainImage y[CH_MAX_STEPS]; int blocks; };
 __global__ void __launch_bounds__(1024) chain_image_kernel(const __grid_constant__ ChainImages a){
     __shared__ float largest[32];
-    __shared__ uint8_t own[2];                                           // of this CTA's two slices of 16 outputs
     int l = 0;
     while(l + 1 < a.n && (int)blockIdx.x >= a.y[l + 1].block_begin) l++;
     const ChainImage& y = a.y[l];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = (blockIdx.x - y.block_begin) * 32 + warp, rows = (y.N + 15) / 16 * 16, pieces = (y.K + 63) / 64;
-    uint8_t* slices = reinterpret_cast<uint8_t*>(y.tail + 516);
+    uint8_t* flags = reinterpret_cast<uint8_t*>(y.tail + 770);
+    float v[4][2];
+#pragma unroll
+    for(int c = 0; c < 4; c++){
+#pragma unroll
+        for(int k = 0; k < 2; k++){
+            const int i = 64 * c + 2 * lane + k;
+            v[c][k] = n < y.N && i < y.K ? __ldg(y.W + (size_t)n * y.stride_n + (size_t)i * y.stride_k) : 0.0f;
+        }
+    }
     float m = 0.0f;
     const int count = y.N * y.K;
     if((reinterpret_cast<uintptr_t>(y.W) & 15u) == 0 && (count & 3) == 0){
@@ -541,20 +542,12 @@ __global__ void __launch_bounds__(1024) chain_image_kernel(const __grid_constant
 #pragma unroll 8
         for(int i = threadIdx.x; i < count; i += 1024) m = fmaxf(m, fabsf(__ldg(y.W + i)));
     }
-    float v[4][2], m_row = 0.0f;
+    float m_row = 0.0f;
 #pragma unroll
-    for(int c = 0; c < 4; c++){
-#pragma unroll
-        for(int k = 0; k < 2; k++){
-            const int i = 64 * c + 2 * lane + k;
-            v[c][k] = n < y.N && i < y.K ? __ldg(y.W + (size_t)n * y.stride_n + (size_t)i * y.stride_k) : 0.0f;
-            m_row = fmaxf(m_row, fabsf(v[c][k]));
-        }
-    }
+    for(int c = 0; c < 4; c++) m_row = fmaxf(m_row, fmaxf(fabsf(v[c][0]), fabsf(v[c][1])));
 #pragma unroll
     for(int o = 16; o > 0; o >>= 1){ m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o)); m_row = fmaxf(m_row, __shfl_xor_sync(0xffffffffu, m_row, o)); }
     if(lane == 0) largest[warp] = m;
-    if(threadIdx.x < 2) own[threadIdx.x] = 0;
     __syncthreads();
     m = largest[lane];
 #pragma unroll
@@ -563,16 +556,17 @@ __global__ void __launch_bounds__(1024) chain_image_kernel(const __grid_constant
     const bool apart = m_row > 0.0f && e_row + CH_OWN_SCALE < e_layer;   // a row of zeros fits any scale
     const uint32_t e = !apart ? e_layer : e_row + 126 < e_layer ? e_layer - 126 : e_row;      // the factor stays a normal number
     const float f = scale_of(e);
-    if(apart && lane == 0) own[warp >> 4] = 1;
-    if((int)blockIdx.x == y.block_begin){
-        for(int i = rows + threadIdx.x; i < 256; i += 1024){ y.tail[i] = 0.0f; y.tail[256 + i] = 0.0f; slices[4 * ((i >> 4) & 3) + (i >> 6)] = 0; }
-        if(threadIdx.x == 0) y.tail[512] = inverse_scale_of(e_layer);
+    const int some_apart = __syncthreads_or(apart);
+    const int cta = blockIdx.x - y.block_begin;
+    if(threadIdx.x == 0) flags[cta] = some_apart ? 1 : 0;
+    if(cta == 0){
+        for(int i = rows + threadIdx.x; i < 256; i += 1024){ y.tail[i] = 0.0f; y.tail[256 + i] = 0.0f; y.tail[512 + i] = 0.0f; }
+        if((int)threadIdx.x >= (rows + 31) / 32 && threadIdx.x < 8) flags[threadIdx.x] = 0;
+        if(threadIdx.x == 0) y.tail[768] = inverse_scale_of(e_layer);
     }
-    __syncthreads();
     if(lane == 0 && n < rows){
-        y.tail[n] = y.bias && n < y.N ? __ldg(y.bias + n) : 0.0f;
-        y.tail[256 + n] = scale_of(e_layer) * inverse_scale_of(e);       // 2^(e - e_layer)
-        if((n & 15) == 0) slices[4 * ((n >> 4) & 3) + (n >> 6)] = own[warp >> 4];
+        const float bias = y.bias && n < y.N ? __ldg(y.bias + n) : 0.0f, lacks = scale_of(e_layer) * inverse_scale_of(e);       // 2^(e - e_layer)
+        y.tail[n] = bias; y.tail[256 + n] = lacks; y.tail[512 + n] = bias - bias * lacks;
     }
     if(n >= rows) return;
     const uint32_t off = (uint32_t)n * 128 + ((((uint32_t)lane >> 2) ^ ((uint32_t)n & 7u)) << 4) + ((uint32_t)lane & 3u) * 4;

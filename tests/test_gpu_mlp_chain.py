@@ -114,12 +114,16 @@ def test_weights_far_below_the_largest_of_their_layer(lib, rows, I, dims):
     of an operand, so a product is off by 2^-21, and the truncating accumulation of a 64-column piece adds about as much: 1e-6 in all, for each product of a chain."""
     import torch
     net = lib.Mlp(I, dims, ["identity"] * len(dims), rows)
-    off, fan_in, weights = 0, I, []
+    off, fan_in, weights, biases = 0, I, [], []
     for l, d in enumerate(dims):
         W = torch.from_numpy(mg.det_uniform(7 + l, d * fan_in).reshape(d, fan_in) / np.float32(np.sqrt(fan_in))).cuda()
         W[::3] *= 2.0 ** -24
         W[:, 1::3] *= 2.0 ** -24
         net.params[off:off + d * fan_in] = W.flatten()
+        bias = torch.from_numpy(mg.det_uniform(17 + l, d)).cuda()
+        bias[::3] *= 2.0 ** -24
+        net.params[off + d * fan_in:off + d * fan_in + d] = bias
+        biases.append(bias.double())
         weights.append(W.double())
         off += d * fan_in + d; fan_in = d
     x = torch.from_numpy(mg.det_normal(1, rows * I).reshape(rows, I)).cuda()
@@ -131,10 +135,10 @@ def test_weights_far_below_the_largest_of_their_layer(lib, rows, I, dims):
     y = net.evaluate(x)
     net.forward(x)
     inp, off = x.double(), 0
-    for W in weights:
+    for W, b in zip(weights, biases):
         got = net.out[off:off + rows * len(W)].view(rows, len(W))
         off += rows * len(W)
-        close(got, inp @ W.T)
+        close(got, inp @ W.T + b)
         inp = got.double()
     close(y, inp)
     d_out = torch.from_numpy(mg.det_normal(2, rows * dims[-1]).reshape(rows, dims[-1])).cuda() / rows

@@ -609,11 +609,9 @@ int mlp_fused_backward(const b200rl_mlp_shape* sh, const float* params, float* g
                        float* d_input, int batch, void* scratch, size_t scratch_bytes, cudaStream_t s);
 
 // all layers of a pass in one tensor-core kernel (mlp_chain.cu)
-bool mlp_chain_eligible(const b200rl_mlp_shape* sh, int batch);
-size_t mlp_chain_workspace_bytes(const b200rl_mlp_shape* sh);
+size_t mlp_chain_workspace_bytes(const b200rl_mlp_shape* sh, int batch);
 int mlp_chain_forward(const b200rl_mlp_shape* sh, const float* params, const float* x, int ldx, float* pre, float* out, float* y, int ldy, int batch, void* workspace,
                       size_t workspace_bytes, cudaStream_t s);
-bool mlp_chain_backward_eligible(const b200rl_mlp_shape* sh, int batch);
 size_t mlp_chain_backward_scratch_bytes(const b200rl_mlp_shape* sh, int batch);
 int mlp_chain_backward(const b200rl_mlp_shape* sh, const float* params, float* grads, const float* x, int ldx, const float* pre, const float* out, const float* d_out,
                        float* d_input, int batch, void* scratch, size_t scratch_bytes, cudaStream_t s);
@@ -736,8 +734,8 @@ size_t b200rl_mlp_forward_workspace_bytes(const b200rl_mlp_shape* sh, int batch)
     if(!valid_shape(sh) || batch < 1) return 0;
     size_t m = 0; int I = sh->input_dim;
     for(int l = 0; l < sh->n_layers; l++){ const size_t b = forward_workspace_bytes(batch, I, sh->dims[l]); if(b > m) m = b; I = sh->dims[l]; }
-    if(mlp_chain_eligible(sh, batch)){ const size_t b = mlp_chain_workspace_bytes(sh); if(b > m) m = b; }
-    return m;
+    const size_t chain = mlp_chain_workspace_bytes(sh, batch);
+    return chain > m ? chain : m;
 }
 
 int b200rl_mlp_evaluate(const b200rl_mlp_shape* sh, const float* params, const float* x, int ldx, float* y, int ldy,
@@ -749,7 +747,7 @@ int b200rl_mlp_evaluate_ws(const b200rl_mlp_shape* sh, const float* params, cons
     if(!valid_shape(sh) || !params || !x || !y || batch < 0 || ldx < sh->input_dim || ldy < sh->dims[sh->n_layers - 1]) return B200RL_ERR_INVALID_ARGUMENT;
     if(sh->n_layers > 1 && (!tick || (sh->n_layers > 2 && !tock))) return B200RL_ERR_INVALID_ARGUMENT;
     if(batch == 0) return B200RL_OK;
-    if(mlp_chain_eligible(sh, batch)){
+    if(mlp_chain_takes(sh, batch, CHAIN_EVALUATE)){
         const int rc = mlp_chain_forward(sh, params, x, ldx, nullptr, nullptr, y, ldy, batch, workspace, workspace_bytes, (cudaStream_t)stream);
         if(rc != B200RL_ERR_UNSUPPORTED) return rc;
     }
@@ -774,7 +772,7 @@ int b200rl_mlp_forward_ws(const b200rl_mlp_shape* sh, const float* params, const
                           int batch, void* workspace, size_t workspace_bytes, b200rl_stream_t stream){
     if(!valid_shape(sh) || !params || !x || !pre || !out || batch < 0 || ldx < sh->input_dim) return B200RL_ERR_INVALID_ARGUMENT;
     if(batch == 0) return B200RL_OK;
-    if(mlp_chain_eligible(sh, batch)){
+    if(mlp_chain_takes(sh, batch, CHAIN_FORWARD)){
         const int rc = mlp_chain_forward(sh, params, x, ldx, pre, out, nullptr, 0, batch, workspace, workspace_bytes, (cudaStream_t)stream);
         if(rc != B200RL_ERR_UNSUPPORTED) return rc;
     }
@@ -809,7 +807,7 @@ int b200rl_mlp_backward(const b200rl_mlp_shape* sh, const float* params, float* 
     int L = sh->n_layers;
     if(L > 1 && (!tick || (L > 2 && !tock))) return B200RL_ERR_INVALID_ARGUMENT;
     if(batch == 0) return B200RL_OK;
-    if(mlp_chain_backward_eligible(sh, batch)){
+    if(mlp_chain_takes(sh, batch, grads ? CHAIN_GRADIENTS : CHAIN_INPUT)){
         const int rc = mlp_chain_backward(sh, params, grads, x, ldx, pre, out, d_out, d_input, batch, scratch, scratch_bytes, (cudaStream_t)stream);
         if(rc != B200RL_ERR_UNSUPPORTED) return rc;
     }

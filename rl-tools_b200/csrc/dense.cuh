@@ -33,4 +33,8 @@ int launch_gemm_tc(const GemmArgs& a, int epilogue, int activation, bool a_kcont
 size_t weight_image_bytes(int N, int K);
 int launch_weight_image(const float* W, long long ld, int N, int K, bool transposed, float* image, cudaStream_t s);
 
+// which passes of a network take the kernels that keep batch rows on the SM through all layers (mlp_chain.cu)
+enum { CHAIN_EVALUATE = 0, CHAIN_FORWARD = 1, CHAIN_GRADIENTS = 2, CHAIN_INPUT = 3 };         // CHAIN_INPUT: the input gradient without the parameters'
+bool mlp_chain_takes(const b200rl_mlp_shape* sh, int batch, int pass);
+
 }  // namespace b200rl

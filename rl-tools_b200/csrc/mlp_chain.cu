@@ -39,6 +39,7 @@
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include "split_f16.cuh"
+#include "dense.cuh"
 #include <atomic>
 
 namespace b200rl {
@@ -582,24 +583,47 @@ __global__ void __launch_bounds__(1024) chain_image_kernel(const __grid_constant
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------------------------------
-// Networks of up to eight layers, no wider than 256. A CTA takes 128 rows through all layers in the same time however few CTAs there are (37 us for
-// 64-256-256-256-16, 56 us when everything is kept; 17 and 21 us for 27-64-64-8), while the kernel per layer gains from a smaller batch: for wide
-// networks the lines cross between 1,024 and 2,048 rows (36 vs 70 us and 56 vs 73 us at 2,048, 36 vs 35 and 57 vs 35 at 512), for networks of up to
-// 128 columns near 8,192 (17 vs 24 and 21 vs 23 us).
-bool mlp_chain_eligible(const b200rl_mlp_shape* sh, int batch){
-    if(sh->n_layers > CH_MAX_STEPS) return false;
+// Which passes run here: networks of two to eight layers, no wider than 256. A CTA takes 128 rows through all layers in the same time however few CTAs there
+// are (34 us for 64-256-256-256-16, 54 us when everything is kept; 14 and 18 us for 27-64-64-8), while the kernels per layer gain from a smaller batch and
+// start sooner; so the lines lie where the rows fill the SMs or the products are many. Measured, these kernels against the kernels per layer, us (graph of ten
+// calls; rows x the network's weights in millions behind the rows):
+//   evaluate            4-256-256-1 at 2,048: 24 and 34; 64-256-16 at 2,048 (42): 17 and 15, at 4,096 (84): 18 and 28; 8-256-4 at 8,192 (25): 14 and 13, at 16,384
+//                       (50): 15 and 20; 64-128-4 at 8,192 (71): 15 and 13, at 16,384 (143): 15 and 17; 3-32-32-1 at 8,192 (9): 13 and 12, at 16,384 (19): 13 and 15
+//   forward             33-200-200-7 at 2,048 (98): 38 and 28, at 4,096 (197): 38 and 39; 64-256-256-256-16 at 2,048 (310): 54 and 60; 27-64-64-8 at 8,192 (52): 18 and 17;
+//                       3-64-64-1 at 16,384 (71): 19 and 24; 3-32-32-1 at 65,536 (75): 50 and 41; 64-128-4 at 65,536 (570): 56 and 49
+//   gradients           17-130-130-3 at 4,096 (80): 59 and 50, at 8,192 (160): 67 and 94; 33-200-200-7 at 2,048 (98): 61 and 66; 64-256-16 at 8,192 (168): 42 and 38, at
+//                       16,384: 48 and 47; 256-256-256 at 2,048: 59 and 83; 64-128-4 at 8,192: 33 and 27, at 16,384: 37 and 40; 10-16-2 at 16,384 (3): 32 and 27
+//   input gradient alone  17-130-130-3 at 2,048 (40): 29 and 18, at 4,096 (80): 29 and 35; 8-256-4 at 4,096 (13): 24 and 16, at 8,192: 22 and 98
+bool mlp_chain_takes(const b200rl_mlp_shape* sh, int batch, int pass){
+    if(sh->n_layers > CH_MAX_STEPS || sh->n_layers < 2) return false;
     int widest = sh->input_dim;
-    for(int l = 0; l < sh->n_layers; l++) if(sh->dims[l] > widest) widest = sh->dims[l];
-    return widest <= 256 && batch >= (widest > 128 ? 2048 : 8192);
+    long long weights = 0;
+    for(int l = 0, I = sh->input_dim; l < sh->n_layers; I = sh->dims[l], l++){
+        if(sh->dims[l] > widest) widest = sh->dims[l];
+        weights += (long long)I * sh->dims[l];
+    }
+    const bool wide = widest > 128, two = sh->n_layers == 2;
+    if(widest > 256 || batch < (wide ? 2048 : 8192)) return false;
+    const long long million = 1000000, work = weights * batch;
+    switch(pass){
+        case CHAIN_EVALUATE: return two ? work >= (wide ? 50 : 72) * million : wide || work >= 16 * million;
+        case CHAIN_FORWARD: return two ? wide && work >= 50 * million : wide ? batch >= 4096 || work >= 200 * million : weights >= 4096 && work >= 64 * million;
+        case CHAIN_GRADIENTS: return two ? weights >= 32768 || (batch >= 16384 && (wide || weights >= 4096)) : !wide || work >= 90 * million;
+        default: return batch >= 8192 || work >= 80 * million;
+    }
 }
 static size_t chain_image_bytes(int N, int K){
     const size_t rows = (N + 15) / 16 * 16;
     return rows * ((K + 63) / 64) * 256 + CH_TAIL;
 }
-size_t mlp_chain_workspace_bytes(const b200rl_mlp_shape* sh){
+static size_t images_bytes(const b200rl_mlp_shape* sh){
     size_t n = 0; int I = sh->input_dim;
     for(int l = 0; l < sh->n_layers; l++){ n += chain_image_bytes(sh->dims[l], I); I = sh->dims[l]; }
     return n;
+}
+size_t mlp_chain_workspace_bytes(const b200rl_mlp_shape* sh, int batch){
+    if(!mlp_chain_takes(sh, batch, CHAIN_EVALUATE) && !mlp_chain_takes(sh, batch, CHAIN_FORWARD)) return 0;
+    return images_bytes(sh);
 }
 // the word that a kernel's expired wait sets, and its reset (b200rl_device_error_state, b200rl_device_error_clear)
 int mlp_chain_error_get(int* word){ B200RL_CUDA_TRY(cudaMemcpyFromSymbol(word, g_chain_error, sizeof(int))); return B200RL_OK; }
@@ -638,7 +662,7 @@ static int launch_chain(ChainArgs& a, const ChainImages& images, cudaStream_t s,
 // pre == NULL: evaluate into y; otherwise forward into the arenas
 int mlp_chain_forward(const b200rl_mlp_shape* sh, const float* params, const float* x, int ldx, float* pre, float* out, float* y, int ldy, int batch, void* workspace,
                       size_t workspace_bytes, cudaStream_t s){
-    if(!workspace || workspace_bytes < mlp_chain_workspace_bytes(sh) || (reinterpret_cast<uintptr_t>(workspace) & 15u)) return B200RL_ERR_UNSUPPORTED;
+    if(!workspace || workspace_bytes < images_bytes(sh) || (reinterpret_cast<uintptr_t>(workspace) & 15u)) return B200RL_ERR_UNSUPPORTED;
     // a CTA reads inputs while another one writes outputs: outputs over the inputs take the kernels per layer. Columns of one matrix do not overlap.
     if(y && y < x + (size_t)batch * ldx && x < y + (size_t)batch * ldy){
         const long long at = ldx == ldy ? ((y - x) % ldx + ldx) % ldx : 0;
@@ -675,7 +699,6 @@ static int chain_backward_rows(int batch){
     const int chunks = (batch + CHAIN_BACKWARD_ROWS - 1) / CHAIN_BACKWARD_ROWS;
     return ((batch + chunks - 1) / chunks + CH_ROWS - 1) / CH_ROWS * CH_ROWS;
 }
-bool mlp_chain_backward_eligible(const b200rl_mlp_shape* sh, int batch){ return sh->n_layers > 1 && mlp_chain_eligible(sh, batch); }
 static size_t aligned256(size_t n){ return (n + 255) / 256 * 256; }
 static long long padded(int columns){ return (columns + 3) / 4 * 4; }           // row pitch for the gradient kernel: rows of whole 16 bytes
 static size_t transposed_images_bytes(const b200rl_mlp_shape* sh){
@@ -684,7 +707,7 @@ static size_t transposed_images_bytes(const b200rl_mlp_shape* sh){
     return aligned256(n);
 }
 size_t mlp_chain_backward_scratch_bytes(const b200rl_mlp_shape* sh, int batch){
-    if(!mlp_chain_backward_eligible(sh, batch)) return 0;
+    if(!mlp_chain_takes(sh, batch, CHAIN_GRADIENTS) && !mlp_chain_takes(sh, batch, CHAIN_INPUT)) return 0;
     size_t columns = padded(sh->input_dim);                                  // padded copies of inputs; whether x needs one depends on where it lies
     bool copies = false;
     for(int l = 0; l < sh->n_layers; l++){

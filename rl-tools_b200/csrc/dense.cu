@@ -617,7 +617,6 @@ int mlp_chain_backward(const b200rl_mlp_shape* sh, const float* params, float* g
                        float* d_input, int batch, void* scratch, size_t scratch_bytes, cudaStream_t s);
 
 // whole training step in one cooperative launch (mlp_team.cu)
-bool mlp_team_eligible(const b200rl_mlp_shape* sh, int rows);
 size_t mlp_team_scratch_bytes(const b200rl_mlp_shape* sh, int rows);
 int mlp_team_step(const b200rl_mlp_shape* sh, float* params, float* grads, float* m, float* v, size_t n_total, const b200rl_adam_hyper& hyper, uint32_t* adam_state,
                   const float* x, int ldx, const float* target, int ldt, int rows, int chunk_rows, float loss_weight, float* pre, float* out, void* scratch, size_t scratch_bytes,
@@ -638,6 +637,22 @@ static size_t outputs_before_last(const b200rl_mlp_shape* sh){
     size_t n = 0;
     for(int l = 0; l + 1 < sh->n_layers; l++) n += (size_t)sh->dims[l];
     return n;
+}
+
+// Which training steps take one launch (mlp_team.cu) rather than a launch per pass: those whose chunk of rows has little work. The one launch's time grows with rows x
+// weights from the start, on CUDA cores; the tensor-core kernels take the same time up to a row tile per SM. Measured, one launch against the sequence, us (rows x weights in
+// millions):
+//   sequence of mlp_chain.cu   64-256-256-256-16 at 1,024 rows (155): 119 and 164, at 2,048 (310): 196 and 163, at 8,192 (1,240): 720 and 208; 64-256-256-16 at 2,048
+//                              (176): 91 and 128, at 3,072 (264): 134 and 130; 33-200-200-7 at 5,003 (240): 117 and 129, at 6,144 (295): 152 and 130; narrower ones
+//                              cross earlier: 64-128-128-16 at 8,192 (218): 99 and 93; 64-100-100-100-16 at 8,192 (229): 123 and 109; 64-100-100-16 (147): 67 and 90
+//   kernels per layer          64-320-320-16 at 2,048 (262): 134 and 187, at 4,096 (524): 229 and 204; 300-256-256-10 at 2,048 (297): 171 and 222, at 4,096 (593): 320 and
+//                              232; 512-128-128-10 at 4,096 (340): 152 and 171, at 8,192 (680): 286 and 190; 17-300-300-300-3 at 2,048 (381): 275 and 291
+static bool mlp_team_is_faster(const b200rl_mlp_shape* sh, int chunk_rows){
+    long long weights = 0;
+    int widest = sh->input_dim;
+    for(int l = 0, I = sh->input_dim; l < sh->n_layers; I = sh->dims[l], l++){ weights += (long long)I * sh->dims[l]; if(sh->dims[l] > widest) widest = sh->dims[l]; }
+    const bool chain = mlp_chain_takes(sh, chunk_rows, CHAIN_FORWARD) && mlp_chain_takes(sh, chunk_rows, CHAIN_GRADIENTS);
+    return weights * chunk_rows <= (!chain ? 400 : widest > 128 ? 245 : 200) * 1000000ll;
 }
 
 }  // namespace b200rl
@@ -841,7 +856,7 @@ int b200rl_mlp_train_step(const b200rl_mlp_shape* sh, float* params, float* grad
         return B200RL_ERR_INVALID_ARGUMENT;
     const int L = sh->n_layers, O = sh->dims[L - 1];
     if(L > 1 && (!tick || (L > 2 && !tock))) return B200RL_ERR_INVALID_ARGUMENT;
-    if(mlp_team_eligible(sh, rows)){
+    if(mlp_team_is_faster(sh, chunk_rows)){
         const int rc = mlp_team_step(sh, params, grads, m, v, n, hyper, state, x, ldx, target, ldt, rows, chunk_rows, loss_weight, pre, out, scratch, scratch_bytes, optimize,
                                      (cudaStream_t)stream);
         if(rc != B200RL_ERR_UNSUPPORTED) return rc;

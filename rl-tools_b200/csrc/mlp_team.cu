@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
 struct TeamChoice { Net net; int C, teams, row_tiles, stage_x, stage_y, y_off, out_off; size_t smem; };
 
 constexpr size_t TEAM_SMEM = 220 * 1024;
-constexpr int TEAM_MAX_ROWS = 8192;          // beyond, the per-layer kernels' larger tiles are the better use of the SMs
+constexpr int TEAM_MAX_ROWS = 8192;          // what was measured; up to there the caller asks for steps of little work only (dense.cu)
 
 // teams of C CTAs that are resident at once on the current device (clusters do not tile every GPC completely); 0: unknown
 static int team_capacity(int C);
@@ -154,10 +154,6 @@ static bool choose_team(const b200rl_mlp_shape* sh, int rows, TeamChoice* out){
     return best > 0.0;
 }
 
-bool mlp_team_eligible(const b200rl_mlp_shape* sh, int rows){
-    TeamChoice c;
-    return rows >= 1 && rows <= TEAM_MAX_ROWS && choose_team(sh, rows, &c);
-}
 // for any number of rows up to the limit (a training step may run over several chunks of the batch the scratch was asked for)
 size_t mlp_team_scratch_bytes(const b200rl_mlp_shape* sh, int rows){
     TeamChoice c;
@@ -232,7 +228,7 @@ int mlp_team_step(const b200rl_mlp_shape* sh, float* params, float* grads, float
                   const float* x, int ldx, const float* target, int ldt, int rows, int chunk_rows, float loss_weight, float* pre, float* out, void* scratch, size_t scratch_bytes,
                   int optimize, cudaStream_t s){
     TeamChoice c;
-    if(!choose_team(sh, rows, &c) || !scratch || (reinterpret_cast<uintptr_t>(scratch) & 15u) || scratch_bytes < sizeof(float4) * (size_t)c.teams * c.C * c.net.n_tiles * 4)
+    if(rows > TEAM_MAX_ROWS || !choose_team(sh, rows, &c) || !scratch || (reinterpret_cast<uintptr_t>(scratch) & 15u) || scratch_bytes < sizeof(float4) * (size_t)c.teams * c.C * c.net.n_tiles * 4)
         return B200RL_ERR_UNSUPPORTED;
     TeamStepArgs a{};
     a.net = c.net;

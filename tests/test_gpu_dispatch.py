@@ -13,6 +13,18 @@ def _network(lib, batch, I, dims):
     return net
 
 
+@pytest.mark.parametrize("batch,chunks,I,dims,one_launch", [
+    (1024, 1, 64, [256, 256, 256, 16], True), (2048, 1, 64, [256, 256, 256, 16], False), (8192, 1, 64, [256, 256, 256, 16], False), (2048, 1, 64, [256, 256, 16], True),
+    (4096, 1, 64, [256, 256, 16], False), (5003, 1, 33, [200, 200, 7], True), (8192, 1, 64, [64, 64, 64, 16], True), (8192, 1, 64, [128, 128, 128, 16], False), (8192, 1, 64, [100, 100, 100, 16], False),
+    (4096, 2, 64, [256, 256, 256, 16], False), (2048, 1, 64, [320, 320, 16], True), (8192, 1, 64, [320, 320, 16], False)])
+def test_training_step_takes_one_launch_where_that_is_faster(lib, batch, chunks, I, dims, one_launch):
+    import torch
+    net = _network(lib, batch, I, dims)
+    x, y = torch.randn(batch * chunks, I, device="cuda"), torch.randn(batch * chunks, dims[-1], device="cuda")
+    names = kernels(lambda: net.train_step(x, y, 1.0 / chunks))
+    assert (len(names) == 1 and "mlp_team_step" in names[0]) == one_launch, names
+
+
 def _chain(names):
     return any("mlp_chain_kernel" in n for n in names)
 

@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
 struct ChainImage { const float* W; const float* bias; uint8_t* image; float* tail; int N, K, block_begin, stride_n, stride_k; };
 struct ChainImages { int n; ChainImage y[CH_MAX_STEPS]; int blocks; };
 __global__ void __launch_bounds__(1024) chain_image_kernel(const __grid_constant__ ChainImages a){
-    __shared__ float largest[32];
+    __shared__ uint32_t largest[32];
     int l = 0;
     while(l + 1 < a.n && (int)blockIdx.x >= a.y[l + 1].block_begin) l++;
     const ChainImage& y = a.y[l];
@@ -546,13 +546,11 @@ __global__ void __launch_bounds__(1024) chain_image_kernel(const __grid_constant
     float m_row = 0.0f;
 #pragma unroll
     for(int c = 0; c < 4; c++) m_row = fmaxf(m_row, fmaxf(fabsf(v[c][0]), fabsf(v[c][1])));
-#pragma unroll
-    for(int o = 16; o > 0; o >>= 1){ m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o)); m_row = fmaxf(m_row, __shfl_xor_sync(0xffffffffu, m_row, o)); }
-    if(lane == 0) largest[warp] = m;
+    // magnitudes compare like their bits (fmaxf has left NaNs out)
+    if(const uint32_t t = __reduce_max_sync(0xffffffffu, __float_as_uint(m)); lane == 0) largest[warp] = t;
+    m_row = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m_row)));
     __syncthreads();
-    m = largest[lane];
-#pragma unroll
-    for(int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    m = __uint_as_float(__reduce_max_sync(0xffffffffu, largest[lane]));
     const uint32_t e_layer = scale_exponent(m), e_row = scale_exponent(m_row);
     const bool apart = m_row > 0.0f && e_row + CH_OWN_SCALE < e_layer;   // a row of zeros fits any scale
     const uint32_t e = !apart ? e_layer : e_row + 126 < e_layer ? e_layer - 126 : e_row;      // the factor stays a normal number

@@ -121,7 +121,8 @@ static int team_capacity(int C);
 // Team size and rows per tile by an estimate of the launch in clock cycles, with constants from timelines of the kernel (64- and 256-wide networks,
 // batches of 256 ... 5,003): a layer of a tile costs its latencies (about 2,000 cycles over both directions, twice that where the team exchanges
 // through cluster barriers) plus its products at a third of the multiply-add peak; loading the weights and adding the teams' sums cost per float.
-static bool choose_team(const b200rl_mlp_shape* sh, int rows, TeamChoice* out){
+// Only plans whose sums fit into scratch_bytes: the scratch of a smaller batch serves a larger one, by its own plan or a better one that fits.
+static bool choose_team(const b200rl_mlp_shape* sh, int rows, size_t scratch_bytes, TeamChoice* out){
     for(int l = 0, I = sh->input_dim; l < sh->n_layers; I = sh->dims[l], l++) if(sh->dims[l] > 512 || I > 512) return false;
     double best = 0.0;
     for(int C = 1; C <= 8; C *= 2){
@@ -141,6 +142,7 @@ static bool choose_team(const b200rl_mlp_shape* sh, int rows, TeamChoice* out){
             if(c.smem > TEAM_SMEM) continue;
             c.row_tiles = (rows + R - 1) / R;
             c.teams = c.row_tiles < max_teams ? c.row_tiles : max_teams;
+            if(sizeof(float4) * (size_t)c.teams * c.C * c.net.n_tiles * 4 > scratch_bytes) continue;
             double weights = 0.0, tile = 0.0;
             for(int l = 0; l < c.net.n_layers; l++){
                 const Layer& y = c.net.layer[l];
@@ -154,10 +156,10 @@ static bool choose_team(const b200rl_mlp_shape* sh, int rows, TeamChoice* out){
     return best > 0.0;
 }
 
-// for any number of rows up to the limit (a training step may run over several chunks of the batch the scratch was asked for)
+// what the plan of this batch needs for any number of rows (a training step may run over several chunks of the batch the scratch was asked for)
 size_t mlp_team_scratch_bytes(const b200rl_mlp_shape* sh, int rows){
     TeamChoice c;
-    if(rows < 1 || !choose_team(sh, rows, &c)) return 0;
+    if(rows < 1 || !choose_team(sh, rows, SIZE_MAX, &c)) return 0;
     return sizeof(float4) * (size_t)team_capacity(c.C) * c.C * c.net.n_tiles * 4;
 }
 
@@ -228,8 +230,7 @@ int mlp_team_step(const b200rl_mlp_shape* sh, float* params, float* grads, float
                   const float* x, int ldx, const float* target, int ldt, int rows, int chunk_rows, float loss_weight, float* pre, float* out, void* scratch, size_t scratch_bytes,
                   int optimize, cudaStream_t s){
     TeamChoice c;
-    if(rows > TEAM_MAX_ROWS || !choose_team(sh, rows, &c) || !scratch || (reinterpret_cast<uintptr_t>(scratch) & 15u) || scratch_bytes < sizeof(float4) * (size_t)c.teams * c.C * c.net.n_tiles * 4)
-        return B200RL_ERR_UNSUPPORTED;
+    if(rows > TEAM_MAX_ROWS || !scratch || (reinterpret_cast<uintptr_t>(scratch) & 15u) || !choose_team(sh, rows, scratch_bytes, &c)) return B200RL_ERR_UNSUPPORTED;
     TeamStepArgs a{};
     a.net = c.net;
     a.params = params; a.grads = grads; a.m = m; a.v = v; a.adam_state = adam_state; a.hyper = hyper;

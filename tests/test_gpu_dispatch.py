@@ -16,6 +16,7 @@ def _network(lib, batch, I, dims):
 @pytest.mark.parametrize("batch,chunks,I,dims,one_launch", [
     (1024, 1, 64, [256, 256, 256, 16], True), (2048, 1, 64, [256, 256, 256, 16], False), (8192, 1, 64, [256, 256, 256, 16], False), (2048, 1, 64, [256, 256, 16], True),
     (4096, 1, 64, [256, 256, 16], False), (5003, 1, 33, [200, 200, 7], True), (8192, 1, 64, [64, 64, 64, 16], True), (8192, 1, 64, [128, 128, 128, 16], False), (8192, 1, 64, [100, 100, 100, 16], False),
+    (1024, 4, 64, [128, 128, 128, 16], True), (512, 8, 64, [256, 256, 16], True),
     (4096, 2, 64, [256, 256, 256, 16], False), (2048, 1, 64, [320, 320, 16], True), (8192, 1, 64, [320, 320, 16], False)])
 def test_training_step_takes_one_launch_where_that_is_faster(lib, batch, chunks, I, dims, one_launch):
     import torch

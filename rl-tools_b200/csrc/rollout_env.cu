@@ -165,8 +165,11 @@ static int launch_env_lanes(const EnvRolloutArgs& a, int sms, cudaStream_t s){
     const int warps = (a.n_envs + PER_WARP - 1) / PER_WARP;
     int per_cta = (warps + sms - 1) / sms;                           // spread over all SMs before CTAs grow
     if(per_cta > ENV_MAX_WARPS) per_cta = ENV_MAX_WARPS;
-    const size_t smem = sizeof(float) * (env_weight_floats(H, ENV::OBS_DIM) + per_cta * PER_WARP * env_pitch(H));
-    if(smem > 48 * 1024) B200RL_CUDA_TRY(cudaFuncSetAttribute(rollout_env_kernel<ENV, H, LANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr size_t per_warp = sizeof(float) * PER_WARP * env_pitch(H), weights = sizeof(float) * env_weight_floats(H, ENV::OBS_DIM), largest = weights + ENV_MAX_WARPS * per_warp;
+    static_assert(largest <= 227 * 1024, "shared memory");
+    const size_t smem = weights + per_cta * per_warp;
+    // always the largest, never this launch's: the limit belongs to the kernel, and another thread may be about to launch it for more environments
+    if constexpr(largest > 48 * 1024) B200RL_CUDA_TRY(cudaFuncSetAttribute(rollout_env_kernel<ENV, H, LANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)largest));
     rollout_env_kernel<ENV, H, LANES><<<(warps + per_cta - 1) / per_cta, 32 * per_cta, smem, s>>>(a);
     B200RL_LAUNCH_CHECK("rollout_env");
     return B200RL_OK;

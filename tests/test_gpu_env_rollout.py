@@ -272,3 +272,18 @@ def test_lanes_per_environment(lib, torch, env, hidden, n):
         assert np.array_equal(a, b)
     want_act = oracle.Oracle().mlp_evaluate(oshape, params, whole[0].reshape(T * n, O)).reshape(-1)
     close(whole[1].reshape(-1), want_act, what="actions on the kernel's observations")
+
+
+def test_a_launch_for_few_environments_leaves_the_kernels_shared_memory_limit(lib, torch):
+    """The shared memory of a launch depends on its number of environments, the kernel's limit must not: another thread may stand between setting the limit for
+    its larger number and its launch, which then fails."""
+    from graph_kernels import dynamic_shared_memory_limits
+    shape = lib.MlpShape.make(6, [128, 128, 1], ["relu", "relu", "tanh"])
+    params = torch.zeros(shape.num_params(), device="cuda")
+
+    def limit(n):
+        state = runner(torch, np.zeros((n, 4), np.float32))
+        (limit,) = dynamic_shared_memory_limits(lambda: lib.env_rollout(lib.ENV_ACROBOT_SWINGUP, shape, params, *state, None, 1, 200))
+        return limit
+    before, after = limit(3500), limit(64)
+    assert before == after

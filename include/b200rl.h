@@ -45,12 +45,13 @@ const char* b200rl_status_string(int status);
 /* text of the last CUDA error seen by this library on the calling thread ("" if none) */
 const char* b200rl_last_cuda_error(void);
 
-/* *status = 1 when a wait of a cooperative launch (the training step of small batches, the PPO epoch) at its grid-wide barrier ever ran into its limit on the
- * current device (the pass's results are then undefined), else 0. Synchronous (a device-to-host copy). */
+/* *status = 1 when a wait of a cooperative launch (the training step of small batches, the PPO epoch) at its grid-wide barrier ran into its limit on the
+ * current device (that launch's results are then undefined), else 0. Waits for the device. Until b200rl_device_error_clear, every further call that needs
+ * such a launch returns B200RL_ERR_DEVICE_FLAG; b200rl_device_error_state reports it too. */
 int b200rl_cooperative_pass_status(int* status);
 
 /* Reads (and synchronises for) the library's device-side error word into *state_host: non-zero after a bounded wait
- * inside a tensor-core dense kernel expired (the kernel then left its loops and released its tensor memory instead of
+ * inside a tensor-core dense kernel or at a cooperative launch's barrier expired (the kernel then left its loops and released its tensor memory instead of
  * spinning). The reference has no counterpart (its asserts are no-ops in kernels, utils/assert/operations_cuda.h:17-21). */
 int b200rl_device_error_state(int* state_host);
 /* Sets that word back to zero on the current device (synchronises), so that a later b200rl_device_error_state reports only what happened since. */

@@ -541,20 +541,24 @@ int launch_gemm_tc(const GemmArgs& a, int epilogue, int activation, bool a_kcont
 
 }  // namespace b200rl
 
-namespace b200rl { int mlp_chain_error_get(int* word); int mlp_chain_error_clear(); int mlp_grad_error_get(int* word); int mlp_grad_error_clear(); }     // mlp_chain.cu, mlp_grad.cu
+namespace b200rl {                                                       // mlp_chain.cu, mlp_grad.cu, grid_barrier.cu
+int mlp_chain_error_get(int* word); int mlp_chain_error_clear(); int mlp_grad_error_get(int* word); int mlp_grad_error_clear();
+int grid_barrier_status(unsigned* status); int grid_barrier_clear();
+}
 
 extern "C" int b200rl_device_error_state(int* state_host){
     if(!state_host) return B200RL_ERR_INVALID_ARGUMENT;
     B200RL_CUDA_TRY(cudaMemcpyFromSymbol(state_host, b200rl::g_dense_tc_error, sizeof(int)));
-    int chain = 0, grad = 0;
+    int chain = 0, grad = 0; unsigned barrier = 0;
     int rc = b200rl::mlp_chain_error_get(&chain);
-    if(rc || (rc = b200rl::mlp_grad_error_get(&grad))) return rc;
-    *state_host |= chain | grad;
+    if(rc || (rc = b200rl::mlp_grad_error_get(&grad)) || (rc = b200rl::grid_barrier_status(&barrier))) return rc;
+    *state_host |= chain | grad | (int)barrier;
     return B200RL_OK;
 }
 extern "C" int b200rl_device_error_clear(void){
     const int zero = 0;
     B200RL_CUDA_TRY(cudaMemcpyToSymbol(b200rl::g_dense_tc_error, &zero, sizeof(int)));
-    const int rc = b200rl::mlp_chain_error_clear();
-    return rc ? rc : b200rl::mlp_grad_error_clear();
+    int rc = b200rl::mlp_chain_error_clear();
+    if(rc || (rc = b200rl::mlp_grad_error_clear())) return rc;
+    return b200rl::grid_barrier_clear();
 }

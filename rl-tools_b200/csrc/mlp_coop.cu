@@ -13,20 +13,12 @@
 // Bound by latency. Measured, 4-256-256-1 at batch 256 in a captured graph: 18 us (one cooperative launch with grid barriers between the layers 24 us: a
 // barrier costs more than a graph's next node, and two such launches take turns on the SMs).
 #include "common.cuh"
-#include "grid_barrier.cuh"
 #include <cstdlib>
-#include <mutex>
-#include <vector>
 
 namespace b200rl {
 
 constexpr int CO_T = 32, CO_KC = 256, CO_THREADS = 256, CO_WARPS = 8;
 constexpr size_t CO_SMEM = sizeof(float) * 2 * CO_KC * CO_T;          // both operand tiles; the eight partial tiles (32 KB) reuse the space
-// Barrier words per device, handed out round-robin per launch (a captured launch keeps the slot it got at capture time). Two launches may
-// share a slot as long as they never run at the same time: launches on one stream never do, and the parallel branches of one captured graph
-// get consecutive slots. What is not supported: two launches whose slots coincide after a wrap of the ring (4,096 launches apart) running
-// concurrently on different streams.
-constexpr int CO_SLOTS = 4096;
 
 struct CoopGemm {                    // C(m, n) = sum_k A(m, k) B(n, k)
     const float* A; const float* B; float* C; const float* aux;
@@ -41,8 +33,6 @@ struct CoopPhase {
 };
 constexpr int CO_MAX_LAYERS = 4, CO_MAX_PHASES = CO_MAX_LAYERS + 1;
 struct CoopArgs { int n_phases; CoopPhase phase[CO_MAX_PHASES]; };
-
-static __device__ unsigned g_coop_barriers[CO_SLOTS * 4];                 // per slot: arrivals, exits, status (sticky), unused
 
 // Operand tiles, brought in by asynchronous copies in the order in which they lie in memory (zeros outside the operand):
 //   summed index contiguous: [row][256], 16-byte pieces swizzled by the row, read four summed indices at a time
@@ -196,25 +186,6 @@ bool mlp_coop_eligible(const b200rl_mlp_shape* sh, int batch){
     return true;
 }
 
-int grid_barrier_slots(int count, unsigned** out){
-    static unsigned* base[MAX_DEVICES] = {};
-    static unsigned next[MAX_DEVICES] = {};
-    static std::mutex mutex;
-    int dev = 0;
-    int rc = current_device(&dev);
-    if(rc) return rc;
-    std::lock_guard<std::mutex> lock(mutex);
-    if(base[dev] == nullptr){
-        void* p = nullptr;
-        B200RL_CUDA_TRY(cudaGetSymbolAddress(&p, g_coop_barriers));
-        base[dev] = static_cast<unsigned*>(p);
-    }
-    if(next[dev] + (unsigned)count > (unsigned)CO_SLOTS) next[dev] = 0;
-    *out = base[dev] + 4 * next[dev];
-    next[dev] += (unsigned)count;
-    return B200RL_OK;
-}
-
 static void set_tiles(CoopGemm& g){ g.tiles_n = (g.N + CO_T - 1) / CO_T; g.tiles = ((g.M + CO_T - 1) / CO_T) * g.tiles_n; }
 
 static int coop_launch(CoopArgs& a, cudaStream_t s){
@@ -271,16 +242,3 @@ int mlp_coop_backward(const b200rl_mlp_shape* sh, const float* params, float* gr
 }
 
 }  // namespace b200rl
-
-// 0: no barrier of a whole-pass launch on the current device ever ran into its limit
-extern "C" int b200rl_cooperative_pass_status(int* status){
-    using namespace b200rl;
-    if(!status) return B200RL_ERR_INVALID_ARGUMENT;
-    void* p = nullptr;
-    B200RL_CUDA_TRY(cudaGetSymbolAddress(&p, g_coop_barriers));
-    std::vector<unsigned> host(CO_SLOTS * 4);
-    B200RL_CUDA_TRY(cudaMemcpy(host.data(), p, host.size() * sizeof(unsigned), cudaMemcpyDeviceToHost));
-    *status = 0;
-    for(int i = 0; i < CO_SLOTS; i++) if(host[4 * i + 2] != 0u) *status = 1;
-    return B200RL_OK;
-}

@@ -19,7 +19,7 @@ struct TeamStepArgs {
     b200rl_adam_hyper hyper;
     const float* x; const float* target; int ldx, ldt;
     float* pre; float* out;
-    float4* partial; unsigned* barrier;
+    float4* partial; GridBarrier barrier;
     int rows, chunk_rows, n_total, optimize, row_tiles, teams, lanes;
     float constant;                          // 2 / (rows of a chunk x columns) x loss weight, evaluated like the reference does
     int stage_x, stage_y, y_off, out_off;    // shared-memory offsets: next tile's rows as they come, this tile's targets and outputs
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
     if(tid == 0){ grid_barrier_arrive(a.barrier); s_ok = grid_barrier_wait(a.barrier, gridDim.x); }
     else if(a.optimize && (tid == 32 || tid == 33)) s_scalars[tid - 32] = adam_bias_correction(tid == 32 ? a.hyper.beta_1 : a.hyper.beta_2, age);
     __syncthreads();
-    if(!s_ok) return;
+    if(!s_ok){ if(tid == 0) grid_barrier_leave(a.barrier, gridDim.x); return; }
     const float c1 = s_scalars[0], c2 = s_scalars[1];
     struct Moments { float p, m, v; };
     auto prefetch = [&](int i){ return a.optimize && i >= 0 ? Moments{a.params[i], a.m[i], a.v[i]} : Moments{0.0f, 0.0f, 0.0f}; };
@@ -243,7 +243,7 @@ int mlp_team_step(const b200rl_mlp_shape* sh, float* params, float* grads, float
     const int quads = c.C * c.net.n_tiles * 4, threads = c.teams * c.C * THREADS;
     a.lanes = 4;
     while(a.lanes < 32 && 2 * a.lanes <= c.teams && (long long)quads * 2 * a.lanes <= threads) a.lanes *= 2;
-    int rc = grid_barrier_slots(1, &a.barrier);
+    int rc = grid_barriers(1, s, &a.barrier);
     if(rc) return rc;
     if(c.C == 1) return launch_team_step_c<1>(a, c.smem, s);
     if(c.C == 2) return launch_team_step_c<2>(a, c.smem, s);

@@ -20,7 +20,7 @@ struct PpoNetArgs {
     Net net;
     float* params; float* grads; float* m; float* v; uint32_t* adam_state;
     b200rl_adam_hyper hyper;
-    float4* partial; float* partial_std; unsigned* barrier;
+    float4* partial; float* partial_std; GridBarrier barrier;
     int ctas, teams, lanes, row_tiles;
     int stage_x, stage_aux, aux, out;        // shared memory: next rows and columns as they come, this tile's columns ([4][R] behind actions [R][S]), outputs [R][S]
 };
@@ -202,7 +202,7 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
         target += (unsigned)w.ctas;
         if(tid == 0){ grid_barrier_arrive(w.barrier); s_ok = grid_barrier_wait(w.barrier, target); }
         __syncthreads();
-        if(!s_ok) return;
+        if(!s_ok) break;
         const float c1 = s_scalars[0][mb & 63], c2 = s_scalars[1][mb & 63];
         {
             float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -248,10 +248,11 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
         target += (unsigned)w.ctas;
         if(tid == 0){ grid_barrier_arrive(w.barrier); s_ok = grid_barrier_wait(w.barrier, target); }
         __syncthreads();
-        if(!s_ok) return;
+        if(!s_ok) break;
         if(has_rows){ load_weights<L>(n, smem, w.params, 0); load_std(); }
     }
     copies_wait();
+    if(!s_ok){ if(tid == 0) grid_barrier_leave(w.barrier, (unsigned)w.ctas); return; }
     if(index >= 0){ w.m[index] = my_m; w.v[index] = my_v; w.grads[index] = my_g; }
     if(cta == 0 && tid == 0){
         const int last_mb = (a.minibatches - 1) & 63;
@@ -370,11 +371,11 @@ extern "C" int b200rl_ppo_train_epoch(const b200rl_mlp_shape* actor, const b200r
     a.epsilon_clip = epsilon_clip; a.entropy_coefficient = entropy_coefficient; a.advantage_epsilon = advantage_epsilon;
     a.neg_log_sqrt_pi = (float)(-0.5 * (double)logf(2.0f * 3.14159265358979323846f));
     a.normalize_advantage = normalize_advantage; a.learn_action_std = learn_action_std;
-    unsigned* bars = nullptr;
-    int rc = grid_barrier_slots(2, &bars);
-    if(rc) return rc;
-    a.actor.barrier = bars; a.critic.barrier = bars + 4;
     cudaStream_t s = (cudaStream_t)stream;
+    GridBarrier bars[2];
+    int rc = grid_barriers(2, s, bars);
+    if(rc) return rc;
+    a.actor.barrier = bars[0]; a.critic.barrier = bars[1];
     if(normalize_advantage){
         ppo_epoch_stats_kernel<<<n_minibatches, 1024, 0, s>>>(advantages, ld, batch, stats);
         B200RL_LAUNCH_CHECK("ppo_epoch_stats");

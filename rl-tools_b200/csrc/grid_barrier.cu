@@ -4,21 +4,24 @@
 
 namespace b200rl {
 
-// Two launches may use one barrier as long as they never run at the same time. Launches take theirs round-robin (a captured one keeps it for its replays): for two
-// of them to meet, one would have to run while BARRIER_RING others are issued and the last of them runs.
-constexpr unsigned BARRIER_RING = 16384;
-static __device__ unsigned g_barriers[BARRIER_RING * 4];
+// Two launches may use one barrier as long as they never run at the same time. Launches outside a capture take theirs round-robin: for two of them to meet, one
+// would have to wait on its stream while BARRIER_RING others are issued and the last of them runs. A captured launch keeps its barrier for every replay, beside
+// whatever runs then, so it gets one that nobody else is given; when those are used up, the caller takes the kernels that need none.
+constexpr unsigned BARRIER_RING = 16384, BARRIER_CAPTURED = 16384;
+static __device__ unsigned g_barriers[(BARRIER_RING + BARRIER_CAPTURED) * 4];
 
 namespace {
-struct DeviceBarriers { unsigned* words; unsigned* status_host; unsigned* status; unsigned next; };
+struct DeviceBarriers { unsigned* words; unsigned* status_host; unsigned* status; unsigned next, next_captured; };
 DeviceBarriers g_device[MAX_DEVICES] = {};
 std::mutex g_mutex;
 }
 
-int grid_barriers(int count, cudaStream_t, GridBarrier* out){
+int grid_barriers(int count, cudaStream_t stream, GridBarrier* out){
     int dev = 0;
     int rc = current_device(&dev);
     if(rc) return rc;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    B200RL_CUDA_TRY(cudaStreamIsCapturing(stream, &capture));
     std::lock_guard<std::mutex> lock(g_mutex);
     DeviceBarriers& d = g_device[dev];
     if(d.words == nullptr){
@@ -36,9 +39,17 @@ int grid_barriers(int count, cudaStream_t, GridBarrier* out){
         d.words = static_cast<unsigned*>(words);
     }
     if(*static_cast<volatile unsigned*>(d.status_host) != 0u) return B200RL_ERR_DEVICE_FLAG;
-    if(d.next + (unsigned)count > BARRIER_RING) d.next = 0;
-    const unsigned first = d.next;
-    d.next += (unsigned)count;
+    unsigned first = 0;
+    if(capture == cudaStreamCaptureStatusNone){
+        if(d.next + (unsigned)count > BARRIER_RING) d.next = 0;
+        first = d.next;
+        d.next += (unsigned)count;
+    }
+    else{
+        if(d.next_captured + (unsigned)count > BARRIER_CAPTURED) return B200RL_ERR_UNSUPPORTED;
+        first = BARRIER_RING + d.next_captured;
+        d.next_captured += (unsigned)count;
+    }
     for(int i = 0; i < count; i++) out[i] = GridBarrier{d.words + 4 * (first + i), d.status};
     return B200RL_OK;
 }

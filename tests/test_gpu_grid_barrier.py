@@ -1,5 +1,5 @@
 """The grid-wide barrier of the cooperative launches: a wait that runs into its limit is reported, leaves the barrier clean for its next launch and stops
-the calls that need one until it is cleared."""
+the calls that need one until it is cleared; captured launches share no barrier with the others."""
 import ctypes as C
 
 import pytest
@@ -88,3 +88,34 @@ def test_the_kernels_that_wait_at_one_leave_no_status(lib, I, dims, batch):
         net.train_step(torch.randn(batch, I, device="cuda"), torch.randn(batch, dims[-1], device="cuda"))
     _epoch(lib, _network(lib, extra=1), _network(lib))
     assert _status(lib) == (0, 0)
+
+
+def test_replays_beside_more_launches_than_there_are_barriers_to_hand_round(lib):
+    """A graph keeps the barrier of its capture. Its replays run beside 20,000 launches on another stream, more than the ring that those take theirs from; both
+    networks end up where they do alone."""
+    import torch
+    x, y = torch.randn(256, 4, device="cuda"), torch.randn(256, 1, device="cuda")
+    side, results = torch.cuda.Stream(), []
+    for together in (False, True):
+        torch.manual_seed(1)
+        a, b = _network(lib), _network(lib)
+        a.train_step(x, y)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            a.train_step(x, y)
+        torch.cuda.synchronize()
+        for k in range(20000):
+            if k % 4 == 0:
+                with torch.cuda.stream(side):
+                    graph.replay()
+                if not together:
+                    torch.cuda.current_stream().wait_stream(side)
+            b.train_step(x, y)
+            if not together and k % 4 == 3:
+                side.wait_stream(torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        results.append([t.clone() for n in (a, b) for t in (n.params, n.m, n.v)])
+        del graph
+    assert _status(lib) == (0, 0)
+    for alone, beside in zip(*results):
+        assert torch.equal(alone, beside)

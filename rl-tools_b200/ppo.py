@@ -38,19 +38,26 @@ def estimate_generalized_advantages(dataset, layout, n_envs, steps, gamma=0.99, 
     return dataset
 
 
-def evaluate_values(critic, dataset, layout):
-    """critic(all observations) -> value column, as the PPO loop does before the advantage estimate
-    (rl/algorithms/ppo/loop/core/operations_generic.h: evaluate(critic, all_observations_privileged, all_values))."""
+def _values_work(critic, n):
+    """Work buffers of evaluate_values for n rows, kept with the critic."""
     import torch
     # As many rows per call as buffers of 32 MB hold, or, below the 8,192 rows from which on one kernel takes any number of them, the 4,096 rows of the
     # kernel for small batches: calls of critic.batch rows are short and many (65,600 rows: 33 of 11 us).
-    n, width = dataset.shape[0], critic.tick.shape[1]
+    width = critic.tick.shape[1]
     chunk = max(critic.batch, min(n, max(1, (1 << 23) // width)) if n >= 8192 else min(n, 4096))
     work = critic.__dict__.setdefault("_values_work", {})
     if work.get("rows") != chunk:
         z = lambda: torch.empty((chunk, width), device=critic.device, dtype=torch.float32)
         work["bytes"] = lib().b200rl_mlp_forward_workspace_bytes(C.byref(critic.shape), chunk)
         work.update(rows=chunk, tick=z(), tock=z(), buffer=torch.empty(max(work["bytes"], 16), device=critic.device, dtype=torch.uint8))
+    return work
+
+
+def evaluate_values(critic, dataset, layout):
+    """critic(all observations) -> value column, as the PPO loop does before the advantage estimate
+    (rl/algorithms/ppo/loop/core/operations_generic.h: evaluate(critic, all_observations_privileged, all_values))."""
+    work = _values_work(critic, dataset.shape[0])
+    n, chunk = dataset.shape[0], work["rows"]
     ld = dataset.stride(0)
     for begin in range(0, n, chunk):
         at = dataset.data_ptr() + 4 * begin * ld
@@ -81,13 +88,27 @@ def _minibatch_update(actor, critic, rows, layout, epsilon_clip=0.2, entropy_coe
 
 
 class MinibatchGraphs:
-    """One captured CUDA graph per minibatch position of a dataset matrix: the ~24 launches of a minibatch update replayed with a
-    single launch. Valid for one (actor, critic, dataset, batch_size) combination; every pointer is baked into the graphs."""
+    """What `train` needs for one (actor, critic, dataset, batch_size) combination, made before its first call: scratch and shuffle buffers, and for networks that
+    the one-launch epoch does not take one captured CUDA graph per minibatch position of the dataset matrix: the ~24 launches of a minibatch update
+    replayed with a single launch. Every pointer is baked into the graphs. Should the epoch decline networks that it takes in general, they are captured then."""
 
     def __init__(self, actor, critic, dataset, layout, n_rows, batch_size, **hyper):
-        import torch
         self.key = (dataset.data_ptr(), n_rows, batch_size)
         self.graphs = []
+        self._capture_arguments = (actor, critic, dataset, layout, n_rows, batch_size, hyper)
+        _values_work(critic, dataset.shape[0])
+        _shuffle(actor, dataset, layout, n_rows)
+        if not _epoch_scratch(actor, critic, dataset, n_rows // batch_size, batch_size)["bytes"]:
+            self._capture()
+
+    def replay(self, b):
+        if not self.graphs:
+            self._capture()
+        self.graphs[b].replay()
+
+    def _capture(self):
+        import torch
+        actor, critic, dataset, layout, n_rows, batch_size, hyper = self._capture_arguments
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         saved = [t.clone() for t in (actor.params, actor.m, actor.v, actor.adam_state, critic.params, critic.m, critic.v, critic.adam_state)]
@@ -103,15 +124,21 @@ class MinibatchGraphs:
             t.copy_(s)                                                                          # the warm-up update is undone
 
 
-def _epoch_call(actor, critic, dataset, layout, n_minibatches, batch_size, epsilon_clip, entropy_coefficient, advantage_epsilon, normalize_advantage, learn_action_std):
-    """All minibatch updates of one epoch as one native call: a function that issues it, made once per train() (an epoch of small networks takes 100 us);
-    None for networks that its kernel does not take."""
+def _epoch_scratch(actor, critic, dataset, n_minibatches, batch_size):
+    """Scratch of the one-launch epoch, kept with the actor; "bytes" is 0 for networks that its kernel does not take."""
     import torch
     work = actor.__dict__.setdefault("_epoch_scratch", {})
     key = (n_minibatches, batch_size, bytes(actor.shape), bytes(critic.shape))
     if work.get("key") != key:
         n = lib().b200rl_ppo_train_epoch_scratch_bytes(C.byref(actor.shape), C.byref(critic.shape), batch_size, n_minibatches)
         work["key"], work["bytes"], work["buffer"] = key, n, torch.empty(n, device=dataset.device, dtype=torch.uint8) if n else None
+    return work
+
+
+def _epoch_call(actor, critic, dataset, layout, n_minibatches, batch_size, epsilon_clip, entropy_coefficient, advantage_epsilon, normalize_advantage, learn_action_std):
+    """All minibatch updates of one epoch as one native call: a function that issues it, made once per train() (an epoch of small networks takes 100 us);
+    None for networks that its kernel does not take."""
+    work = _epoch_scratch(actor, critic, dataset, n_minibatches, batch_size)
     if not work["bytes"]:
         return None
     base, ld = dataset.data_ptr(), dataset.stride(0)
@@ -132,29 +159,44 @@ def _epoch_call(actor, critic, dataset, layout, n_minibatches, batch_size, epsil
 
 class _Shuffle:
     """The epoch shuffle: the next epoch's permutation is drawn and sent, on a stream of its own and into the other of two buffers, while this one's kernels
-    run (a copy in the stream of the kernels held the epoch up by 25 to 40 us). Pinned memory comes from torch's pool, which waits for copies under way."""
+    run (a copy in the stream of the kernels held the epoch up by 25 to 40 us). Both pairs of buffers, device and pinned, are kept: the host draws into a
+    pinned one once the copy out of it, two epochs before, has completed."""
 
     def __init__(self, dataset, n_rows, columns):
         import torch
         self.n_rows, self.columns, self.epoch = n_rows, columns, 0
         self.scratch = _permute_rows_scratch(dataset, n_rows, columns)
         self.perm = torch.empty((2, n_rows), device=dataset.device, dtype=torch.int32)
+        self.host = torch.empty((2, n_rows), dtype=torch.int32, pin_memory=True)
         self.used = [torch.cuda.current_stream().record_event()] * 2
+        self.sent = [None, None]
         self.stream = torch.cuda.Stream(device=dataset.device)
 
     def __call__(self, dataset, rng_state):
         import torch
         main, k = torch.cuda.current_stream(), self.epoch & 1
-        host = torch.empty(self.n_rows, dtype=torch.int32, pin_memory=True)
-        _shuffle_permutation_host(rng_state, self.n_rows, host.data_ptr())
+        if self.sent[k] is not None:
+            self.sent[k].synchronize()
+        _shuffle_permutation_host(rng_state, self.n_rows, self.host[k].data_ptr())
         with torch.cuda.stream(self.stream):
             self.stream.wait_event(self.used[k])
-            self.perm[k].copy_(host, non_blocking=True)
-            ready = self.stream.record_event()
-        main.wait_event(ready)
+            self.perm[k].copy_(self.host[k], non_blocking=True)
+            self.sent[k] = self.stream.record_event()
+        main.wait_event(self.sent[k])
         _permute_rows(dataset, self.n_rows, self.perm[k], self.columns, self.scratch)
         self.used[k] = main.record_event()
         self.epoch += 1
+
+
+def _shuffle(actor, dataset, layout, n_rows):
+    """The shuffle of the columns that an update reads, kept with the actor."""
+    columns = list(range(layout.observations.start, layout.observations.stop)) + list(range(layout.actions.start, layout.actions.stop)) + \
+        [layout.action_log_probs, layout.advantages, layout.target_values]
+    key, work = (dataset.device, n_rows, tuple(columns)), actor.__dict__.setdefault("_shuffle", {})
+    if key not in work:
+        work.clear()
+        work[key] = _Shuffle(dataset, n_rows, columns)
+    return work[key]
 
 
 def _train_epoch(*networks_and_sizes, **hyper):
@@ -172,28 +214,20 @@ def train(actor, critic, dataset, layout, n_rows, batch_size, n_epochs=10, epsil
     layers), `critic` an Mlp with one output; both built for batch_size rows. An epoch is one native call where its kernel takes the networks
     (small ones: up to three layers and about 18,000 parameters); otherwise graphs = a MinibatchGraphs built for these arguments replays each
     minibatch update as one CUDA graph launch instead of ~24 kernel launches (same kernels, same results)."""
-    import torch
     assert actor.batch == batch_size and critic.batch == batch_size and actor.n_extra == layout.action_dim
     hyper = dict(epsilon_clip=epsilon_clip, entropy_coefficient=entropy_coefficient, advantage_epsilon=advantage_epsilon,
                  normalize_advantage=normalize_advantage, learn_action_std=learn_action_std)
     if graphs is not None:
         assert graphs.key == (dataset.data_ptr(), n_rows, batch_size), "graphs were captured for another dataset matrix"
-    shuffled = list(range(layout.observations.start, layout.observations.stop)) + list(range(layout.actions.start, layout.actions.stop)) + \
-        [layout.action_log_probs, layout.advantages, layout.target_values]
     epoch = _epoch_call(actor, critic, dataset, layout, n_rows // batch_size, batch_size, **hyper)
-    if shuffle_rng_state is not None:
-        key, work = (dataset.device, n_rows, tuple(shuffled)), actor.__dict__.setdefault("_shuffle", {})
-        if key not in work:
-            work.clear()
-            work[key] = _Shuffle(dataset, n_rows, shuffled)
-        shuffle = work[key]
+    shuffle = _shuffle(actor, dataset, layout, n_rows) if shuffle_rng_state is not None else None
     for _ in range(n_epochs):
-        if shuffle_rng_state is not None:
+        if shuffle is not None:
             shuffle(dataset, shuffle_rng_state)
         if epoch is not None and epoch():
             continue
         for b in range(n_rows // batch_size):
             if graphs is not None:
-                graphs.graphs[b].replay()
+                graphs.replay(b)
             else:
                 _minibatch_update(actor, critic, dataset[b * batch_size:(b + 1) * batch_size], layout, **hyper)

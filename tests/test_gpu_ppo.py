@@ -279,3 +279,51 @@ def test_ppo_loop_learns_the_pendulum(lib, torch):
     first, last = float(np.mean(returns[:3])), float(np.mean(returns[-5:]))
     print(f"PPO loop: mean episode return {first:.0f} -> {last:.0f} over {len(returns)} iterations; log_std {loop.actor.extra('params').item():.3f}")
     assert first < -900 and last > -700 and last > first + 400
+
+
+def _update_pair(lib, torch, hidden, batch, rows, seed):
+    """An actor and a critic with 5 observations and 2 actions, and a dataset matrix for them, all from the seed."""
+    from rl_tools_b200 import ppo
+    layout = ppo.DatasetLayout(5, 2)
+    gen = torch.Generator(device="cuda"); gen.manual_seed(seed)
+    acts = ["tanh", "tanh", "identity"]
+    actor, critic = lib.Mlp(5, [hidden, hidden, 2], acts, batch, extra_params=2), lib.Mlp(5, [hidden, hidden, 1], acts, batch)
+    for net in (actor, critic):
+        net.params.copy_((torch.rand(net.params.shape, device="cuda", generator=gen) - 0.5) * 0.2)
+    dataset = torch.randn((rows + 64, layout.data_dim), device="cuda", generator=gen)
+    dataset[:, layout.action_log_probs] -= 2
+    dataset[:, layout.terminated:layout.reset + 1] = 0
+    return actor, critic, dataset, layout
+
+
+def test_minibatch_graphs_captured_late(lib, torch):
+    """Networks that the epoch kernel takes have no graphs, until one is asked for: it does what the separate launches do."""
+    from rl_tools_b200 import ppo
+    batch, rows, results = 256, 1024, []
+    for use_graphs in (False, True):
+        actor, critic, dataset, layout = _update_pair(lib, torch, 64, batch, rows, 4)
+        graphs = ppo.MinibatchGraphs(actor, critic, dataset, layout, rows, batch)
+        assert graphs.graphs == []
+        for b in range(rows // batch):
+            if use_graphs:
+                graphs.replay(b)
+            else:
+                ppo._minibatch_update(actor, critic, dataset[b * batch:(b + 1) * batch], layout)
+        results.append([t.clone() for t in (actor.params, actor.m, actor.v, critic.params, critic.m, critic.v)])
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
+def test_first_ppo_update_of_a_new_pair_allocates_nothing(lib, torch):
+    """What an update needs is made with its MinibatchGraphs: the first one takes no memory, on the device or pinned."""
+    from rl_tools_b200 import ppo
+    batch, rows = 256, 1024
+    actor, critic, dataset, layout = _update_pair(lib, torch, 64, batch, rows, 6)
+    graphs = ppo.MinibatchGraphs(actor, critic, dataset, layout, rows, batch)
+    rng = lib.rng_init_host(1)
+    counts = lambda: (torch.cuda.memory_stats()["allocation.all.allocated"], torch.cuda.host_memory_stats()["allocations.allocated"])
+    before = counts()
+    ppo.evaluate_values(critic, dataset, layout)
+    ppo.estimate_generalized_advantages(dataset, layout, 64, rows // 64)
+    ppo.train(actor, critic, dataset, layout, rows, batch, n_epochs=10, shuffle_rng_state=rng, graphs=graphs)
+    assert counts() == before

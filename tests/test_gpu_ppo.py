@@ -296,6 +296,20 @@ def _update_pair(lib, torch, hidden, batch, rows, seed):
     return actor, critic, dataset, layout
 
 
+def test_ppo_train_graph_replay_of_networks_beyond_the_epoch_kernel(lib, torch):
+    """Networks that the one-launch epoch does not take: the captured minibatch graphs leave behind the bits that the separate launches do."""
+    from rl_tools_b200 import ppo
+    batch, rows, results = 256, 1024, []
+    for use_graphs in (False, True):
+        actor, critic, dataset, layout = _update_pair(lib, torch, 256, batch, rows, 3)
+        graphs = ppo.MinibatchGraphs(actor, critic, dataset, layout, rows, batch) if use_graphs else None
+        assert ppo._epoch_scratch(actor, critic, dataset, rows // batch, batch)["bytes"] == 0 and (graphs is None or len(graphs.graphs) == rows // batch)
+        ppo.train(actor, critic, dataset, layout, rows, batch, n_epochs=3, shuffle_rng_state=lib.rng_init_host(5), graphs=graphs)
+        results.append([t.clone() for t in (actor.params, actor.m, actor.v, critic.params, critic.m, critic.v, dataset)])
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
 def test_minibatch_graphs_captured_late(lib, torch):
     """Networks that the epoch kernel takes have no graphs, until one is asked for: it does what the separate launches do."""
     from rl_tools_b200 import ppo

@@ -341,3 +341,28 @@ def test_first_ppo_update_of_a_new_pair_allocates_nothing(lib, torch):
     ppo.estimate_generalized_advantages(dataset, layout, 64, rows // 64)
     ppo.train(actor, critic, dataset, layout, rows, batch, n_epochs=10, shuffle_rng_state=rng, graphs=graphs)
     assert counts() == before
+
+
+@pytest.mark.parametrize("pitch", [1, 13])
+@pytest.mark.parametrize("N,steps,kernel", [(4095, 16, "gae_kernel"), (4096, 16, "gae_many"), (4097, 17, "gae_kernel"), (8191, 33, "gae_kernel"), (8192, 256, "gae_many"),
+                                            (8193, 257, "gae_kernel"), (20001, 3, "gae_many"), (8192, 1, "gae_many")])
+def test_gae_of_many_environments(lib, orc, torch, N, steps, kernel, pitch):
+    """A thread per environment and a CTA per environment, on both sides of the line between them: the oracle's bits."""
+    from graph_kernels import kernels
+    rng = np.random.default_rng(N + steps)
+    rows = (steps + 1) * N
+    values, rewards = rng.normal(size=rows).astype(np.float32), rng.normal(size=rows).astype(np.float32)
+    terminated = (rng.random(rows) < 0.05).astype(np.uint8)
+    truncated = ((rng.random(rows) < 0.05) | (terminated == 1)).astype(np.uint8)
+    columns = [dev(torch, a.astype(np.float32)) for a in (rewards, values, terminated, truncated)] + [torch.zeros(rows, device="cuda") for _ in range(2)]
+    if pitch > 1:
+        matrix = torch.zeros(rows, pitch, device="cuda")
+        for k, c in enumerate(columns):
+            matrix[:, k] = c
+        columns = [matrix[:, k] for k in range(6)]
+    n = steps * N
+    call = lambda: lib.gae(*columns[:4], N, steps, advantages=columns[4][:n], target_values=columns[5][:n])
+    assert [kernel in name for name in kernels(call)] == [True]
+    call()
+    adv, tgt = orc.gae(rewards[:n], values, terminated[:n], truncated[:n], N, steps)
+    assert np.array_equal(columns[4][:n].cpu().numpy(), adv) and np.array_equal(columns[5][:n].cpu().numpy(), tgt)

@@ -622,9 +622,9 @@ int mlp_team_step(const b200rl_mlp_shape* sh, float* params, float* grads, float
                   const float* x, int ldx, const float* target, int ldt, int rows, int chunk_rows, float loss_weight, float* pre, float* out, void* scratch, size_t scratch_bytes,
                   int optimize, cudaStream_t s);
 
-// backward pass of wide networks at small batches, a launch per layer (mlp_coop.cu)
-bool mlp_coop_eligible(const b200rl_mlp_shape* sh, int batch);
-int mlp_coop_backward(const b200rl_mlp_shape* sh, const float* params, float* grads, const float* x, int ldx, const float* pre, const float* out,
+// backward pass of wide networks at small batches, a launch per layer (mlp_phase.cu)
+bool mlp_phase_eligible(const b200rl_mlp_shape* sh, int batch);
+int mlp_phase_backward(const b200rl_mlp_shape* sh, const float* params, float* grads, const float* x, int ldx, const float* pre, const float* out,
                       float* d_out, float* d_input, float* tick, float* tock, int batch, cudaStream_t s);
 
 static bool valid_shape(const b200rl_mlp_shape* sh){
@@ -829,7 +829,7 @@ int b200rl_mlp_backward(const b200rl_mlp_shape* sh, const float* params, float* 
     // small batches: the whole pass in two launches, when the caller's scratch has room for the gradients of all layers
     if(mlp_fused_eligible(sh, batch) && scratch && scratch_bytes >= mlp_fused_backward_scratch_bytes(sh, batch))
         return mlp_fused_backward(sh, params, grads, x, ldx, pre, out, d_out, d_input, batch, scratch, scratch_bytes, (cudaStream_t)stream);
-    if(mlp_coop_eligible(sh, batch)) return mlp_coop_backward(sh, params, grads, x, ldx, pre, out, d_out, d_input, tick, tock, batch, (cudaStream_t)stream);
+    if(mlp_phase_eligible(sh, batch)) return mlp_phase_backward(sh, params, grads, x, ldx, pre, out, d_out, d_input, tick, tock, batch, (cudaStream_t)stream);
     size_t poff[B200RL_MAX_LAYERS], aoff[B200RL_MAX_LAYERS]; int Is[B200RL_MAX_LAYERS];
     { size_t po = 0, ao = 0; int I = sh->input_dim;
       for(int l = 0; l < L; l++){ poff[l] = po; aoff[l] = ao; Is[l] = I; po += (size_t)sh->dims[l] * I + sh->dims[l]; ao += (size_t)batch * sh->dims[l]; I = sh->dims[l]; } }

@@ -259,9 +259,9 @@ def test_mlp_backward_large_batch_against_the_oracle(lib, orc, torch, hidden_act
     (512, 300, [512, 260], ["fast_tanh", "identity"]),              # two chunks of the summed index, the largest batch and width
 ])
 def test_mlp_backward_in_one_cooperative_launch(lib, orc, torch, B, I, dims, acts):
-    """Wide networks at small batches take the backward pass as one cooperative launch (phases with grid-wide barriers): parameter
-    gradients on top of existing values and the input gradient against the oracle's per-layer recursion; the input-gradient-only pass;
-    two passes in a row give the same bits (the partial tiles are added in a fixed order); no barrier wait ran into its limit."""
+    """The backward pass of wide networks at small batches (a launch per layer): parameter gradients on top of existing values and the input
+    gradient against the oracle's per-layer recursion; the input-gradient-only pass; two passes in a row give the same bits (the partial tiles are
+    added in a fixed order); no barrier of another launch ran into its limit (the pass itself has none)."""
     import ctypes
     shape = oracle.MlpShape.make(I, dims, acts)
     params = mg.det_uniform(91, shape.num_params()) * np.float32(0.1)

@@ -415,12 +415,20 @@ class Mlp:
         self.adam_state = torch.zeros(4, device=device, dtype=torch.int32)
         nbytes = lib().b200rl_mlp_backward_scratch_bytes(C.byref(self.shape), batch)
         self.scratch_bytes = nbytes
-        self.scratch = torch.empty(max(nbytes, 4), device=device, dtype=torch.uint8)
+        # the scratch of large batches (0.8 GB for 64-256-256-256-16 from 2^18 rows on) is for those that train: it is made with the first backward pass
+        self._scratch = torch.empty(max(nbytes, 4), device=device, dtype=torch.uint8) if nbytes <= 1 << 26 else None
         # forward workspace: the weights' tensor-core operand image of the layer in flight (0 bytes for small batches)
         self.workspace_bytes = lib().b200rl_mlp_forward_workspace_bytes(C.byref(self.shape), batch)
         self.workspace = torch.empty(max(self.workspace_bytes, 16), device=device, dtype=torch.uint8)
         self.hyper = AdamHyper()
         self.reset_optimizer_state()
+
+    @property
+    def scratch(self):
+        if self._scratch is None:
+            import torch
+            self._scratch = torch.empty(self.scratch_bytes, device=self.device, dtype=torch.uint8)
+        return self._scratch
 
     def extra(self, arena="params"):
         """View of the extra parameters (or their gradient / moments) behind the layers."""

@@ -154,3 +154,18 @@ def test_weights_far_below_the_largest_of_their_layer(lib, rows, I, dims):
             assert float(((net.grads[poff:poff + o * i].view(o, i).double() - d.T @ x.double()).abs() / size).max()) <= 2e-6
         d = d @ weights[l]
     close(d_input, d, products=len(dims))
+
+
+def test_a_network_that_only_evaluates_holds_no_backward_scratch(lib):
+    """64-256-256-256-16 at 2^18 rows: 0.8 GB that only the backward pass uses."""
+    import torch
+    rows, dims = 1 << 18, [256, 256, 256, 16]
+    before = torch.cuda.memory_allocated()
+    net = lib.Mlp(64, dims, ["relu"] * 3 + ["identity"], rows)
+    x = torch.zeros(rows, 64, device="cuda")
+    net.evaluate(x)
+    net.forward(x)
+    arenas = sum(t.numel() * t.element_size() for t in (net.params, net.grads, net.m, net.v, net.tick, net.tock, net.pre, net.out, net.workspace, x))
+    assert net.scratch_bytes > 1 << 29 and torch.cuda.memory_allocated() - before < arenas + (1 << 26)
+    net.backward(x, torch.zeros(rows, 16, device="cuda"))
+    assert net.scratch.numel() == net.scratch_bytes

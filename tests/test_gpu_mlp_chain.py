@@ -169,3 +169,29 @@ def test_a_network_that_only_evaluates_holds_no_backward_scratch(lib):
     assert net.scratch_bytes > 1 << 29 and torch.cuda.memory_allocated() - before < arenas + (1 << 26)
     net.backward(x, torch.zeros(rows, 16, device="cuda"))
     assert net.scratch.numel() == net.scratch_bytes
+
+
+def test_bias_gradients_of_many_rows(lib):
+    """2^18 rows in one chunk: a bias gradient sums 12,500 of them per CTA. In sums of 256 values and sums of those it loses what the d_pre themselves lack, 3e-7
+    in all; 6e-7 leaves room for other seeds (one running sum: 1.2e-6)."""
+    import torch
+    rows, I, dims, acts = 1 << 18, 64, [256, 256, 256, 16], ["tanh", "tanh", "tanh", "identity"]
+    net = lib.Mlp(I, dims, acts, rows)
+    gen = torch.Generator(device="cuda"); gen.manual_seed(3)
+    off, fan_in = 0, I
+    for d in dims:
+        n = d * fan_in + d
+        net.params[off:off + n] = (torch.rand(n, device="cuda", generator=gen) * 2 - 1) / fan_in ** 0.5
+        off += n; fan_in = d
+    x, d_out = torch.randn(rows, I, device="cuda", generator=gen), torch.randn(rows, dims[-1], device="cuda", generator=gen) / rows
+    net.forward(x)
+    net.zero_gradient()
+    net.backward(x, d_out.clone())
+    d, poff, aoff = d_out.double(), net.n_mlp, net.pre.numel()
+    for l in range(len(dims) - 1, -1, -1):
+        o, i = dims[l], dims[l - 1] if l else I
+        poff -= o * i + o; aoff -= rows * o
+        d = d * DERIVATIVE[acts[l]](net.pre[aoff:aoff + rows * o].view(rows, o).double())
+        want = d.sum(0)
+        assert float((net.grads[poff + o * i:poff + o * i + o].double() - want).norm() / want.norm()) <= 6e-7
+        d = d @ net.params[poff:poff + o * i].double().view(o, i)

@@ -1,8 +1,8 @@
 """The on-policy training loop around the path: state, init and step of rl/algorithms/ppo/loop/core (operations_generic.h:20-58 malloc,
 :66-85 init, :88-131 step) for the Pendulum, composed of the library's pieces -- nothing in a step leaves the GPU except the statistics the
 caller asks for. One `step()` = collect (fused actor inference + environment steps into the dataset matrix), the critic's values of all
-observations, generalized advantage estimation, `train` (epochs x minibatches of the clipped-surrogate update, each minibatch one CUDA-graph
-replay). Observation normalisation (NORMALIZE_OBSERVATIONS) is off, as in the loop's default parameters (config.h:42-43); the
+observations, generalized advantage estimation, `train` (epochs x minibatches of the clipped-surrogate update, an epoch in one launch for the networks that its
+kernel takes, else a CUDA-graph replay per minibatch). Observation normalisation (NORMALIZE_OBSERVATIONS) is off, as in the loop's default parameters (config.h:42-43); the
 RunningNormalizer / standardize pieces exist separately (rl_tools_b200.RunningNormalizer).
 
 Randomness: initial weights and the epoch shuffles come from the reference-compatible host engine (so a loop seeded like the reference's

@@ -127,31 +127,10 @@ __global__ void __launch_bounds__(GR_THREADS, 1) mlp_grad_kernel(const __grid_co
         for(int p = 0; p < 8; p++)
 #pragma unroll
             for(int i = 0; i < 8; i++) acc[p][i] = zero;
-        // this range's record
-        auto store_record = [&](bool add){
-            const int r = 32 * q + lane;
-            if(r >= M) return;
-            float* to = a.partial + split * a.record + y.at + r * y.stride_m;
-#pragma unroll
-            for(int p = 0; p < 8; p++){
-                float old[16];
-#pragma unroll
-                for(int i = 0; i < 16; i++){ const int c = 16 * (2 * p + g) + i; old[i] = add && c < N ? to[c * y.stride_n] : 0.0f; }
-#pragma unroll
-                for(int i = 0; i < 16; i++){ const int c = 16 * (2 * p + g) + i; if(c < N) to[c * y.stride_n] = add ? old[i] + (i & 1 ? acc[p][i >> 1].y : acc[p][i >> 1].x) : (i & 1 ? acc[p][i >> 1].y : acc[p][i >> 1].x); }
-            }
-        };
-        const int segment = (units + (units + GR_SEGMENT - 1) / GR_SEGMENT - 1) / max(1, (units + GR_SEGMENT - 1) / GR_SEGMENT);
-        bool add = a.accumulate != 0;
-        for(int d = 0, next = segment; d < units; d++){
-            if(d == next){
-                store_record(add);
-                add = true; next += segment;
-#pragma unroll
-                for(int p = 0; p < 8; p++)
-#pragma unroll
-                    for(int i = 0; i < 8; i++) acc[p][i] = zero;
-            }
+        const int segments = (units + GR_SEGMENT - 1) / GR_SEGMENT, segment = (units + segments - 1) / max(1, segments);
+        for(int begin = 0; ; begin += segment){
+        const int end = min(units, begin + segment);
+        for(int d = begin; d < end; d++){
             if(!wait(acc_full + (d & 1), (d >> 1) & 1u)) break;
             tc::fence_after_thread_sync();
             const float* inverse = scales + (d % GR_SCALE_BUFFERS) * GR_SCALES;
@@ -175,7 +154,30 @@ __global__ void __launch_bounds__(GR_THREADS, 1) mlp_grad_kernel(const __grid_co
             __syncwarp();
             if(lane == 0) tc::mbar_arrive(acc_empty + (d & 1));
         }
-        store_record(add);
+        // ---- this range's record ----
+        if(32 * q + lane < M){
+            float* to = a.partial + split * a.record + y.at + (32 * q + lane) * y.stride_m;
+            const bool add = begin > 0 || a.accumulate;
+#pragma unroll
+            for(int p = 0; p < 8; p++){
+                if(16 * (2 * p + g) >= N) break;
+                float old[16];                                           // all of them asked for before the first store
+#pragma unroll
+                for(int i = 0; i < 16; i++){ const int c = 16 * (2 * p + g) + i; old[i] = add && c < N ? to[c * y.stride_n] : 0.0f; }
+#pragma unroll
+                for(int i = 0; i < 16; i++){
+                    const int c = 16 * (2 * p + g) + i;
+                    const float v = i & 1 ? acc[p][i >> 1].y : acc[p][i >> 1].x;
+                    if(c < N) to[c * y.stride_n] = add ? old[i] + v : v;
+                }
+            }
+        }
+        if(end >= units || *abort_flag) break;
+#pragma unroll
+        for(int p = 0; p < 8; p++)
+#pragma unroll
+            for(int i = 0; i < 8; i++) acc[p][i] = zero;
+        }
     }
     else if(warp >= GR_SUM_WARPS + GR_STAGING_WARPS){
         tc::setmaxnreg_dec<24>();

@@ -588,7 +588,8 @@ __global__ void __launch_bounds__(1024) chain_image_kernel(const __grid_constant
 //   evaluate            4-256-256-1 at 2,048: 24 and 34; 64-256-16 at 2,048 (42): 17 and 15, at 4,096 (84): 18 and 28; 8-256-4 at 8,192 (25): 14 and 13, at 16,384
 //                       (50): 15 and 20; 64-128-4 at 8,192 (71): 15 and 13, at 16,384 (143): 15 and 17; 3-32-32-1 at 8,192 (9): 13 and 12, at 16,384 (19): 13 and 15
 //   forward             33-200-200-7 at 2,048 (98): 38 and 28, at 4,096 (197): 38 and 39; 64-256-256-256-16 at 2,048 (310): 54 and 60; 27-64-64-8 at 8,192 (52): 18 and 17;
-//                       3-64-64-1 at 16,384 (71): 19 and 24; 3-32-32-1 at 65,536 (75): 50 and 41; 64-128-4 at 65,536 (570): 56 and 49
+//                       3-64-64-1 at 16,384 (71): 19 and 24; 20-32-32-32-8 at 16,384 (48): 25 and 33; 3-50-50-1 at 16,384 (44): 23 and 29; 3-32-32-1 at 65,536
+//                       (75): 50 and 41; 64-128-4 at 65,536 (570): 56 and 49
 //   gradients           17-130-130-3 at 4,096 (80): 59 and 50, at 8,192 (160): 67 and 94; 33-200-200-7 at 2,048 (98): 61 and 66; 64-256-16 at 8,192 (168): 42 and 38, at
 //                       16,384: 48 and 47; 256-256-256 at 2,048: 59 and 83; 64-128-4 at 8,192: 33 and 27, at 16,384: 37 and 40; 10-16-2 at 16,384 (3): 32 and 27
 //   input gradient alone  17-130-130-3 at 2,048 (40): 29 and 18, at 4,096 (80): 29 and 35; 8-256-4 at 4,096 (13): 24 and 16, at 8,192: 22 and 98
@@ -605,7 +606,7 @@ bool mlp_chain_takes(const b200rl_mlp_shape* sh, int batch, int pass){
     const long long million = 1000000, work = weights * batch;
     switch(pass){
         case CHAIN_EVALUATE: return two ? work >= (wide ? 50 : 72) * million : wide || work >= 16 * million;
-        case CHAIN_FORWARD: return two ? wide && work >= 50 * million : wide ? batch >= 4096 || work >= 200 * million : weights >= 4096 && work >= 64 * million;
+        case CHAIN_FORWARD: return two ? wide && work >= 50 * million : wide ? batch >= 4096 || work >= 200 * million : weights >= 2048 && (batch >= 16384 || work >= 64 * million);
         case CHAIN_GRADIENTS: return two ? weights >= 32768 || (batch >= 16384 && (wide || weights >= 4096)) : !wide || work >= 90 * million;
         default: return batch >= 8192 || work >= 80 * million;
     }

@@ -35,7 +35,8 @@ def _chain(names):
     (4096, 33, [200, 200, 7], True, True, True, True), (2048, 17, [130, 130, 3], True, False, False, False), (8192, 17, [130, 130, 3], True, True, True, True),
     (4096, 64, [256, 16], True, True, False, True), (8192, 8, [256, 4], False, False, False, True), (16384, 8, [256, 4], True, True, True, True), (16384, 64, [256], False, False, False, False),
     (8191, 27, [64, 64, 8], False, False, False, False), (8192, 27, [64, 64, 8], True, False, True, True), (16384, 27, [64, 64, 8], True, True, True, True),
-    (8192, 64, [64, 4], False, False, False, True), (65536, 64, [64, 4], True, False, True, True)])
+    (8192, 64, [64, 4], False, False, False, True), (16384, 20, [32, 32, 32, 8], True, True, True, True), (65536, 4, [32, 32, 15], True, False, True, True),
+    (65536, 64, [64, 4], True, False, True, True)])
 def test_passes_of_a_network_take_the_chain_kernels_where_those_are_faster(lib, rows, I, dims, evaluate, forward, gradients, d_input):
     import torch
     net = _network(lib, rows, I, dims)

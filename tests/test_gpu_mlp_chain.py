@@ -1,5 +1,6 @@
-"""All layers of a forward pass in one tensor-core kernel against fp64: the least rows it serves, rows that fill no tile of 128, more row tiles than
-SMs, widths on both sides of the 64-column pieces and of the 128-column stacking, one and eight layers, strided and unaligned operands."""
+"""All layers of a forward pass in one tensor-core kernel against fp64, and the passes that take the kernels per layer beside it (test_gpu_dispatch.py says which):
+the least rows it serves, rows that fill no tile of 128, more row tiles than SMs, widths on both sides of the 64-column pieces and of the 128-column
+stacking, one to eight layers, strided and unaligned operands."""
 import numpy as np
 import pytest
 
@@ -107,7 +108,7 @@ def test_backward_matches_fp64(lib, rows, I, dims, acts, mode):
         assert float((err - 1e-5 * size).max()) <= 1e-6 / rows
 
 
-@pytest.mark.parametrize("rows,I,dims", [(2048, 64, [256, 256, 16]), (2100, 200, [130, 129]), (8192, 27, [64, 64, 8]), (8200, 100, [33, 128, 7])])
+@pytest.mark.parametrize("rows,I,dims", [(2048, 64, [256, 256, 16]), (4099, 64, [256, 256, 16]), (2100, 200, [130, 129]), (8192, 27, [64, 64, 8]), (16390, 27, [64, 64, 8]), (8200, 100, [33, 128, 7])])
 def test_weights_far_below_the_largest_of_their_layer(lib, rows, I, dims):
     """Every third output of a layer has weights 2^-24 of the layer's largest, and so has every third input (a column, which is an output of the
     backward chain): each output column, input-gradient column and gradient row is as close to fp64 as its own size asks for. Two fp16 parts hold 22 bits

@@ -21,11 +21,12 @@ struct TeamStepArgs {
     float* pre; float* out;
     float4* partial; GridBarrier barrier;
     int rows, chunk_rows, n_total, optimize, row_tiles, teams, lanes;
+    Divisor by_S;
     float constant;                          // 2 / (rows of a chunk x columns) x loss weight, evaluated like the reference does
-    int stage_x, stage_y, y_off, out_off;    // shared-memory offsets: next tile's rows as they come, this tile's targets and outputs
+    int y_off, y_alt, out_off;               // shared-memory offsets: targets of a tile, distance of the next tile's, outputs
 };
 
-template <int C, int L, int TPT>
+template <int C, int L, int N, int PO, int PI>
 __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_constant__ TeamStepArgs a){
     extern __shared__ __align__(16) float smem[];
     __shared__ float s_scalars[2];
@@ -34,57 +35,66 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
     const int tid = threadIdx.x, rank = C == 1 ? 0 : (int)cluster_rank(), t = blockIdx.x / C;
     const Layer& last = n.layer[L - 1];
     const int I0 = n.layer[0].I, R = n.R;
-    auto stage = [&](int tile){              // the tile's input rows and this CTA's target columns, zero beyond the batch
-        const int row0 = tile * R;
-        for(int i = tid; i < R * I0; i += THREADS){
-            const int r = quotient(i, n.by_I0), k = i - r * I0;
-            if(row0 + r < a.rows) copy4_async(smem + a.stage_x + i, a.x + (size_t)(row0 + r) * a.ldx + k);
-            else smem[a.stage_x + i] = 0.0f;
+    auto stage = [&](int tile, bool other){  // the tile's input rows and this CTA's target columns, zero beyond the batch
+        const int row0 = tile * R, P = n.layer[0].P;
+        float* rows = smem + n.layer[0].a + (other ? n.a_alt : 0);
+        if(((I0 | a.ldx) & 3) == 0 && (reinterpret_cast<uintptr_t>(a.x) & 15u) == 0){
+#pragma unroll 1
+            for(int i = tid; i < R * (I0 >> 2); i += THREADS){
+                const int r = quotient(i, n.layer[0].by_row), k = 4 * (i - r * (I0 >> 2));
+                if(row0 + r < a.rows) copy16_async(rows + r * P + k, a.x + (size_t)(row0 + r) * a.ldx + k);
+                else *reinterpret_cast<float4*>(rows + r * P + k) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
         }
+        else{
+#pragma unroll 1
+            for(int i = tid; i < R * I0; i += THREADS){
+                const int r = quotient(i, n.by_I0), k = i - r * I0;
+                if(row0 + r < a.rows) copy4_async(rows + r * P + k, a.x + (size_t)(row0 + r) * a.ldx + k);
+                else rows[r * P + k] = 0.0f;
+            }
+        }
+#pragma unroll 1
         for(int i = tid; i < R * last.S; i += THREADS){
-            const int r = quotient(i, last.by_S), unit = rank * last.S + i - r * last.S;
-            if(row0 + r < a.rows && unit < last.O) copy4_async(smem + a.stage_y + i, a.target + (size_t)(row0 + r) * a.ldt + unit);
+            const int r = quotient(i, a.by_S), unit = rank * last.S + i - r * last.S;
+            if(row0 + r < a.rows && unit < last.O) copy4_async(smem + a.y_off + (other ? a.y_alt : 0) + i, a.target + (size_t)(row0 + r) * a.ldt + unit);
         }
     };
-    stage(t);
     clear_rows<L>(n, smem);
+    __syncthreads();
+    stage(t, false);
     load_weights<L>(n, smem, a.params, rank);
-    Patch patches[TPT];
-    float2 acc[TPT][4][2];
+    Patch patches[N];
+    Sums<N, PO, PI> acc;
 #pragma unroll
-    for(int k = 0; k < TPT; k++){
-        patches[k] = patch<L>(n, k * THREADS + tid);
-#pragma unroll
-        for(int i = 0; i < 4; i++){ acc[k][i][0] = make_float2(0.0f, 0.0f); acc[k][i][1] = make_float2(0.0f, 0.0f); }
-    }
+    for(int k = 0; k < N; k++) patches[k] = patch<L>(n, k * THREADS + tid);
+    clear_sums(acc);
     const int keep_from = a.rows - a.chunk_rows;          // the activations of the last chunk stay behind in pre / out
-    for(int tile = t; tile < a.row_tiles; tile += a.teams){
+    bool other = false;                                   // which of the two buffers this tile's rows are in
+    for(int tile = t; tile < a.row_tiles; tile += a.teams, other = !other){
         copies_wait();
-        __syncthreads();
-        for(int i = tid; i < R * I0; i += THREADS){ const int r = quotient(i, n.by_I0), k = i - r * I0; smem[n.layer[0].a + r * n.layer[0].P + k] = smem[a.stage_x + i]; }
-        for(int i = tid; i < R * last.S; i += THREADS) smem[a.y_off + i] = smem[a.stage_y + i];
-        sync_team<C>();                                   // also: every CTA of the team has set its buffers up before the first remote store
-        if(tile + a.teams < a.row_tiles) stage(tile + a.teams);
+        sync_team<C>();                                   // the rows are there; every CTA of the team has left the previous tile (or set its buffers up)
+        if(tile + a.teams < a.row_tiles) stage(tile + a.teams, !other);
         const int row0 = tile * R;
-#pragma unroll
+        const float* y = smem + a.y_off + (other ? a.y_alt : 0);
+#pragma unroll 1
         for(int l = 0; l < L; l++){
-            const Layer& y = n.layer[l];
-            forward_layer<C, L>(n, l, smem, rank, [&](int r, int unit, int idx, float value, float derivative){
-                if(l == L - 1){
-                    smem[y.d + idx] = row0 + r < a.rows ? __fmul_rn(__fsub_rn(value, smem[a.y_off + idx]), a.constant) * derivative : 0.0f;
-                    smem[a.out_off + idx] = value;
-                }
+            forward_layer<C, L, true>(n, l, n.layer[l].a + (l == 0 && other ? n.a_alt : 0), smem, rank, [&](int r, int unit, float4 value, float4 derivative){
+                const int at = r * last.S + unit;
+                const float4 target = *reinterpret_cast<const float4*>(y + at);
+                auto d = [&](float v, float wanted, float dv){ return row0 + r < a.rows && dv != 0.0f ? __fmul_rn(__fsub_rn(v, wanted), a.constant) * dv : 0.0f; };
+                *reinterpret_cast<float4*>(smem + last.d + at) = make_float4(d(value.x, target.x, derivative.x), d(value.y, target.y, derivative.y), d(value.z, target.z, derivative.z), d(value.w, target.w, derivative.w));
+                *reinterpret_cast<float4*>(smem + a.out_off + at) = value;
             });
             if(l == L - 1) __syncthreads();
             else sync_team<C>();
         }
-#pragma unroll
+#pragma unroll 1
         for(int l = L - 1; l > 0; l--) backward_layer<C>(n, l, smem, rank, (L - l) & 1);
         store_activations<L>(n, smem, smem + a.out_off, rank, row0, a.rows, keep_from, a.chunk_rows, a.pre, a.out);
-        accumulate_gradients<TPT>(n, smem, patches, acc);
-        sync_team<C>();
+        accumulate_gradients<N, PO, PI>(n, smem, patches, acc, other);
     }
-    store_gradients<C, TPT>(n, a.partial + (size_t)t * C * n.n_tiles * 4, rank, acc);
+    store_gradients<N, PO, PI>(n, a.partial + (size_t)t * C * n.quads, rank, acc);
     __syncthreads();
     const uint32_t age = a.optimize ? *reinterpret_cast<volatile uint32_t*>(a.adam_state) : 1u;
     if(tid == 0){ grid_barrier_arrive(a.barrier); s_ok = grid_barrier_wait(a.barrier, gridDim.x); }
@@ -110,7 +120,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------------------------------
-struct TeamChoice { Net net; int C, teams, row_tiles, stage_x, stage_y, y_off, out_off; size_t smem; };
+struct TeamChoice { Net net; int C, teams, row_tiles, y_off, y_alt, out_off; size_t smem; };
 
 constexpr size_t TEAM_SMEM = 220 * 1024;
 constexpr int TEAM_MAX_ROWS = 8192;          // what was measured; up to there the caller asks for steps of little work only (dense.cu)
@@ -118,9 +128,9 @@ constexpr int TEAM_MAX_ROWS = 8192;          // what was measured; up to there t
 // teams of C CTAs that are resident at once on the current device (clusters do not tile every GPC completely); 0: unknown
 static int team_capacity(int C);
 
-// Team size and rows per tile by an estimate of the launch in clock cycles, with constants from timelines of the kernel (64- and 256-wide networks,
-// batches of 256 ... 5,003): a layer of a tile costs its latencies (about 2,000 cycles over both directions, twice that where the team exchanges
-// through cluster barriers) plus its products at a third of the multiply-add peak; loading the weights and adding the teams' sums cost per float.
+// Team size and rows per tile by an estimate of the launch: a layer of a tile costs its latencies (twice as much where the team exchanges through cluster barriers) and its
+// products, loading the weights and storing and adding the teams' sums cost per float. The constants, in no unit but their own, are fitted to all teams and tiles of 24 shapes (32 ... 256
+// wide, 2 to 4 layers, 32 ... 8,192 rows): 22 choices within 2 % of the fastest, the worst 7 % off (8-64-64-64-4 at 64 rows: 17.7 and 16.6 us).
 // Only plans whose sums fit into scratch_bytes: the scratch of a smaller batch serves a larger one, by its own plan or a better one that fits.
 static bool choose_team(const b200rl_mlp_shape* sh, int rows, size_t scratch_bytes, TeamChoice* out){
     for(int l = 0, I = sh->input_dim; l < sh->n_layers; I = sh->dims[l], l++) if(sh->dims[l] > 512 || I > 512) return false;
@@ -130,26 +140,25 @@ static bool choose_team(const b200rl_mlp_shape* sh, int rows, size_t scratch_byt
         if(max_teams < 1) continue;
         for(int R = 4; R <= 32; R += 4){
             TeamChoice c{};
-            if(!plan(sh, C, R, 0, &c.net)) continue;
+            if(!plan(sh, C, R, 0, true, 0, &c.net)) continue;
             c.C = C;
             const Layer& last = c.net.layer[c.net.n_layers - 1];
             int off = (c.net.end + 3) / 4 * 4;
-            c.stage_x = off; off += (R * sh->input_dim + 3) / 4 * 4;
-            c.stage_y = off; off += R * last.S;
-            c.y_off = off; off += R * last.S;
+            c.y_off = off; c.y_alt = R * last.S; off += 2 * R * last.S;
             c.out_off = off; off += R * last.S;
             c.smem = sizeof(float) * (size_t)off;
             if(c.smem > TEAM_SMEM) continue;
             c.row_tiles = (rows + R - 1) / R;
             c.teams = c.row_tiles < max_teams ? c.row_tiles : max_teams;
-            if(sizeof(float4) * (size_t)c.teams * c.C * c.net.n_tiles * 4 > scratch_bytes) continue;
+            if(sizeof(float4) * (size_t)c.teams * c.C * c.net.quads > scratch_bytes) continue;
             double weights = 0.0, tile = 0.0;
             for(int l = 0; l < c.net.n_layers; l++){
                 const Layer& y = c.net.layer[l];
                 weights += (double)y.S * y.P;
-                tile += (C == 1 ? 2000.0 : 4000.0) + 3.0 * R * y.S * y.P / 42.0;
+                tile += (C == 1 ? 3800.0 : 7700.0) + 0.12 * R * y.S * y.P;
             }
-            const double cost = 0.15 * weights + tile * ((c.row_tiles + c.teams - 1) / c.teams) + 64.0 * C * c.net.n_tiles * c.teams / (12.0 * c.teams * C);
+            double cost = 0.15 * weights + tile * ((c.row_tiles + c.teams - 1) / c.teams) + 1.8 * c.net.quads + 0.0016 * C * c.net.quads * c.teams;
+            if(c.net.n_patches > THREADS) cost *= 1.5;                   // two patches a thread do not fit its registers (64-256-256-256-16 at 1,024 rows: 146 us, 102 with teams of eight)
             if(best == 0.0 || cost < best){ best = cost; *out = c; }
         }
     }
@@ -160,7 +169,7 @@ static bool choose_team(const b200rl_mlp_shape* sh, int rows, size_t scratch_byt
 size_t mlp_team_scratch_bytes(const b200rl_mlp_shape* sh, int rows){
     TeamChoice c;
     if(rows < 1 || !choose_team(sh, rows, SIZE_MAX, &c)) return 0;
-    return sizeof(float4) * (size_t)team_capacity(c.C) * c.C * c.net.n_tiles * 4;
+    return sizeof(float4) * (size_t)team_capacity(c.C) * c.C * c.net.quads;
 }
 
 static void team_attributes(cudaLaunchAttribute (&attr)[2], int C){
@@ -174,8 +183,8 @@ static int query_capacity(){
     cudaLaunchAttribute attr[2];
     team_attributes(attr, C);
     cfg.gridDim = dim3(NUM_SMS / C * C); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = TEAM_SMEM; cfg.attrs = attr; cfg.numAttrs = 1;
-    if(cudaFuncSetAttribute(mlp_team_step_kernel<C, 3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TEAM_SMEM) != cudaSuccess ||
-       cudaOccupancyMaxActiveClusters(&n, mlp_team_step_kernel<C, 3, 1>, &cfg) != cudaSuccess){ cudaGetLastError(); return 0; }
+    if(cudaFuncSetAttribute(mlp_team_step_kernel<C, 3, 1, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TEAM_SMEM) != cudaSuccess ||
+       cudaOccupancyMaxActiveClusters(&n, mlp_team_step_kernel<C, 3, 1, 1, 1>, &cfg) != cudaSuccess){ cudaGetLastError(); return 0; }
     return n;
 }
 static int team_capacity(int C){
@@ -191,30 +200,29 @@ static int team_capacity(int C){
     return n - 1;
 }
 
-template <int C, int L, int TPT>
+template <int C, int L, int N, int PO, int PI>
 static int launch_team_step(const TeamStepArgs& a, size_t smem, cudaStream_t s){
     static std::atomic<bool> configured[MAX_DEVICES];
     int dev = 0;
     int rc = current_device(&dev);
     if(rc) return rc;
     if(!configured[dev].load(std::memory_order_acquire)){
-        B200RL_CUDA_TRY(cudaFuncSetAttribute(mlp_team_step_kernel<C, L, TPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TEAM_SMEM));
+        B200RL_CUDA_TRY(cudaFuncSetAttribute(mlp_team_step_kernel<C, L, N, PO, PI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TEAM_SMEM));
         configured[dev].store(true, std::memory_order_release);
     }
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[2];
     team_attributes(attr, C);
     cfg.gridDim = dim3(a.teams * C); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = s; cfg.attrs = attr; cfg.numAttrs = 2;
-    B200RL_CUDA_TRY(cudaLaunchKernelEx(&cfg, mlp_team_step_kernel<C, L, TPT>, a));
+    B200RL_CUDA_TRY(cudaLaunchKernelEx(&cfg, mlp_team_step_kernel<C, L, N, PO, PI>, a));
     return B200RL_OK;
 }
 template <int C, int L>
 static int launch_team_step_l(const TeamStepArgs& a, size_t smem, cudaStream_t s){
-    const int per_thread = (a.net.n_tiles + THREADS - 1) / THREADS;
-    if(per_thread <= 1) return launch_team_step<C, L, 1>(a, smem, s);
-    if(per_thread <= 2) return launch_team_step<C, L, 2>(a, smem, s);
-    if(per_thread <= 4) return launch_team_step<C, L, 4>(a, smem, s);
-    return launch_team_step<C, L, 8>(a, smem, s);
+    if(a.net.n_patches > THREADS) return launch_team_step<C, L, 2, 2, 2>(a, smem, s);
+    if(a.net.patch_i == 2) return launch_team_step<C, L, 1, 2, 2>(a, smem, s);
+    if(a.net.patch_o == 2) return launch_team_step<C, L, 1, 2, 1>(a, smem, s);
+    return launch_team_step<C, L, 1, 1, 1>(a, smem, s);
 }
 template <int C>
 static int launch_team_step_c(const TeamStepArgs& a, size_t smem, cudaStream_t s){
@@ -238,9 +246,9 @@ int mlp_team_step(const b200rl_mlp_shape* sh, float* params, float* grads, float
     a.partial = static_cast<float4*>(scratch);
     a.rows = rows; a.chunk_rows = chunk_rows; a.n_total = (int)n_total; a.optimize = optimize; a.row_tiles = c.row_tiles; a.teams = c.teams;
     a.constant = 2.0f / ((float)chunk_rows * (float)sh->dims[sh->n_layers - 1]) * loss_weight;
-    a.stage_x = c.stage_x; a.stage_y = c.stage_y; a.y_off = c.y_off; a.out_off = c.out_off;
+    a.y_off = c.y_off; a.y_alt = c.y_alt; a.out_off = c.out_off; a.by_S = divisor(c.net.layer[c.net.n_layers - 1].S);
     // threads per quad of the reduction: as many as let the grid take all quads in one pass, no more than there are sums to add
-    const int quads = c.C * c.net.n_tiles * 4, threads = c.teams * c.C * THREADS;
+    const int quads = c.C * c.net.quads, threads = c.teams * c.C * THREADS;
     a.lanes = 4;
     while(a.lanes < 32 && 2 * a.lanes <= c.teams && (long long)quads * 2 * a.lanes <= threads) a.lanes *= 2;
     int rc = grid_barriers(1, s, &a.barrier);

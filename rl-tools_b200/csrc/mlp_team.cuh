@@ -10,93 +10,118 @@
 //     (distributed shared memory), one cluster barrier per layer;
 //   - backward: the input gradient is a sum over the units, i.e. over the team: each CTA forms the partial sums of its own units for all inputs
 //     and stores each part into the CTA that owns that input, which adds the parts in a fixed order;
-//   - parameter gradients: 4 x 4 patches per thread, in registers over all row tiles of the launch. The bias is column I of the weight row
-//     (its input is the constant 1 in column I of the activation rows), so it needs no code of its own in either direction.
-// Every product runs as 4 x 4 register tiles on packed multiply-adds with 16-byte shared-memory operands; where a product has fewer tiles than
-// the CTA has threads, the summed index is split over thread groups and the parts are added in group order.
+//   - parameter gradients: a patch of 4, 8 outputs x 4, 8 inputs per thread, in registers over all row tiles of the launch. The bias is column I of the
+//     weight row (its input is the constant 1 in column I of the activation rows).
+// A product of a layer is 4 x 4 register tiles with 16-byte shared-memory operands; the summed index of a tile is shared out over 1 ... 16 lanes of ONE warp, which
+// add their parts by shuffles and go on with what follows the product (bias, activation, derivative; derivative of the layer below) on the sums in
+// their registers: nothing but finished rows passes through shared memory, and a layer is one phase with one barrier behind it.
 // Teams write their gradient sums to scratch memory; after a grid-wide barrier all CTAs share out the parameters, add the teams' sums in a fixed
 // order and apply the optimizer step.
 //
-// Loops over elements and layers stay rolled: a minibatch walks the whole code once, and what does not fit the instruction caches is fetched anew for every one of
-// them (PPO epoch kernel 220 -> 108 KB of code: 27-64-64-8, 2,048 rows 22.4 -> 20.3 us per minibatch).
+// Bound by shared-memory reads: a 16-byte read takes 4 cycles of an SM for a warp, 2 where all lanes of each half-phase read the same, so a 4 x 4 x 4 step costs 24 cycles of
+// reads against 16 of multiply-adds; eight lanes in a row share the tile's rows (2 cycles) and read eight weight rows an odd number of 16 bytes apart
+// (4 cycles, no conflicts). Patches of 8 x 8 read 12 cycles for 32 of multiply-adds.
+//
+// Loops over elements stay rolled: a minibatch walks the whole code once, and what does not fit the instruction caches is fetched anew for every one of them.
+// Measured against products whose parts met in shared memory, element-wise passes behind them, 256 threads: 4-256-256-1 at 256 rows 28.7 -> 24.6 us a training step, 33-200-200-7 at 5,003 rows
+// 121 -> 103, PPO epochs of 27-64-64-8 with 2,048 rows 20.3 -> 15.9 us per minibatch. Packed multiply-adds (two per instruction) were slower here: 135 us for the second one, because the pairs
+// take twice the registers.
 #pragma once
 #include "common.cuh"
 
 namespace b200rl { namespace team {
 
-// 256 threads: a tile of a few rows is bound by the latency of its phases and by instruction issue (address arithmetic around short products), which
-// more warps only repeat. Measured with 512: 64-wide networks 12.8 -> 15.7 us per step at batch 512, 18.1 -> 19.8 us at batch 2,048.
-constexpr int THREADS = 256, MAX_LAYERS = 4, MAX_TILES_PER_THREAD = 8;
+// Four warps per scheduler: with the products' sums in registers until they are finished, more warps hide the shared-memory latencies.
+// (Half as many for networks without work for more, by a number in the plan instead of a constant: no faster there, 3 to 8 % slower elsewhere.)
+constexpr int THREADS = 512, WARPS = THREADS / 32, MAX_LAYERS = 4, MAX_PATCHES_PER_THREAD = 2;
 
-// quotient by a divisor known on the host (both below 2^16): one multiplication instead of a division's ~40 instructions, which on the path of a
+// quotient by a divisor known on the host (n d < 2^32): one multiplication instead of a division's ~40 instructions, which on the path of a
 // few microseconds per layer would be most of the time
 struct Divisor { unsigned m; };
 inline Divisor divisor(int d){ return Divisor{d <= 1 ? 0u : (unsigned)((0x100000000ull + (unsigned)d - 1) / (unsigned)d)}; }
 
 struct Layer {
     int O, I, act;
-    int S;                      // units per CTA (multiple of 4)
+    int S;                      // units per CTA (multiple of 4); unit u's weight row lies at row (u & 3) S / 4 + u / 4, so that the four units of a tile are S / 4 rows apart
     int P;                      // pitch of weight and activation rows in floats: I + 1 rounded up to four, an odd number of 16-byte pieces
-    int K4;                     // 16-byte pieces of a row that hold data
+    int K4;                     // 16-byte pieces of the summed index of a forward product (with the bias column, unless that starts a piece of its own)
     long long poff, aoff;       // offset in the parameter arena (weights, then bias), in the activation arenas (x batch)
     int w, a, p, g, d;          // shared-memory offsets (floats): weight rows [S][P], input rows [R][P]; [R][S]: pre-activations, activation derivatives, d_pre
-    int fwd_threads, fwd_groups, bwd_threads, bwd_groups;      // threads of one pass over all tiles, groups that share out the summed index
-    int tile_begin, tiles_i;    // gradient patches: first index of this layer, patches along the inputs
-    Divisor by_S, by_S4, by_fwd, by_bwd, by_I, by_row, by_I4, by_tiles_i;
+    int fwd_tiles, fwd_shift, bwd_tiles, bwd_shift;            // 4 x 4 tiles of a product; 2^shift lanes share out its summed index
+    int patch_begin, across;    // gradient patches: first index of this layer, patches along the inputs
+    Divisor by_S4, by_I, by_row, by_I4, by_across, by_owner;
 };
 struct Net {
-    int n_layers, R, n_tiles, n_params;      // n_tiles: gradient patches per CTA
-    Divisor by_tiles, by_I0;
+    int n_layers, R, n_params;
+    int patch_o, patch_i, n_patches, quads;  // a patch is patch_o x patch_i pieces of four (1 x 1, 2 x 1, 2 x 2); patches per CTA; 16-byte pieces of gradient sums per CTA
+    int a_alt;                               // the first layer's second buffer of input rows lies this much behind the first
+    Divisor by_quads, by_patches, by_I0;
     int zero_begin, zero_end;                // weight and input rows of all layers (offsets, multiples of four floats)
-    int rb[2];                               // exchange buffers (offsets); rb_floats each
+    int rb[2];                               // exchange buffers of teams of several CTAs (offsets)
     int end;                                 // end of the network's shared memory (floats)
     Layer layer[MAX_LAYERS];
 };
 
+// lanes that share out the K4 pieces of a tile's summed index, as a power of two: by an estimate in cycles of an SM, reads or latencies of the steps, then the exchange
+// and what follows the product (a lane keeps 4, 2, 1 of the tile's rows)
+inline int lanes_of_a_tile(int tiles, int K4){
+    int best = 0; double cost = 0.0;
+    for(int s = 0; s <= 4; s++){
+        const int warps = (tiles + (32 >> s) - 1) / (32 >> s), rounds = (warps + WARPS - 1) / WARPS, steps = (K4 + (1 << s) - 1) >> s, rows = s == 0 ? 4 : s == 1 ? 2 : 1;
+        const double reads = 24.0 * warps * steps, latency = 70.0 * rounds * steps;
+        const double c = (reads > latency ? reads : latency) + rounds * (80.0 * rows + 25.0 * s) + 8.0 * rows * warps;
+        if(s == 0 || c < cost){ best = s; cost = c; }
+    }
+    return best;
+}
+
 // host: lays a network out for teams of C CTAs and R rows per tile, from shared-memory offset `base` on. False: a shape these kernels do not take.
-inline bool plan(const b200rl_mlp_shape* sh, int C, int R, int base, Net* out){
+// `least`: 0, or patches of at least 2 x 1 (1), 2 x 2 (2).
+inline bool plan(const b200rl_mlp_shape* sh, int C, int R, int base, bool keep_pre, int least, Net* out){
     if(sh->n_layers > MAX_LAYERS) return false;
     Net n{};
     n.n_layers = sh->n_layers; n.R = R;
     int I = sh->input_dim, off = base, rb = 0;
     long long po = 0, ao = 0;
-    for(int l = 0, i = sh->input_dim; l < sh->n_layers; i = sh->dims[l], l++){            // what has to start at zero lies together
-        const int S = ((sh->dims[l] + C - 1) / C + 3) / 4 * 4, P = 4 * (((i + 1 + 3) / 4) | 1);
-        n.layer[l].w = off; off += S * P;
-        n.layer[l].a = off; off += R * P;
+    for(int l = 0; l < sh->n_layers; l++){                               // what has to start at zero lies together
+        Layer& y = n.layer[l];
+        y.O = sh->dims[l]; y.I = I; y.act = sh->acts[l];
+        y.S = ((y.O + C - 1) / C + 3) / 4 * 4; y.P = 4 * (((I + 1 + 3) / 4) | 1); y.K4 = (I + 3) / 4;
+        y.w = off; off += y.S * y.P;
+        y.a = off; off += R * y.P;
+        if(l == 0){ n.a_alt = R * y.P; off += R * y.P; }
+        I = y.O;
     }
     n.zero_begin = base; n.zero_end = off;
     for(int l = 0; l < sh->n_layers; l++){
         Layer& y = n.layer[l];
-        y.O = sh->dims[l]; y.I = I; y.act = sh->acts[l];
-        y.S = ((y.O + C - 1) / C + 3) / 4 * 4;
-        y.K4 = (I + 1 + 3) / 4;
-        y.P = 4 * (y.K4 | 1);
         y.poff = po; y.aoff = ao;
-        po += (long long)y.O * I + y.O; ao += y.O;
-        y.p = off; off += R * y.S;
+        po += (long long)y.O * y.I + y.O; ao += y.O;
+        if(keep_pre){ y.p = off; off += R * y.S; }
         y.g = off; off += R * y.S;
         y.d = off; off += R * y.S;
-        y.fwd_threads = (R / 4) * (y.S / 4);
-        y.fwd_groups = 1;
-        while(2 * y.fwd_groups * y.fwd_threads <= THREADS && 4 * y.fwd_groups <= y.K4) y.fwd_groups *= 2;
-        if(y.fwd_groups * R * y.S > rb) rb = y.fwd_groups * R * y.S;
-        if(l > 0){
-            y.bwd_threads = (R / 4) * ((I + 3) / 4);
-            y.bwd_groups = 1;
-            while(2 * y.bwd_groups * y.bwd_threads <= THREADS && 2 * y.bwd_groups <= y.S / 4) y.bwd_groups *= 2;
-            const int need = C * y.bwd_groups * R * n.layer[l - 1].S;
-            if(need > rb) rb = need;
-        }
-        y.tile_begin = n.n_tiles; y.tiles_i = y.K4;
-        n.n_tiles += (y.S / 4) * y.tiles_i;
-        y.by_S = divisor(y.S); y.by_S4 = divisor(y.S / 4); y.by_fwd = divisor(y.fwd_threads); y.by_bwd = divisor(l > 0 ? y.bwd_threads : 1); y.by_I4 = divisor((I + 3) / 4);
-        y.by_tiles_i = divisor(y.tiles_i); y.by_I = divisor(I); y.by_row = divisor(I / 4);
-        I = y.O;
+        const int I4 = (y.I + 3) / 4;
+        y.fwd_tiles = (R / 4) * (y.S / 4); y.fwd_shift = lanes_of_a_tile(y.fwd_tiles, y.K4);
+        y.bwd_tiles = (R / 4) * I4; y.bwd_shift = lanes_of_a_tile(y.bwd_tiles, y.S / 4);
+        if(l > 0 && C > 1 && C * R * n.layer[l - 1].S > rb) rb = C * R * n.layer[l - 1].S;
+        y.by_S4 = divisor(y.S / 4); y.by_I4 = divisor(I4); y.by_I = divisor(y.I); y.by_row = divisor(y.I / 4); y.by_owner = divisor(l > 0 ? n.layer[l - 1].S : 1);
     }
-    if(n.n_tiles > MAX_TILES_PER_THREAD * THREADS || off % 4 != 0) return false;
+    // the smallest patch that gives every thread at most one; shapes that exceed the largest patch take two of those
+    bool fits = false;
+    for(int k = least; k < 4 && !fits; k++){
+        n.patch_o = k > 0 ? 2 : 1; n.patch_i = k > 1 ? 2 : 1; n.n_patches = 0;
+        for(int l = 0; l < n.n_layers; l++){
+            Layer& y = n.layer[l];
+            y.patch_begin = n.n_patches; y.across = ((y.I + 1 + 3) / 4 + n.patch_i - 1) / n.patch_i; y.by_across = divisor(y.across);
+            n.n_patches += (y.S / 4 + n.patch_o - 1) / n.patch_o * y.across;
+        }
+        fits = n.n_patches <= (k == 3 ? MAX_PATCHES_PER_THREAD : 1) * THREADS;
+    }
+    if(!fits || off % 4 != 0) return false;
+    n.quads = n.n_patches * n.patch_o * 4 * n.patch_i;
     n.n_params = (int)po;
-    n.by_tiles = divisor(n.n_tiles); n.by_I0 = divisor(sh->input_dim);
+    n.by_quads = divisor(n.quads); n.by_patches = divisor(n.n_patches); n.by_I0 = divisor(sh->input_dim);
+    off += 4;                                                            // a patch at the end of a row reads the piece behind it (into sums that nobody uses)
     n.rb[0] = off; off += rb;
     n.rb[1] = off; off += rb;
     n.end = off;
@@ -106,6 +131,10 @@ inline bool plan(const b200rl_mlp_shape* sh, int C, int R, int base, Net* out){
 
 #ifdef __CUDACC__
 __device__ __forceinline__ int quotient(int n, Divisor d){ return d.m ? (int)__umulhi((unsigned)n, d.m) : n; }
+
+// threadIdx.x, as a value that the compiler does not take out of the loop around: what a thread does in each of the layers, kept from one minibatch to the next, would
+// cost the registers of the gradient sums
+__device__ __forceinline__ int thread_here(){ int t = threadIdx.x; asm volatile("" : "+r"(t)); return t; }
 
 // ---- cluster primitives -----------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_rank(){ uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
@@ -122,8 +151,8 @@ __device__ __forceinline__ void store_remote(float* p, int rank, float v){ asm v
 __device__ __forceinline__ void store_remote(float* p, int rank, float4 v){
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" :: "r"(remote(p, rank)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
-template <int C, typename T> __device__ __forceinline__ void store_to(float* p, int rank, T v){
-    if constexpr(C == 1) *reinterpret_cast<T*>(p) = v;
+template <int C, typename V> __device__ __forceinline__ void store_to(float* p, int rank, V v){
+    if constexpr(C == 1) *reinterpret_cast<V*>(p) = v;
     else store_remote(p, rank, v);
 }
 __device__ __forceinline__ void copy4_async(float* smem, const float* gmem){
@@ -134,14 +163,17 @@ __device__ __forceinline__ void copy16_async(float* smem, const float* gmem){
 }
 __device__ __forceinline__ void copies_wait(){ asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory"); }
 
-// activation and its derivative in one evaluation (the derivatives of nn/activation_functions.h:57-85 in terms of the value)
-__device__ __forceinline__ float activate(float x, int act, float& derivative){
+// activation and its derivative in one evaluation (the derivatives of nn/activation_functions.h:57-85 in terms of the value), on four units
+template <typename F> __device__ __forceinline__ float4 each(float4 x, float4& derivative, F f){
+    return make_float4(f(x.x, derivative.x), f(x.y, derivative.y), f(x.z, derivative.z), f(x.w, derivative.w));
+}
+__device__ __forceinline__ float4 activate(float4 x, int act, float4& derivative){
     switch(act){
-        case B200RL_ACT_IDENTITY: derivative = 1.0f; return x;
-        case B200RL_ACT_RELU: derivative = x > 0.0f ? 1.0f : 0.0f; return x > 0.0f ? x : 0.0f;
-        case B200RL_ACT_TANH: { const float a = tanhf(x); derivative = 1.0f - a * a; return a; }
-        case B200RL_ACT_FAST_TANH: { const float a = fast_tanh_dev(x); derivative = 1.0f - a * a; return a; }
-        default: { const float a = 1.0f / (1.0f + expf(-x)); derivative = a * (1.0f - a); return a; }
+        case B200RL_ACT_IDENTITY: derivative = make_float4(1.0f, 1.0f, 1.0f, 1.0f); return x;
+        case B200RL_ACT_RELU: return each(x, derivative, [](float v, float& d){ d = v > 0.0f ? 1.0f : 0.0f; return v > 0.0f ? v : 0.0f; });
+        case B200RL_ACT_TANH: return each(x, derivative, [](float v, float& d){ const float a = tanhf(v); d = 1.0f - a * a; return a; });
+        case B200RL_ACT_FAST_TANH: return each(x, derivative, [](float v, float& d){ const float a = fast_tanh_dev(v); d = 1.0f - a * a; return a; });
+        default: return each(x, derivative, [](float v, float& d){ const float a = 1.0f / (1.0f + expf(-v)); d = a * (1.0f - a); return a; });
     }
 }
 
@@ -150,10 +182,10 @@ __device__ __forceinline__ float activate(float x, int act, float& derivative){
 template <int L>
 __device__ __forceinline__ void clear_rows(const Net& n, float* smem){
     for(int i = n.zero_begin + 4 * (int)threadIdx.x; i < n.zero_end; i += 4 * THREADS) *reinterpret_cast<float4*>(smem + i) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for(int i = threadIdx.x; i < n.R * n.layer[L - 1].S; i += THREADS) smem[n.layer[L - 1].d + i] = 0.0f;      // columns beyond the output stay zero
     __syncthreads();
 #pragma unroll
     for(int l = 0; l < L; l++) if((int)threadIdx.x < n.R) smem[n.layer[l].a + threadIdx.x * n.layer[l].P + n.layer[l].I] = 1.0f;
+    if((int)threadIdx.x < n.R) smem[n.layer[0].a + n.a_alt + threadIdx.x * n.layer[0].P + n.layer[0].I] = 1.0f;
 }
 // this CTA's weight rows of every layer into shared memory by asynchronous copies; the caller waits for them
 template <int L>
@@ -163,36 +195,80 @@ __device__ __forceinline__ void load_weights(const Net& n, float* smem, const fl
         const Layer& y = n.layer[l];
         const float* W = params + y.poff + (size_t)rank * y.S * y.I;
         float* sw = smem + y.w;
-        const int rows = min(y.S, y.O - rank * y.S);
+        const int rows = min(y.S, y.O - rank * y.S), S4 = y.S >> 2;
         if((y.I & 3) == 0 && (reinterpret_cast<uintptr_t>(W) & 15u) == 0){
             const int q = y.I >> 2;
 #pragma unroll 2
-            for(int i = threadIdx.x; i < rows * q; i += THREADS) copy16_async(sw + 4 * i + quotient(i, y.by_row) * (y.P - y.I), W + 4 * i);
+            for(int i = threadIdx.x; i < rows * q; i += THREADS){
+                const int o = quotient(i, y.by_row), k = i - o * q;
+                copy16_async(sw + ((o & 3) * S4 + (o >> 2)) * y.P + 4 * k, W + 4 * i);
+            }
         }
         else{
 #pragma unroll 2
-            for(int i = threadIdx.x; i < rows * y.I; i += THREADS) copy4_async(sw + i + quotient(i, y.by_I) * (y.P - y.I), W + i);
+            for(int i = threadIdx.x; i < rows * y.I; i += THREADS){
+                const int o = quotient(i, y.by_I), k = i - o * y.I;
+                copy4_async(sw + ((o & 3) * S4 + (o >> 2)) * y.P + k, W + i);
+            }
         }
 #pragma unroll 1
-        for(int o = threadIdx.x; o < rows; o += THREADS) copy4_async(sw + o * y.P + y.I, params + y.poff + (size_t)y.O * y.I + rank * y.S + o);
+        for(int o = threadIdx.x; o < rows; o += THREADS) copy4_async(sw + ((o & 3) * S4 + (o >> 2)) * y.P + y.I, params + y.poff + (size_t)y.O * y.I + rank * y.S + o);
     }
 }
 
-// partial sums of one layer's pre-activations for the CTA's units: exchange buffer [group][R][S]
-__device__ __forceinline__ void forward_products(const Net& n, const Layer& y, const float* smem, float* rb){
-    const int g = quotient(threadIdx.x, y.by_fwd), S4 = y.S >> 2, P4 = y.P >> 2;
-    if(g >= y.fwd_groups) return;
-    for(int t = threadIdx.x - g * y.fwd_threads; t < y.fwd_threads; t += THREADS){           // more than one round only with a single group
-        const int rg = quotient(t, y.by_S4), og = t - rg * S4;      // unit og + S4 j: the weight rows of consecutive lanes lie in different banks
-        const float4* a = reinterpret_cast<const float4*>(smem + y.a) + rg * 4 * P4;
+// the lanes' parts of a 4 x 4 tile are added: v[0 ... rows - 1] of the tile's rows from `first` on stay with a lane (4, 2, 1 of them). Lanes beyond four per tile all
+// get the sums.
+struct Share { int tile, part, first, rows, copy, copies; };     // tile of the round, part of the summed index; kept rows; which of `copies` lanes with the same sums this is
+__device__ __forceinline__ Share share(int shift, int lane){
+    Share s;
+    const int per_warp = 32 >> shift;
+    s.tile = lane & (per_warp - 1); s.part = lane >> (5 - shift);
+    s.first = (shift >= 1 ? (lane >> 3) & 2 : 0) + (shift >= 2 ? (lane >> 3) & 1 : 0);
+    s.rows = shift == 0 ? 4 : shift == 1 ? 2 : 1;
+    s.copies = shift > 2 ? 1 << (shift - 2) : 1; s.copy = s.part & (s.copies - 1);
+    return s;
+}
+__device__ __forceinline__ void add_parts(float4 (&v)[4], int shift, int lane){
+    auto add_to = [](float4& a, float4 b){ a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; };
+    auto exchange = [](float4 a, int mask){
+        return make_float4(__shfl_xor_sync(0xffffffffu, a.x, mask), __shfl_xor_sync(0xffffffffu, a.y, mask), __shfl_xor_sync(0xffffffffu, a.z, mask), __shfl_xor_sync(0xffffffffu, a.w, mask));
+    };
+    if(shift >= 1){
+        const bool upper = lane & 16;
+        const float4 s0 = upper ? v[0] : v[2], s1 = upper ? v[1] : v[3];
+        v[0] = upper ? v[2] : v[0]; v[1] = upper ? v[3] : v[1];
+        add_to(v[0], exchange(s0, 16)); add_to(v[1], exchange(s1, 16));
+    }
+    if(shift >= 2){
+        const bool upper = lane & 8;
+        const float4 s0 = upper ? v[0] : v[1];
+        v[0] = upper ? v[1] : v[0];
+        add_to(v[0], exchange(s0, 8));
+    }
+    if(shift >= 3) add_to(v[0], exchange(v[0], 4));
+    if(shift >= 4) add_to(v[0], exchange(v[0], 2));
+}
+
+// One layer of the forward pass; `a`: where its input rows lie. The values go into the next layer's input rows of the whole team; after the last layer
+// finish(row, first unit, values, derivatives) runs for every row and four units of this CTA (derivatives of units beyond the layer are 0). Ends without a barrier.
+template <int C, int L, bool KEEP_PRE, typename FINISH>
+__device__ __forceinline__ void forward_layer(const Net& n, int l, int a_rows, float* smem, int rank, FINISH finish){
+    const Layer& y = n.layer[l];
+    const int tid = thread_here(), lane = tid & 31, warp = tid >> 5, S4 = y.S >> 2, P4 = y.P >> 2, shift = y.fwd_shift, G = 1 << shift;
+    const Share sh = share(shift, lane);
+#pragma unroll 1
+    for(int t0 = warp << (5 - shift); t0 < y.fwd_tiles; t0 += WARPS << (5 - shift)){
+        const int t = min(t0 + sh.tile, y.fwd_tiles - 1), rg = quotient(t, y.by_S4), og = t - rg * S4;
+        const bool mine = t0 + sh.tile < y.fwd_tiles;
+        const float4* a = reinterpret_cast<const float4*>(smem + a_rows) + rg * 4 * P4;
         const float4* w = reinterpret_cast<const float4*>(smem + y.w) + og * P4;
-        float2 acc[4][4];
+        float acc[4][4];
 #pragma unroll
         for(int i = 0; i < 4; i++)
 #pragma unroll
-            for(int j = 0; j < 4; j++) acc[i][j] = make_float2(0.0f, 0.0f);
-#pragma unroll 2
-        for(int k = g; k < y.K4; k += y.fwd_groups){
+            for(int j = 0; j < 4; j++) acc[i][j] = 0.0f;
+#pragma unroll 1
+        for(int k = sh.part; k < y.K4; k += G){
             float4 xv[4], wv[4];
 #pragma unroll
             for(int i = 0; i < 4; i++) xv[i] = a[i * P4 + k];
@@ -202,47 +278,49 @@ __device__ __forceinline__ void forward_products(const Net& n, const Layer& y, c
             for(int i = 0; i < 4; i++)
 #pragma unroll
                 for(int j = 0; j < 4; j++){
-                    acc[i][j] = __ffma2_rn(make_float2(xv[i].x, xv[i].y), make_float2(wv[j].x, wv[j].y), acc[i][j]);
-                    acc[i][j] = __ffma2_rn(make_float2(xv[i].z, xv[i].w), make_float2(wv[j].z, wv[j].w), acc[i][j]);
+                    acc[i][j] = fmaf(xv[i].x, wv[j].x, acc[i][j]); acc[i][j] = fmaf(xv[i].y, wv[j].y, acc[i][j]);
+                    acc[i][j] = fmaf(xv[i].z, wv[j].z, acc[i][j]); acc[i][j] = fmaf(xv[i].w, wv[j].w, acc[i][j]);
                 }
         }
-        float* dst = rb + (g * n.R + rg * 4) * y.S + og;
+        float4 v[4];
 #pragma unroll
-        for(int i = 0; i < 4; i++)
-#pragma unroll
-            for(int j = 0; j < 4; j++) dst[i * y.S + j * S4] = acc[i][j].x + acc[i][j].y;
-    }
-}
-
-// One layer of the forward pass. epilogue(r, unit, index in [R][S], value, derivative) runs once per row and own unit; the value goes into the
-// next layer's input rows of the whole team (unless this is the last layer). Ends without a barrier.
-template <int C, int L, typename EPILOGUE>
-__device__ __forceinline__ void forward_layer(const Net& n, int l, float* smem, int rank, EPILOGUE epilogue){
-    const Layer& y = n.layer[l];
-    float* rb = smem + n.rb[0];
-    forward_products(n, y, smem, rb);
-    __syncthreads();
-    const int count = n.R * y.S, next_a = l + 1 < L ? n.layer[l + 1].a : 0, next_p = l + 1 < L ? n.layer[l + 1].P : 0;
+        for(int i = 0; i < 4; i++) v[i] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        add_parts(v, shift, lane);
+        if(!mine) continue;                                              // no barrier or exchange below
+        float4 bias = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if((y.I & 3) == 0){                                              // the bias column is not among the pieces summed
+            const float* b = smem + y.w + og * y.P + y.I;
+            bias = make_float4(b[0], b[S4 * y.P], b[2 * S4 * y.P], b[3 * S4 * y.P]);
+        }
+        const int unit = rank * y.S + 4 * og, beyond = unit + 4 - y.O;   // how many of the four units lie beyond the layer
+        float* next = nullptr;
+        if(l + 1 < L) next = smem + n.layer[l + 1].a + unit;
 #pragma unroll 1
-    for(int idx = threadIdx.x; idx < count; idx += THREADS){
-        const int r = quotient(idx, y.by_S), o = idx - r * y.S, unit = rank * y.S + o;
-        float v = rb[idx], dv;
-#pragma unroll 4
-        for(int g = 1; g < y.fwd_groups; g++) v += rb[g * count + idx];
-        const float value = activate(v, y.act, dv);
-        if(unit >= y.O) dv = 0.0f;
-        smem[y.g + idx] = dv;
-        smem[y.p + idx] = v;
-        if(unit < y.O){
+        for(int i = 0; i < sh.rows; i++){
+            const int r = rg * 4 + sh.first + i;
+            const float4 pre = make_float4(v[0].x + bias.x, v[0].y + bias.y, v[0].z + bias.z, v[0].w + bias.w);
+            v[0] = v[1]; v[1] = v[2]; v[2] = v[3];
+            float4 dv;
+            const float4 value = activate(pre, y.act, dv);
+            if(beyond > 0){ dv.w = 0.0f; if(beyond > 1) dv.z = 0.0f; if(beyond > 2) dv.y = 0.0f; if(beyond > 3) dv.x = 0.0f; }
+            const int at = r * y.S + 4 * og;
+            if(sh.copy == 0){
+                *reinterpret_cast<float4*>(smem + y.g + at) = dv;
+                if constexpr(KEEP_PRE) *reinterpret_cast<float4*>(smem + y.p + at) = pre;
+                if(l + 1 == L) finish(r, 4 * og, value, dv);
+            }
             if(l + 1 < L){
-                float* dst = smem + next_a + r * next_p + unit;
-                if constexpr(C == 1) *dst = value;
-                else{
-#pragma unroll
-                    for(int c = 0; c < C; c++) store_remote(dst, c, value);
+                float* dst = next + r * n.layer[l + 1].P;
+#pragma unroll 1
+                for(int c = sh.copy; c < C; c += sh.copies){
+                    if(beyond <= 0) store_to<C>(dst, c, value);
+                    else{
+                        if(beyond < 4) store_to<C>(dst, c, value.x);
+                        if(beyond < 3) store_to<C>(dst + 1, c, value.y);
+                        if(beyond < 2) store_to<C>(dst + 2, c, value.z);
+                    }
                 }
             }
-            epilogue(r, unit, idx, value, dv);
         }
     }
 }
@@ -251,138 +329,193 @@ __device__ __forceinline__ void forward_layer(const Net& n, int l, float* smem, 
 template <int L>
 __device__ __forceinline__ void store_activations(const Net& n, const float* smem, const float* last_out, int rank, int row0, int rows, int keep_from, int stride, float* pre, float* out){
     if(row0 + n.R <= keep_from) return;
-#pragma unroll
+#pragma unroll 1
     for(int l = 0; l < L; l++){
         const Layer& y = n.layer[l];
-        const int count = n.R * y.S;
+        const int S4 = y.S >> 2, count = n.R * S4;
         const size_t base = (size_t)y.aoff * stride;
-        for(int idx = threadIdx.x; idx < count; idx += THREADS){
-            const int r = quotient(idx, y.by_S), unit = rank * y.S + idx - r * y.S, row = row0 + r;
+        const bool quads = (y.O & 3) == 0 && (base & 3) == 0 && ((reinterpret_cast<uintptr_t>(pre) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
+#pragma unroll 2
+        for(int i = threadIdx.x; i < count; i += THREADS){
+            const int r = quotient(i, y.by_S4), og = i - r * S4, unit = rank * y.S + 4 * og, row = row0 + r;
             if(unit >= y.O || row >= rows || row < keep_from) continue;
             const size_t at = base + (size_t)(row - keep_from) * y.O + unit;
-            pre[at] = smem[y.p + idx];
-            out[at] = l + 1 < L ? smem[n.layer[l + 1].a + r * n.layer[l + 1].P + unit] : last_out[idx];
+            const float* p = smem + y.p + 4 * i;
+            const float* o = l + 1 < L ? smem + n.layer[l + 1].a + r * n.layer[l + 1].P + unit : last_out + 4 * i;
+            if(quads){ *reinterpret_cast<float4*>(pre + at) = *reinterpret_cast<const float4*>(p); *reinterpret_cast<float4*>(out + at) = *reinterpret_cast<const float4*>(o); }
+            else for(int k = 0; k < min(4, y.O - unit); k++){ pre[at + k] = p[k]; out[at + k] = o[k]; }
         }
     }
 }
 
-// Input gradient of layer l > 0 from its d_pre (own units): partial sums to the owners of the inputs, then d_pre of layer l - 1 (own units).
-// `turn` alternates between the two exchange buffers.
+// Input gradient of layer l > 0 from its d_pre (own units), then d_pre of layer l - 1 (own units): in teams of several CTAs by way of the owners of the inputs, through
+// one of two exchange buffers (`turn` alternates).
 template <int C>
 __device__ __forceinline__ void backward_layer(const Net& n, int l, float* smem, int rank, int turn){
     const Layer& y = n.layer[l];
     const Layer& z = n.layer[l - 1];
     float* rb = smem + n.rb[turn];
-    const int g = quotient(threadIdx.x, y.by_bwd), I4 = (y.I + 3) >> 2, S4 = y.S >> 2, P4 = y.P >> 2;
-    for(int t = g < y.bwd_groups ? threadIdx.x - g * y.bwd_threads : y.bwd_threads; t < y.bwd_threads; t += THREADS){
-        const int rg = quotient(t, y.by_I4), i4 = t - rg * I4;
+    const int tid = thread_here(), lane = tid & 31, warp = tid >> 5, I4 = (y.I + 3) >> 2, S4 = y.S >> 2, P4 = y.P >> 2, shift = y.bwd_shift, G = 1 << shift;
+    const Share sh = share(shift, lane);
+    auto below = [&](int at, float4 v){                                  // units beyond the layer's width have derivative 0
+        const float4 dv = *reinterpret_cast<const float4*>(smem + z.g + at);
+        *reinterpret_cast<float4*>(smem + z.d + at) = make_float4(dv.x != 0.0f ? v.x * dv.x : 0.0f, dv.y != 0.0f ? v.y * dv.y : 0.0f, dv.z != 0.0f ? v.z * dv.z : 0.0f, dv.w != 0.0f ? v.w * dv.w : 0.0f);
+    };
+#pragma unroll 1
+    for(int t0 = warp << (5 - shift); t0 < y.bwd_tiles; t0 += WARPS << (5 - shift)){
+        const int t = min(t0 + sh.tile, y.bwd_tiles - 1), rg = quotient(t, y.by_I4), i4 = t - rg * I4;
+        const bool mine = t0 + sh.tile < y.bwd_tiles;
         const float4* d = reinterpret_cast<const float4*>(smem + y.d) + rg * 4 * S4;
         const float4* w = reinterpret_cast<const float4*>(smem + y.w) + i4;
-        float2 acc[4][2];
+        float4 v[4];
 #pragma unroll
-        for(int i = 0; i < 4; i++){ acc[i][0] = make_float2(0.0f, 0.0f); acc[i][1] = make_float2(0.0f, 0.0f); }
-#pragma unroll 2
-        for(int o4 = g; o4 < S4; o4 += y.bwd_groups){
+        for(int i = 0; i < 4; i++) v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+        for(int o4 = sh.part; o4 < S4; o4 += G){
             float4 dv[4], wv[4];
 #pragma unroll
             for(int i = 0; i < 4; i++) dv[i] = d[i * S4 + o4];
 #pragma unroll
-            for(int q = 0; q < 4; q++) wv[q] = w[(o4 * 4 + q) * P4];
+            for(int q = 0; q < 4; q++) wv[q] = w[(q * S4 + o4) * P4];
 #pragma unroll
             for(int i = 0; i < 4; i++){
                 const float e[4] = {dv[i].x, dv[i].y, dv[i].z, dv[i].w};
 #pragma unroll
-                for(int q = 0; q < 4; q++){
-                    acc[i][0] = __ffma2_rn(make_float2(e[q], e[q]), make_float2(wv[q].x, wv[q].y), acc[i][0]);
-                    acc[i][1] = __ffma2_rn(make_float2(e[q], e[q]), make_float2(wv[q].z, wv[q].w), acc[i][1]);
-                }
+                for(int q = 0; q < 4; q++) v[i] = make_float4(fmaf(e[q], wv[q].x, v[i].x), fmaf(e[q], wv[q].y, v[i].y), fmaf(e[q], wv[q].z, v[i].z), fmaf(e[q], wv[q].w, v[i].w));
             }
         }
-        const int owner = C == 1 ? 0 : quotient(i4 * 4, z.by_S), col = i4 * 4 - owner * z.S;
-        float* dst = rb + ((rank * y.bwd_groups + g) * n.R + rg * 4) * z.S + col;
-#pragma unroll
-        for(int i = 0; i < 4; i++) store_to<C>(dst + i * z.S, owner, make_float4(acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y));
-    }
-    sync_team<C>();
-    const int count = n.R * z.S, parts = C * y.bwd_groups;
+        add_parts(v, shift, lane);
+        if(!mine || sh.copy != 0) continue;
+        const int owner = C == 1 ? 0 : quotient(i4 * 4, y.by_owner), col = i4 * 4 - owner * z.S;
 #pragma unroll 1
-    for(int idx = threadIdx.x; idx < count; idx += THREADS){
-        const float dv = smem[z.g + idx];
-        float v = 0.0f;
-#pragma unroll 4
-        for(int p = 0; p < parts; p++) v += rb[p * count + idx];
-        smem[z.d + idx] = dv != 0.0f ? v * dv : 0.0f;             // units beyond the layer's width have derivative 0
+        for(int i = 0; i < sh.rows; i++){
+            const int r = rg * 4 + sh.first + i;
+            if constexpr(C == 1) below(r * z.S + col, v[0]);
+            else store_remote(rb + (rank * n.R + r) * z.S + col, owner, v[0]);
+            v[0] = v[1]; v[1] = v[2]; v[2] = v[3];
+        }
+    }
+    if constexpr(C > 1){
+        sync_team<C>();
+        const int count = n.R * z.S;
+#pragma unroll 1
+        for(int at = 4 * threadIdx.x; at < count; at += 4 * THREADS){
+            float4 v = *reinterpret_cast<const float4*>(rb + at);
+#pragma unroll
+            for(int p = 1; p < C; p++){ const float4 t = *reinterpret_cast<const float4*>(rb + p * count + at); v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w; }
+            below(at, v);
+        }
     }
     __syncthreads();
 }
 
-// ---- parameter gradients: thread t owns the patches t, t + THREADS, ... of the CTA's weight rows -------------------------------------------
-struct Patch { int d, a, pitch; };                      // pitch: of the d_pre rows in the low half, of the input rows in the high half
-// layer, output quad and input quad of a patch; tiles ascend over the layers
+// ---- parameter gradients: thread t owns the patch t (and t + THREADS) of the CTA's weight rows ---------------------------------------------
+struct Patch { int d, a, pitch, alt; };                 // pitch: of the d_pre rows in the low half, of the input rows in the high half; alt: distance of the other input buffer
+// layer, first output quad and first input quad of a patch; patches ascend over the layers
 template <int L>
-__device__ __forceinline__ void locate(const Net& n, int tile, int& l, int& o4, int& i4){
+__device__ __forceinline__ void locate(const Net& n, int at, int& l, int& o4, int& i4){
     l = 0;
 #pragma unroll
-    for(int k = 1; k < L; k++) if(tile >= n.layer[k].tile_begin) l = k;
-    int begin = n.layer[0].tile_begin, tiles_i = n.layer[0].tiles_i; Divisor by = n.layer[0].by_tiles_i;
+    for(int k = 1; k < L; k++) if(at >= n.layer[k].patch_begin) l = k;
+    int begin = n.layer[0].patch_begin, across = n.layer[0].across; Divisor by = n.layer[0].by_across;
 #pragma unroll
-    for(int k = 1; k < L; k++) if(l == k){ begin = n.layer[k].tile_begin; tiles_i = n.layer[k].tiles_i; by = n.layer[k].by_tiles_i; }
-    o4 = quotient(tile - begin, by); i4 = tile - begin - o4 * tiles_i;
+    for(int k = 1; k < L; k++) if(l == k){ begin = n.layer[k].patch_begin; across = n.layer[k].across; by = n.layer[k].by_across; }
+    const int o = quotient(at - begin, by);
+    o4 = o * n.patch_o; i4 = (at - begin - o * across) * n.patch_i;
 }
 template <int L>
-__device__ __forceinline__ Patch patch(const Net& n, int tile){
-    Patch p{0, 0, 0};
-    if(tile >= n.n_tiles) return p;
+__device__ __forceinline__ Patch patch(const Net& n, int at){
+    Patch p{0, 0, 0, 0};
+    if(at >= n.n_patches) return p;
     int l, o4, i4;
-    locate<L>(n, tile, l, o4, i4);
+    locate<L>(n, at, l, o4, i4);
 #pragma unroll
-    for(int k = 0; k < L; k++) if(l == k){ const Layer& y = n.layer[k]; p.d = y.d + 4 * o4; p.a = y.a + 4 * i4; p.pitch = y.S | (y.P << 16); }
+    for(int k = 0; k < L; k++) if(l == k){ const Layer& y = n.layer[k]; p.d = y.d + 4 * o4; p.a = y.a + 4 * i4; p.pitch = y.S | (y.P << 16); p.alt = k == 0 ? n.a_alt : 0; }
     return p;
 }
-template <int TPT>
-__device__ __forceinline__ void accumulate_gradients(const Net& n, const float* smem, const Patch (&p)[TPT], float2 (&acc)[TPT][4][2]){
+// a thread's sums: N patches of PO x PI pieces
+template <int N, int PO, int PI> struct Sums { float4 v[N][4 * PO][PI]; };
+template <int N, int PO, int PI>
+__device__ __forceinline__ void clear_sums(Sums<N, PO, PI>& acc){
 #pragma unroll
-    for(int k = 0; k < TPT; k++){
-        if(k * THREADS + (int)threadIdx.x >= n.n_tiles) continue;
-        const float* d = smem + p[k].d; const float* a = smem + p[k].a;
+    for(int k = 0; k < N; k++)
+#pragma unroll
+        for(int o = 0; o < 4 * PO; o++)
+#pragma unroll
+            for(int i = 0; i < PI; i++) acc.v[k][o][i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+}
+// `other`: the first layer's rows lie in its second buffer
+template <int N, int PO, int PI>
+__device__ __forceinline__ void accumulate_gradients(const Net& n, const float* smem, const Patch (&p)[N], Sums<N, PO, PI>& acc, bool other){
+#pragma unroll
+    for(int k = 0; k < N; k++){
+        if(k * THREADS + (int)threadIdx.x >= n.n_patches) continue;
+        const float* d = smem + p[k].d; const float* a = smem + p[k].a + (other ? p[k].alt : 0);
         const int ds = p[k].pitch & 0xFFFF, as = p[k].pitch >> 16;
-#pragma unroll 4
+#pragma unroll (PO * PI == 1 ? 4 : PO * PI == 2 ? 2 : 1)
         for(int r = 0; r < n.R; r++){
-            const float4 dv = *reinterpret_cast<const float4*>(d + r * ds), av = *reinterpret_cast<const float4*>(a + r * as);
-            const float e[4] = {dv.x, dv.y, dv.z, dv.w};
+            float4 dv[PO], av[PI];
 #pragma unroll
-            for(int i = 0; i < 4; i++){
-                acc[k][i][0] = __ffma2_rn(make_float2(e[i], e[i]), make_float2(av.x, av.y), acc[k][i][0]);
-                acc[k][i][1] = __ffma2_rn(make_float2(e[i], e[i]), make_float2(av.z, av.w), acc[k][i][1]);
+            for(int o = 0; o < PO; o++) dv[o] = *reinterpret_cast<const float4*>(d + r * ds + 4 * o);
+#pragma unroll
+            for(int i = 0; i < PI; i++) av[i] = *reinterpret_cast<const float4*>(a + r * as + 4 * i);
+#pragma unroll
+            for(int o = 0; o < PO; o++){
+                const float e[4] = {dv[o].x, dv[o].y, dv[o].z, dv[o].w};
+#pragma unroll
+                for(int q = 0; q < 4; q++)
+#pragma unroll
+                    for(int i = 0; i < PI; i++){
+                        float4& s = acc.v[k][4 * o + q][i];
+                        s.x = fmaf(e[q], av[i].x, s.x); s.y = fmaf(e[q], av[i].y, s.y); s.z = fmaf(e[q], av[i].z, s.z); s.w = fmaf(e[q], av[i].w, s.w);
+                    }
             }
         }
     }
 }
-// gradient sums of one team: [CTA of the team][patch][output of the patch] x 16 bytes
-template <int C, int TPT>
-__device__ __forceinline__ void store_gradients(const Net& n, float4* partial, int rank, const float2 (&acc)[TPT][4][2]){
+// gradient sums of one CTA of a team: [output of the patch][piece of the inputs][patch] x 16 bytes, so that the lanes of a warp write neighbouring pieces
+template <int N, int PO, int PI>
+__device__ __forceinline__ void store_gradients(const Net& n, float4* partial, int rank, const Sums<N, PO, PI>& acc){
 #pragma unroll
-    for(int k = 0; k < TPT; k++){
-        const int tile = k * THREADS + (int)threadIdx.x;
-        if(tile >= n.n_tiles) continue;
-        float4* dst = partial + ((size_t)rank * n.n_tiles + tile) * 4;
+    for(int k = 0; k < N; k++){
+        const int at = k * THREADS + (int)threadIdx.x;
+        if(at >= n.n_patches) continue;
+        float4* dst = partial + (size_t)rank * n.quads + at;
 #pragma unroll
-        for(int i = 0; i < 4; i++) __stcg(dst + i, make_float4(acc[k][i][0].x, acc[k][i][0].y, acc[k][i][1].x, acc[k][i][1].y));
+        for(int o = 0; o < 4 * PO; o++)
+#pragma unroll
+            for(int i = 0; i < PI; i++) __stcg(dst + (o * PI + i) * n.n_patches, acc.v[k][o][i]);
     }
 }
-// arena index of component `comp` of quad `u` (= (CTA of the team, patch, output)); -1 where the patch reaches beyond the layer
+// arena index of component `comp` of quad `u` (= (CTA of the team, output of the patch, piece of the inputs, patch)); -1 where the patch reaches beyond the layer
 template <int L>
 __device__ __forceinline__ int arena_index(const Net& n, int u, int comp){
-    const int q = u & 3, rank = quotient(u >> 2, n.by_tiles), tile = (u >> 2) - rank * n.n_tiles;
+    const int rank = quotient(u, n.by_quads), rest = u - rank * n.quads, j = quotient(rest, n.by_patches), at = rest - j * n.n_patches;
     int l, o4, i4, index = -1;
-    locate<L>(n, tile, l, o4, i4);
+    locate<L>(n, at, l, o4, i4);
+    const int out = n.patch_i == 2 ? j >> 1 : j, piece = n.patch_i == 2 ? j & 1 : 0;
 #pragma unroll
     for(int k = 0; k < L; k++) if(l == k){
         const Layer& y = n.layer[k];
-        const int o = rank * y.S + o4 * 4 + q, i = i4 * 4 + comp;
-        if(o < y.O && i <= y.I) index = (int)y.poff + (i < y.I ? o * y.I + i : y.O * y.I + o);
+        const int unit = o4 * 4 + out, o = rank * y.S + unit, i = (i4 + piece) * 4 + comp;
+        if(unit < y.S && o < y.O && i <= y.I) index = (int)y.poff + (i < y.I ? o * y.I + i : y.O * y.I + o);
     }
     return index;
+}
+
+// shared-memory offset of the four weights that quad `u` of a team of one CTA holds the gradients of; -1 where the patch reaches beyond the layer
+template <int L>
+__device__ __forceinline__ int weights_of_quad(const Net& n, int u){
+    const int j = quotient(u, n.by_patches), at = u - j * n.n_patches, out = n.patch_i == 2 ? j >> 1 : j, piece = n.patch_i == 2 ? j & 1 : 0;
+    int l, o4, i4, off = -1;
+    locate<L>(n, at, l, o4, i4);
+#pragma unroll
+    for(int k = 0; k < L; k++) if(l == k){
+        const Layer& y = n.layer[k];
+        const int unit = o4 * 4 + out, i = (i4 + piece) * 4;
+        if(unit < y.O && i <= y.I) off = y.w + ((unit & 3) * (y.S >> 2) + (unit >> 2)) * y.P + i;
+    }
+    return off;
 }
 
 static __device__ __noinline__ float adam_bias_correction(float beta, uint32_t age){
@@ -397,32 +530,42 @@ __device__ __forceinline__ float adam_update(float p, float g, float& m, float& 
     return __fsub_rn(p, __fdiv_rn(__fmul_rn(__fmul_rn(h.alpha, c1), m), __fadd_rn(__fsqrt_rn(pre_sqrt), h.epsilon)));
 }
 
-// All CTAs of the grid (cta of ctas) share out the parameters: `lanes` threads per quad (a power of two from 4 on) add the teams' sums (lane y
-// takes teams y, y + lanes, ... ascending, then the lanes pairwise: a fixed order), the first four lanes each finish one parameter:
-// sink(arena index, gradient, what prefetch(arena index) returned before the sums were loaded).
+// All CTAs of the grid share out the parameters: `lanes` threads per quad (a power of two from 4 on) add the teams' sums (thread y of a quad takes teams y, y + lanes, ... ascending,
+// then they are added pairwise: a fixed order), the first four each finish one parameter. Lanes of neighbouring quads lie side by side.
+struct Owner { int quad, part, step; };
+__device__ __forceinline__ Owner owner(int lanes, int cta, int ctas){
+    const int bits = __popc(lanes - 1), per_warp = 32 >> bits, lane = threadIdx.x & 31;
+    return Owner{(cta * WARPS + ((int)threadIdx.x >> 5)) * per_warp + (lane & (per_warp - 1)), lane >> (5 - bits), ctas * WARPS * per_warp};
+}
+__device__ __forceinline__ float sum_of_teams(const float4* partial, int u, int quads, int teams, int part, int lanes){
+    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if(u < quads){
+        const float4* src = partial + u;
+        for(int t = part; t < teams; t += 8 * lanes){
+            float4 v[8];
+#pragma unroll
+            for(int k = 0; k < 8; k++) v[k] = t + k * lanes < teams ? __ldcg(src + (size_t)(t + k * lanes) * quads) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+            for(int k = 0; k < 8; k++){ s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
+        }
+    }
+    for(int o = 32 / lanes; o < 32; o <<= 1){
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o); s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+        s.z += __shfl_xor_sync(0xffffffffu, s.z, o); s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
+    }
+    return part == 0 ? s.x : part == 1 ? s.y : part == 2 ? s.z : s.w;
+}
+// sink(arena index, gradient, what prefetch(arena index) returned before the sums were loaded)
 template <int C, int L, typename PREFETCH, typename SINK>
 __device__ __forceinline__ void reduce_gradients(const Net& n, const float4* partial, int teams, int cta, int ctas, int lanes, PREFETCH prefetch, SINK sink){
-    const int quads = C * n.n_tiles * 4, lane = threadIdx.x & (lanes - 1), lane_bits = __popc(lanes - 1), per_cta = THREADS >> lane_bits;
-    for(int u0 = cta * per_cta; u0 < quads; u0 += ctas * per_cta){
-        const int u = u0 + ((int)threadIdx.x >> lane_bits);
-        const int index = u < quads && lane < 4 ? arena_index<L>(n, u, lane) : -1;
+    const int quads = C * n.quads;
+    const Owner me = owner(lanes, cta, ctas);
+    const int first = me.quad - (threadIdx.x & 31 & ((32 / lanes) - 1));                 // the same for all lanes of a warp
+    for(int u0 = first; u0 < quads; u0 += me.step){
+        const int u = u0 + me.quad - first, index = u < quads && me.part < 4 ? arena_index<L>(n, u, me.part) : -1;
         const auto early = prefetch(index);
-        float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if(u < quads){
-            const float4* src = partial + u;
-            for(int t = lane; t < teams; t += 8 * lanes){
-                float4 v[8];
-#pragma unroll
-                for(int k = 0; k < 8; k++) v[k] = t + k * lanes < teams ? __ldcg(src + (size_t)(t + k * lanes) * quads) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-                for(int k = 0; k < 8; k++){ s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
-            }
-        }
-        for(int o = lanes >> 1; o > 0; o >>= 1){
-            s.x += __shfl_xor_sync(0xffffffffu, s.x, o); s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-            s.z += __shfl_xor_sync(0xffffffffu, s.z, o); s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
-        }
-        if(index >= 0) sink(index, lane == 0 ? s.x : lane == 1 ? s.y : lane == 2 ? s.z : s.w, early);
+        const float g = sum_of_teams(partial, u, quads, teams, me.part, lanes);
+        if(index >= 0) sink(index, g, early);
     }
 }
 #endif

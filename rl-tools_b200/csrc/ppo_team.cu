@@ -5,8 +5,8 @@
 // takes its rows of a minibatch through the network (mlp_team.cuh, teams of one CTA), the row-wise loss gradient of the clipped surrogate or of
 // the value regression in between, writes its gradient sums, and behind a barrier over the network's CTAs every thread adds the sums of the one
 // parameter it owns and steps the optimizer for it, with the moments in registers for the whole epoch. A second barrier publishes the new
-// parameters. Replaces the per-minibatch body of train (rl/algorithms/ppo/operations_generic.h:159-336), per sample :214-296; Gaussian head
-// random/operations_generic.h:87-121.
+// parameters, in quads of four neighbours of a weight row whose places in shared memory every CTA has a table of. log_std is a quad like the weights. Replaces the
+// per-minibatch body of train (rl/algorithms/ppo/operations_generic.h:159-336), per sample :214-296; Gaussian head random/operations_generic.h:87-121.
 #include "common.cuh"
 #include "grid_barrier.cuh"
 #include "mlp_team.cuh"
@@ -20,9 +20,13 @@ struct PpoNetArgs {
     Net net;
     float* params; float* grads; float* m; float* v; uint32_t* adam_state;
     b200rl_adam_hyper hyper;
-    float4* partial; float* partial_std; GridBarrier barrier;
+    float4* partial; float* fresh; GridBarrier barrier;       // gradient sums [team][quad] x 16 bytes; parameters on their way to all CTAs [quad] x 16 bytes
     int ctas, teams, lanes, row_tiles;
-    int stage_x, stage_aux, aux, out;        // shared memory: next rows and columns as they come, this tile's columns ([4][R] behind actions [R][S]), outputs [R][S]
+    int quads;                               // those of the layers and, behind them, of log_std
+    int aux, aux_alt, out;                   // shared memory: columns of a tile (actions [R][S], log-probabilities [R], advantages [R]; targets [R]), distance of the next tile's; outputs [R][S]
+    int places, log_std;                     // where the weights of every quad go [quads]; log_std [action dimension rounded up to four]
+    int lp, ps, dl;                          // the surrogate's log-probability terms [R][S], (action - mean) / std [R][S], dL / d log-probability [R]
+    Divisor by_S;
 };
 struct PpoEpochArgs {
     PpoNetArgs actor, critic;
@@ -33,7 +37,7 @@ struct PpoEpochArgs {
     int normalize_advantage, learn_action_std;
 };
 
-constexpr int PPO_TEAM_MAX_ACTIONS = 64;
+constexpr int PPO_TEAM_MAX_ACTIONS = 64, PPO_TEAM_MAX_PARAMS = 18944;       // parameters of a network's layers: what was measured
 
 // mean and standard deviation of every minibatch's advantages (:173-184), one CTA each
 __global__ void __launch_bounds__(1024) ppo_epoch_stats_kernel(const float* __restrict__ advantages, int ld, int batch, float* __restrict__ stats){
@@ -52,121 +56,123 @@ __global__ void __launch_bounds__(1024) ppo_epoch_stats_kernel(const float* __re
     }
 }
 
-template <bool ACTOR, int L, int TPT>
+template <bool ACTOR, int L, int N, int PO, int PI>
 __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArgs& w, int cta, float* smem){
     __shared__ float s_scalars[2][64];       // bias corrections of the next minibatches
-    __shared__ float s_log_std[PPO_TEAM_MAX_ACTIONS], s_std[PPO_TEAM_MAX_ACTIONS];
+    __shared__ float s_std[PPO_TEAM_MAX_ACTIONS];
     __shared__ int s_ok;
     const Net& n = w.net;
     const Layer& last = n.layer[L - 1];
     const int tid = threadIdx.x, R = n.R, I0 = n.layer[0].I, A = a.action_dim, S = last.S;
     const bool has_rows = cta < w.row_tiles;
-    auto stage = [&](int minibatch, int tile){
+    auto stage = [&](int minibatch, int tile, bool other){
+        const int tid = thread_here();
         const int row0 = tile * R;
         const size_t base = (size_t)minibatch * a.batch + row0;
         const int rows = min(R, a.batch - row0);
+        float* in = smem + n.layer[0].a + (other ? n.a_alt : 0);
+        float* aux = smem + w.aux + (other ? w.aux_alt : 0);
 #pragma unroll 1
         for(int i = tid; i < R * I0; i += THREADS){
             const int r = quotient(i, n.by_I0), k = i - r * I0;
-            if(r < rows) copy4_async(smem + w.stage_x + i, a.observations + (base + r) * a.ld + k);
-            else smem[w.stage_x + i] = 0.0f;
+            if(r < rows) copy4_async(in + r * n.layer[0].P + k, a.observations + (base + r) * a.ld + k);
+            else in[r * n.layer[0].P + k] = 0.0f;
         }
         if constexpr(ACTOR){
 #pragma unroll 1
             for(int i = tid; i < R * S; i += THREADS){
-                const int r = quotient(i, last.by_S), k = i - r * S;
-                if(r < rows && k < A) copy4_async(smem + w.stage_aux + i, a.actions + (base + r) * a.ld + k);
+                const int r = quotient(i, w.by_S), k = i - r * S;
+                if(r < rows && k < A) copy4_async(aux + i, a.actions + (base + r) * a.ld + k);
             }
             if(tid < rows){
-                copy4_async(smem + w.stage_aux + R * S + tid, a.log_probs + (base + tid) * a.ld);
-                copy4_async(smem + w.stage_aux + R * S + R + tid, a.advantages + (base + tid) * a.ld);
+                copy4_async(aux + R * S + tid, a.log_probs + (base + tid) * a.ld);
+                copy4_async(aux + R * S + R + tid, a.advantages + (base + tid) * a.ld);
             }
         }
-        else if(tid < rows) copy4_async(smem + w.stage_aux + tid, a.targets + (base + tid) * a.ld);
+        else if(tid < rows) copy4_async(aux + tid, a.targets + (base + tid) * a.ld);
     };
-    if(has_rows) stage(0, cta);
     clear_rows<L>(n, smem);
+    __syncthreads();
+    if(has_rows) stage(0, cta, false);
     load_weights<L>(n, smem, w.params, 0);
-    auto load_std = [&](){
-        if(ACTOR && tid < A){ const float ls = __ldcg(w.params + n.n_params + tid); s_log_std[tid] = ls; s_std[tid] = expf(ls); }
-    };
-    load_std();
+    if(ACTOR && tid < A) smem[w.log_std + tid] = w.params[n.n_params + tid];
     // the parameter this thread owns: `lanes` threads per quad, one pass over all quads (guaranteed by the host's choice of lanes)
-    const int quads = n.n_tiles * 4, lane = tid & (w.lanes - 1), lane_bits = __popc(w.lanes - 1), u = cta * (THREADS >> lane_bits) + (tid >> lane_bits);
-    const int index = u < quads && lane < 4 ? arena_index<L>(n, u, lane) : -1;
+    const Owner me = owner(w.lanes, cta, w.ctas);
+    const int quads = w.quads, u = me.quad;
+    auto place_of_quad = [&](int q){ return ACTOR && q >= n.quads ? w.log_std + 4 * (q - n.quads) : weights_of_quad<L>(n, q); };
+    int* places = reinterpret_cast<int*>(smem + w.places);
+    for(int i = tid; i < quads; i += THREADS) places[i] = place_of_quad(i);
+    const bool adds = u < quads && place_of_quad(u) >= 0;
+    int index = -1;
+    if(adds && me.part < 4){
+        if(!ACTOR || u < n.quads) index = arena_index<L>(n, u, me.part);
+        else if(4 * (u - n.quads) + me.part < A) index = n.n_params + 4 * (u - n.quads) + me.part;
+    }
     float my_p = 0.0f, my_m = 0.0f, my_v = 0.0f, my_g = 0.0f;
     if(index >= 0){ my_p = w.params[index]; my_m = w.m[index]; my_v = w.v[index]; }
-    const uint32_t age0 = *reinterpret_cast<volatile uint32_t*>(w.adam_state);
-    Patch patches[TPT];
-#pragma unroll
-    for(int k = 0; k < TPT; k++) patches[k] = patch<L>(n, k * THREADS + tid);
-    const float value_constant = 2.0f / ((float)a.batch * 1.0f) * 0.5f;
     unsigned target = 0;
+    const uint32_t age0 = *reinterpret_cast<volatile uint32_t*>(w.adam_state);
+    Patch patches[N];
+#pragma unroll
+    for(int k = 0; k < N; k++) patches[k] = patch<L>(n, k * THREADS + tid);
+    bool other = false;                      // which of the two buffers this tile's rows are in
+    const float value_constant = 2.0f / ((float)a.batch * 1.0f) * 0.5f;
     for(int mb = 0; mb < a.minibatches; mb++){
-        if((mb & 63) == 0 && tid < 128) s_scalars[tid & 1][tid >> 1] = adam_bias_correction(tid & 1 ? w.hyper.beta_2 : w.hyper.beta_1, age0 + (uint32_t)(mb + (tid >> 1)));
-        float2 acc[TPT][4][2];
+        const int tid = thread_here();
+        if((mb & 63) == 0){
+            __syncthreads();                                              // the last of the old ones have been read
+            if(tid < 128) s_scalars[tid & 1][tid >> 1] = adam_bias_correction(tid & 1 ? w.hyper.beta_2 : w.hyper.beta_1, age0 + (uint32_t)(mb + (tid >> 1)));
+            __syncthreads();
+        }
+        Sums<N, PO, PI> acc;
+        clear_sums(acc);
         float std_gradient = 0.0f;
-#pragma unroll
-        for(int k = 0; k < TPT; k++)
-#pragma unroll
-            for(int i = 0; i < 4; i++){ acc[k][i][0] = make_float2(0.0f, 0.0f); acc[k][i][1] = make_float2(0.0f, 0.0f); }
         float mean = 0.0f, deviation = 1.0f;
         if(ACTOR && a.normalize_advantage){ mean = __ldg(a.stats + 2 * mb); deviation = __fadd_rn(__ldg(a.stats + 2 * mb + 1), a.advantage_epsilon); }
-        for(int tile = cta; tile < w.row_tiles; tile += w.teams){
+        for(int tile = cta; tile < w.row_tiles; tile += w.teams, other = !other){
             const int rows = min(R, a.batch - tile * R);
+            const float* aux = smem + w.aux + (other ? w.aux_alt : 0);
             copies_wait();
             __syncthreads();
-#pragma unroll 1
-            for(int i = tid; i < R * I0; i += THREADS){ const int r = quotient(i, n.by_I0), k = i - r * I0; smem[n.layer[0].a + r * n.layer[0].P + k] = smem[w.stage_x + i]; }
-            if constexpr(ACTOR){
-#pragma unroll 1
-                for(int i = tid; i < R * S + 2 * R; i += THREADS) smem[w.aux + i] = smem[w.stage_aux + i];
-            }
-            else if(tid < R) smem[w.aux + tid] = smem[w.stage_aux + tid];
-            __syncthreads();
-            {
-                const bool more = tile + w.teams < w.row_tiles;
-                if(more) stage(mb, tile + w.teams);
-                else if(mb + 1 < a.minibatches) stage(mb + 1, cta);
-            }
-#pragma unroll 1
+            if(ACTOR && tid < A) s_std[tid] = expf(smem[w.log_std + tid]);
+            if(tile + w.teams < w.row_tiles) stage(mb, tile + w.teams, !other);
+            else if(mb + 1 < a.minibatches) stage(mb + 1, cta, !other);
+#pragma unroll
             for(int l = 0; l < L; l++){
-                forward_layer<1, L>(n, l, smem, 0, [&](int r, int unit, int idx, float value, float derivative){
-                    if(l == L - 1){
-                        if constexpr(ACTOR) smem[w.out + idx] = value;
-                        else smem[last.d + idx] = r < rows ? __fmul_rn(__fsub_rn(value, smem[w.aux + r]), value_constant) * derivative : 0.0f;
-                    }
+                forward_layer<1, L, false>(n, l, n.layer[l].a + (l == 0 && other ? n.a_alt : 0), smem, 0, [&](int r, int unit, float4 value, float4 derivative){
+                    if constexpr(ACTOR) *reinterpret_cast<float4*>(smem + w.out + r * S + unit) = value;
+                    else *reinterpret_cast<float4*>(smem + last.d + r * S + unit) =
+                        make_float4(r < rows ? __fmul_rn(__fsub_rn(value.x, aux[r]), value_constant) * derivative.x : 0.0f, 0.0f, 0.0f, 0.0f);       // one output
                 });
                 __syncthreads();
             }
             if constexpr(ACTOR){
-                float* lp = smem + n.rb[1];                      // [R][S] log-probability terms, then [R][S] (action - mean) / std, then [R] dL / d log-probability
-                float* ps = lp + R * S;
-                float* dl = ps + R * S;
+                // eight lanes a row; what one of them needs from the others of its row goes through shared memory
+                float* lp = smem + w.lp; float* ps = smem + w.ps; float* dl = smem + w.dl;
+                const int part = tid & 7;
 #pragma unroll 1
-                for(int i = tid; i < R * S; i += THREADS){
-                    const int r = quotient(i, last.by_S), k = i - r * S;
-                    if(k < A){
-                        const float p = __fdiv_rn(__fsub_rn(smem[w.aux + i], smem[w.out + i]), s_std[k]);
+                for(int r = tid >> 3; r < R; r += THREADS / 8){          // the same number of rounds for all lanes of a warp: R is a multiple of four
+#pragma unroll 1
+                    for(int k = part; k < A; k += 8){
+                        const int i = r * S + k;
+                        const float p = __fdiv_rn(__fsub_rn(aux[i], smem[w.out + i]), s_std[k]);
                         // (constant - log_std) - 0.5 p^2 rounded once: p^2 as an exact float pair (see ppo.cu)
                         const float h = __fmul_rn(p, p), lo = __fmaf_rn(p, p, -h);
-                        const float c = __fsub_rn(a.neg_log_sqrt_pi, s_log_std[k]), hh = __fmul_rn(0.5f, h);
+                        const float c = __fsub_rn(a.neg_log_sqrt_pi, smem[w.log_std + k]), hh = __fmul_rn(0.5f, h);
                         const float d = __fsub_rn(c, hh), db = __fsub_rn(d, c);
                         const float de = __fsub_rn(__fsub_rn(c, __fsub_rn(d, db)), __fadd_rn(hh, db));
                         lp[i] = __fadd_rn(d, __fmaf_rn(-0.5f, lo, de));
                         ps[i] = p;
                     }
-                }
-                __syncthreads();
-                if(tid < R){
+                    __syncwarp();
                     float d = 0.0f;
-                    if(tid < rows){
+                    if(r < rows){
                         float log_prob = 0.0f;
-#pragma unroll 1
-                        for(int k = 0; k < A; k++) log_prob = __fadd_rn(log_prob, lp[tid * S + k]);
-                        float advantage = smem[w.aux + R * S + R + tid];
+#pragma unroll 4
+                        for(int k = 0; k < A; k++) log_prob = __fadd_rn(log_prob, lp[r * S + k]);
+                        float advantage = aux[R * S + R + r];
                         if(a.normalize_advantage) advantage = __fdiv_rn(__fsub_rn(advantage, mean), deviation);
-                        const float ratio = expf(__fsub_rn(log_prob, smem[w.aux + R * S + tid]));
+                        const float ratio = expf(__fsub_rn(log_prob, aux[R * S + r]));
                         const float lo = 1.0f - a.epsilon_clip, hi = 1.0f + a.epsilon_clip;
                         const float clipped_ratio = ratio < lo ? lo : (ratio > hi ? hi : ratio);
                         const bool clipped = ratio != clipped_ratio;
@@ -174,29 +180,27 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
                         const float d_ratio = unclipped_is_smaller ? advantage : (clipped ? 0.0f : advantage);
                         d = __fmul_rn(__fmul_rn(-1.0f / (float)a.batch, d_ratio), ratio);
                     }
-                    dl[tid] = d;
+                    if(part == 0) dl[r] = d;
+#pragma unroll 1
+                    for(int k = part; k < S; k += 8){
+                        const int i = r * S + k;
+                        smem[last.d + i] = r < rows && k < A ? __fmul_rn(__fdiv_rn(ps[i], s_std[k]), d) * smem[last.g + i] : 0.0f;
+                    }
                 }
                 __syncthreads();
-#pragma unroll 1
-                for(int i = tid; i < R * S; i += THREADS){
-                    const int r = quotient(i, last.by_S), k = i - r * S;
-                    if(k < A) smem[last.d + i] = r < rows ? __fmul_rn(__fdiv_rn(ps[i], s_std[k]), dl[r]) * smem[last.g + i] : 0.0f;
-                }
-                if(tid >= 128 && tid < 128 + A){                 // the log_std gradient of the CTA's rows, in row order
-                    const int k = tid - 128;
+                if(tid >= THREADS - 64 && tid < THREADS - 64 + A){       // the log_std gradient of the CTA's rows, in row order
+                    const int k = tid - (THREADS - 64);
 #pragma unroll 4
                     for(int r = 0; r < rows; r++) std_gradient += __fmul_rn(dl[r], __fadd_rn(-1.0f, __fmul_rn(ps[r * S + k], ps[r * S + k])));
                 }
-                __syncthreads();
             }
-#pragma unroll 1
-            for(int l = L - 1; l > 0; l--) backward_layer<1>(n, l, smem, 0, (L - 1 - l) & 1);
-            accumulate_gradients<TPT>(n, smem, patches, acc);
-            if(tile + w.teams < w.row_tiles) __syncthreads();
+#pragma unroll
+            for(int l = L - 1; l > 0; l--) backward_layer<1>(n, l, smem, 0, 0);
+            accumulate_gradients<N, PO, PI>(n, smem, patches, acc, other);
         }
         if(has_rows){
-            store_gradients<1, TPT>(n, w.partial + (size_t)cta * quads, 0, acc);
-            if(ACTOR && a.learn_action_std && tid >= 128 && tid < 128 + A) __stcg(w.partial_std + (size_t)cta * A + tid - 128, std_gradient);
+            store_gradients<N, PO, PI>(n, w.partial + (size_t)cta * quads, 0, acc);
+            if(ACTOR && tid >= THREADS - 64 && tid - (THREADS - 64) < 4 * (quads - n.quads)) __stcg(reinterpret_cast<float*>(w.partial + (size_t)cta * quads + n.quads) + tid - (THREADS - 64), std_gradient);
         }
         __syncthreads();
         target += (unsigned)w.ctas;
@@ -204,56 +208,27 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
         __syncthreads();
         if(!s_ok) break;
         const float c1 = s_scalars[0][mb & 63], c2 = s_scalars[1][mb & 63];
-        {
-            float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if(u < quads){
-                const float4* src = w.partial + u;
-                for(int t = lane; t < w.teams; t += 8 * w.lanes){
-                    float4 v[8];
-#pragma unroll
-                    for(int k = 0; k < 8; k++) v[k] = t + k * w.lanes < w.teams ? __ldcg(src + (size_t)(t + k * w.lanes) * quads) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-                    for(int k = 0; k < 8; k++){ s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
-                }
-            }
-            for(int o = w.lanes >> 1; o > 0; o >>= 1){
-                s.x += __shfl_xor_sync(0xffffffffu, s.x, o); s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-                s.z += __shfl_xor_sync(0xffffffffu, s.z, o); s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
-            }
-            if(index >= 0){
-                my_g = lane == 0 ? s.x : lane == 1 ? s.y : lane == 2 ? s.z : s.w;
-                my_p = adam_update(my_p, my_g, my_m, my_v, w.hyper, c1, c2);
-                __stcg(w.params + index, my_p);
-            }
-            if(ACTOR && cta == w.ctas - 1){                      // log_std: a warp per action, teams over the lanes
-                for(int k = tid >> 5; k < A; k += THREADS / 32){
-                    float g = 0.0f;
-                    if(a.learn_action_std){
-                        for(int t = tid & 31; t < w.teams; t += 32) g += __ldcg(w.partial_std + (size_t)t * A + k);
-#pragma unroll
-                        for(int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
-                        g += (float)a.batch * (-1.0f / (float)a.batch * a.entropy_coefficient);      // the entropy bonus of every sample (:262-266)
-                    }
-                    if((tid & 31) == 0){
-                        const int i = n.n_params + k;
-                        float mm = w.m[i], vv = w.v[i];
-                        __stcg(w.params + i, adam_update(__ldcg(w.params + i), g, mm, vv, w.hyper, c1, c2));
-                        w.m[i] = mm; w.v[i] = vv; w.grads[i] = g;
-                    }
-                }
-            }
+        const float g = sum_of_teams(w.partial, adds ? u : quads, quads, w.teams, me.part, w.lanes);
+        if(index >= 0){
+            // log_std: the entropy bonus of every sample (:262-266); no gradient where it is not learnt
+            my_g = !ACTOR || index < n.n_params ? g : a.learn_action_std ? g + (float)a.batch * (-1.0f / (float)a.batch * a.entropy_coefficient) : 0.0f;
+            my_p = adam_update(my_p, my_g, my_m, my_v, w.hyper, c1, c2);
         }
+        if(adds && me.part < 4) __stcg(w.fresh + 4 * u + me.part, my_p);
         if(mb + 1 == a.minibatches) break;
         __syncthreads();
         target += (unsigned)w.ctas;
         if(tid == 0){ grid_barrier_arrive(w.barrier); s_ok = grid_barrier_wait(w.barrier, target); }
         __syncthreads();
         if(!s_ok) break;
-        if(has_rows){ load_weights<L>(n, smem, w.params, 0); load_std(); }
+        if(has_rows){
+#pragma unroll 4
+            for(int q = tid; q < quads; q += THREADS){ const int at = places[q]; if(at >= 0) copy16_async(smem + at, w.fresh + 4 * q); }
+        }
     }
     copies_wait();
     if(!s_ok){ if(tid == 0) grid_barrier_leave(w.barrier, (unsigned)w.ctas); return; }
-    if(index >= 0){ w.m[index] = my_m; w.v[index] = my_v; w.grads[index] = my_g; }
+    if(index >= 0){ w.params[index] = my_p; w.m[index] = my_m; w.v[index] = my_v; w.grads[index] = my_g; }
     if(cta == 0 && tid == 0){
         const int last_mb = (a.minibatches - 1) & 63;
         w.adam_state[0] = age0 + (uint32_t)a.minibatches; w.adam_state[1] = 0u;
@@ -262,35 +237,36 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
     if(tid == 0) grid_barrier_leave(w.barrier, (unsigned)w.ctas);
 }
 
-template <int L, int TPT>
+template <int L, int PO, int PI>
 __global__ void __launch_bounds__(THREADS, 1) ppo_epoch_kernel(const __grid_constant__ PpoEpochArgs a){
     extern __shared__ __align__(16) float smem[];
-    if((int)blockIdx.x < a.actor.ctas) ppo_epoch<true, L, TPT>(a, a.actor, blockIdx.x, smem);
-    else ppo_epoch<false, L, TPT>(a, a.critic, blockIdx.x - a.actor.ctas, smem);
+    if((int)blockIdx.x < a.actor.ctas) ppo_epoch<true, L, 1, PO, PI>(a, a.actor, blockIdx.x, smem);
+    else ppo_epoch<false, L, 1, PO, PI>(a, a.critic, blockIdx.x - a.actor.ctas, smem);
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------------------------------
-constexpr size_t PPO_TEAM_SMEM = 200 * 1024;
+constexpr size_t PPO_TEAM_SMEM = 220 * 1024;
 
 // rows per tile: one tile per CTA where the batch allows it
-static bool plan_ppo_net(const b200rl_mlp_shape* sh, int batch, int ctas, bool actor, PpoNetArgs* w, size_t* smem){
+static bool plan_ppo_net(const b200rl_mlp_shape* sh, int batch, int ctas, bool actor, int least, PpoNetArgs* w, size_t* smem){
     const int want = (batch + ctas - 1) / ctas, A = sh->dims[sh->n_layers - 1];
     for(int R = want >= 32 ? 32 : (want + 3) / 4 * 4; R >= 4; R -= 4){
         Net n;
-        if(!team::plan(sh, 1, R, 0, &n)) continue;
+        if(!team::plan(sh, 1, R, 0, false, least, &n)) continue;
+        if(n.n_patches > THREADS || n.n_params > PPO_TEAM_MAX_PARAMS || A > PPO_TEAM_MAX_ACTIONS) return false;
         const int S = n.layer[n.n_layers - 1].S;
-        // the surrogate's work area lies in the second exchange buffer
-        if(actor && n.end - n.rb[1] < 2 * R * S + R) n.end = n.rb[1] + 2 * R * S + R;
         int off = (n.end + 3) / 4 * 4;
-        w->stage_x = off; off += (R * sh->input_dim + 3) / 4 * 4;
-        w->stage_aux = off; off += R * S + 2 * R;
-        w->aux = off; off += R * S + 2 * R;
+        w->quads = n.quads + (actor ? (A + 3) / 4 : 0);
+        w->aux = off; w->aux_alt = R * S + 2 * R; off += 2 * w->aux_alt;
         w->out = off; off += R * S;
+        w->places = off; off += (w->quads + 3) / 4 * 4;
+        if(actor){ w->log_std = off; off += (A + 3) / 4 * 4; w->lp = off; off += R * S; w->ps = off; off += R * S; w->dl = off; off += R; }
+        w->by_S = divisor(S);
         if(sizeof(float) * (size_t)off > PPO_TEAM_SMEM) continue;
         w->net = n; w->ctas = ctas; w->row_tiles = (batch + R - 1) / R; w->teams = w->row_tiles < ctas ? w->row_tiles : ctas;
         // one parameter per thread, one pass: lanes x quads within the threads of the network's CTAs
-        const int quads = n.n_tiles * 4, threads = ctas * THREADS;
-        if(4ll * quads > threads || A > PPO_TEAM_MAX_ACTIONS) return false;
+        const int quads = w->quads, threads = ctas * THREADS;
+        if(4ll * quads > threads) return false;
         w->lanes = 4;
         while(w->lanes < 32 && 2 * w->lanes <= w->teams && 2ll * w->lanes * quads <= threads) w->lanes *= 2;
         *smem = sizeof(float) * (size_t)off;
@@ -298,40 +274,47 @@ static bool plan_ppo_net(const b200rl_mlp_shape* sh, int batch, int ctas, bool a
     }
     return false;
 }
+// gradient sums of the teams and the parameters on their way
+static size_t ppo_exchange_bytes(const PpoNetArgs& w){ return sizeof(float4) * (size_t)(w.teams + 1) * w.quads; }
 struct PpoChoice { PpoNetArgs actor, critic; size_t smem, bytes; };
 static bool choose_ppo(const b200rl_mlp_shape* actor, const b200rl_mlp_shape* critic, int batch, int minibatches, PpoChoice* out){
     int sms = 0;
     if(!actor || !critic || actor->n_layers != critic->n_layers || actor->n_layers < 1 || actor->n_layers > 3 || batch < 1 || sm_count(&sms) != B200RL_OK) return false;
     PpoChoice c{};
     size_t sa = 0, sc = 0;
-    if(!plan_ppo_net(actor, batch, sms / 2, true, &c.actor, &sa) || !plan_ppo_net(critic, batch, sms / 2, false, &c.critic, &sc)) return false;
-    if(c.actor.net.n_tiles > 4 * THREADS || c.critic.net.n_tiles > 4 * THREADS) return false;
+    int least = 0;                           // both networks take patches of the same size
+    for(int k = 0; k < 2; k++){
+        if(!plan_ppo_net(actor, batch, sms / 2, true, least, &c.actor, &sa) || !plan_ppo_net(critic, batch, sms / 2, false, least, &c.critic, &sc)) return false;
+        const int pa = c.actor.net.patch_o + c.actor.net.patch_i, pc = c.critic.net.patch_o + c.critic.net.patch_i;
+        if(pa == pc) break;
+        least = (pa > pc ? pa : pc) - 2;
+    }
     c.smem = sa > sc ? sa : sc;
-    c.bytes = sizeof(float4) * 4 * ((size_t)c.actor.teams * c.actor.net.n_tiles + (size_t)c.critic.teams * c.critic.net.n_tiles) +
-              sizeof(float) * ((size_t)c.actor.teams * actor->dims[actor->n_layers - 1] + 2 * (size_t)minibatches);
+    c.bytes = ppo_exchange_bytes(c.actor) + ppo_exchange_bytes(c.critic) + sizeof(float) * 2 * (size_t)minibatches;
     *out = c;
     return true;
 }
 
-template <int L, int TPT>
+template <int L, int PO, int PI>
 static int launch_ppo_epoch(const PpoEpochArgs& a, size_t smem, cudaStream_t s){
     static std::atomic<bool> configured[MAX_DEVICES];
     int dev = 0;
     int rc = current_device(&dev);
     if(rc) return rc;
     if(!configured[dev].load(std::memory_order_acquire)){
-        B200RL_CUDA_TRY(cudaFuncSetAttribute(ppo_epoch_kernel<L, TPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PPO_TEAM_SMEM));
+        B200RL_CUDA_TRY(cudaFuncSetAttribute(ppo_epoch_kernel<L, PO, PI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PPO_TEAM_SMEM));
         configured[dev].store(true, std::memory_order_release);
     }
     PpoEpochArgs copy = a;
     void* params[] = { &copy };
-    B200RL_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(ppo_epoch_kernel<L, TPT>), dim3(a.actor.ctas + a.critic.ctas), dim3(THREADS), params, smem, s));
+    B200RL_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(ppo_epoch_kernel<L, PO, PI>), dim3(a.actor.ctas + a.critic.ctas), dim3(THREADS), params, smem, s));
     return B200RL_OK;
 }
 template <int L>
 static int launch_ppo_epoch_l(const PpoEpochArgs& a, size_t smem, cudaStream_t s){
-    const int tiles = a.actor.net.n_tiles > a.critic.net.n_tiles ? a.actor.net.n_tiles : a.critic.net.n_tiles;
-    return tiles <= 2 * THREADS ? launch_ppo_epoch<L, 2>(a, smem, s) : launch_ppo_epoch<L, 4>(a, smem, s);
+    if(a.actor.net.patch_i == 2) return launch_ppo_epoch<L, 2, 2>(a, smem, s);
+    if(a.actor.net.patch_o == 2) return launch_ppo_epoch<L, 2, 1>(a, smem, s);
+    return launch_ppo_epoch<L, 1, 1>(a, smem, s);
 }
 
 }  // namespace b200rl
@@ -359,13 +342,14 @@ extern "C" int b200rl_ppo_train_epoch(const b200rl_mlp_shape* actor, const b200r
     if(!scratch || scratch_bytes < c.bytes || (reinterpret_cast<uintptr_t>(scratch) & 15u)) return B200RL_ERR_INVALID_ARGUMENT;
     PpoEpochArgs a{};
     a.actor = c.actor; a.critic = c.critic;
-    float4* p = static_cast<float4*>(scratch);
     auto arenas = [](PpoNetArgs& w, const b200rl_mlp_arenas* r){ w.params = r->params; w.grads = r->grads; w.m = r->m; w.v = r->v; w.adam_state = r->adam_state; w.hyper = r->hyper; };
     arenas(a.actor, actor_arenas); arenas(a.critic, critic_arenas);
-    a.actor.partial = p; p += (size_t)c.actor.teams * c.actor.net.n_tiles * 4;
-    a.critic.partial = p; p += (size_t)c.critic.teams * c.critic.net.n_tiles * 4;
-    a.actor.partial_std = reinterpret_cast<float*>(p);
-    float* stats = a.actor.partial_std + (size_t)c.actor.teams * A;
+    uint8_t* p = static_cast<uint8_t*>(scratch);
+    for(PpoNetArgs* w : {&a.actor, &a.critic}){
+        w->partial = reinterpret_cast<float4*>(p); w->fresh = reinterpret_cast<float*>(w->partial + (size_t)w->teams * w->quads);
+        p += ppo_exchange_bytes(*w);
+    }
+    float* stats = reinterpret_cast<float*>(p);
     a.observations = observations; a.actions = actions; a.log_probs = log_probs; a.advantages = advantages; a.targets = target_values; a.stats = stats;
     a.ld = ld; a.batch = batch; a.minibatches = n_minibatches; a.action_dim = A;
     a.epsilon_clip = epsilon_clip; a.entropy_coefficient = entropy_coefficient; a.advantage_epsilon = advantage_epsilon;

@@ -649,6 +649,11 @@ int b200rl_shuffle_permutation_host(uint32_t* rng_state_host, int n_rows, int32_
 size_t b200rl_permute_rows_scratch_bytes(int n_rows, unsigned long long column_mask);
 int b200rl_permute_rows(float* data, int ld, int n_rows, const int32_t* perm, unsigned long long column_mask, void* scratch, size_t scratch_bytes,
                         b200rl_stream_t stream);
+/* Both for one epoch of a loop that shuffles again and again: the permutation is drawn into perm_host (page-locked) and sent to perm on copy_stream while kernels of
+ * the epoch before run on `stream`, which waits for it and permutes. sent, used: CUDA events that exist; with two sets of (perm_host, perm, sent, used) taken in turn, the
+ * host draws as soon as the copy of two epochs before is through (sent), the copy waits until the permutation of two epochs before has been applied (used). */
+int b200rl_shuffle_rows(float* data, int ld, int n_rows, unsigned long long column_mask, uint32_t* rng_state_host, int32_t* perm_host, int32_t* perm, void* scratch,
+                        size_t scratch_bytes, void* sent, void* used, b200rl_stream_t copy_stream, b200rl_stream_t stream);
 
 #ifdef __cplusplus
 }

@@ -180,6 +180,7 @@ def lib():
         L.b200rl_permute_rows_scratch_bytes.argtypes = [i, C.c_uint64]
         L.b200rl_permute_rows_scratch_bytes.restype = sz
         L.b200rl_permute_rows.argtypes = [vp, i, i, vp, C.c_uint64, vp, sz, vp]
+        L.b200rl_shuffle_rows.argtypes = [vp, i, i, C.c_uint64, vp, vp, vp, vp, sz, vp, vp, vp, vp]
         L.b200rl_pendulum_offpolicy_step.argtypes = [shape_p, vp, vp, vp, vp, vp, vp, vp, i, i, vp, vp, vp, vp, C.POINTER(ReplayLayout), vp, vp, vp, vp]
         L.b200rl_collect_tables_host.argtypes = [vp, i, i, vp, vp, i, vp, i, C.POINTER(i), vp]
         L.b200rl_sample_and_squash_forward.argtypes = [vp, i, vp, i, i, i, vp, vp, i, vp, vp]

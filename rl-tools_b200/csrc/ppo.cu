@@ -304,3 +304,21 @@ extern "C" int b200rl_permute_rows(float* data, int ld, int n_rows, const int32_
     B200RL_LAUNCH_CHECK("permute_rows");
     return B200RL_OK;
 }
+
+// Native, because a loop of small networks calls it every 100 us: as a dozen calls from Python it took 92 us of the host, more than an epoch's kernels (64 x 64 networks, 4,096 rows).
+extern "C" int b200rl_shuffle_rows(float* data, int ld, int n_rows, unsigned long long column_mask, uint32_t* rng, int32_t* perm_host, int32_t* perm, void* scratch,
+                                   size_t scratch_bytes, void* sent, void* used, b200rl_stream_t copy_stream, b200rl_stream_t stream){
+    if(!data || !rng || !perm_host || !perm || !sent || !used || n_rows < 0 || ld < 1 || (ld < 64 && (column_mask >> ld) != 0) ||
+       (n_rows > 0 && column_mask != 0 && (!scratch || scratch_bytes < b200rl_permute_rows_scratch_bytes(n_rows, column_mask)))) return B200RL_ERR_INVALID_ARGUMENT;
+    cudaStream_t copies = (cudaStream_t)copy_stream, s = (cudaStream_t)stream;
+    B200RL_CUDA_TRY(cudaEventSynchronize((cudaEvent_t)sent));
+    int rc = b200rl_shuffle_permutation_host(rng, n_rows, perm_host);
+    if(rc) return rc;
+    B200RL_CUDA_TRY(cudaStreamWaitEvent(copies, (cudaEvent_t)used, 0));
+    B200RL_CUDA_TRY(cudaMemcpyAsync(perm, perm_host, sizeof(int32_t) * (size_t)n_rows, cudaMemcpyHostToDevice, copies));
+    B200RL_CUDA_TRY(cudaEventRecord((cudaEvent_t)sent, copies));
+    B200RL_CUDA_TRY(cudaStreamWaitEvent(s, (cudaEvent_t)sent, 0));
+    if((rc = b200rl_permute_rows(data, ld, n_rows, perm, column_mask, scratch, scratch_bytes, stream))) return rc;
+    B200RL_CUDA_TRY(cudaEventRecord((cudaEvent_t)used, s));
+    return B200RL_OK;
+}

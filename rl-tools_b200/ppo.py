@@ -6,7 +6,7 @@ parameters of rl/algorithms/ppo/ppo.h:13-38. Everything runs on the GPU on torch
 """
 import ctypes as C
 
-from . import lib, check, _ptr, _stream, gae as _gae, mse_gradient as _mse_gradient, ppo_policy_gradient as _ppo_policy_gradient, permute_rows as _permute_rows, permute_rows_scratch as _permute_rows_scratch, shuffle_permutation_host as _shuffle_permutation_host
+from . import lib, check, _ptr, _stream, gae as _gae, mse_gradient as _mse_gradient, ppo_policy_gradient as _ppo_policy_gradient, permute_rows_scratch as _permute_rows_scratch
 
 
 class DatasetLayout:
@@ -160,31 +160,23 @@ def _epoch_call(actor, critic, dataset, layout, n_minibatches, batch_size, epsil
 class _Shuffle:
     """The epoch shuffle: the next epoch's permutation is drawn and sent, on a stream of its own and into the other of two buffers, while this one's kernels
     run (a copy in the stream of the kernels held the epoch up by 25 to 40 us). Both pairs of buffers, device and pinned, are kept: the host draws into a
-    pinned one once the copy out of it, two epochs before, has completed."""
+    pinned one once the copy out of it, two epochs before, has completed. An epoch is one native call."""
 
     def __init__(self, dataset, n_rows, columns):
         import torch
-        self.n_rows, self.columns, self.epoch = n_rows, columns, 0
+        self.n_rows, self.epoch = n_rows, 0
         self.scratch = _permute_rows_scratch(dataset, n_rows, columns)
         self.perm = torch.empty((2, n_rows), device=dataset.device, dtype=torch.int32)
         self.host = torch.empty((2, n_rows), dtype=torch.int32, pin_memory=True)
-        self.used = [torch.cuda.current_stream().record_event()] * 2
-        self.sent = [None, None]
         self.stream = torch.cuda.Stream(device=dataset.device)
+        self.used = [torch.cuda.current_stream().record_event() for _ in range(2)]
+        self.sent = [self.stream.record_event() for _ in range(2)]
 
     def __call__(self, dataset, rng_state):
-        import torch
-        main, k = torch.cuda.current_stream(), self.epoch & 1
-        if self.sent[k] is not None:
-            self.sent[k].synchronize()
-        _shuffle_permutation_host(rng_state, self.n_rows, self.host[k].data_ptr())
-        with torch.cuda.stream(self.stream):
-            self.stream.wait_event(self.used[k])
-            self.perm[k].copy_(self.host[k], non_blocking=True)
-            self.sent[k] = self.stream.record_event()
-        main.wait_event(self.sent[k])
-        _permute_rows(dataset, self.n_rows, self.perm[k], self.columns, self.scratch)
-        self.used[k] = main.record_event()
+        k = self.epoch & 1
+        mask, scratch, nbytes = self.scratch
+        check(lib().b200rl_shuffle_rows(dataset.data_ptr(), dataset.stride(0), self.n_rows, mask, rng_state.ctypes.data, self.host[k].data_ptr(), self.perm[k].data_ptr(),
+                                        scratch.data_ptr(), nbytes, self.sent[k].cuda_event, self.used[k].cuda_event, self.stream.cuda_stream, _stream()), "b200rl_shuffle_rows")
         self.epoch += 1
 
 

@@ -32,9 +32,15 @@
 // exactly the shared-memory tiles, stream through three 32 KB slots by bulk copies (every CTA reads all weights from L2 for each of its row tiles: 592
 // KB per tile of 64-256-256-256-16).
 //
+// Networks of at most 64 columns, input and outputs included (NARROW): a layer is one unit, 8 MMAs, and what a tile waits for is its own chain of MMAs, tensor-memory reads and splits,
+// not any unit's rate. Two CTAs of eight element-wise warps share an SM (80 KB of shared memory, half the tensor memory, 104 registers), a tile each, so that one's chain
+// fills the other's gaps; a warp owns columns 16 g ... + 15 of both halves of the piece, and two warps share a row. Wider networks need more than half an SM's shared memory.
+// Measured, one CTA of 16 warps / this: evaluate 27-64-64-8 at 524,288 rows 214 / 118 us (11 us at the copy bandwidth); forward and backward chain 29-64-64-5 at 404,405
+// rows 303 / 187 and 272 / 193 us (73 and 68), 31-32-32-32-1 at 251,600 rows 226 / 121 and 203 / 101 us.
+//
 // Bound by the tensor core and, between layers, by what the 16 warps do to a row tile before the next layer can start (about a third of the time), in
 // the forward pass by the stores. Measured, 64-256-256-256-16 at 1,048,576 rows: evaluate 3,236 -> 1,450 us (0.58 ms at the rate of three fp16
-// passes), forward 3,366 -> 2,850 us (6.8 GB, 1.0 ms at the copy bandwidth); 27-64-64-8 at 524,288 rows: evaluate 336 -> 218 us, forward 367 -> 369.
+// passes), forward 3,366 -> 2,850 us (6.8 GB, 1.0 ms at the copy bandwidth).
 // Backward, 64-256-256-256-16 at 1,048,576 rows: 3.04 ms for the chain of d_pre (6.5 GB; the products per layer and the passes over d_pre took 4.1 ms).
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -45,13 +51,20 @@
 namespace b200rl {
 
 namespace {
-constexpr int CH_ROWS = 128, CH_WARPS = 16, CH_THREADS = 32 * (CH_WARPS + 4), CH_MAX_STEPS = 8, CH_STAGES = 3;
+constexpr int CH_ROWS = 128, CH_MAX_STEPS = 8, CH_STAGES = 3, CH_NARROW = 64;
 constexpr uint32_t CH_TILE = 128 * 128;                           // one fp16 operand tile: 128 rows x 64 columns
-constexpr uint32_t CH_STAGE = 2 * CH_TILE;                        // a slot of the weights; a piece of the activations: both parts
-constexpr uint32_t CH_A = 4 * CH_STAGE;                           // both parts of four 64-column pieces of the activations
-constexpr uint32_t CH_EXP = 4 * CH_ROWS + 2 * 4 * CH_ROWS;        // exponents of the pieces' scales; two buffers of the four warps' exponents per row
-constexpr uint32_t CH_SMEM = CH_A + CH_STAGES * CH_STAGE + CH_EXP + 256 + 1024;
-static_assert(CH_SMEM <= 227 * 1024, "shared memory");
+constexpr uint32_t CH_PIECE = 2 * CH_TILE;                        // a piece of the activations: both parts
+constexpr uint32_t CH_EXP = 4 * CH_ROWS + 2 * 4 * CH_ROWS;        // exponents of the pieces' scales; two buffers of the warps' exponents per row
+// What a CTA consists of: an SM's worth, or half of it for networks of at most 64 columns (one piece, weights of one 64-row tile per part)
+template <bool NARROW> struct Chain {
+    static constexpr int WARPS = NARROW ? 8 : 16, THREADS = 32 * (WARPS + 4), PER_SM = NARROW ? 2 : 1;
+    static constexpr int REGISTERS = NARROW ? 104 : 112;          // of the element-wise warps; 32 of the others: together what the CTA is launched with (80, 96 per thread)
+    static constexpr int SLICES = NARROW ? 2 : 4, STEP = NARROW ? 32 : 64;   // slices of 16 columns of a warp; their distance
+    static constexpr uint32_t A = NARROW ? CH_PIECE : 4 * CH_PIECE, STAGE = NARROW ? CH_TILE : 2 * CH_TILE;
+    static constexpr uint32_t ACCUMULATOR = NARROW ? 128 : 256;   // columns of one of the two
+    static constexpr uint32_t SMEM = A + CH_STAGES * STAGE + CH_EXP + 256 + 1024;
+};
+static_assert(Chain<false>::SMEM <= 227 * 1024 && Chain<true>::SMEM <= 113 * 1024, "shared memory");
 constexpr size_t CH_TAIL = (3 * 256 + 4) * sizeof(float);        // behind an image: see ChainStep::tail
 constexpr uint32_t CH_OWN_SCALE = 12;                             // powers of two below the layer's largest weight from which on an output has its own scale
 constexpr long long CH_WAIT_LIMIT = 2000000000LL;
@@ -202,12 +215,15 @@ __device__ __forceinline__ void prefetch_rows(const float* p, long long ld, int 
 }
 }  // namespace
 
-template <int MODE>
-__global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_constant__ ChainArgs a){
+template <int MODE, bool NARROW>
+__global__ void __launch_bounds__(Chain<NARROW>::THREADS, Chain<NARROW>::PER_SM) mlp_chain_kernel(const __grid_constant__ ChainArgs a){
+    typedef Chain<NARROW> H;
     constexpr bool ROWS = MODE == CH_EVALUATE;                          // only the last outputs go to memory
+    constexpr int CH_WARPS = H::WARPS;
+    constexpr uint32_t CH_STAGE = H::STAGE;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
-    uint8_t* stages = base + CH_A;
+    uint8_t* stages = base + H::A;
     uint8_t* exps = stages + CH_STAGES * CH_STAGE;                      // [piece][row], then two exchange buffers [row][warp of the row]
     uint64_t* bars = reinterpret_cast<uint64_t*>(exps + CH_EXP);
     uint64_t* w_full = bars; uint64_t* w_empty = bars + CH_STAGES; uint64_t* acc_full = bars + 2 * CH_STAGES; uint64_t* acc_empty = acc_full + 2;
@@ -224,7 +240,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
         for(int i = 0; i < 4; i++) tc::mbar_init(a_full + i, CH_WARPS);
         tc::fence_mbar_init(); *abort_flag = 0;
     }
-    if(warp == CH_WARPS){ tc::tmem_alloc(slot, 512); tc::tmem_relinquish(); }
+    if(warp == CH_WARPS){ tc::tmem_alloc(slot, 2 * H::ACCUMULATOR); tc::tmem_relinquish(); }
     tc::fence_before_thread_sync();
     __syncthreads();
     tc::fence_after_thread_sync();
@@ -248,15 +264,15 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
                 for(int st = 0; st < a.n_steps && ok; st++){
                     const ChainStep& y = a.step[st];
                     const int pieces = y.pieces, K = y.K, n = y.n;
-                    const bool stacked = n <= 128;
+                    const bool stacked = NARROW || n <= 128;
                     const uint32_t idesc = tc::make_idesc_f16(CH_ROWS, stacked ? 2 * n : n);
                     for(int c = 0; c < pieces; c++, u++, w += stacked ? 1u : 2u){
                         if(!(ok = wait(a_full + c, (ready >> c) & 1u))) break;
                         ready ^= 1u << c;
                         if((u & 1u) != mine) continue;
                         const int ksteps = min(4, (K - 64 * c + 15) / 16);
-                        const uint64_t lead = tc::make_desc_kmajor_sw128(tc::smem_u32(base + c * CH_STAGE)), rest = lead + (CH_TILE >> 4);
-                        const uint32_t d = tmem + (u & 1u) * 256, s0 = w % CH_STAGES;
+                        const uint64_t lead = tc::make_desc_kmajor_sw128(tc::smem_u32(base + c * CH_PIECE)), rest = lead + (CH_TILE >> 4);
+                        const uint32_t d = tmem + (u & 1u) * H::ACCUMULATOR, s0 = w % CH_STAGES;
                         if(!(ok = wait(acc_empty + (u & 1u), ((u >> 1) & 1u) ^ 1u))) break;
                         if(!(ok = wait(w_full + s0, (w / CH_STAGES) & 1u))) break;
                         const uint32_t s1 = (w + 1) % CH_STAGES;
@@ -295,7 +311,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
                 for(int st = 0; st < a.n_steps && ok; st++){
                     const ChainStep& y = a.step[st];
                     const uint32_t part = (uint32_t)y.n * 128;
-                    const bool stacked = y.n <= 128;
+                    const bool stacked = NARROW || y.n <= 128;
                     const uint8_t* unit = y.image;
                     if constexpr(MODE == CH_BACKWARD){                  // what the element-wise part will read, into L2 about a layer's MMAs ahead of it
                         if(y.act != B200RL_ACT_IDENTITY) prefetch_rows(y.pre_in, y.N, tile * CH_ROWS, a.rows);
@@ -320,56 +336,68 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
         }
     }
     else{
-        tc::setmaxnreg_inc<112>();
-        const int q = warp & 3, g = warp >> 2;                          // rows (TMEM lanes) 32 q ... + 31; columns 16 g ... + 15 of every piece
+        tc::setmaxnreg_inc<H::REGISTERS>();
+        const int q = warp & 3, g = warp >> 2;                          // rows (TMEM lanes) 32 q ... + 31; columns 16 g ... + 15 of every piece, of every half of the only piece
         const uint32_t tmem_lane = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(16 * g);
         uint32_t u = 0, exchange = 0;                                   // running unit; running exchange of exponents
         bool ok = true;
-        // this warp's slice of a piece of the next operand: scaled by the largest magnitude of each row in the piece, split, stored
-        auto store_operand = [&](int piece, const Slice& v){
-            uint8_t* buffer = exps + 4 * CH_ROWS + (exchange & 1u) * 4 * CH_ROWS + 4 * q * 32;
+        // this warp's slices of a piece of the next operand (one, or the first `n` of a narrow network's two): scaled by the largest magnitude of each row in the piece, split, stored
+        auto store_operand = [&](int piece, const Slice* v, int n){
+            constexpr int PER_ROW = NARROW ? 2 : 4;                      // warps that share a row
+            uint8_t* buffer = exps + 4 * CH_ROWS + (exchange & 1u) * 4 * CH_ROWS + PER_ROW * q * 32;
             exchange++;
             constexpr int SLOTS = ROWS ? 1 : 4, PER = 8 / SLOTS;
 #pragma unroll
             for(int s = 0; s < SLOTS; s++){
                 float m0 = 0.0f, m1 = 0.0f;
 #pragma unroll
-                for(int j = 0; j < PER; j++){ m0 = fmaxf(m0, fabsf(v[s * PER + j].x)); m1 = fmaxf(m1, fabsf(v[s * PER + j].y)); }
+                for(int p = 0; p < (NARROW ? 2 : 1); p++){
+                    if(p >= n) break;
+#pragma unroll
+                    for(int j = 0; j < PER; j++){ m0 = fmaxf(m0, fabsf(v[p][s * PER + j].x)); m1 = fmaxf(m1, fabsf(v[p][s * PER + j].y)); }
+                }
                 float m = fmaxf(m0, m1);
                 if constexpr(!ROWS){
                     m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
                     m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
                 }
-                if(ROWS || (lane & 3) == 0) buffer[4 * Spread<ROWS>::row(lane, s * PER) + g] = (uint8_t)scale_exponent(m);
+                if(ROWS || (lane & 3) == 0) buffer[PER_ROW * Spread<ROWS>::row(lane, s * PER) + g] = (uint8_t)scale_exponent(m);
             }
-            tc::named_barrier_sync(1 + q, 128);                          // the four warps of these rows; all of them have read the previous layer's sums
-            uint8_t* tile_lead = base + piece * CH_STAGE;
+            tc::named_barrier_sync(1 + q, 32 * PER_ROW);                 // the warps of these rows; all of them have read the previous layer's sums
+            uint8_t* tile_lead = base + piece * CH_PIECE;
             const float2 zero = make_float2(0.0f, 0.0f);
 #pragma unroll
             for(int s = 0; s < SLOTS; s++){
                 const int r = Spread<ROWS>::row(lane, s * PER);
-                const uint32_t four = *reinterpret_cast<const uint32_t*>(buffer + 4 * r);
-                const uint32_t e = max(max(four & 0xFFu, (four >> 8) & 0xFFu), max((four >> 16) & 0xFFu, four >> 24));
+                uint32_t e;
+                if constexpr(NARROW){
+                    const uint32_t two = *reinterpret_cast<const uint16_t*>(buffer + 2 * r);
+                    e = max(two & 0xFFu, two >> 8);
+                }
+                else{
+                    const uint32_t four = *reinterpret_cast<const uint32_t*>(buffer + 4 * r);
+                    e = max(max(four & 0xFFu, (four >> 8) & 0xFFu), max((four >> 16) & 0xFFu, four >> 24));
+                }
                 if(g == 0 && (ROWS || (lane & 3) == 0)) exps[piece * CH_ROWS + q * 32 + r] = (uint8_t)e;
                 const float2 f = make_float2(scale_of(e), scale_of(e));
                 const uint32_t row = (uint32_t)(q * 32 + r), x = row & 7u;
-                uint32_t lead[PER], rest[PER];
 #pragma unroll
-                for(int j = 0; j < PER; j++) split_pair(__ffma2_rn(v[s * PER + j], f, zero), lead[j], rest[j]);
-                if constexpr(ROWS){
+                for(int p = 0; p < (NARROW ? 2 : 1); p++){
+                    if(p >= n) break;
+                    uint32_t lead[PER], rest[PER];
 #pragma unroll
-                    for(int j = 0; j < 2; j++){
-                        const uint32_t off = row * 128 + (((uint32_t)(2 * g + j) ^ x) << 4);
-                        *reinterpret_cast<uint4*>(tile_lead + off) = make_uint4(lead[4 * j], lead[4 * j + 1], lead[4 * j + 2], lead[4 * j + 3]);
-                        *reinterpret_cast<uint4*>(tile_lead + CH_TILE + off) = make_uint4(rest[4 * j], rest[4 * j + 1], rest[4 * j + 2], rest[4 * j + 3]);
-                    }
-                }
-                else{
+                    for(int j = 0; j < PER; j++) split_pair(__ffma2_rn(v[p][s * PER + j], f, zero), lead[j], rest[j]);
 #pragma unroll
                     for(int j = 0; j < 2; j++){
-                        const uint32_t off = row * 128 + (((uint32_t)(2 * g + j) ^ x) << 4) + (uint32_t)(lane & 3) * 4;
-                        *reinterpret_cast<uint32_t*>(tile_lead + off) = lead[j];
-                        *reinterpret_cast<uint32_t*>(tile_lead + CH_TILE + off) = rest[j];
+                        const uint32_t off = row * 128 + (((uint32_t)(4 * p + 2 * g + j) ^ x) << 4) + (ROWS ? 0u : (uint32_t)(lane & 3) * 4);
+                        if constexpr(ROWS){
+                            *reinterpret_cast<uint4*>(tile_lead + off) = make_uint4(lead[4 * j], lead[4 * j + 1], lead[4 * j + 2], lead[4 * j + 3]);
+                            *reinterpret_cast<uint4*>(tile_lead + CH_TILE + off) = make_uint4(rest[4 * j], rest[4 * j + 1], rest[4 * j + 2], rest[4 * j + 3]);
+                        }
+                        else{
+                            *reinterpret_cast<uint32_t*>(tile_lead + off) = lead[j];
+                            *reinterpret_cast<uint32_t*>(tile_lead + CH_TILE + off) = rest[j];
+                        }
                     }
                 }
             }
@@ -377,9 +405,12 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
             __syncwarp();
             if(lane == 0) tc::mbar_arrive(a_full + piece);
         };
+        const int column = 16 * g;                                       // of slice p: column + STEP p
+        // pieces of STEP columns in n of them
+        auto slices = [](int n){ return (n + H::STEP - 1) / H::STEP; };
         // this warp's slice of a piece of a tile's inputs
         auto load_input = [&](int tile, int piece, Slice& v){
-            load_slice<ROWS>(Place{tile * CH_ROWS + q * 32, 64 * piece + 16 * g, a.rows, a.in_cols, a.ld_in}, a.in, lane, v);
+            load_slice<ROWS>(Place{tile * CH_ROWS + q * 32, H::STEP * piece + column, a.rows, a.in_cols, a.ld_in}, a.in, lane, v);
         };
         const bool some_own = __any_sync(0xffffffffu, (own_flags.x | own_flags.y) != 0u);        // some output of the network has a scale of its own
         Slice acc[4];                                                   // this layer's sums, a slice per piece
@@ -387,32 +418,41 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
         for(int tile = blockIdx.x; tile < a.tiles && ok; tile += gridDim.x){
             const int row0 = tile * CH_ROWS + q * 32;
             // ---- the first layer's input (every MMA of the previous tile has completed: its last unit was drained) ----
+            const int ins = slices(a.in_cols);
 #pragma unroll
-            for(int p = 0; p < 4; p++){
-                if(p >= a.step[0].pieces) break;
+            for(int p = 0; p < H::SLICES; p++){
+                if(p >= ins) break;
+                Slice& v = NARROW ? acc[MODE == CH_BACKWARD ? p : 2 + p] : acc[MODE == CH_BACKWARD ? 0 : p < 2 ? 2 + p : p - 2];
                 if constexpr(MODE == CH_BACKWARD){
-                    const Place at{row0, 64 * p + 16 * g, a.rows, a.in_cols, a.ld_in};
-                    load_slice<ROWS>(at, a.in, lane, acc[0]);
+                    const Place at{row0, H::STEP * p + column, a.rows, a.in_cols, a.ld_in};
+                    load_slice<ROWS>(at, a.in, lane, v);
                     if(a.in_act != B200RL_ACT_IDENTITY){
-                        load_slice<ROWS>(Place{at.row0, at.col0, a.rows, a.in_cols, a.in_cols}, a.in_pre, lane, acc[1]);
-                        differentiate_slice_rt(acc[0], acc[1], a.in_act);
-                        clear_beyond<ROWS>(at.col0, a.in_cols, lane, acc[0]);
+                        Slice& pre = acc[NARROW ? 2 : 1];
+                        load_slice<ROWS>(Place{at.row0, at.col0, a.rows, a.in_cols, a.in_cols}, a.in_pre, lane, pre);
+                        differentiate_slice_rt(v, pre, a.in_act);
+                        clear_beyond<ROWS>(at.col0, a.in_cols, lane, v);
                     }
-                    store_operand(p, acc[0]);
-                    if(a.in_out) store_slice<ROWS>(Place{at.row0, at.col0, a.rows, a.in_cols, a.ld_in_out}, a.in_out, lane, acc[0]);
                 }
-                else if(p < 2){ if(!loaded) load_input(tile, p, acc[2 + p]); store_operand(p, acc[2 + p]); }
-                else{ load_input(tile, p, acc[p - 2]); store_operand(p, acc[p - 2]); }
+                else if(p >= 2 || !loaded) load_input(tile, p, v);
+                if(!NARROW) store_operand(p, &v, 1);
+                if(!NARROW && MODE == CH_BACKWARD && a.in_out) store_slice<ROWS>(Place{row0, H::STEP * p + column, a.rows, a.in_cols, a.ld_in_out}, a.in_out, lane, v);
+            }
+            if constexpr(NARROW){
+                store_operand(0, acc + (MODE == CH_BACKWARD ? 0 : 2), ins);
+                if(MODE == CH_BACKWARD && a.in_out){
+#pragma unroll
+                    for(int p = 0; p < H::SLICES; p++) if(p < ins) store_slice<ROWS>(Place{row0, H::STEP * p + column, a.rows, a.in_cols, a.ld_in_out}, a.in_out, lane, acc[p]);
+                }
             }
             loaded = false;
             for(int st = 0; st < a.n_steps && ok; st++){
                 const ChainStep& y = a.step[st];
-                const bool last = st + 1 == a.n_steps, stacked = y.n <= 128;
-                const int outs = (y.N + 63) / 64;                       // pieces of the output
+                const bool last = st + 1 == a.n_steps, stacked = NARROW || y.n <= 128;
+                const int outs = slices(y.N);                           // of the output
 #pragma unroll
-                for(int p = 0; p < 4; p++){                              // the sums start with the bias
+                for(int p = 0; p < H::SLICES; p++){                      // the sums start with the bias
                     if(p >= outs) break;
-                    const float* at = y.tail + 64 * p + 16 * g;
+                    const float* at = y.tail + H::STEP * p + column;
                     if constexpr(ROWS){
 #pragma unroll
                         for(int j = 0; j < 4; j++){
@@ -431,14 +471,14 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
                 }
                 if(MODE != CH_BACKWARD && last && stacked && tile + (int)gridDim.x < a.tiles){  // a narrow last layer leaves room for the next tile's inputs
                     load_input(tile + gridDim.x, 0, acc[2]);
-                    if(a.step[0].pieces > 1) load_input(tile + gridDim.x, 1, acc[3]);
+                    if(ins > 1) load_input(tile + gridDim.x, 1, acc[3]);
                     loaded = true;
                 }
                 const float weights = __ldg(y.tail + 768);              // inverse of the weights' scale
                 Slice below;                                             // backward: pre-activations of the next piece
                 for(int c = 0; c < y.pieces; c++, u++){
                     if constexpr(MODE == CH_BACKWARD){
-                        if(c + 1 == y.pieces && y.act != B200RL_ACT_IDENTITY) load_slice<ROWS>(Place{row0, 16 * g, a.rows, y.N, y.N}, y.pre_in, lane, below);
+                        if(c + 1 == y.pieces && y.act != B200RL_ACT_IDENTITY) load_slice<ROWS>(Place{row0, column, a.rows, y.N, y.N}, y.pre_in, lane, below);
                     }
                     if(!(ok = wait(acc_full + (u & 1u), (u >> 1) & 1u))) break;
                     tc::fence_after_thread_sync();
@@ -446,17 +486,17 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
                     float inv[ROWS ? 1 : 4];
 #pragma unroll
                     for(int s = 0; s < (ROWS ? 1 : 4); s++) inv[s] = weights * inverse_scale_of(e[Spread<ROWS>::row(lane, 2 * s)]);
-                    const uint32_t from = tmem_lane + (u & 1u) * 256;
+                    const uint32_t from = tmem_lane + (u & 1u) * H::ACCUMULATOR;
 #pragma unroll
-                    for(int p = 0; p < 4; p++){
+                    for(int p = 0; p < H::SLICES; p++){
                         if(p >= outs) break;
                         uint32_t d[16], d2[16];
                         auto read = [&](uint32_t column, uint32_t (&r)[16]){
                             if constexpr(ROWS) ld_32x32b_x16(from + column, r);
                             else{ ld_16x256b_x2(from + column, r); ld_16x256b_x2(from + column + (16u << 16), r + 8); }
                         };
-                        read((uint32_t)(64 * p), d);
-                        if(p < 2 && stacked) read((uint32_t)(64 * p + y.n), d2);       // stacked parts: both column ranges
+                        read((uint32_t)(H::STEP * p), d);
+                        if(p < 2 && stacked) read((uint32_t)(H::STEP * p + y.n), d2);  // stacked parts: both column ranges
                         tc::tmem_wait_ld();
 #pragma unroll
                         for(int i = 0; i < 8; i++){
@@ -475,33 +515,34 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
                 if(!ok) break;
                 if(some_own){                                           // one test per layer: it stands between this layer's MMAs and the next one's
 #pragma unroll
-                    for(int p = 0; p < 4; p++){
+                    for(int p = 0; p < H::SLICES; p++){
                         if(p >= outs) break;
-                        finish_sums<ROWS>(y.tail + 256 + 64 * p + 16 * g, lane, acc[p]);
+                        finish_sums<ROWS>(y.tail + 256 + H::STEP * p + column, lane, acc[p]);
                     }
                 }
                 // every MMA of this layer has completed: its input may be overwritten
 #pragma unroll
-                for(int p = 0; p < 4; p++){
+                for(int p = 0; p < H::SLICES; p++){
                     if(p >= outs) break;
-                    const Place at{row0, 64 * p + 16 * g, a.rows, y.N, y.ld};
+                    const Place at{row0, H::STEP * p + column, a.rows, y.N, y.ld};
                     if constexpr(MODE == CH_FORWARD) store_slice<ROWS>(at, y.pre, lane, acc[p]);
                     if constexpr(MODE == CH_BACKWARD){
                         if(y.act != B200RL_ACT_IDENTITY){
                             differentiate_slice_rt(acc[p], below, y.act);
-                            if(p + 1 < outs) load_slice<ROWS>(Place{row0, at.col0 + 64, a.rows, y.N, y.N}, y.pre_in, lane, below);
+                            if(p + 1 < outs) load_slice<ROWS>(Place{row0, at.col0 + H::STEP, a.rows, y.N, y.N}, y.pre_in, lane, below);
                         }
                     }
                     else activate_slice_rt(acc[p], y.act);
                     clear_beyond<ROWS>(at.col0, y.N, lane, acc[p]);
-                    if(!last) store_operand(p, acc[p]);
+                    if(!last){ if(!NARROW) store_operand(p, acc + p, 1); }
                     else if(MODE != CH_BACKWARD || y.out) store_slice<ROWS>(at, y.out, lane, acc[p]);
                 }
+                if(NARROW && !last) store_operand(0, acc, outs);
                 if(MODE != CH_EVALUATE && !last && (MODE == CH_FORWARD || y.out)){
 #pragma unroll
-                    for(int p = 0; p < 4; p++){
+                    for(int p = 0; p < H::SLICES; p++){
                         if(p >= outs) break;
-                        store_slice<ROWS>(Place{row0, 64 * p + 16 * g, a.rows, y.N, y.ld}, y.out, lane, acc[p]);
+                        store_slice<ROWS>(Place{row0, H::STEP * p + column, a.rows, y.N, y.ld}, y.out, lane, acc[p]);
                     }
                 }
             }
@@ -509,7 +550,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) mlp_chain_kernel(const __grid_c
     }
     tc::fence_before_thread_sync();
     __syncthreads();
-    if(warp == CH_WARPS) tc::tmem_dealloc(tmem, 512);
+    if(warp == CH_WARPS) tc::tmem_dealloc(tmem, 2 * H::ACCUMULATOR);
 }
 
 // ---- weight images: a CTA per 32 output rows of a product, a warp per row. Every CTA finds the
@@ -637,25 +678,33 @@ static void chain_step(ChainStep& y, ChainImages& images, const float* W, const 
     y.image = m.image; y.tail = m.tail;
     ws += chain_image_bytes(N, K);
 }
-template <int MODE>
-static int launch_chain(ChainArgs& a, const ChainImages& images, cudaStream_t s, bool with_images = true){
+template <int MODE, bool NARROW>
+static int launch_chain_kernel(ChainArgs& a, cudaStream_t s){
+    typedef Chain<NARROW> H;
     static std::atomic<bool> configured[MAX_DEVICES];
     int dev = 0, sms = 0;
     int rc = current_device(&dev);
     if(rc) return rc;
     if((rc = sm_count(&sms))) return rc;
     if(!configured[dev].load(std::memory_order_acquire)){
-        B200RL_CUDA_TRY(cudaFuncSetAttribute(mlp_chain_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_SMEM));
+        B200RL_CUDA_TRY(cudaFuncSetAttribute((mlp_chain_kernel<MODE, NARROW>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)H::SMEM));
         configured[dev].store(true, std::memory_order_release);
     }
+    a.tiles = (a.rows + CH_ROWS - 1) / CH_ROWS;
+    const int ctas = H::PER_SM * sms;
+    mlp_chain_kernel<MODE, NARROW><<<a.tiles < ctas ? a.tiles : ctas, H::THREADS, H::SMEM, s>>>(a);
+    B200RL_LAUNCH_CHECK("mlp_chain");
+    return B200RL_OK;
+}
+template <int MODE>
+static int launch_chain(ChainArgs& a, const ChainImages& images, cudaStream_t s, bool with_images = true){
     if(with_images){
         chain_image_kernel<<<images.blocks, 1024, 0, s>>>(images);
         B200RL_LAUNCH_CHECK("chain_image");
     }
-    a.tiles = (a.rows + CH_ROWS - 1) / CH_ROWS;
-    mlp_chain_kernel<MODE><<<a.tiles < sms ? a.tiles : sms, CH_THREADS, CH_SMEM, s>>>(a);
-    B200RL_LAUNCH_CHECK("mlp_chain");
-    return B200RL_OK;
+    bool narrow = true;
+    for(int l = 0; l < a.n_steps; l++) narrow = narrow && a.step[l].N <= CH_NARROW && a.step[l].K <= CH_NARROW;
+    return narrow ? launch_chain_kernel<MODE, true>(a, s) : launch_chain_kernel<MODE, false>(a, s);
 }
 
 // pre == NULL: evaluate into y; otherwise forward into the arenas

@@ -108,6 +108,15 @@ def test_backward_matches_fp64(lib, rows, I, dims, acts, mode):
         assert float((err - 1e-5 * size).max()) <= 1e-6 / rows
 
 
+@pytest.mark.parametrize("rows,I,dims,acts", [
+    (16385, 64, [64, 64, 64], ["tanh", "relu", "identity"]), (16400, 1, [16, 32, 17, 33, 48, 64, 64, 1], ["tanh"] * 8), (2 * 2 * 148 * 128 + 5, 33, [32, 31, 64, 2], ["sigmoid", "tanh", "fast_tanh", "tanh"]),
+    (16385, 65, [64, 64, 3], ["tanh", "tanh", "identity"]), (16385, 64, [64, 65, 3], ["tanh", "tanh", "identity"])])
+def test_networks_of_at_most_64_columns(lib, rows, I, dims, acts):
+    """The kernels of two CTAs per SM: both sides of their line, operands of one and of both halves of a piece, more row tiles than two per SM; with the tolerances of the tests above."""
+    test_forward_and_evaluate_match_fp64(lib, rows, I, dims, acts, False)
+    test_backward_matches_fp64(lib, rows, I, dims, acts, "both")
+
+
 @pytest.mark.parametrize("rows,I,dims", [(2048, 64, [256, 256, 16]), (4099, 64, [256, 256, 16]), (2100, 200, [130, 129]), (8192, 27, [64, 64, 8]), (16390, 27, [64, 64, 8]), (8200, 100, [33, 128, 7])])
 def test_weights_far_below_the_largest_of_their_layer(lib, rows, I, dims):
     """Every third output of a layer has weights 2^-24 of the layer's largest, and so has every third input (a column, which is an output of the

@@ -8,6 +8,7 @@
 // association, division and square root are IEEE, so a step gives the reference's CPU bits.
 #include "common.cuh"
 #include "rollout.cuh"
+#include <atomic>
 
 namespace b200rl {
 
@@ -30,8 +31,18 @@ __device__ __forceinline__ void l2f_matvec(const float (&A)[3][3], const float* 
 }
 __device__ __forceinline__ float l2f_clamp(float x, float lo, float hi){ return x < lo ? lo : (x > hi ? hi : x); }
 
+// what the constant disturbances add to every evaluation of the dynamics in a step (StateRandomForce, 60_dynamics.h:77-88)
+struct L2fDisturbance { float inverse_mass, acceleration[3], angular_acceleration[3]; };
+__device__ __forceinline__ L2fDisturbance l2f_disturbance(const L2fDynamics& p, const L2fState& s){
+    L2fDisturbance c;
+    c.inverse_mass = 1 / p.mass;
+#pragma unroll
+    for(int i = 0; i < 3; i++) c.acceleration[i] = s.force[i] / p.mass;
+    l2f_matvec(p.J_inv, s.torque, c.angular_acceleration);
+    return c;
+}
 // 60_dynamics.h: the rotor speeds in the state drive the body, the set-points drive the rotors
-__device__ __forceinline__ void l2f_dynamics(const L2fDynamics& p, const L2fState& s, const float (&setpoint)[4], L2fState& d){
+__device__ __forceinline__ void l2f_dynamics(const L2fDynamics& p, const L2fState& s, const float (&setpoint)[4], const L2fDisturbance& c, L2fState& d){
     float thrust[3] = {0, 0, 0}, torque[3] = {0, 0, 0};
 #pragma unroll
     for(int r = 0; r < 4; r++){
@@ -66,9 +77,8 @@ __device__ __forceinline__ void l2f_dynamics(const L2fDynamics& p, const L2fStat
     for(int i = 0; i < 3; i++) rotated[i] += var[i] * q[0];
 #pragma unroll
     for(int i = 0; i < 3; i++) rotated[i] += thrust[i];
-    const float inverse_mass = 1 / p.mass;
 #pragma unroll
-    for(int i = 0; i < 3; i++) d.linear_velocity[i] = rotated[i] * inverse_mass;
+    for(int i = 0; i < 3; i++) d.linear_velocity[i] = rotated[i] * c.inverse_mass;
 #pragma unroll
     for(int i = 0; i < 3; i++) d.linear_velocity[i] += p.gravity[i];
     float v1[3], v2[3];
@@ -78,11 +88,7 @@ __device__ __forceinline__ void l2f_dynamics(const L2fDynamics& p, const L2fStat
     for(int i = 0; i < 3; i++) v1[i] = torque[i] - v2[i];
     l2f_matvec(p.J_inv, v1, d.angular_velocity);
 #pragma unroll
-    for(int i = 0; i < 3; i++) d.linear_velocity[i] += s.force[i] / p.mass;      // StateRandomForce, 60_dynamics.h:77-88
-    float extra[3];
-    l2f_matvec(p.J_inv, s.torque, extra);
-#pragma unroll
-    for(int i = 0; i < 3; i++) d.angular_velocity[i] += extra[i];
+    for(int i = 0; i < 3; i++){ d.linear_velocity[i] += c.acceleration[i]; d.angular_velocity[i] += c.angular_acceleration[i]; }
 #pragma unroll
     for(int r = 0; r < 4; r++){                                                  // StateRotors, :89-101
         const float tau = setpoint[r] >= s.rpm[r] ? p.rotor_time_constants_rising[r] : p.rotor_time_constants_falling[r];
@@ -114,13 +120,18 @@ __device__ __forceinline__ void l2f_step(const L2fArgs& a, const L2fState& s, co
         setpoint[i] = act * half_range + p.action_min + half_range;
     }
     const float dt = a.dt;
-    L2fState k1 = s, k2 = s, k3 = s, k4 = s, t;
-    l2f_dynamics(p, s, setpoint, k1);
-    t = s; l2f_axpy(k1, dt / 2, t); l2f_dynamics(p, t, setpoint, k2);
-    t = s; l2f_axpy(k2, dt / 2, t); l2f_dynamics(p, t, setpoint, k3);
-    t = s; l2f_axpy(k3, dt, t);     l2f_dynamics(p, t, setpoint, k4);
+    const L2fDisturbance c = l2f_disturbance(p, s);
+    // The four stages in a loop, and the sum over them as they come: k1 dt / 6, then k2 dt / 3, k3 dt / 3, k4 dt / 6. Unrolled, the code of a step is too long for the
+    // instruction caches near a warp and fetching it takes longer than executing it (50 steps of 32,768 quadrotors 1,225 -> 1,060 us, of 16,384 734 -> 684).
+    L2fState t = s, k = s;
     next = s;
-    l2f_axpy(k1, dt / 6, next); l2f_axpy(k2, dt / 3, next); l2f_axpy(k3, dt / 3, next); l2f_axpy(k4, dt / 6, next);
+#pragma unroll 1
+    for(int stage = 0; stage < 4; stage++){
+        l2f_dynamics(p, t, setpoint, c, k);
+        l2f_axpy(k, stage == 0 || stage == 3 ? dt / 6 : dt / 3, next);
+        t = s;
+        l2f_axpy(k, stage == 2 ? dt : dt / 2, t);
+    }
     float norm = 0;                                                          // 70_post_integration.h:21-34
 #pragma unroll
     for(int i = 0; i < 4; i++) norm += next.orientation[i] * next.orientation[i];
@@ -305,7 +316,7 @@ __device__ __forceinline__ float l2f_reward(const L2fArgs& a, const float (&mdp)
 }
 
 // One CTA of up to 14 warps per SM: 448 quadrotors, so 65536 of them (443 per SM) are resident at once; fewer quadrotors take CTAs of as many
-// warps as spread them over all SMs (launch_l2f_rollout). A lane owns one quadrotor for the
+// warps as spread them over all SMs (launch_l2f_rollout), few ones the kernel behind this one's helpers. A lane owns one quadrotor for the
 // environment part (reset, observe, step, reward) and, for the two hidden layers, a register tile of 8 quadrotors x H/8 units of its warp's
 // 32 x H product: operands come from shared memory as 16-byte loads that each feed 32 multiply-adds (one broadcast weight per multiply-add,
 // as a thread-per-quadrotor layer would load it, leaves the kernel bound by shared-memory wavefronts). Every unit still accumulates
@@ -364,6 +375,160 @@ __device__ __forceinline__ void l2f_tile_store(float* hid, float2 (&acc)[8][H / 
     }
 }
 
+// The same rollout for fewer quadrotors: up to 128 per SM, where a warp for each 32 of them leaves every scheduler with one warp, and a step lasts as long as that one takes
+// for the actor and the dynamics one after the other. Four warps share 32 quadrotors: each computes a quarter of a layer's units (a lane four quadrotors x H / 16 units) and
+// one of the four actions; the first one owns the states and does the environment part, while the others write the observations out, in memory order. Sums in the same
+// order, so the same bits. Bound by the latency of the dynamics' chain in the owner's warp. us for 50 steps, a warp / four warps per 32 quadrotors:
+//   64 x 64 actor   64: 607 / 381, 9,000: 610 / 430, 16,384: 684 / 542, 18,944: 686 / 561       32 x 32 actor   500: 394 / 301, 9,000: 401 / 339, 16,384: 417 / 382
+//   16 x 16 actor   500: 308 / 290, 5,000: 317 / 313, 9,000: 322 / 323, 16,384: 341 / 366 (little to share out): up to 64 per SM
+constexpr int L2F_SHARED_WARPS = 4, L2F_SHARED_GROUPS = 4, L2F_SHARED_THREADS = 32 * L2F_SHARED_WARPS * L2F_SHARED_GROUPS;
+template <int H>
+struct L2fSharedLayout {
+    static constexpr int O = 18, A = 4, UNITS = H / 16, PITCH = 36;      // units per lane: those from (H / 4) warp + UNITS (lane & 3) on
+    static constexpr int W1T = 0, B1 = W1T + O * H, W2T = B1 + H, B2 = W2T + H * H, W3T = B2 + H, B3 = W3T + A * H, GROUP0 = B3 + A;       // weights transposed: [k][unit], the last [unit][4]
+    static constexpr int OBS = 0, HID1 = 2 * O * 32, HID2 = HID1 + H * PITCH, OUT = HID2 + H * PITCH, PER_GROUP = OUT + A * 32;           // observations of this step and of the next
+    static constexpr size_t bytes(int groups){ return sizeof(float) * (GROUP0 + (size_t)groups * PER_GROUP); }
+};
+template <int H, int K, int ACT_PITCH>
+__device__ __forceinline__ void l2f_shared_layer(const float* __restrict__ in, const float* __restrict__ wT, const float* __restrict__ bias, float* __restrict__ out, int first_unit, int eg, int act){
+    using L = L2fSharedLayout<H>;
+    constexpr int U = L::UNITS, PAIRS = (U + 1) / 2;
+    float2 acc[4][PAIRS];
+#pragma unroll
+    for(int p = 0; p < PAIRS; p++){
+        const float2 b = make_float2(bias[first_unit + 2 * p], U > 1 ? bias[first_unit + 2 * p + 1] : 0.0f);
+#pragma unroll
+        for(int ee = 0; ee < 4; ee++) acc[ee][p] = b;
+    }
+#pragma unroll 4
+    for(int k = 0; k < K; k++){
+        const float4 xv = *reinterpret_cast<const float4*>(in + k * ACT_PITCH + 4 * eg);
+        const float x[4] = {xv.x, xv.y, xv.z, xv.w};
+        const float* src = wT + k * H + first_unit;
+        float2 w[PAIRS];
+        if constexpr(U == 4){ const float4 t = *reinterpret_cast<const float4*>(src); w[0] = make_float2(t.x, t.y); w[1] = make_float2(t.z, t.w); }
+        else if constexpr(U == 2) w[0] = *reinterpret_cast<const float2*>(src);
+        else w[0] = make_float2(src[0], 0.0f);
+#pragma unroll
+        for(int ee = 0; ee < 4; ee++){
+#pragma unroll
+            for(int p = 0; p < PAIRS; p++){
+                if constexpr(U == 1) acc[ee][p].x = fmaf(w[p].x, x[ee], acc[ee][p].x);
+                else acc[ee][p] = __ffma2_rn(w[p], make_float2(x[ee], x[ee]), acc[ee][p]);
+            }
+        }
+    }
+#pragma unroll
+    for(int u = 0; u < U; u++){
+        float v[4];
+#pragma unroll
+        for(int ee = 0; ee < 4; ee++) v[ee] = activation_rt(u & 1 ? acc[ee][u / 2].y : acc[ee][u / 2].x, act);
+        *reinterpret_cast<float4*>(out + (first_unit + u) * L::PITCH + 4 * eg) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+// a quadrotor's reset where its episode has ended (operations_generic_per_env.h:8-61)
+__device__ __forceinline__ void l2f_rollout_reset(const L2fRolloutArgs& a, int t, int e, int& resets, L2fState& s){
+    if(a.device_rng){
+        float uu[17], nn[6];
+        l2f_reset_draws(a.rng_seed, a.rng_step0 + (unsigned long long)t, (uint32_t)e, a.init[9] != 0.0f || a.init[11] != 0.0f, uu, nn);
+        l2f_initial_state(a.init, a.env.p.action_min, a.env.p.action_max, uu, nn, s);
+    }
+    else if(a.reset_states != nullptr && resets < a.n_reset_rounds){
+        const float* src = a.reset_states + ((size_t)resets * a.n_envs + e) * 23;
+        float* dst = reinterpret_cast<float*>(&s);
+#pragma unroll
+        for(int k = 0; k < 23; k++) dst[k] = __ldg(src + k);
+    }
+    else if(a.error_flag) *a.error_flag = 1;
+    resets++;
+}
+
+template <int H>
+__global__ void __launch_bounds__(L2F_SHARED_THREADS, 1) l2f_rollout_shared_kernel(L2fRolloutArgs a){
+    using L = L2fSharedLayout<H>;
+    constexpr int O = L::O, A = L::A;
+    extern __shared__ __align__(16) float smem[];
+    {
+        constexpr int W1_END = O * H, B1_END = W1_END + H, W2_END = B1_END + H * H, B2_END = W2_END + H, W3_END = B2_END + A * H;
+        for(int i = threadIdx.x; i < W3_END + A; i += blockDim.x){
+            int dst = i;                                                                       // biases keep their place
+            if(i < W1_END) dst = L::W1T + (i % O) * H + i / O;                                 // W1[j][k]
+            else if(i >= B1_END && i < W2_END){ const int r = i - B1_END; dst = L::W2T + (r % H) * H + r / H; }                  // W2[j][k]
+            else if(i >= B2_END && i < W3_END){ const int r = i - B2_END; dst = L::W3T + (r % H) * A + r / H; }                  // W3[c][j]
+            smem[dst] = __ldg(a.params + i);
+        }
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = warp / L2F_SHARED_WARPS, member = (warp + group) % L2F_SHARED_WARPS;      // the groups' owners on a scheduler each
+    const int e0 = (blockIdx.x * (blockDim.x / (32 * L2F_SHARED_WARPS)) + group) * 32, e = e0 + lane, eg = lane >> 2, first_unit = member * (H / 4) + L::UNITS * (lane & 3);
+    float* tiles = smem + L::GROUP0 + group * L::PER_GROUP;
+    const bool owner = member == 0, active = owner && e < a.n_envs;
+    auto meet = [&](){ asm volatile("bar.sync %0, %1;" :: "r"(1 + group), "n"(32 * L2F_SHARED_WARPS) : "memory"); };
+    L2fState s;
+    {
+        float* dst = reinterpret_cast<float*>(&s);
+#pragma unroll
+        for(int k = 0; k < 23; k++) dst[k] = active ? a.states[(size_t)e * 23 + k] : 0.0f;
+    }
+    int es = active ? a.episode_step[e] : 0, resets = 0;
+    bool trunc = active ? a.truncated[e] != 0 : false;
+    float er = active ? a.episode_return[e] : 0.0f;
+    for(int t = 0; t < a.n_steps; t++){
+        const size_t row = (size_t)t * a.n_envs + e;
+        float* obs = tiles + L::OBS + (t & 1) * O * 32;                  // the other warps may still be writing the last step's out
+        if(owner){
+            float o[O];
+#pragma unroll
+            for(int k = 0; k < O; k++) o[k] = 0.0f;
+            if(active){
+                if(trunc){ l2f_rollout_reset(a, t, e, resets, s); es = 0; er = 0.0f; }
+                l2f_observe(s, o);
+            }
+#pragma unroll
+            for(int k = 0; k < O; k++) obs[k * 32 + lane] = o[k];
+        }
+        meet();
+        l2f_shared_layer<H, O, 32>(obs, smem + L::W1T, smem + L::B1, tiles + L::HID1, first_unit, eg, a.acts[0]);
+        meet();
+        l2f_shared_layer<H, H, L::PITCH>(tiles + L::HID1, smem + L::W2T, smem + L::B2, tiles + L::HID2, first_unit, eg, a.acts[1]);
+        meet();
+        {
+            float out = smem[L::B3 + member];
+#pragma unroll 16
+            for(int j = 0; j < H; j++) out = fmaf(smem[L::W3T + j * A + member], tiles[L::HID2 + j * L::PITCH + lane], out);
+            tiles[L::OUT + member * 32 + lane] = activation_rt(out, a.acts[2]);
+        }
+        meet();
+        if(!owner){
+            const int n = min(32, a.n_envs - e0) * O;
+            float* to = a.obs + ((size_t)t * a.n_envs + e0) * O;
+            for(int i = 32 * (member - 1) + lane; i < n; i += 32 * (L2F_SHARED_WARPS - 1)) to[i] = obs[(i % O) * 32 + i / O];
+        }
+        else if(active){
+            float action[A];
+#pragma unroll
+            for(int c = 0; c < A; c++){ action[c] = tiles[L::OUT + c * 32 + lane]; a.act[row * A + c] = action[c]; }
+            L2fState next;
+            l2f_step(a.env, s, action, next);
+            const bool term = l2f_terminated(a.mdp, next);
+            const float r = l2f_reward(a.env, a.mdp, s, action, next, term);
+            es += 1; er = __fadd_rn(er, r);
+            trunc = term || (es == a.step_limit);
+            a.rew[row] = r;
+            if(a.terminated) a.terminated[row] = term ? 1 : 0;
+            s = next;
+        }
+    }
+    if(active){
+        float* dst = a.states + (size_t)e * 23;
+        const float* src = reinterpret_cast<const float*>(&s);
+#pragma unroll
+        for(int k = 0; k < 23; k++) dst[k] = src[k];
+        a.episode_step[e] = es; a.truncated[e] = trunc ? 1 : 0; a.episode_return[e] = er;
+    }
+}
+
 template <int H>
 __global__ void __launch_bounds__(L2F_ROLLOUT_THREADS, 1) l2f_rollout_kernel(L2fRolloutArgs a){
     using L = L2fRolloutLayout<H>;
@@ -398,21 +563,7 @@ __global__ void __launch_bounds__(L2F_ROLLOUT_THREADS, 1) l2f_rollout_kernel(L2f
     for(int t = 0; t < a.n_steps; t++){
         const size_t row = (size_t)t * a.n_envs + e;
         if(active){
-            if(trunc){                                   // operations_generic_per_env.h:8-61
-                if(a.device_rng){
-                    float uu[17], nn[6];
-                    l2f_reset_draws(a.rng_seed, a.rng_step0 + (unsigned long long)t, (uint32_t)e, a.init[9] != 0.0f || a.init[11] != 0.0f, uu, nn);
-                    l2f_initial_state(a.init, a.env.p.action_min, a.env.p.action_max, uu, nn, s);
-                }
-                else if(a.reset_states != nullptr && resets < a.n_reset_rounds){
-                    const float* src = a.reset_states + ((size_t)resets * a.n_envs + e) * 23;
-                    float* dst = reinterpret_cast<float*>(&s);
-#pragma unroll
-                    for(int k = 0; k < 23; k++) dst[k] = __ldg(src + k);
-                }
-                else if(a.error_flag) *a.error_flag = 1;
-                resets++; es = 0; er = 0.0f;
-            }
+            if(trunc){ l2f_rollout_reset(a, t, e, resets, s); es = 0; er = 0.0f; }
             float o[O];
             l2f_observe(s, o);
 #pragma unroll
@@ -489,6 +640,18 @@ static int launch_l2f_rollout(const L2fRolloutArgs& a, cudaStream_t s){
     if(rc) return rc;
     const int total = (a.n_envs + 31) / 32;
     int warps = (total + sms - 1) / sms;
+    if(warps <= (H == 16 ? L2F_SHARED_GROUPS / 2 : L2F_SHARED_GROUPS)){
+        static std::atomic<bool> configured[MAX_DEVICES];
+        int dev = 0;
+        if((rc = current_device(&dev))) return rc;
+        if(!configured[dev].load(std::memory_order_acquire)){
+            B200RL_CUDA_TRY(cudaFuncSetAttribute(l2f_rollout_shared_kernel<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L2fSharedLayout<H>::bytes(L2F_SHARED_GROUPS)));
+            configured[dev].store(true, std::memory_order_release);
+        }
+        l2f_rollout_shared_kernel<H><<<(total + warps - 1) / warps, 32 * L2F_SHARED_WARPS * warps, L2fSharedLayout<H>::bytes(warps), s>>>(a);
+        B200RL_LAUNCH_CHECK("l2f_rollout_shared");
+        return B200RL_OK;
+    }
     if(warps > L2F_ROLLOUT_WARPS) warps = L2F_ROLLOUT_WARPS;
     B200RL_CUDA_TRY(cudaFuncSetAttribute(l2f_rollout_kernel<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L2fRolloutLayout<H>::bytes(L2F_ROLLOUT_WARPS)));
     l2f_rollout_kernel<H><<<(total + warps - 1) / warps, 32 * warps, L2fRolloutLayout<H>::bytes(warps), s>>>(a);

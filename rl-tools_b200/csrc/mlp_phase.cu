@@ -10,7 +10,8 @@
 // at once (one L2 round trip per tile), its eight warps take every eighth group of four summed indices and each lane a 4 x 8 patch,
 // and the eight partial tiles are added in warp order (deterministic).
 //
-// Bound by latency. Measured, 4-256-256-1 at batch 256 in a captured graph: 18 us (one cooperative launch with grid barriers between the layers 24 us: a
+// Bound by latency, so what the epilogues read (old gradients, pre-activations) and a column's rows for the bias sums are under way together with the operands (a launch of the critic's backward
+// pass 6.0 -> 5.6 us on average). Measured, 4-256-256-1 at batch 256 in a captured graph: 16.7 us (one cooperative launch with grid barriers between the layers 24 us: a
 // barrier costs more than a graph's next node, and two such launches take turns on the SMs).
 #include "common.cuh"
 #include <atomic>
@@ -80,6 +81,18 @@ __device__ __forceinline__ void phase_product_tile(const PhaseProduct& g, int ti
     for(int i = 0; i < 4; i++)
 #pragma unroll
         for(int j = 0; j < 4; j++) acc[i][j] = make_float2(0.0f, 0.0f);
+    // what the epilogue reads, asked for while the operands are on their way: the old gradients, the pre-activations of the layer below
+    const int r = tid >> 3, c4 = (tid & 7) * 4, m = m0 + r;
+    float early[4];
+#pragma unroll
+    for(int j = 0; j < 4; j++){
+        const int n = n0 + c4 + j;
+        early[j] = 0.0f;
+        if(m < g.M && n < g.N){
+            if(!A_KCONTIG) early[j] = g.C[(size_t)m * g.ldc + n];
+            else if(g.aux) early[j] = __ldg(g.aux + (size_t)m * g.ldaux + n);
+        }
+    }
     for(int k0 = 0; k0 < g.K; k0 += PH_KC){
         const int kc = min(PH_KC, g.K - k0);
         if(k0) __syncthreads();                            // whoever read the previous chunk is done
@@ -115,7 +128,6 @@ __device__ __forceinline__ void phase_product_tile(const PhaseProduct& g, int ti
         *reinterpret_cast<float4*>(row + 4) = make_float4(acc[i][2].x, acc[i][2].y, acc[i][3].x, acc[i][3].y);
     }
     __syncthreads();
-    const int r = tid >> 3, c4 = (tid & 7) * 4, m = m0 + r;
     float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
     for(int w = 0; w < PH_WARPS; w++){
@@ -129,22 +141,26 @@ __device__ __forceinline__ void phase_product_tile(const PhaseProduct& g, int ti
         if(n >= g.N) continue;
         float s = v[j];
         if(A_KCONTIG){                                     // input gradient, through the activation below
-            if(g.aux) s *= d_activation_rt(__ldg(g.aux + (size_t)m * g.ldaux + n), g.act);
+            if(g.aux) s *= d_activation_rt(early[j], g.act);
             g.C[(size_t)m * g.ldc + n] = s;
         }
-        else{
-            float* dst = g.C + (size_t)m * g.ldc + n;
-            *dst += s;
-        }
+        else g.C[(size_t)m * g.ldc + n] = early[j] + s;
     }
 }
 
 // 32 columns of the bias gradient: eight row lanes per column, added in lane order
 __device__ void phase_bias_item(const Phase& p, int item, float* smem){
     const int tid = threadIdx.x, c = tid & 31, seg = tid >> 5, col = item * 32 + c;
+    const float old = seg == 0 && col < p.bias_cols ? p.bias_dst[col] : 0.0f;
     float s = 0.0f;
     if(col < p.bias_cols)
-        for(int b = seg; b < p.bias_rows; b += PH_WARPS) s += p.bias_src[(size_t)b * p.bias_ld + col];
+        for(int b = seg; b < p.bias_rows; b += 32 * PH_WARPS){         // 32 loads under way, added in order
+            float v[32];
+#pragma unroll
+            for(int k = 0; k < 32; k++) v[k] = b + k * PH_WARPS < p.bias_rows ? p.bias_src[(size_t)(b + k * PH_WARPS) * p.bias_ld + col] : 0.0f;
+#pragma unroll
+            for(int k = 0; k < 32; k++) s += v[k];
+        }
     __syncthreads();
     smem[seg * 32 + c] = s;
     __syncthreads();
@@ -152,7 +168,7 @@ __device__ void phase_bias_item(const Phase& p, int item, float* smem){
         float t = 0.0f;
 #pragma unroll
         for(int w = 0; w < PH_WARPS; w++) t += smem[w * 32 + tid];
-        p.bias_dst[col] += t;
+        p.bias_dst[col] = old + t;
     }
 }
 

@@ -25,6 +25,8 @@ __device__ __forceinline__ void adam_one(float& p, float g, float& m, float& v, 
 __global__ void __launch_bounds__(256) adam_step_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
                                                         size_t n, b200rl_adam_hyper h, AdamState* state, int vec_ok){
     __shared__ float sc[2];
+    after_predecessor();
+    p = opaque(p); g = opaque(g); m = opaque(m); v = opaque(v); state = opaque(state);
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x, n4 = vec_ok ? n / 4 : 0;
     float4* p4 = reinterpret_cast<float4*>(p); const float4* g4 = reinterpret_cast<const float4*>(g);
     float4* m4 = reinterpret_cast<float4*>(m); float4* v4 = reinterpret_cast<float4*>(v);
@@ -73,6 +75,8 @@ __global__ void adam_reset_kernel(AdamState* s){ s->age = 1; s->ticket = 0; s->c
 
 __global__ void __launch_bounds__(256) mse_gradient_kernel(const float* __restrict__ a, long long lda, const float* __restrict__ b, long long ldb, float* d, long long ldd,
                                                            int rows, int cols, float constant){
+    after_predecessor();
+    a = opaque(a); b = opaque(b);
     long long n = (long long)rows * cols;
     for(long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x){
         long long r = i / cols; int c = (int)(i - r * cols);
@@ -102,6 +106,7 @@ __global__ void __launch_bounds__(1024) mse_evaluate_kernel(const float* __restr
     if(threadIdx.x == 0) *out = __fdiv_rn(__fmul_rn((float)part[0], loss_weight), (float)n);     // acc * loss_weight / (ROWS * COLS)
 }
 __global__ void __launch_bounds__(256) fill_kernel(float* dst, size_t n, float value, int vec_ok){
+    after_predecessor();
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
     if(vec_ok){
         size_t n4 = n / 4; float4 v4 = make_float4(value, value, value, value);
@@ -125,6 +130,8 @@ static bool aligned16(const void* p){ return (reinterpret_cast<uintptr_t>(p) & 1
 template <bool SQUARE>
 __global__ void __launch_bounds__(256) polyak_kernel(const float* __restrict__ source, int ld_source, float* __restrict__ target, int ld_target,
                                                      int rows, int cols, float polyak, float one_minus){
+    after_predecessor();
+    source = opaque(source); target = opaque(target);
     const size_t n = (size_t)rows * cols, stride = (size_t)gridDim.x * blockDim.x;
     for(size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += stride){
         const size_t r = i / cols, c = i - r * cols;
@@ -187,8 +194,8 @@ int b200rl_polyak_update(const float* source, int ld_source, float* target, int 
     if(!source || !target || rows < 0 || cols < 1 || ld_source < cols || ld_target < cols) return B200RL_ERR_INVALID_ARGUMENT;
     if(rows == 0) return B200RL_OK;
     const int grid = grid_for((size_t)rows * cols, 256);
-    if(square) polyak_kernel<true><<<grid, 256, 0, (cudaStream_t)stream>>>(source, ld_source, target, ld_target, rows, cols, polyak, 1.0f - polyak);
-    else polyak_kernel<false><<<grid, 256, 0, (cudaStream_t)stream>>>(source, ld_source, target, ld_target, rows, cols, polyak, 1.0f - polyak);
+    B200RL_CUDA_TRY(launch_after(square ? polyak_kernel<true> : polyak_kernel<false>, dim3(grid), dim3(256), 0, (cudaStream_t)stream, source, ld_source, target, ld_target, rows, cols, polyak,
+                                 1.0f - polyak));
     B200RL_LAUNCH_CHECK("polyak_update");
     return B200RL_OK;
 }
@@ -205,8 +212,7 @@ int b200rl_adam_step(float* params, const float* grads, float* m, float* v, size
     if(n == 0) return B200RL_OK;
     int vec_ok = aligned16(params) && aligned16(grads) && aligned16(m) && aligned16(v);
     int grid = grid_for(vec_ok ? (n + 3) / 4 : n, 256);
-    adam_step_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(params, grads, m, v, n, hyper, reinterpret_cast<AdamState*>(state), vec_ok);
-    B200RL_LAUNCH_CHECK("adam_step");
+    B200RL_CUDA_TRY(launch_after(adam_step_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, params, grads, m, v, n, hyper, reinterpret_cast<AdamState*>(state), vec_ok));
     return B200RL_OK;
 }
 
@@ -229,8 +235,7 @@ int b200rl_mse_gradient(const float* a, int lda, const float* b, int ldb, float*
     if(rows == 0) return B200RL_OK;
     // nn/loss_functions/mse/operations_generic.h:49: (T)2 / ((T)ROWS * COLS) * loss_weight, evaluated in float
     float constant = 2.0f / ((float)rows * (float)cols) * loss_weight;
-    mse_gradient_kernel<<<grid_for((size_t)rows * cols, 256), 256, 0, (cudaStream_t)stream>>>(a, lda, b, ldb, d_a, ldd, rows, cols, constant);
-    B200RL_LAUNCH_CHECK("mse_gradient");
+    B200RL_CUDA_TRY(launch_after(mse_gradient_kernel, dim3(grid_for((size_t)rows * cols, 256)), dim3(256), 0, (cudaStream_t)stream, a, lda, b, ldb, d_a, ldd, rows, cols, constant));
     return B200RL_OK;
 }
 
@@ -250,8 +255,7 @@ int b200rl_fill(float* dst, size_t n, float value, b200rl_stream_t stream){
     if(!dst) return B200RL_ERR_INVALID_ARGUMENT;
     if(n == 0) return B200RL_OK;
     int vec_ok = aligned16(dst);
-    fill_kernel<<<grid_for(vec_ok ? (n + 3) / 4 : n, 256), 256, 0, (cudaStream_t)stream>>>(dst, n, value, vec_ok);
-    B200RL_LAUNCH_CHECK("fill");
+    B200RL_CUDA_TRY(launch_after(fill_kernel, dim3(grid_for(vec_ok ? (n + 3) / 4 : n, 256)), dim3(256), 0, (cudaStream_t)stream, dst, n, value, vec_ok));
     return B200RL_OK;
 }
 

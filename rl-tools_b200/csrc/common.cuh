@@ -22,6 +22,25 @@ int cuda_fail(cudaError_t e, const char* where);
 #define B200RL_CUDA_TRY(expr) do { cudaError_t _e = (expr); if(_e != cudaSuccess) return ::b200rl::cuda_fail(_e, #expr); } while(0)
 #define B200RL_LAUNCH_CHECK(where) do { cudaError_t _e = cudaPeekAtLastError(); if(_e != cudaSuccess) return ::b200rl::cuda_fail(_e, where); } while(0)
 
+// ---- launches that follow one another closely ------------------------------------------------------------------------------------------------
+// The passes of small networks are chains of dependent kernels of two to six microseconds, of which one is the way from the end of a kernel to the first instruction of the next.
+// A kernel launched by launch_after may start while the kernel before it on its stream still runs (programmatic stream serialization, also inside a captured graph). It opens with
+// after_predecessor(), in front of its first access to memory: every grid before it has then completed and its writes are visible. What it reads goes through opaque(), so that no
+// load through a read-only pointer can be moved in front of that. In the chain of kernels every one that was launched this way waits, so "before" reaches back to the first.
+__device__ __forceinline__ void after_predecessor(){
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename T> __device__ __forceinline__ T* opaque(T* p){ asm volatile("" : "+l"(p) :: "memory"); return p; }
+template <typename... P, typename... A>
+inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args){
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s; cfg.attrs = attr; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // nn/activation_functions.h:25-55 and math/operations_cuda.h (precise ::tanhf / ::expf, no fast-math intrinsics);
 // fast_tanh: math/operations_generic.h:247-251.
 __device__ __forceinline__ float fast_tanh_dev(float x){

@@ -147,6 +147,10 @@ __global__ void __launch_bounds__(256) small_forward_kernel(GemmArgs a, int vec_
     __shared__ __align__(16) float S[(SF_M + SF_N) * SF_KC];                      // [row][piece ^ (row & 7)][4]; later the partial sums [warp][32][20]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = lane >> 2, cg = lane & 3;
     const int m0 = blockIdx.y * SF_M, n0 = blockIdx.x * SF_N;
+    after_predecessor();
+    a.A = opaque(a.A); a.B = opaque(a.B);
+    const float* bias_at = opaque(a.bias) + n0 + 2 * (tid & 7);                   // of this thread's two outputs, asked for before the operands
+    const float2 bias = make_float2(n0 + 2 * (tid & 7) < a.N ? __ldg(bias_at) : 0.0f, n0 + 2 * (tid & 7) + 1 < a.N ? __ldg(bias_at + 1) : 0.0f);
     float2 acc[4][4];                                                             // sums over even and odd k
 #pragma unroll
     for(int i = 0; i < 4; i++)
@@ -202,7 +206,7 @@ __global__ void __launch_bounds__(256) small_forward_kernel(GemmArgs a, int vec_
     for(int j = 0; j < 2; j++){
         const int n = n0 + c + j;
         if(n >= a.N) continue;
-        const float s = (j ? v.y : v.x) + __ldg(a.bias + n);
+        const float s = j ? v.y + bias.y : v.x + bias.x;
         if(a.pre) a.pre[(long long)m * a.ldpre + n] = s;
         a.C[(long long)m * a.ldc + n] = activation<ACT>(s);
     }
@@ -435,7 +439,7 @@ static int dense_forward_impl(const float* W, const float* bias, const float* x,
     if(small_tiles(a.M, a.N, 1)){
         auto vec = [&](const float* p, long long ld){ return a.K % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
         const dim3 grid((a.N + SF_N - 1) / SF_N, (a.M + SF_M - 1) / SF_M);
-        B200RL_DISPATCH_ACT(act, (small_forward_kernel<ACT><<<grid, 256, 0, s>>>(a, vec(a.A, a.lda), vec(a.B, a.ldb))));
+        B200RL_DISPATCH_ACT(act, B200RL_CUDA_TRY(launch_after(small_forward_kernel<ACT>, grid, dim3(256), 0, s, a, (int)vec(a.A, a.lda), (int)vec(a.B, a.ldb))));
     }
     else{
         const dim3 grid((a.N + 63) / 64, (a.M + 63) / 64);

@@ -698,6 +698,8 @@ __device__ __forceinline__ void l2f_replay_append(int e, const float (&obs)[18],
 // prologue: reset-if-truncated (from reset_states [n, 23], or drawn in the kernel from `init`), counters of a fresh episode, observation
 __global__ void __launch_bounds__(128) l2f_offpolicy_prologue_kernel(L2fRolloutArgs a, const unsigned long long* __restrict__ call_counter, float* __restrict__ observations,
                                                                      uint8_t* __restrict__ was_truncated){
+    after_predecessor();
+    a.reset_states = opaque(a.reset_states); call_counter = opaque(call_counter);
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if(e >= a.n_envs) return;
     L2fState s;
@@ -729,6 +731,8 @@ __global__ void __launch_bounds__(128) l2f_offpolicy_prologue_kernel(L2fRolloutA
 template <typename INDEX>
 __global__ void __launch_bounds__(128) l2f_offpolicy_epilogue_kernel(L2fRolloutArgs a, const float* __restrict__ actions, float* __restrict__ next_observations,
                                                                      const uint8_t* __restrict__ was_truncated, unsigned char* replay, b200rl_replay_layout L){
+    after_predecessor();
+    actions = opaque(actions); was_truncated = opaque(was_truncated);
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if(e >= a.n_envs) return;
     L2fState s, next;
@@ -845,8 +849,7 @@ extern "C" int b200rl_l2f_offpolicy_prologue(const b200rl_l2f_parameters* parame
     if(init) memcpy(a.init, init, sizeof(a.init));
     a.states = states; a.episode_step = episode_step; a.truncated = const_cast<uint8_t*>(truncated); a.episode_return = episode_return; a.reset_states = reset_states;
     a.n_envs = n_envs; a.rng_seed = seed; a.rng_step0 = call;
-    l2f_offpolicy_prologue_kernel<<<(n_envs + 127) / 128, 128, 0, (cudaStream_t)stream>>>(a, call_counter, observations, was_truncated_scratch);
-    B200RL_LAUNCH_CHECK("l2f_offpolicy_prologue");
+    B200RL_CUDA_TRY(launch_after(l2f_offpolicy_prologue_kernel, dim3((n_envs + 127) / 128), dim3(128), 0, (cudaStream_t)stream, a, call_counter, observations, was_truncated_scratch));
     return B200RL_OK;
 }
 
@@ -864,10 +867,7 @@ extern "C" int b200rl_l2f_offpolicy_epilogue(const b200rl_l2f_parameters* parame
     a.states = states; a.episode_step = episode_step; a.truncated = truncated; a.episode_return = episode_return; a.n_envs = n_envs; a.step_limit = step_limit;
     cudaStream_t s = (cudaStream_t)stream;
     const int blocks = (n_envs + 127) / 128;
-    if(layout->index_bytes == 4)
-        l2f_offpolicy_epilogue_kernel<uint32_t><<<blocks, 128, 0, s>>>(a, actions, next_observations, was_truncated_scratch, static_cast<unsigned char*>(replay_buffers), *layout);
-    else
-        l2f_offpolicy_epilogue_kernel<unsigned long long><<<blocks, 128, 0, s>>>(a, actions, next_observations, was_truncated_scratch, static_cast<unsigned char*>(replay_buffers), *layout);
-    B200RL_LAUNCH_CHECK("l2f_offpolicy_epilogue");
+    B200RL_CUDA_TRY(launch_after(layout->index_bytes == 4 ? l2f_offpolicy_epilogue_kernel<uint32_t> : l2f_offpolicy_epilogue_kernel<unsigned long long>, dim3(blocks), dim3(128), 0, s, a, actions,
+                                 next_observations, was_truncated_scratch, static_cast<unsigned char*>(replay_buffers), *layout));
     return B200RL_OK;
 }

@@ -57,6 +57,8 @@ template <int ROWS, bool SAVE>
 __global__ void __launch_bounds__(FUSED_THREADS) mlp_fused_forward_kernel(FusedShape sh, const float* __restrict__ params, const float* __restrict__ x, long long ldx,
                                                                           float* __restrict__ pre, float* __restrict__ out, float* __restrict__ y, long long ldy){
     extern __shared__ __align__(16) float fused_smem[];
+    after_predecessor();
+    params = opaque(params); x = opaque(x);
     float* s_par = fused_smem;
     float (*act)[ROWS][FUSED_MAX_WIDTH] = reinterpret_cast<float (*)[ROWS][FUSED_MAX_WIDTH]>(fused_smem + sh.smem_params);
     const int tid = threadIdx.x;
@@ -150,6 +152,8 @@ __global__ void __launch_bounds__(FUSED_THREADS) mlp_fused_backward_chain_kernel
                                                                                  float* d_out, long long ldd, float* __restrict__ dpre, float* d_input, long long ldi,
                                                                                  unsigned int* counters, int n_counters){
     extern __shared__ __align__(16) float fused_smem[];
+    after_predecessor();
+    params = opaque(params); pre = opaque(pre);
     float* s_par = fused_smem;                                   // the parameter arena as it is: W_l row-major, b_l behind
     float (*d)[ROWS][FUSED_MAX_WIDTH] = reinterpret_cast<float (*)[ROWS][FUSED_MAX_WIDTH]>(fused_smem + ((sh.n_params + 3) & ~3));
     const int tid = threadIdx.x;
@@ -233,6 +237,8 @@ __global__ void __launch_bounds__(256) mlp_fused_grads_kernel(FusedShape sh, con
                                                               const float* __restrict__ dpre, float* grads, float* partial, unsigned int* counters, int n_slices){
     __shared__ __align__(16) float s_all[2 * GRADS_ROWS * GRADS_PITCH];          // d_pre rows, then input rows; the eight partial tiles reuse it
     __shared__ bool is_last;
+    after_predecessor();
+    x = opaque(x); outs = opaque(outs); dpre = opaque(dpre);
     float (*s_d)[GRADS_PITCH] = reinterpret_cast<float (*)[GRADS_PITCH]>(s_all);
     float (*s_in)[GRADS_PITCH] = s_d + GRADS_ROWS;
     static_assert(8 * 32 * 32 <= 2 * GRADS_ROWS * GRADS_PITCH, "partial tiles");
@@ -397,8 +403,7 @@ static int launch_fused_forward(const FusedShape& f, const float* params, const 
     const size_t bytes = ((size_t)f.smem_params + 2 * ROWS * FUSED_MAX_WIDTH) * sizeof(float);
     int rc = allow_shared_memory(mlp_fused_forward_kernel<ROWS, SAVE>, granted, bytes);
     if(rc) return rc;
-    mlp_fused_forward_kernel<ROWS, SAVE><<<(f.batch + ROWS - 1) / ROWS, FUSED_THREADS, bytes, s>>>(f, params, x, ldx, pre, out, y, ldy);
-    B200RL_LAUNCH_CHECK("mlp_fused_forward");
+    B200RL_CUDA_TRY(launch_after(mlp_fused_forward_kernel<ROWS, SAVE>, dim3((f.batch + ROWS - 1) / ROWS), dim3(FUSED_THREADS), bytes, s, f, params, x, ldx, pre, out, y, ldy));
     return B200RL_OK;
 }
 template <int ROWS>
@@ -408,8 +413,8 @@ static int launch_fused_chain(const FusedShape& f, const float* params, const fl
     const size_t bytes = ((size_t)((f.n_params + 3) & ~3) + 2 * ROWS * FUSED_MAX_WIDTH) * sizeof(float);
     int rc = allow_shared_memory(mlp_fused_backward_chain_kernel<ROWS>, granted, bytes);
     if(rc) return rc;
-    mlp_fused_backward_chain_kernel<ROWS><<<(f.batch + ROWS - 1) / ROWS, FUSED_THREADS, bytes, s>>>(f, params, pre, d_out, ldd, dpre, d_input, ldi, counters, n_counters);
-    B200RL_LAUNCH_CHECK("mlp_fused_backward_chain");
+    B200RL_CUDA_TRY(launch_after(mlp_fused_backward_chain_kernel<ROWS>, dim3((f.batch + ROWS - 1) / ROWS), dim3(FUSED_THREADS), bytes, s, f, params, pre, d_out, ldd, dpre, d_input, ldi,
+                                 counters, n_counters));
     return B200RL_OK;
 }
 
@@ -443,8 +448,7 @@ int mlp_fused_backward(const b200rl_mlp_shape* sh, const float* params, float* g
     else rc = launch_fused_chain<8>(f, params, pre, d_out, ldd, dpre, d_input, sh->input_dim, cnt, (int)fs.counters, s);
     if(rc) return rc;
     if(grads){
-        mlp_fused_grads_kernel<<<dim3(fs.tiles, fs.slices), 256, 0, s>>>(f, x, ldx, out, dpre, grads, partial, counters, fs.slices);
-        B200RL_LAUNCH_CHECK("mlp_fused_grads");
+        B200RL_CUDA_TRY(launch_after(mlp_fused_grads_kernel, dim3(fs.tiles, fs.slices), dim3(256), 0, s, f, x, ldx, out, dpre, grads, partial, counters, fs.slices));
     }
     return B200RL_OK;
 }

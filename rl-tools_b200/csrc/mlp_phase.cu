@@ -72,6 +72,7 @@ __device__ __forceinline__ void phase_load(float* S, const float* P, int ld, boo
 // the first operand in either order, the second with its rows contiguous
 template <bool A_KCONTIG>
 __device__ __forceinline__ void phase_product_tile(const PhaseProduct& g, int tile, float* smem){
+    const float* A = opaque(g.A); const float* B = opaque(g.B); const float* aux = opaque(g.aux); float* C = opaque(g.C);
     float* As = smem;
     float* Bs = smem + PH_T * PH_KC;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rg = lane >> 2, cg = lane & 3;
@@ -89,15 +90,15 @@ __device__ __forceinline__ void phase_product_tile(const PhaseProduct& g, int ti
         const int n = n0 + c4 + j;
         early[j] = 0.0f;
         if(m < g.M && n < g.N){
-            if(!A_KCONTIG) early[j] = g.C[(size_t)m * g.ldc + n];
-            else if(g.aux) early[j] = __ldg(g.aux + (size_t)m * g.ldaux + n);
+            if(!A_KCONTIG) early[j] = C[(size_t)m * g.ldc + n];
+            else if(g.aux) early[j] = __ldg(aux + (size_t)m * g.ldaux + n);
         }
     }
     for(int k0 = 0; k0 < g.K; k0 += PH_KC){
         const int kc = min(PH_KC, g.K - k0);
         if(k0) __syncthreads();                            // whoever read the previous chunk is done
-        phase_load(As, g.A, g.lda, A_KCONTIG, m0, g.M, k0, kc);
-        phase_load(Bs, g.B, g.ldb, false, n0, g.N, k0, kc);
+        phase_load(As, A, g.lda, A_KCONTIG, m0, g.M, k0, kc);
+        phase_load(Bs, B, g.ldb, false, n0, g.N, k0, kc);
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         for(int c = warp; c < (kc + 3) / 4; c += PH_WARPS){
@@ -142,22 +143,23 @@ __device__ __forceinline__ void phase_product_tile(const PhaseProduct& g, int ti
         float s = v[j];
         if(A_KCONTIG){                                     // input gradient, through the activation below
             if(g.aux) s *= d_activation_rt(early[j], g.act);
-            g.C[(size_t)m * g.ldc + n] = s;
+            C[(size_t)m * g.ldc + n] = s;
         }
-        else g.C[(size_t)m * g.ldc + n] = early[j] + s;
+        else C[(size_t)m * g.ldc + n] = early[j] + s;
     }
 }
 
 // 32 columns of the bias gradient: eight row lanes per column, added in lane order
 __device__ void phase_bias_item(const Phase& p, int item, float* smem){
     const int tid = threadIdx.x, c = tid & 31, seg = tid >> 5, col = item * 32 + c;
+    const float* src = opaque(p.bias_src);
     const float old = seg == 0 && col < p.bias_cols ? p.bias_dst[col] : 0.0f;
     float s = 0.0f;
     if(col < p.bias_cols)
         for(int b = seg; b < p.bias_rows; b += 32 * PH_WARPS){         // 32 loads under way, added in order
             float v[32];
 #pragma unroll
-            for(int k = 0; k < 32; k++) v[k] = b + k * PH_WARPS < p.bias_rows ? p.bias_src[(size_t)(b + k * PH_WARPS) * p.bias_ld + col] : 0.0f;
+            for(int k = 0; k < 32; k++) v[k] = b + k * PH_WARPS < p.bias_rows ? src[(size_t)(b + k * PH_WARPS) * p.bias_ld + col] : 0.0f;
 #pragma unroll
             for(int k = 0; k < 32; k++) s += v[k];
         }
@@ -174,12 +176,13 @@ __device__ void phase_bias_item(const Phase& p, int item, float* smem){
 
 __global__ void __launch_bounds__(PH_THREADS, 2) mlp_phase_kernel(const __grid_constant__ Phase p){
     extern __shared__ __align__(16) float smem[];
+    after_predecessor();
     if(p.type == PH_PHASE_DPRE){
         const int total = p.ew_rows * p.ew_cols, idx = blockIdx.x * PH_THREADS + threadIdx.x;
         if(idx >= total) return;
         const int r = idx / p.ew_cols, c = idx % p.ew_cols;
-        float* d = p.d_out + (size_t)r * p.ew_ldd + c;
-        *d = *d * d_activation_rt(p.pre[(size_t)r * p.ew_ldpre + c], p.ew_act);
+        float* d = opaque(p.d_out) + (size_t)r * p.ew_ldd + c;
+        *d = *d * d_activation_rt(opaque(p.pre)[(size_t)r * p.ew_ldpre + c], p.ew_act);
     }
     else{
         const int item = blockIdx.x, t0 = p.dx.tiles, t1 = p.dw.tiles;
@@ -216,8 +219,7 @@ static int launch_phases(PhaseArgs& a, cudaStream_t s){
         const Phase& p = a.phase[ph];
         const int items = p.type == PH_PHASE_DPRE ? (p.ew_rows * p.ew_cols + PH_THREADS - 1) / PH_THREADS
                                                   : p.dx.tiles + p.dw.tiles + p.bias_items;
-        mlp_phase_kernel<<<items, PH_THREADS, PH_SMEM, s>>>(p);
-        B200RL_LAUNCH_CHECK("mlp_phase");
+        B200RL_CUDA_TRY(launch_after(mlp_phase_kernel, dim3(items), dim3(PH_THREADS), PH_SMEM, s, p));
     }
     return B200RL_OK;
 }

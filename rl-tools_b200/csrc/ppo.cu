@@ -270,6 +270,8 @@ template <bool GATHER>
 __global__ void __launch_bounds__(256) permute_rows_kernel(float* __restrict__ data, int ld, int n_rows, const int32_t* __restrict__ perm, unsigned long long mask, int n_cols,
                                     float* __restrict__ scratch){
     __shared__ int s_col[64], s_row[PERMUTE_ROWS];
+    after_predecessor();
+    data = opaque(data); perm = opaque(perm); scratch = opaque(scratch);
     const int row0 = blockIdx.x * PERMUTE_ROWS, rows = min(PERMUTE_ROWS, n_rows - row0);
     if(threadIdx.x < 64 && (mask >> threadIdx.x & 1)) s_col[__popcll(mask & ((1ull << threadIdx.x) - 1))] = threadIdx.x;
     if(threadIdx.x < rows) s_row[threadIdx.x] = GATHER ? perm[row0 + threadIdx.x] : row0 + threadIdx.x;
@@ -299,9 +301,8 @@ extern "C" int b200rl_permute_rows(float* data, int ld, int n_rows, const int32_
     const int threads = 256;
     const unsigned blocks = (unsigned)((n_rows + b200rl::PERMUTE_ROWS - 1) / b200rl::PERMUTE_ROWS);
     cudaStream_t s = (cudaStream_t)stream;
-    b200rl::permute_rows_kernel<true><<<blocks, threads, 0, s>>>(data, ld, n_rows, perm, column_mask, n_cols, static_cast<float*>(scratch));
-    b200rl::permute_rows_kernel<false><<<blocks, threads, 0, s>>>(data, ld, n_rows, perm, column_mask, n_cols, static_cast<float*>(scratch));
-    B200RL_LAUNCH_CHECK("permute_rows");
+    for(auto kernel : {b200rl::permute_rows_kernel<true>, b200rl::permute_rows_kernel<false>})
+        B200RL_CUDA_TRY(b200rl::launch_after(kernel, dim3(blocks), dim3(threads), 0, s, data, ld, n_rows, perm, column_mask, n_cols, static_cast<float*>(scratch)));
     return B200RL_OK;
 }
 

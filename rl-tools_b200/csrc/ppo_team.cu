@@ -42,7 +42,8 @@ constexpr int PPO_TEAM_MAX_ACTIONS = 64, PPO_TEAM_MAX_PARAMS = 18944;       // p
 // mean and standard deviation of every minibatch's advantages (:173-184), one CTA each
 __global__ void __launch_bounds__(1024) ppo_epoch_stats_kernel(const float* __restrict__ advantages, int ld, int batch, float* __restrict__ stats){
     __shared__ float s_sum[32], s_sq[32];
-    const float* adv = advantages + (size_t)blockIdx.x * batch * ld;
+    after_predecessor();
+    const float* adv = opaque(advantages) + (size_t)blockIdx.x * batch * ld;
     float sum = 0.0f, sq = 0.0f;
     for(int b = threadIdx.x; b < batch; b += blockDim.x){ const float a = adv[(size_t)b * ld]; sum += a; sq = fmaf(a, a, sq); }
     for(int o = 16; o > 0; o >>= 1){ sum += __shfl_xor_sync(0xffffffffu, sum, o); sq += __shfl_xor_sync(0xffffffffu, sq, o); }
@@ -361,8 +362,7 @@ extern "C" int b200rl_ppo_train_epoch(const b200rl_mlp_shape* actor, const b200r
     if(rc) return rc;
     a.actor.barrier = bars[0]; a.critic.barrier = bars[1];
     if(normalize_advantage){
-        ppo_epoch_stats_kernel<<<n_minibatches, 1024, 0, s>>>(advantages, ld, batch, stats);
-        B200RL_LAUNCH_CHECK("ppo_epoch_stats");
+        B200RL_CUDA_TRY(launch_after(ppo_epoch_stats_kernel, dim3(n_minibatches), dim3(1024), 0, s, advantages, ld, batch, stats));
     }
     switch(actor->n_layers){
         case 1: return launch_ppo_epoch_l<1>(a, c.smem, s);

@@ -212,6 +212,8 @@ __global__ void replay_add_kernel(int n_envs, const float* __restrict__ states, 
 __global__ void offpolicy_prologue_kernel(int n_envs, float* __restrict__ states, int32_t* __restrict__ episode_step, const uint8_t* __restrict__ truncated,
                                           float* __restrict__ episode_return, const float* __restrict__ reset_states, unsigned long long seed, unsigned long long call,
                                           const unsigned long long* __restrict__ call_counter, float* __restrict__ observations, uint8_t* __restrict__ was_truncated){
+    after_predecessor();
+    truncated = opaque(truncated); reset_states = opaque(reset_states); call_counter = opaque(call_counter);
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if(e >= n_envs) return;
     float theta = states[2 * e], theta_dot = states[2 * e + 1];
@@ -235,6 +237,8 @@ template <typename INDEX>
 __global__ void offpolicy_epilogue_kernel(int n_envs, int step_limit, float* __restrict__ states, int32_t* __restrict__ episode_step, uint8_t* __restrict__ truncated,
                                           float* __restrict__ episode_return, const float* __restrict__ observations, const float* __restrict__ actions,
                                           float* __restrict__ next_observations, const uint8_t* __restrict__ was_truncated, unsigned char* replay, b200rl_replay_layout L){
+    after_predecessor();
+    observations = opaque(observations); actions = opaque(actions); was_truncated = opaque(was_truncated);
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if(e >= n_envs) return;
     const float theta = states[2 * e], theta_dot = states[2 * e + 1], action = actions[e];
@@ -295,9 +299,8 @@ extern "C" int b200rl_pendulum_offpolicy_prologue(float* states, int32_t* episod
     if(!states || !episode_step || !truncated || !episode_return || !observations || !was_truncated_scratch || n_envs < 0) return B200RL_ERR_INVALID_ARGUMENT;
     if(n_envs == 0) return B200RL_OK;
     const int threads = 128, blocks = (n_envs + threads - 1) / threads;
-    offpolicy_prologue_kernel<<<blocks, threads, 0, (cudaStream_t)stream>>>(n_envs, states, episode_step, truncated, episode_return, reset_states, seed, call, call_counter,
-                                                                           observations, was_truncated_scratch);
-    B200RL_LAUNCH_CHECK("offpolicy_prologue");
+    B200RL_CUDA_TRY(launch_after(offpolicy_prologue_kernel, dim3(blocks), dim3(threads), 0, (cudaStream_t)stream, n_envs, states, episode_step, truncated, episode_return, reset_states, seed,
+                                 call, call_counter, observations, was_truncated_scratch));
     return B200RL_OK;
 }
 
@@ -311,13 +314,9 @@ extern "C" int b200rl_pendulum_offpolicy_epilogue(float* states, int32_t* episod
     if(n_envs == 0) return B200RL_OK;
     const int threads = 128, blocks = (n_envs + threads - 1) / threads;
     cudaStream_t s = (cudaStream_t)stream;
-    if(layout->index_bytes == 4)
-        offpolicy_epilogue_kernel<uint32_t><<<blocks, threads, 0, s>>>(n_envs, step_limit, states, episode_step, truncated, episode_return, observations, actions,
-                                                                      next_observations, was_truncated_scratch, static_cast<unsigned char*>(replay_buffers), *layout);
-    else
-        offpolicy_epilogue_kernel<unsigned long long><<<blocks, threads, 0, s>>>(n_envs, step_limit, states, episode_step, truncated, episode_return, observations, actions,
-                                                                                next_observations, was_truncated_scratch, static_cast<unsigned char*>(replay_buffers), *layout);
-    B200RL_LAUNCH_CHECK("offpolicy_epilogue");
+    B200RL_CUDA_TRY(launch_after(layout->index_bytes == 4 ? offpolicy_epilogue_kernel<uint32_t> : offpolicy_epilogue_kernel<unsigned long long>, dim3(blocks), dim3(threads), 0, s, n_envs,
+                                 step_limit, states, episode_step, truncated, episode_return, observations, actions, next_observations, was_truncated_scratch,
+                                 static_cast<unsigned char*>(replay_buffers), *layout));
     return B200RL_OK;
 }
 
@@ -350,6 +349,7 @@ struct GatherArgs {
 // one warp per batch element: lanes stride over the columns of the transition row
 template <typename INDEX>
 __global__ void gather_batch_kernel(GatherArgs a){
+    after_predecessor();
     const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if(b >= a.batch) return;
     int e, offset = 0;
@@ -546,9 +546,7 @@ static int gather_launch(const void* replay_buffers, const b200rl_replay_layout*
     a.device_rng = rng.enabled; a.seed = rng.seed; a.call = rng.step0; a.call_counter = call_counter;
     const int threads = 128, blocks = (int)(((size_t)batch * 32 + threads - 1) / threads);
     cudaStream_t s = (cudaStream_t)stream;
-    if(layout->index_bytes == 4) gather_batch_kernel<uint32_t><<<blocks, threads, 0, s>>>(a);
-    else gather_batch_kernel<unsigned long long><<<blocks, threads, 0, s>>>(a);
-    B200RL_LAUNCH_CHECK("gather_batch");
+    B200RL_CUDA_TRY(launch_after(layout->index_bytes == 4 ? gather_batch_kernel<uint32_t> : gather_batch_kernel<unsigned long long>, dim3(blocks), dim3(threads), 0, s, a));
     return B200RL_OK;
 }
 
@@ -574,11 +572,13 @@ extern "C" int b200rl_gather_batch_device_rng(const void* replay_buffers, const 
 // every replay of the same graph draws fresh numbers.
 // ---------------------------------------------------------------------------------------------------------------
 namespace b200rl {
-__global__ void counter_advance_kernel(unsigned long long* counter, unsigned long long increment){ *counter += increment; }
+__global__ void counter_advance_kernel(unsigned long long* counter, unsigned long long increment){ after_predecessor(); counter = opaque(counter); *counter += increment; }
 
 // four standard normals per Philox block: counter (element / 4, call low, call high, 2 + stream_id), Box-Muller on word pairs
 __global__ void randn_kernel(float* __restrict__ dst, size_t n, unsigned long long seed, uint32_t stream_id, unsigned long long call,
                              const unsigned long long* __restrict__ call_counter){
+    after_predecessor();
+    call_counter = opaque(call_counter);
     const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if(q * 4 >= n) return;
     call += call_counter ? *call_counter : 0ull;
@@ -598,8 +598,7 @@ __global__ void randn_kernel(float* __restrict__ dst, size_t n, unsigned long lo
 
 extern "C" int b200rl_counter_advance(unsigned long long* counter, unsigned long long increment, b200rl_stream_t stream){
     if(!counter) return B200RL_ERR_INVALID_ARGUMENT;
-    counter_advance_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(counter, increment);
-    B200RL_LAUNCH_CHECK("counter_advance");
+    B200RL_CUDA_TRY(launch_after(counter_advance_kernel, dim3(1), dim3(1), 0, (cudaStream_t)stream, counter, increment));
     return B200RL_OK;
 }
 
@@ -608,8 +607,7 @@ extern "C" int b200rl_randn_device_rng(float* dst, size_t n, unsigned long long 
     if(!dst || n > ((size_t)1 << 33)) return B200RL_ERR_INVALID_ARGUMENT;
     if(n == 0) return B200RL_OK;
     const size_t quads = (n + 3) / 4;
-    randn_kernel<<<(unsigned)((quads + 127) / 128), 128, 0, (cudaStream_t)stream>>>(dst, n, seed, stream_id, call_index, call_counter);
-    B200RL_LAUNCH_CHECK("randn_device_rng");
+    B200RL_CUDA_TRY(launch_after(randn_kernel, dim3((unsigned)((quads + 127) / 128)), dim3(128), 0, (cudaStream_t)stream, dst, n, seed, stream_id, call_index, call_counter));
     return B200RL_OK;
 }
 

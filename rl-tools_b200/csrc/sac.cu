@@ -31,6 +31,8 @@ struct NormalTerms {
 __global__ void sas_forward_kernel(const float* __restrict__ input, int ld_in, const float* __restrict__ noise, int ld_noise, int B, int A,
                                    float* __restrict__ pre_squashing, float* __restrict__ output, int ld_out, float* __restrict__ log_probs,
                                    float neg_half_log_2pi){
+    after_predecessor();
+    input = opaque(input); noise = opaque(noise);
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if(b >= B) return;
     float log_prob = 0.0f;
@@ -54,6 +56,8 @@ __global__ void sas_backward_kernel(const float* __restrict__ input, int ld_in, 
                                     const float* __restrict__ output, int ld_out, const float* __restrict__ d_output, int ld_dout, const float* __restrict__ log_alpha,
                                     float target_entropy, int B, int A, float* __restrict__ d_input, int ld_din, float* __restrict__ d_log_alpha_per_sample,
                                     float neg_half_log_2pi){
+    after_predecessor();
+    input = opaque(input); noise = opaque(noise); pre_squashing = opaque(pre_squashing); output = opaque(output); d_output = opaque(d_output); log_alpha = opaque(log_alpha);
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if(b >= B) return;
     const float alpha = exp_once(__ldg(log_alpha));
@@ -85,6 +89,8 @@ __global__ void sas_backward_kernel(const float* __restrict__ input, int ld_in, 
 // backward_full (:384-397): the per-sample terms summed in sample order (one thread adds, from shared memory that all fill: 4.5 us at 256 samples with a
 // shuffle per sample), divided by the batch size (the number of resets at sequence length 1) and added to the gradient
 __global__ void sas_log_alpha_gradient_kernel(const float* __restrict__ per_sample, int B, float* __restrict__ gradient){
+    after_predecessor();
+    per_sample = opaque(per_sample); gradient = opaque(gradient);
     __shared__ __align__(16) float s[256];
     float acc = 0.0f;
     for(int base = 0; base < B; base += 256){
@@ -111,6 +117,8 @@ __global__ void sac_target_kernel(const float* __restrict__ q1, int ld_q1, const
                                   const uint8_t* __restrict__ terminated, const float* __restrict__ next_log_probs, const float* __restrict__ log_alpha,
                                   float gamma, int ignore_termination, int entropy_bonus, int entropy_bonus_next_step, float* __restrict__ target,
                                   int ld_target, int B){
+    after_predecessor();
+    q1 = opaque(q1); q2 = opaque(q2); rewards = opaque(rewards); terminated = opaque(terminated); next_log_probs = opaque(next_log_probs); log_alpha = opaque(log_alpha);
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if(b >= B) return;
     const float alpha = exp_once(__ldg(log_alpha));
@@ -126,6 +134,8 @@ __global__ void sac_target_kernel(const float* __restrict__ q1, int ld_q1, const
 // min_value_d_output_per_sample (:341-365): the action part of the input gradient of whichever critic has the smaller value
 __global__ void sac_min_value_kernel(const float* __restrict__ q1, int ld_q1, const float* __restrict__ q2, int ld_q2, const float* __restrict__ d_in_1,
                                      const float* __restrict__ d_in_2, int ld_d_in, int action_offset, int A, float* __restrict__ d_actor_output, int ld_out, int B){
+    after_predecessor();
+    q1 = opaque(q1); q2 = opaque(q2); d_in_1 = opaque(d_in_1); d_in_2 = opaque(d_in_2);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= B * A) return;
     const int b = i / A, a = i - b * A;
@@ -144,9 +154,8 @@ int b200rl_sample_and_squash_forward(const float* input, int ld_in, const float*
                                      float* output, int ld_out, float* log_probs, b200rl_stream_t stream){
     if(!input || !noise || !output || batch < 0 || action_dim < 1 || ld_in < 2 * action_dim || ld_noise < action_dim || ld_out < action_dim) return B200RL_ERR_INVALID_ARGUMENT;
     if(batch == 0) return B200RL_OK;
-    sas_forward_kernel<<<(batch + 127) / 128, 128, 0, (cudaStream_t)stream>>>(input, ld_in, noise, ld_noise, batch, action_dim, pre_squashing, output, ld_out, log_probs,
-                                                                           neg_half_log_2pi_host());
-    B200RL_LAUNCH_CHECK("sample_and_squash_forward");
+    B200RL_CUDA_TRY(launch_after(sas_forward_kernel, dim3((batch + 127) / 128), dim3(128), 0, (cudaStream_t)stream, input, ld_in, noise, ld_noise, batch, action_dim, pre_squashing, output, ld_out, log_probs,
+                                                                           neg_half_log_2pi_host()));
     return B200RL_OK;
 }
 
@@ -158,12 +167,10 @@ int b200rl_sample_and_squash_backward(const float* input, int ld_in, const float
         return B200RL_ERR_INVALID_ARGUMENT;
     if(batch == 0) return B200RL_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    sas_backward_kernel<<<(batch + 127) / 128, 128, 0, s>>>(input, ld_in, noise, ld_noise, pre_squashing, output, ld_out, d_output, ld_dout, log_alpha, target_entropy,
-                                                            batch, action_dim, d_input, ld_din, d_log_alpha_per_sample, neg_half_log_2pi_host());
-    B200RL_LAUNCH_CHECK("sample_and_squash_backward");
+    B200RL_CUDA_TRY(launch_after(sas_backward_kernel, dim3((batch + 127) / 128), dim3(128), 0, s, input, ld_in, noise, ld_noise, pre_squashing, output, ld_out, d_output, ld_dout, log_alpha, target_entropy,
+                                                            batch, action_dim, d_input, ld_din, d_log_alpha_per_sample, neg_half_log_2pi_host()));
     if(log_alpha_gradient){
-        sas_log_alpha_gradient_kernel<<<1, 256, 0, s>>>(d_log_alpha_per_sample, batch, log_alpha_gradient);
-        B200RL_LAUNCH_CHECK("sample_and_squash_log_alpha_gradient");
+        B200RL_CUDA_TRY(launch_after(sas_log_alpha_gradient_kernel, dim3(1), dim3(256), 0, s, d_log_alpha_per_sample, batch, log_alpha_gradient));
     }
     return B200RL_OK;
 }
@@ -174,9 +181,8 @@ int b200rl_sac_target_action_values(const float* q1_next, int ld_q1, const float
     if(!q1_next || !q2_next || !rewards || !terminated || !next_log_probs || !log_alpha || !target || batch < 0 || ld_q1 < 1 || ld_q2 < 1 || ld_target < 1)
         return B200RL_ERR_INVALID_ARGUMENT;
     if(batch == 0) return B200RL_OK;
-    sac_target_kernel<<<(batch + 127) / 128, 128, 0, (cudaStream_t)stream>>>(q1_next, ld_q1, q2_next, ld_q2, rewards, terminated, next_log_probs, log_alpha, gamma,
-                                                                          ignore_termination, entropy_bonus, entropy_bonus_next_step, target, ld_target, batch);
-    B200RL_LAUNCH_CHECK("sac_target_action_values");
+    B200RL_CUDA_TRY(launch_after(sac_target_kernel, dim3((batch + 127) / 128), dim3(128), 0, (cudaStream_t)stream, q1_next, ld_q1, q2_next, ld_q2, rewards, terminated, next_log_probs, log_alpha, gamma,
+                                                                          ignore_termination, entropy_bonus, entropy_bonus_next_step, target, ld_target, batch));
     return B200RL_OK;
 }
 
@@ -187,9 +193,8 @@ int b200rl_sac_min_value_d_output(const float* q1, int ld_q1, const float* q2, i
         return B200RL_ERR_INVALID_ARGUMENT;
     if(batch == 0) return B200RL_OK;
     const int n = batch * action_dim;
-    sac_min_value_kernel<<<(n + 127) / 128, 128, 0, (cudaStream_t)stream>>>(q1, ld_q1, q2, ld_q2, d_critic_1_input, d_critic_2_input, ld_d_input, action_offset, action_dim,
-                                                                         d_actor_output, ld_out, batch);
-    B200RL_LAUNCH_CHECK("sac_min_value_d_output");
+    B200RL_CUDA_TRY(launch_after(sac_min_value_kernel, dim3((n + 127) / 128), dim3(128), 0, (cudaStream_t)stream, q1, ld_q1, q2, ld_q2, d_critic_1_input, d_critic_2_input, ld_d_input, action_offset, action_dim,
+                                                                         d_actor_output, ld_out, batch));
     return B200RL_OK;
 }
 

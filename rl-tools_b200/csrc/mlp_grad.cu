@@ -293,14 +293,21 @@ __global__ void __launch_bounds__(GR_THREADS, 1) mlp_grad_kernel(const __grid_co
     if(warp == 0) tc::tmem_dealloc(tmem, 512);
 }
 
-// rows of `from` with row pitch ld into rows of a pitch that is a multiple of four, zeros behind the columns
-__global__ void __launch_bounds__(256) pad_rows_kernel(const float* __restrict__ from, long long ld, int rows, int cols, float* __restrict__ to){
-    const int pitch = (cols + 3) / 4 * 4;
-    const long long n = (long long)rows * pitch;
-    for(long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += gridDim.x * 256ll){
-        const int r = (int)(i / pitch), c = (int)(i - (long long)r * pitch);
-        to[i] = c < cols ? __ldg(from + r * ld + c) : 0.0f;
+// Rows of `from` with row pitch ld into rows of a pitch that is a multiple of four, zeros behind the columns. A thread takes four 16-byte pieces of the result, with all of their
+// loads under way; bound by HBM (202,203 rows of 29 columns, 49 MB: 21.9 us with an element and a 64-bit division at a time, 9.1 us this way).
+constexpr int PAD_PIECES = 4;
+__global__ void __launch_bounds__(256) pad_rows_kernel(const float* __restrict__ from, long long ld, unsigned pieces, unsigned per_row, int cols, float4* __restrict__ to){
+    const unsigned first = blockIdx.x * (256u * PAD_PIECES) + threadIdx.x;
+    float v[PAD_PIECES][4];
+#pragma unroll
+    for(int k = 0; k < PAD_PIECES; k++){
+        const unsigned i = first + 256u * k, r = i / per_row;
+        const int c = 4 * (int)(i - r * per_row);
+#pragma unroll
+        for(int j = 0; j < 4; j++) v[k][j] = i < pieces && c + j < cols ? __ldg(from + (long long)r * ld + c + j) : 0.0f;
     }
+#pragma unroll
+    for(int k = 0; k < PAD_PIECES; k++) if(first + 256u * k < pieces) to[first + 256u * k] = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------------------------------
@@ -309,8 +316,8 @@ int mlp_grad_error_get(int* word){ B200RL_CUDA_TRY(cudaMemcpyFromSymbol(word, g_
 int mlp_grad_error_clear(){ const int zero = 0; B200RL_CUDA_TRY(cudaMemcpyToSymbol(g_grad_error, &zero, sizeof(int))); return B200RL_OK; }
 
 int pad_rows(const float* from, long long ld, int rows, int cols, float* to, cudaStream_t s){
-    const long long n = (long long)rows * ((cols + 3) / 4 * 4), blocks = (n + 1023) / 1024;
-    pad_rows_kernel<<<(unsigned)(blocks < 16 * NUM_SMS ? blocks : 16 * NUM_SMS), 256, 0, s>>>(from, ld, rows, cols, to);
+    const unsigned per_row = (unsigned)(cols + 3) / 4, pieces = (unsigned)rows * per_row;            // at most 2^18 rows (a chunk of the backward pass) of 64 pieces
+    pad_rows_kernel<<<(pieces + 256 * PAD_PIECES - 1) / (256 * PAD_PIECES), 256, 0, s>>>(from, ld, pieces, per_row, cols, reinterpret_cast<float4*>(to));
     B200RL_LAUNCH_CHECK("pad_rows");
     return B200RL_OK;
 }

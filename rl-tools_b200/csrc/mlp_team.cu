@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
         if(tile + a.teams < a.row_tiles) stage(tile + a.teams, !other);
         const int row0 = tile * R;
         const float* y = smem + a.y_off + (other ? a.y_alt : 0);
-#pragma unroll 1
+#pragma unroll
         for(int l = 0; l < L; l++){
             forward_layer<C, L, true>(n, l, n.layer[l].a + (l == 0 && other ? n.a_alt : 0), smem, rank, [&](int r, int unit, float4 value, float4 derivative){
                 const int at = r * last.S + unit;
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
             if(l == L - 1) __syncthreads();
             else sync_team<C>();
         }
-#pragma unroll 1
+#pragma unroll
         for(int l = L - 1; l > 0; l--) backward_layer<C>(n, l, smem, rank, (L - l) & 1);
         store_activations<L>(n, smem, smem + a.out_off, rank, row0, a.rows, keep_from, a.chunk_rows, a.pre, a.out);
         accumulate_gradients<N, PO, PI>(n, smem, patches, acc, other);

@@ -326,6 +326,8 @@ __global__ void reduce_partials_kernel(float* dst, const float* __restrict__ par
 // (stride: floats from one segment's record to the next; O for densely packed segments)
 __global__ void __launch_bounds__(256) reduce_strided_partials_kernel(float* dst, const float* __restrict__ partial, int O, long long stride, int segs){
     __shared__ float red[8][33];
+    after_predecessor();
+    partial = opaque(partial);
     const int o = blockIdx.x * 32 + threadIdx.x;
     float s = 0.0f;
     if(o < O){
@@ -600,8 +602,7 @@ static int dense_backward_impl(const float* W, const float* x, int ldx, const fl
 
 // dst[i] += the sum of `segments` partial sums `stride` apart, in a fixed order
 int reduce_partials_into(float* dst, const float* partial, int n, long long stride, int segments, cudaStream_t s){
-    reduce_strided_partials_kernel<<<(n + 31) / 32, dim3(32, 8), 0, s>>>(dst, partial, n, stride, segments);
-    B200RL_LAUNCH_CHECK("reduce_partials");
+    B200RL_CUDA_TRY(launch_after(reduce_strided_partials_kernel, dim3((n + 31) / 32), dim3(32, 8), 0, s, dst, partial, n, stride, segments));
     return B200RL_OK;
 }
 

@@ -27,9 +27,10 @@
 namespace b200rl {
 
 namespace {
-constexpr int GR_SUM_WARPS = 8, GR_STAGING_WARPS = 12, GR_THREADS = 32 * (GR_SUM_WARPS + GR_STAGING_WARPS + 4), GR_UNIT = 32, GR_MAX_STAGES = 4, GR_MAX_JOBS = 2 * 8;
+constexpr int GR_SUM_WARPS = 8, GR_STAGING_WARPS = 12, GR_THREADS = 32 * (GR_SUM_WARPS + GR_STAGING_WARPS + 4), GR_UNIT = 32, GR_MAX_STAGES = 6, GR_MAX_JOBS = 2 * 8;
 constexpr uint32_t GR_BLOCK = GR_UNIT * 128;                     // one part of 64 columns of a unit: 32 rows x 128 bytes
-constexpr uint32_t GR_TILES = 2 * 48 * 1024, GR_RAW = 2 * 48 * 1024;        // two stages of tiles and two slots of fp32 rows of 128 + 256 columns; up to four of narrower ones
+constexpr uint32_t GR_TILES = 2 * 48 * 1024, GR_RAW = 2 * 48 * 1024;        // two stages of tiles and two slots of fp32 rows of 128 + 256 columns; up to six of narrower ones
+                                                                              // (64 + 64 columns: a copy takes longer than a unit; 202,203 rows of 29-64-64-5 114 us with four, 102 with six)
 // inverse scales of the columns, by unit: who stages unit u has waited for the MMAs of a unit at least u - GR_MAX_STAGES, which have waited for
 // the accumulator of the unit two before it to be read
 constexpr uint32_t GR_SCALES = 128 + 256, GR_SCALE_BUFFERS = GR_MAX_STAGES + 2;
@@ -88,6 +89,7 @@ __global__ void __launch_bounds__(GR_THREADS, 1) mlp_grad_kernel(const __grid_co
     uint32_t* slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(slot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    after_predecessor();
     const int split = blockIdx.x / a.n_jobs;
     const GradJob& y = a.job[blockIdx.x - split * a.n_jobs];
     const int M = y.M, N = y.N, n = (N + 15) / 16 * 16;
@@ -297,6 +299,8 @@ __global__ void __launch_bounds__(GR_THREADS, 1) mlp_grad_kernel(const __grid_co
 // loads under way; bound by HBM (202,203 rows of 29 columns, 49 MB: 21.9 us with an element and a 64-bit division at a time, 9.1 us this way).
 constexpr int PAD_PIECES = 4;
 __global__ void __launch_bounds__(256) pad_rows_kernel(const float* __restrict__ from, long long ld, unsigned pieces, unsigned per_row, int cols, float4* __restrict__ to){
+    after_predecessor();
+    from = opaque(from);
     const unsigned first = blockIdx.x * (256u * PAD_PIECES) + threadIdx.x;
     float v[PAD_PIECES][4];
 #pragma unroll
@@ -317,8 +321,7 @@ int mlp_grad_error_clear(){ const int zero = 0; B200RL_CUDA_TRY(cudaMemcpyToSymb
 
 int pad_rows(const float* from, long long ld, int rows, int cols, float* to, cudaStream_t s){
     const unsigned per_row = (unsigned)(cols + 3) / 4, pieces = (unsigned)rows * per_row;            // at most 2^18 rows (a chunk of the backward pass) of 64 pieces
-    pad_rows_kernel<<<(pieces + 256 * PAD_PIECES - 1) / (256 * PAD_PIECES), 256, 0, s>>>(from, ld, pieces, per_row, cols, reinterpret_cast<float4*>(to));
-    B200RL_LAUNCH_CHECK("pad_rows");
+    B200RL_CUDA_TRY(launch_after(pad_rows_kernel, dim3((pieces + 256 * PAD_PIECES - 1) / (256 * PAD_PIECES)), dim3(256), 0, s, from, ld, pieces, per_row, cols, reinterpret_cast<float4*>(to)));
     return B200RL_OK;
 }
 // Which operand gives the 128 rows of an accumulator: the input, whose gradient elements then lie next to each other in memory, unless that takes more jobs
@@ -391,7 +394,7 @@ int mlp_grad_launch(const b200rl_mlp_shape* sh, const float* const* input, const
         I = O;
     }
     if(!encoded) return B200RL_ERR_INVALID_ARGUMENT;
-    mlp_grad_kernel<<<a.n_jobs * a.splits, GR_THREADS, GR_SMEM, s>>>(a);
+    B200RL_CUDA_TRY(launch_after(mlp_grad_kernel, dim3(a.n_jobs * a.splits), dim3(GR_THREADS), GR_SMEM, s, a));
     B200RL_LAUNCH_CHECK("mlp_grad");
     return B200RL_OK;
 }

@@ -647,17 +647,19 @@ static size_t outputs_before_last(const b200rl_mlp_shape* sh){
 // Which training steps take one launch (mlp_team.cu) rather than a launch per pass: those whose chunk of rows has little work. The one launch's time grows with rows x
 // weights from the start, on CUDA cores; the tensor-core kernels take the same time up to a row tile per SM. Measured, one launch against the sequence, us (rows x weights in
 // millions):
-//   sequence of mlp_chain.cu   64-256-256-256-16 at 1,024 rows (155): 119 and 164, at 2,048 (310): 196 and 163, at 8,192 (1,240): 720 and 208; 64-256-256-16 at 2,048
-//                              (176): 91 and 128, at 3,072 (264): 134 and 130; 33-200-200-7 at 5,003 (240): 117 and 129, at 6,144 (295): 152 and 130; narrower ones
-//                              cross earlier: 64-128-128-16 at 8,192 (218): 99 and 93; 64-100-100-100-16 at 8,192 (229): 123 and 109; 64-100-100-16 (147): 67 and 90
-//   kernels per layer          64-320-320-16 at 2,048 (262): 134 and 187, at 4,096 (524): 229 and 204; 300-256-256-10 at 2,048 (297): 171 and 222, at 4,096 (593): 320 and
-//                              232; 512-128-128-10 at 4,096 (340): 152 and 171, at 8,192 (680): 286 and 190; 17-300-300-300-3 at 2,048 (381): 275 and 291
+//   sequence of mlp_chain.cu   64-256-256-16 at 2,048 (176): 78 and 103, at 3,072 (264): 106 and 111, at 4,096 (352): 143 and 113; 33-200-200-7 at 5,003 (240): 100 and 107, at 6,144
+//                              (295): 137 and 108; 33-200-200-200-7 at 2,048 (180): 101 and 122, at 3,072 (270): 140 and 136; 64-256-256-256-16 at 2,048 (310): 176 and 144;
+//                              narrower ones cross earlier: 64-128-128-16 at 8,192 (218): 70 and 74; 64-100-100-100-16 at 8,192 (229): 94 and 88; 64-100-100-16 (147): 50 and 72
+//   kernels per layer          up to 128 wide: 64-128-128-128-16 at 6,144 (264): 99 and 141; wider ones: 64-320-320-16 at 1,024 (131): 70 and 92, at 2,048 (262): 126 and 120;
+//                              300-256-256-10 at 1,024 (148): 97 and 84, at 3,072 (445): 235 and 163; 512-128-128-10 at 3,072 (255): 104 and 119, at 4,096 (340): 135 and 122
+//   above 160,000 weights      (they fill a team of eight): 128-350-350-10 at 512 (87): 68 and 72, at 1,024 (175): 118 and 108; 250-250-250-250-5 at 512 (97): 85 and 90, at 1,024
+//                              (193): 155 and 124; 17-300-300-300-3 at 256 (48): 59 and 57, at 1,024 (190): 148 and 134; 100-256-256-256-256 at 128 (28): 39 and 48, at 512 (114): 81 and 64
 static bool mlp_team_is_faster(const b200rl_mlp_shape* sh, int chunk_rows){
     long long weights = 0;
     int widest = sh->input_dim;
     for(int l = 0, I = sh->input_dim; l < sh->n_layers; I = sh->dims[l], l++){ weights += (long long)I * sh->dims[l]; if(sh->dims[l] > widest) widest = sh->dims[l]; }
     const bool chain = mlp_chain_takes(sh, chunk_rows, CHAIN_FORWARD) && mlp_chain_takes(sh, chunk_rows, CHAIN_GRADIENTS);
-    return weights * chunk_rows <= (!chain ? 400 : widest > 128 ? 245 : 200) * 1000000ll;
+    return weights * chunk_rows <= (chain ? (widest > 128 ? 245 : 200) : weights > 160000 ? 100 : widest > 128 ? 265 : 400) * 1000000ll;
 }
 
 }  // namespace b200rl

@@ -158,7 +158,6 @@ static bool choose_team(const b200rl_mlp_shape* sh, int rows, size_t scratch_byt
                 tile += (C == 1 ? 3800.0 : 7700.0) + 0.12 * R * y.S * y.P;
             }
             double cost = 0.15 * weights + tile * ((c.row_tiles + c.teams - 1) / c.teams) + 1.8 * c.net.quads + 0.0016 * C * c.net.quads * c.teams;
-            if(c.net.n_patches > THREADS) cost *= 1.5;                   // two patches a thread do not fit its registers (64-256-256-256-16 at 1,024 rows: 146 us, 102 with teams of eight)
             if(best == 0.0 || cost < best){ best = cost; *out = c; }
         }
     }
@@ -219,7 +218,7 @@ static int launch_team_step(const TeamStepArgs& a, size_t smem, cudaStream_t s){
 }
 template <int C, int L>
 static int launch_team_step_l(const TeamStepArgs& a, size_t smem, cudaStream_t s){
-    if(a.net.n_patches > THREADS) return launch_team_step<C, L, 2, 2, 2>(a, smem, s);
+    if(a.net.n_patches > THREADS) return launch_team_step<C, L, MAX_PATCHES_PER_THREAD, 1, 1>(a, smem, s);
     if(a.net.patch_i == 2) return launch_team_step<C, L, 1, 2, 2>(a, smem, s);
     if(a.net.patch_o == 2) return launch_team_step<C, L, 1, 2, 1>(a, smem, s);
     return launch_team_step<C, L, 1, 1, 1>(a, smem, s);

@@ -35,7 +35,7 @@ namespace b200rl { namespace team {
 
 // Four warps per scheduler: with the products' sums in registers until they are finished, more warps hide the shared-memory latencies.
 // (Half as many for networks without work for more, by a number in the plan instead of a constant: no faster there, 3 to 8 % slower elsewhere.)
-constexpr int THREADS = 512, WARPS = THREADS / 32, MAX_LAYERS = 4, MAX_PATCHES_PER_THREAD = 2;
+constexpr int THREADS = 512, WARPS = THREADS / 32, MAX_LAYERS = 4, MAX_PATCHES_PER_THREAD = 4;
 
 // quotient by a divisor known on the host (n d < 2^32): one multiplication instead of a division's ~40 instructions, which on the path of a
 // few microseconds per layer would be most of the time
@@ -108,10 +108,12 @@ inline bool plan(const b200rl_mlp_shape* sh, int C, int R, int base, bool keep_p
         if(l > 0 && C > 1 && C * R * n.layer[l - 1].S > rb) rb = C * R * n.layer[l - 1].S;
         y.by_S4 = divisor(y.S / 4); y.by_I4 = divisor(I4); y.by_I = divisor(y.I); y.by_row = divisor(y.I / 4); y.by_owner = divisor(l > 0 ? n.layer[l - 1].S : 1);
     }
-    // the smallest patch that gives every thread at most one; shapes that exceed the largest patch take two of those
+    // the smallest patch that gives every thread at most one; shapes that exceed the largest patch (layers of which its edges waste much) take up to four of the smallest: the same sums
+    // in registers, twice the reads. 64-320-320-16 by teams of four (541 of the largest, 2,041 of the smallest): 70 us at 1,024 rows, 91 by teams of eight with one patch a
+    // thread; 33-240-240-240-7: 87 and 107. Two of the largest do not fit the registers (32-512-512-4 at 256 rows: 102 us, 46 as a launch per pass)
     bool fits = false;
     for(int k = least; k < 4 && !fits; k++){
-        n.patch_o = k > 0 ? 2 : 1; n.patch_i = k > 1 ? 2 : 1; n.n_patches = 0;
+        n.patch_o = k == 1 || k == 2 ? 2 : 1; n.patch_i = k == 2 ? 2 : 1; n.n_patches = 0;
         for(int l = 0; l < n.n_layers; l++){
             Layer& y = n.layer[l];
             y.patch_begin = n.n_patches; y.across = ((y.I + 1 + 3) / 4 + n.patch_i - 1) / n.patch_i; y.by_across = divisor(y.across);

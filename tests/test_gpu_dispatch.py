@@ -26,6 +26,13 @@ def test_training_step_takes_one_launch_where_that_is_faster(lib, batch, chunks,
     assert (len(names) == 1 and "mlp_team_step" in names[0]) == one_launch, names
 
 
+@pytest.mark.parametrize("batch,I,dims,one_launch", [
+    (3072, 64, [320, 320, 16], False), (3072, 512, [128, 128, 10], True), (6144, 64, [128, 128, 128, 16], True), (512, 128, [350, 350, 10], True), (1024, 128, [350, 350, 10], False),
+    (256, 100, [256, 256, 256, 256], True), (512, 100, [256, 256, 256, 256], False), (128, 32, [512, 512, 4], False)])
+def test_training_step_beside_kernels_per_layer_takes_one_launch_where_that_is_faster(lib, batch, I, dims, one_launch):
+    test_training_step_takes_one_launch_where_that_is_faster(lib, batch, 1, I, dims, one_launch)
+
+
 def _chain(names):
     return any("mlp_chain_kernel" in n for n in names)
 

@@ -87,7 +87,8 @@ def test_ppo_epoch_equals_the_separate_calls(lib, batch, minibatches, obs, actio
 @pytest.mark.parametrize("batch,I,dims,acts", [
     (3, 1, [1], ["tanh"]), (33, 4, [4, 4], ["tanh", "identity"]), (300, 3, [5, 9, 2], ["tanh", "sigmoid", "identity"]), (1024, 16, [64, 64, 6], ["tanh", "tanh", "tanh"]),
     (2049, 31, [30, 66, 3], ["fast_tanh", "tanh", "identity"]), (64, 200, [130, 17, 8], ["tanh", "tanh", "identity"]), (1025, 12, [96, 100, 104, 1], ["tanh", "tanh", "sigmoid", "identity"]),
-    (700, 64, [256, 256, 256, 5], ["tanh", "tanh", "tanh", "identity"]), (400, 511, [508, 12], ["tanh", "identity"])])
+    (700, 64, [256, 256, 256, 5], ["tanh", "tanh", "tanh", "identity"]), (400, 511, [508, 12], ["tanh", "identity"]),
+    (700, 64, [320, 320, 16], ["tanh", "tanh", "identity"]), (259, 13, [309, 311, 3], ["tanh", "tanh", "tanh"])])
 def test_train_step_of_tiles_and_patches(lib, batch, I, dims, acts):
     """Sizes at which the walk's tiles have remainders: one unit, inputs that are and are not whole pieces of four (the bias lies in a piece of its own or in the last one), a summed index
     shared out over one to sixteen lanes, each size of gradient patch, odd numbers of patches, aligned and unaligned input rows."""

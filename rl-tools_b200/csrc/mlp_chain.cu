@@ -626,14 +626,14 @@ __global__ void __launch_bounds__(1024) chain_image_kernel(const __grid_constant
 // are (34 us for 64-256-256-256-16, 54 us when everything is kept; 14 and 18 us for 27-64-64-8), while the kernels per layer gain from a smaller batch and
 // start sooner; so the lines lie where the rows fill the SMs or the products are many. Measured, these kernels against the kernels per layer, us (graph of ten
 // calls; rows x the network's weights in millions behind the rows):
-//   evaluate            4-256-256-1 at 2,048: 24 and 34; 64-256-16 at 2,048 (42): 17 and 15, at 4,096 (84): 18 and 28; 8-256-4 at 8,192 (25): 14 and 13, at 16,384
-//                       (50): 15 and 20; 64-128-4 at 8,192 (71): 15 and 13, at 16,384 (143): 15 and 17; 3-32-32-1 at 8,192 (9): 13 and 12, at 16,384 (19): 13 and 15
-//   forward             33-200-200-7 at 2,048 (98): 38 and 28, at 4,096 (197): 38 and 39; 64-256-256-256-16 at 2,048 (310): 54 and 60; 27-64-64-8 at 8,192 (52): 18 and 17;
-//                       3-64-64-1 at 16,384 (71): 19 and 24; 20-32-32-32-8 at 16,384 (48): 25 and 33; 3-50-50-1 at 16,384 (44): 23 and 29; 3-32-32-1 at 65,536
-//                       (75): 50 and 41; 64-128-4 at 65,536 (570): 56 and 49
-//   gradients           17-130-130-3 at 4,096 (80): 59 and 50, at 8,192 (160): 67 and 94; 33-200-200-7 at 2,048 (98): 61 and 66; 64-256-16 at 8,192 (168): 42 and 38, at
-//                       16,384: 48 and 47; 256-256-256 at 2,048: 59 and 83; 64-128-4 at 8,192: 33 and 27, at 16,384: 37 and 40; 10-16-2 at 16,384 (3): 32 and 27
-//   input gradient alone  17-130-130-3 at 2,048 (40): 29 and 18, at 4,096 (80): 29 and 35; 8-256-4 at 4,096 (13): 24 and 16, at 8,192: 22 and 98
+//   evaluate            4-256-256-1 at 2,048: 23 and 29; 64-256-16 at 2,048 (42): 17 and 15, at 4,096 (84): 17 and 28; 8-256-4 at 8,192 (25): 15 and 13, at 16,384
+//                       (50): 15 and 20; 64-128-4 at 8,192 (71): 14 and 13, at 16,384 (143): 15 and 17; 3-32-32-1 at 8,192 (9): 11 and 12, at 16,384 (19): 11 and 15
+//   forward             33-200-200-7 at 2,048 (98): 37 and 23, at 4,096 (197): 37 and 34; 64-256-256-256-16 at 2,048 (310): 54 and 55; 27-64-64-8 at 8,192 (52): 17 and 17;
+//                       3-64-64-1 at 16,384 (71): 17 and 24; 20-32-32-32-8 at 16,384 (48): 17 and 25; 3-50-50-1 at 16,384 (44): 17 and 24; 3-32-32-1 at 65,536
+//                       (75): 28 and 42 (below the line of 2,048 weights; 50 and 41 with one tile per SM); 64-128-4 at 65,536 (570): 51 and 49
+//   gradients           17-130-130-3 at 4,096 (80): 51 and 49, at 8,192 (160): 57 and 81; 33-200-200-7 at 2,048 (98): 58 and 53; 64-256-16 at 8,192 (168): 42 and 39, at
+//                       16,384: 48 and 48; 256-256-256 at 2,048: 58 and 83; 64-128-4 at 8,192: 31 and 28, at 16,384: 34 and 40; 10-16-2 at 16,384 (3): 25 and 27
+//   input gradient alone  17-130-130-3 at 2,048 (40): 27 and 18, at 4,096 (80): 27 and 35; 8-256-4 at 4,096 (13): 22 and 17, at 8,192: 22 and 99
 bool mlp_chain_takes(const b200rl_mlp_shape* sh, int batch, int pass){
     if(sh->n_layers > CH_MAX_STEPS || sh->n_layers < 2) return false;
     int widest = sh->input_dim;

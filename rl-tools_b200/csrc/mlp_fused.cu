@@ -397,13 +397,18 @@ static int allow_shared_memory(KERNEL kernel, std::atomic<int>* granted, size_t 
     return B200RL_OK;
 }
 
+// Whether a launch may start under the kernel before it: only where its blocks find room beside that one's, one per SM; blocks that come early otherwise pile up on the SMs that are free, and
+// the launch ends with them. us, ordinary / early always / early up to a block per SM: forward 3-64-64-10, 4,096 rows (512 blocks) 12.2 / 14.1 / 12.1, 2,374 rows with backward 29.1 / 35.2
+// / 28.3; 24-64-64-64-8, 2,374 rows 13.7 / 15.3 / 13.7. The backward chain holds the most shared memory and comes between two kernels of as many blocks: half as many (8-128-128-2,
+// forward and backward, 290 rows, 145 blocks: 22.6 ordinary, 24.5 early, 21.1 with this line; 100 rows, 50 blocks: 17.4 ordinary, 17.3 early).
+static bool early_launch_pays(int blocks, int most = NUM_SMS){ return blocks <= most; }
 template <int ROWS, bool SAVE>
 static int launch_fused_forward(const FusedShape& f, const float* params, const float* x, int ldx, float* pre, float* out, float* y, int ldy, cudaStream_t s){
     static std::atomic<int> granted[MAX_DEVICES];
     const size_t bytes = ((size_t)f.smem_params + 2 * ROWS * FUSED_MAX_WIDTH) * sizeof(float);
     int rc = allow_shared_memory(mlp_fused_forward_kernel<ROWS, SAVE>, granted, bytes);
     if(rc) return rc;
-    B200RL_CUDA_TRY(launch_after(mlp_fused_forward_kernel<ROWS, SAVE>, dim3((f.batch + ROWS - 1) / ROWS), dim3(FUSED_THREADS), bytes, s, f, params, x, ldx, pre, out, y, ldy));
+    B200RL_CUDA_TRY(launch_after_if(early_launch_pays((f.batch + ROWS - 1) / ROWS), mlp_fused_forward_kernel<ROWS, SAVE>, dim3((f.batch + ROWS - 1) / ROWS), dim3(FUSED_THREADS), bytes, s, f, params, x, ldx, pre, out, y, ldy));
     return B200RL_OK;
 }
 template <int ROWS>
@@ -413,7 +418,7 @@ static int launch_fused_chain(const FusedShape& f, const float* params, const fl
     const size_t bytes = ((size_t)((f.n_params + 3) & ~3) + 2 * ROWS * FUSED_MAX_WIDTH) * sizeof(float);
     int rc = allow_shared_memory(mlp_fused_backward_chain_kernel<ROWS>, granted, bytes);
     if(rc) return rc;
-    B200RL_CUDA_TRY(launch_after(mlp_fused_backward_chain_kernel<ROWS>, dim3((f.batch + ROWS - 1) / ROWS), dim3(FUSED_THREADS), bytes, s, f, params, pre, d_out, ldd, dpre, d_input, ldi,
+    B200RL_CUDA_TRY(launch_after_if(early_launch_pays((f.batch + ROWS - 1) / ROWS, NUM_SMS / 2), mlp_fused_backward_chain_kernel<ROWS>, dim3((f.batch + ROWS - 1) / ROWS), dim3(FUSED_THREADS), bytes, s, f, params, pre, d_out, ldd, dpre, d_input, ldi,
                                  counters, n_counters));
     return B200RL_OK;
 }
@@ -448,7 +453,7 @@ int mlp_fused_backward(const b200rl_mlp_shape* sh, const float* params, float* g
     else rc = launch_fused_chain<8>(f, params, pre, d_out, ldd, dpre, d_input, sh->input_dim, cnt, (int)fs.counters, s);
     if(rc) return rc;
     if(grads){
-        B200RL_CUDA_TRY(launch_after(mlp_fused_grads_kernel, dim3(fs.tiles, fs.slices), dim3(256), 0, s, f, x, ldx, out, dpre, grads, partial, counters, fs.slices));
+        B200RL_CUDA_TRY(launch_after_if(early_launch_pays(fs.tiles * fs.slices), mlp_fused_grads_kernel, dim3(fs.tiles, fs.slices), dim3(256), 0, s, f, x, ldx, out, dpre, grads, partial, counters, fs.slices));
     }
     return B200RL_OK;
 }

@@ -129,7 +129,8 @@ __global__ void __launch_bounds__(GR_THREADS, 1) mlp_grad_kernel(const __grid_co
         for(int p = 0; p < 8; p++)
 #pragma unroll
             for(int i = 0; i < 8; i++) acc[p][i] = zero;
-        const int segments = (units + GR_SEGMENT - 1) / GR_SEGMENT, segment = (units + segments - 1) / max(1, segments);
+        // A range may have no unit (2,048 rows of 128-256-16: 64 units for 74 ranges): one segment of none, whose record is zeros
+        const int segments = max(1, (units + GR_SEGMENT - 1) / GR_SEGMENT), segment = (units + segments - 1) / segments;
         for(int begin = 0; ; begin += segment){
         const int end = min(units, begin + segment);
         for(int d = begin; d < end; d++){

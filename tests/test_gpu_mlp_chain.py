@@ -108,6 +108,12 @@ def test_backward_matches_fp64(lib, rows, I, dims, acts, mode):
         assert float((err - 1e-5 * size).max()) <= 1e-6 / rows
 
 
+@pytest.mark.parametrize("rows", [2048, 2051, 2080, 2367, 2368, 2369])
+def test_gradients_of_fewer_units_than_ranges(lib, rows):
+    """Two layers, each of whose gradients is one job: 74 ranges of the rows for the 148 SMs, more than the batch has units of 32 rows. A range without a unit leaves zeros."""
+    test_backward_matches_fp64(lib, rows, 128, [256, 16], ["tanh", "identity"], "gradients")
+
+
 @pytest.mark.parametrize("rows,I,dims,acts", [
     (16385, 64, [64, 64, 64], ["tanh", "relu", "identity"]), (16400, 1, [16, 32, 17, 33, 48, 64, 64, 1], ["tanh"] * 8), (2 * 2 * 148 * 128 + 5, 33, [32, 31, 64, 2], ["sigmoid", "tanh", "fast_tanh", "tanh"]),
     (16385, 65, [64, 64, 3], ["tanh", "tanh", "identity"]), (16385, 64, [64, 65, 3], ["tanh", "tanh", "identity"])])

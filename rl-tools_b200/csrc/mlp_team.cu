@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
             forward_layer<C, L, true>(n, l, n.layer[l].a + (l == 0 && other ? n.a_alt : 0), smem, rank, [&](int r, int unit, float4 value, float4 derivative){
                 const int at = r * last.S + unit;
                 const float4 target = *reinterpret_cast<const float4*>(y + at);
-                auto d = [&](float v, float wanted, float dv){ return row0 + r < a.rows && dv != 0.0f ? __fmul_rn(__fsub_rn(v, wanted), a.constant) * dv : 0.0f; };
+                auto d = [&](float v, float wanted, float dv){ return row0 + r < a.rows ? d_pre(__fmul_rn(__fsub_rn(v, wanted), a.constant), dv) : 0.0f; };
                 *reinterpret_cast<float4*>(smem + last.d + at) = make_float4(d(value.x, target.x, derivative.x), d(value.y, target.y, derivative.y), d(value.z, target.z, derivative.z), d(value.w, target.w, derivative.w));
                 *reinterpret_cast<float4*>(smem + a.out_off + at) = value;
             });

@@ -181,6 +181,11 @@ __device__ __forceinline__ float4 activate(float4 x, int act, float4& derivative
     }
 }
 
+// Units beyond a layer's width carry the derivative -0, which no activation has, and their d_pre is 0 whatever stands in their place (targets that were never copied; in the layers below the sums
+// of the bias column). A derivative of 0 is not that: it is a factor like any other, so that what is not finite stays so.
+constexpr float BEYOND = -0.0f;
+__device__ __forceinline__ float d_pre(float d_out, float derivative){ return __float_as_uint(derivative) == 0x80000000u ? 0.0f : d_out * derivative; }
+
 // Once per launch: the weight and input rows start at zero (the padding behind a row and the rows beyond the layer's width stay so), with the
 // constant 1 in the bias column of every input row. A CTA-wide barrier, then load_weights.
 template <int L>
@@ -254,7 +259,7 @@ __device__ __forceinline__ void add_parts(float4 (&v)[4], int shift, int lane){
 }
 
 // One layer of the forward pass; `a`: where its input rows lie. The values go into the next layer's input rows of the whole team; after the last layer
-// finish(row, first unit, values, derivatives) runs for every row and four units of this CTA (derivatives of units beyond the layer are 0). Ends without a barrier.
+// finish(row, first unit, values, derivatives) runs for every row and four units of this CTA. Ends without a barrier.
 template <int C, int L, bool KEEP_PRE, typename FINISH>
 __device__ __forceinline__ void forward_layer(const Net& n, int l, int a_rows, float* smem, int rank, FINISH finish){
     const Layer& y = n.layer[l];
@@ -306,7 +311,7 @@ __device__ __forceinline__ void forward_layer(const Net& n, int l, int a_rows, f
             v[0] = v[1]; v[1] = v[2]; v[2] = v[3];
             float4 dv;
             const float4 value = activate(pre, y.act, dv);
-            if(beyond > 0){ dv.w = 0.0f; if(beyond > 1) dv.z = 0.0f; if(beyond > 2) dv.y = 0.0f; if(beyond > 3) dv.x = 0.0f; }
+            if(beyond > 0){ dv.w = BEYOND; if(beyond > 1) dv.z = BEYOND; if(beyond > 2) dv.y = BEYOND; if(beyond > 3) dv.x = BEYOND; }
             const int at = r * y.S + 4 * og;
             if(sh.copy == 0){
                 *reinterpret_cast<float4*>(smem + y.g + at) = dv;
@@ -361,9 +366,9 @@ __device__ __forceinline__ void backward_layer(const Net& n, int l, float* smem,
     float* rb = smem + n.rb[turn];
     const int tid = thread_here(), lane = tid & 31, warp = tid >> 5, I4 = (y.I + 3) >> 2, S4 = y.S >> 2, P4 = y.P >> 2, shift = y.bwd_shift, G = 1 << shift;
     const Share sh = share(shift, lane);
-    auto below = [&](int at, float4 v){                                  // units beyond the layer's width have derivative 0
+    auto below = [&](int at, float4 v){
         const float4 dv = *reinterpret_cast<const float4*>(smem + z.g + at);
-        *reinterpret_cast<float4*>(smem + z.d + at) = make_float4(dv.x != 0.0f ? v.x * dv.x : 0.0f, dv.y != 0.0f ? v.y * dv.y : 0.0f, dv.z != 0.0f ? v.z * dv.z : 0.0f, dv.w != 0.0f ? v.w * dv.w : 0.0f);
+        *reinterpret_cast<float4*>(smem + z.d + at) = make_float4(d_pre(v.x, dv.x), d_pre(v.y, dv.y), d_pre(v.z, dv.z), d_pre(v.w, dv.w));
     };
 #pragma unroll 1
     for(int t0 = warp << (5 - shift); t0 < y.bwd_tiles; t0 += WARPS << (5 - shift)){

@@ -94,3 +94,31 @@ def test_train_step_of_tiles_and_patches(lib, batch, I, dims, acts):
     shared out over one to sixteen lanes, each size of gradient patch, odd numbers of patches, aligned and unaligned input rows."""
     test_train_step_equals_the_separate_calls(lib, batch, 1, I, dims, acts)
     test_train_step_equals_the_separate_calls(lib, batch, 2, I, dims, acts)
+
+
+@pytest.mark.parametrize("batch,I,dims,acts", [
+    (40, 5, [16, 6], ["tanh", "relu"]), (40, 5, [16, 6], ["tanh", "tanh"]), (40, 5, [16, 6], ["relu", "identity"]), (256, 4, [256, 256, 1], ["relu", "relu", "relu"]),
+    (256, 4, [256, 255, 3], ["relu", "tanh", "fast_tanh"])])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_train_step_keeps_what_is_not_finite(lib, batch, I, dims, acts, value):
+    """A target that is not finite reaches the gradient also where the derivative of its output, or of the units below it, is 0 (inactive ReLU, saturated tanh): the same entries are finite
+    and the same are NaN as after the separate calls."""
+    import torch
+    x = torch.from_numpy(mg.det_normal(1, batch * I).reshape(batch, I)).cuda()
+    a, b = _net(lib, torch, batch, I, dims, acts, 5), _net(lib, torch, batch, I, dims, acts, 5)
+    n_last = dims[-1] * dims[-2] + dims[-1]
+    for net in (a, b):
+        net.params[-dims[-1]:] = -40.0                                    # every output far on the side where its derivative is 0, if its activation has one
+    y = torch.from_numpy(mg.det_normal(2, batch * dims[-1]).reshape(batch, dims[-1])).cuda()
+    y[batch // 2, dims[-1] // 2] = value
+    a.train_step(x, y, 1.0)
+    b.zero_gradient()
+    out = b.forward(x)
+    b.backward(x, lib.mse_gradient(out, y, 1.0, d_a=b.d_out_buffer()))
+    b.step()
+    assert not torch.isfinite(b.grads[-n_last:]).all()
+    for name in ("grads", "params", "m", "v"):
+        got, want = getattr(a, name), getattr(b, name)
+        assert torch.equal(torch.isfinite(got), torch.isfinite(want)), name
+        if value != value:
+            assert torch.equal(torch.isnan(got), torch.isnan(want)), name

@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------------------------------
-struct TeamChoice { Net net; int C, teams, row_tiles, y_off, y_alt, out_off; size_t smem; };
+struct TeamChoice { Net net; int teams, row_tiles, y_off, y_alt, out_off; size_t smem; };
 
 constexpr size_t TEAM_SMEM = 220 * 1024;
 constexpr int TEAM_MAX_ROWS = 8192;          // what was measured; up to there the caller asks for steps of little work only (dense.cu)
@@ -137,30 +137,27 @@ static bool choose_team(const b200rl_mlp_shape* sh, int rows, size_t scratch_byt
     double best = 0.0;
     for(int C = 1; C <= 8; C *= 2){
         const int max_teams = team_capacity(C);
-        if(max_teams < 1) continue;
+        TeamChoice c{};
+        if(max_teams < 1 || !spread(sh, C, 0, &c.net)) continue;
+        double weights = 0.0;
+        for(int l = 0; l < c.net.n_layers; l++) weights += (double)c.net.layer[l].S * c.net.layer[l].P;
+        const Layer& last = c.net.layer[c.net.n_layers - 1];
         for(int R = 4; R <= 32; R += 4){
-            TeamChoice c{};
-            if(!plan(sh, C, R, 0, true, 0, &c.net)) continue;
-            c.C = C;
-            const Layer& last = c.net.layer[c.net.n_layers - 1];
+            place(c.net, R, true);
             int off = (c.net.end + 3) / 4 * 4;
             c.y_off = off; c.y_alt = R * last.S; off += 2 * R * last.S;
             c.out_off = off; off += R * last.S;
             c.smem = sizeof(float) * (size_t)off;
-            if(c.smem > TEAM_SMEM) continue;
+            if(c.smem > TEAM_SMEM) break;                                // more rows take more
             c.row_tiles = (rows + R - 1) / R;
             c.teams = c.row_tiles < max_teams ? c.row_tiles : max_teams;
-            if(sizeof(float4) * (size_t)c.teams * c.C * c.net.quads > scratch_bytes) continue;
-            double weights = 0.0, tile = 0.0;
-            for(int l = 0; l < c.net.n_layers; l++){
-                const Layer& y = c.net.layer[l];
-                weights += (double)y.S * y.P;
-                tile += (C == 1 ? 3800.0 : 7700.0) + 0.12 * R * y.S * y.P;
-            }
-            double cost = 0.15 * weights + tile * ((c.row_tiles + c.teams - 1) / c.teams) + 1.8 * c.net.quads + 0.0016 * C * c.net.quads * c.teams;
+            if(sizeof(float4) * (size_t)c.teams * C * c.net.quads > scratch_bytes) continue;
+            const double tile = (C == 1 ? 3800.0 : 7700.0) * c.net.n_layers + 0.12 * R * weights;
+            const double cost = 0.15 * weights + tile * ((c.row_tiles + c.teams - 1) / c.teams) + 1.8 * c.net.quads + 0.0016 * C * c.net.quads * c.teams;
             if(best == 0.0 || cost < best){ best = cost; *out = c; }
         }
     }
+    if(best > 0.0) complete(out->net);
     return best > 0.0;
 }
 
@@ -168,7 +165,7 @@ static bool choose_team(const b200rl_mlp_shape* sh, int rows, size_t scratch_byt
 size_t mlp_team_scratch_bytes(const b200rl_mlp_shape* sh, int rows){
     TeamChoice c;
     if(rows < 1 || !choose_team(sh, rows, SIZE_MAX, &c)) return 0;
-    return sizeof(float4) * (size_t)team_capacity(c.C) * c.C * c.net.quads;
+    return sizeof(float4) * (size_t)team_capacity(c.net.C) * c.net.C * c.net.quads;
 }
 
 static void team_attributes(cudaLaunchAttribute (&attr)[2], int C){
@@ -247,14 +244,14 @@ int mlp_team_step(const b200rl_mlp_shape* sh, float* params, float* grads, float
     a.constant = 2.0f / ((float)chunk_rows * (float)sh->dims[sh->n_layers - 1]) * loss_weight;
     a.y_off = c.y_off; a.y_alt = c.y_alt; a.out_off = c.out_off; a.by_S = divisor(c.net.layer[c.net.n_layers - 1].S);
     // threads per quad of the reduction: as many as let the grid take all quads in one pass, no more than there are sums to add
-    const int quads = c.C * c.net.quads, threads = c.teams * c.C * THREADS;
+    const int quads = c.net.C * c.net.quads, threads = c.teams * c.net.C * THREADS;
     a.lanes = 4;
     while(a.lanes < 32 && 2 * a.lanes <= c.teams && (long long)quads * 2 * a.lanes <= threads) a.lanes *= 2;
     int rc = grid_barriers(1, s, &a.barrier);
     if(rc) return rc;
-    if(c.C == 1) return launch_team_step_c<1>(a, c.smem, s);
-    if(c.C == 2) return launch_team_step_c<2>(a, c.smem, s);
-    if(c.C == 4) return launch_team_step_c<4>(a, c.smem, s);
+    if(c.net.C == 1) return launch_team_step_c<1>(a, c.smem, s);
+    if(c.net.C == 2) return launch_team_step_c<2>(a, c.smem, s);
+    if(c.net.C == 4) return launch_team_step_c<4>(a, c.smem, s);
     return launch_team_step_c<8>(a, c.smem, s);
 }
 

@@ -54,7 +54,7 @@ struct Layer {
     Divisor by_S4, by_I, by_row, by_I4, by_across, by_owner;
 };
 struct Net {
-    int n_layers, R, n_params;
+    int n_layers, C, R, n_params;            // C: CTAs per team
     int patch_o, patch_i, n_patches, quads;  // a patch is patch_o x patch_i pieces of four (1 x 1, 2 x 1, 2 x 2); patches per CTA; 16-byte pieces of gradient sums per CTA
     int a_alt;                               // the first layer's second buffer of input rows lies this much behind the first
     Divisor by_quads, by_patches, by_I0;
@@ -77,60 +77,76 @@ inline int lanes_of_a_tile(int tiles, int K4){
     return best;
 }
 
-// host: lays a network out for teams of C CTAs and R rows per tile, from shared-memory offset `base` on. False: a shape these kernels do not take.
-// `least`: 0, or patches of at least 2 x 1 (1), 2 x 2 (2).
-inline bool plan(const b200rl_mlp_shape* sh, int C, int R, int base, bool keep_pre, int least, Net* out){
+// host: a plan is made in three parts, so that a search over team sizes and tiles pays for each of them once: what follows from the team size, what follows from the rows of a tile, and what
+// only the chosen plan needs (32 candidates of 4-256-256-1: 0.5 us, 6.7 with everything made for each of them).
+//
+// Units, pitches and gradient patches for teams of C CTAs. False: a shape these kernels do not take. `least`: 0, or patches of at least 2 x 1 (1), 2 x 2 (2).
+inline bool spread(const b200rl_mlp_shape* sh, int C, int least, Net* out){
     if(sh->n_layers > MAX_LAYERS) return false;
     Net n{};
-    n.n_layers = sh->n_layers; n.R = R;
-    int I = sh->input_dim, off = base, rb = 0;
+    n.n_layers = sh->n_layers; n.C = C;
+    int I = sh->input_dim;
     long long po = 0, ao = 0;
-    for(int l = 0; l < sh->n_layers; l++){                               // what has to start at zero lies together
+    for(int l = 0; l < sh->n_layers; l++){
         Layer& y = n.layer[l];
         y.O = sh->dims[l]; y.I = I; y.act = sh->acts[l];
         y.S = ((y.O + C - 1) / C + 3) / 4 * 4; y.P = 4 * (((I + 1 + 3) / 4) | 1); y.K4 = (I + 3) / 4;
-        y.w = off; off += y.S * y.P;
-        y.a = off; off += R * y.P;
-        if(l == 0){ n.a_alt = R * y.P; off += R * y.P; }
-        I = y.O;
-    }
-    n.zero_begin = base; n.zero_end = off;
-    for(int l = 0; l < sh->n_layers; l++){
-        Layer& y = n.layer[l];
         y.poff = po; y.aoff = ao;
         po += (long long)y.O * y.I + y.O; ao += y.O;
-        if(keep_pre){ y.p = off; off += R * y.S; }
-        y.g = off; off += R * y.S;
-        y.d = off; off += R * y.S;
-        const int I4 = (y.I + 3) / 4;
-        y.fwd_tiles = (R / 4) * (y.S / 4); y.fwd_shift = lanes_of_a_tile(y.fwd_tiles, y.K4);
-        y.bwd_tiles = (R / 4) * I4; y.bwd_shift = lanes_of_a_tile(y.bwd_tiles, y.S / 4);
-        if(l > 0 && C > 1 && C * R * n.layer[l - 1].S > rb) rb = C * R * n.layer[l - 1].S;
-        y.by_S4 = divisor(y.S / 4); y.by_I4 = divisor(I4); y.by_I = divisor(y.I); y.by_row = divisor(y.I / 4); y.by_owner = divisor(l > 0 ? n.layer[l - 1].S : 1);
+        I = y.O;
     }
+    n.n_params = (int)po;
     // the smallest patch that gives every thread at most one; shapes that exceed the largest patch (layers of which its edges waste much) take up to four of the smallest: the same sums
     // in registers, twice the reads. 64-320-320-16 by teams of four (541 of the largest, 2,041 of the smallest): 70 us at 1,024 rows, 91 by teams of eight with one patch a
     // thread; 33-240-240-240-7: 87 and 107. Two of the largest do not fit the registers (32-512-512-4 at 256 rows: 102 us, 46 as a launch per pass)
     bool fits = false;
     for(int k = least; k < 4 && !fits; k++){
-        n.patch_o = k == 1 || k == 2 ? 2 : 1; n.patch_i = k == 2 ? 2 : 1; n.n_patches = 0;
+        const int more_o = k == 1 || k == 2, more_i = k == 2;
+        n.patch_o = 1 + more_o; n.patch_i = 1 + more_i; n.n_patches = 0;
         for(int l = 0; l < n.n_layers; l++){
             Layer& y = n.layer[l];
-            y.patch_begin = n.n_patches; y.across = ((y.I + 1 + 3) / 4 + n.patch_i - 1) / n.patch_i; y.by_across = divisor(y.across);
-            n.n_patches += (y.S / 4 + n.patch_o - 1) / n.patch_o * y.across;
+            y.patch_begin = n.n_patches; y.across = (y.I / 4 + 1 + more_i) >> more_i;
+            n.n_patches += ((y.S / 4 + more_o) >> more_o) * y.across;
         }
         fits = n.n_patches <= (k == 3 ? MAX_PATCHES_PER_THREAD : 1) * THREADS;
     }
-    if(!fits || off % 4 != 0) return false;
     n.quads = n.n_patches * n.patch_o * 4 * n.patch_i;
-    n.n_params = (int)po;
-    n.by_quads = divisor(n.quads); n.by_patches = divisor(n.n_patches); n.by_I0 = divisor(sh->input_dim);
+    *out = n;
+    return fits;
+}
+// Where everything lies for tiles of R rows (a multiple of four)
+inline void place(Net& n, int R, bool keep_pre){
+    n.R = R;
+    int off = 0, rb = 0;
+    for(int l = 0; l < n.n_layers; l++){                                 // what has to start at zero lies together
+        Layer& y = n.layer[l];
+        y.w = off; off += y.S * y.P;
+        y.a = off; off += R * y.P;
+        if(l == 0){ n.a_alt = R * y.P; off += R * y.P; }
+    }
+    n.zero_begin = 0; n.zero_end = off;
+    for(int l = 0; l < n.n_layers; l++){
+        Layer& y = n.layer[l];
+        if(keep_pre){ y.p = off; off += R * y.S; }
+        y.g = off; off += R * y.S;
+        y.d = off; off += R * y.S;
+        if(l > 0 && n.C > 1 && n.C * R * n.layer[l - 1].S > rb) rb = n.C * R * n.layer[l - 1].S;
+    }
     off += 4;                                                            // a patch at the end of a row reads the piece behind it (into sums that nobody uses)
     n.rb[0] = off; off += rb;
     n.rb[1] = off; off += rb;
     n.end = off;
-    *out = n;
-    return true;
+}
+// What only the kernel reads: tiles, lanes and divisors
+inline void complete(Net& n){
+    for(int l = 0; l < n.n_layers; l++){
+        Layer& y = n.layer[l];
+        const int I4 = (y.I + 3) / 4;
+        y.fwd_tiles = (n.R / 4) * (y.S / 4); y.fwd_shift = lanes_of_a_tile(y.fwd_tiles, y.K4);
+        y.bwd_tiles = (n.R / 4) * I4; y.bwd_shift = l > 0 ? lanes_of_a_tile(y.bwd_tiles, y.S / 4) : 0;
+        y.by_S4 = divisor(y.S / 4); y.by_I4 = divisor(I4); y.by_I = divisor(y.I); y.by_row = divisor(y.I / 4); y.by_owner = divisor(l > 0 ? n.layer[l - 1].S : 1); y.by_across = divisor(y.across);
+    }
+    n.by_quads = divisor(n.quads); n.by_patches = divisor(n.n_patches); n.by_I0 = divisor(n.layer[0].I);
 }
 
 #ifdef __CUDACC__

@@ -251,10 +251,10 @@ constexpr size_t PPO_TEAM_SMEM = 220 * 1024;
 // rows per tile: one tile per CTA where the batch allows it
 static bool plan_ppo_net(const b200rl_mlp_shape* sh, int batch, int ctas, bool actor, int least, PpoNetArgs* w, size_t* smem){
     const int want = (batch + ctas - 1) / ctas, A = sh->dims[sh->n_layers - 1];
+    Net n;
+    if(!spread(sh, 1, least, &n) || n.n_patches > THREADS || n.n_params > PPO_TEAM_MAX_PARAMS || A > PPO_TEAM_MAX_ACTIONS) return false;
     for(int R = want >= 32 ? 32 : (want + 3) / 4 * 4; R >= 4; R -= 4){
-        Net n;
-        if(!team::plan(sh, 1, R, 0, false, least, &n)) continue;
-        if(n.n_patches > THREADS || n.n_params > PPO_TEAM_MAX_PARAMS || A > PPO_TEAM_MAX_ACTIONS) return false;
+        place(n, R, false);
         const int S = n.layer[n.n_layers - 1].S;
         int off = (n.end + 3) / 4 * 4;
         w->quads = n.quads + (actor ? (A + 3) / 4 : 0);
@@ -290,6 +290,7 @@ static bool choose_ppo(const b200rl_mlp_shape* actor, const b200rl_mlp_shape* cr
         if(pa == pc) break;
         least = (pa > pc ? pa : pc) - 2;
     }
+    complete(c.actor.net); complete(c.critic.net);
     c.smem = sa > sc ? sa : sc;
     c.bytes = ppo_exchange_bytes(c.actor) + ppo_exchange_bytes(c.critic) + sizeof(float) * 2 * (size_t)minibatches;
     *out = c;

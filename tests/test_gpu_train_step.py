@@ -122,3 +122,23 @@ def test_train_step_keeps_what_is_not_finite(lib, batch, I, dims, acts, value):
         assert torch.equal(torch.isfinite(got), torch.isfinite(want)), name
         if value != value:
             assert torch.equal(torch.isnan(got), torch.isnan(want)), name
+
+
+@pytest.mark.parametrize("rows,I,dims", [(256, 4, [256, 256, 1]), (5003, 33, [200, 200, 7]), (1024, 64, [64, 64, 64, 16]), (337, 8, [256, 256, 256, 3])])
+def test_the_plan_of_a_step_costs_little(lib, rows, I, dims):
+    """Every one-launch step looks for its plan among 32 candidates; the size query does nothing else of weight. 0.7 to 0.9 us, 4.9 to 7.2 where everything the kernel needs was made for each
+    of the candidates (least of many calls, less those of a call that returns at once)."""
+    import ctypes
+    import time
+    shape = lib.MlpShape.make(I, dims, ["tanh"] * len(dims))
+    query = lib.lib().b200rl_mlp_backward_scratch_bytes
+
+    def least(batch):
+        best = 1.0
+        for _ in range(100):
+            begin = time.perf_counter()
+            for _ in range(50):
+                query(ctypes.byref(shape), batch)
+            best = min(best, (time.perf_counter() - begin) / 50)
+        return best
+    assert least(rows) - least(0) < 2e-6

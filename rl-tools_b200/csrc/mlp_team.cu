@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
         const float* y = smem + a.y_off + (other ? a.y_alt : 0);
 #pragma unroll
         for(int l = 0; l < L; l++){
-            forward_layer<C, L, true>(n, l, n.layer[l].a + (l == 0 && other ? n.a_alt : 0), smem, rank, [&](int r, int unit, float4 value, float4 derivative){
+            forward_layer<C, L, true, false>(n, l, n.layer[l].a + (l == 0 && other ? n.a_alt : 0), smem, rank, nullptr, [&](int r, int unit, float4 value, float4 derivative){
                 const int at = r * last.S + unit;
                 const float4 target = *reinterpret_cast<const float4*>(y + at);
                 auto d = [&](float v, float wanted, float dv){ return row0 + r < a.rows ? d_pre(__fmul_rn(__fsub_rn(v, wanted), a.constant), dv) : 0.0f; };
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
             else sync_team<C>();
         }
 #pragma unroll
-        for(int l = L - 1; l > 0; l--) backward_layer<C>(n, l, smem, rank, (L - l) & 1);
+        for(int l = L - 1; l > 0; l--) backward_layer<C, false>(n, l, smem, rank, (L - l) & 1, nullptr);
         store_activations<L>(n, smem, smem + a.out_off, rank, row0, a.rows, keep_from, a.chunk_rows, a.pre, a.out);
         accumulate_gradients<N, PO, PI>(n, smem, patches, acc, other);
     }
@@ -157,7 +157,7 @@ static bool choose_team(const b200rl_mlp_shape* sh, int rows, size_t scratch_byt
             if(best == 0.0 || cost < best){ best = cost; *out = c; }
         }
     }
-    if(best > 0.0) complete(out->net);
+    if(best > 0.0) complete(out->net, false);
     return best > 0.0;
 }
 

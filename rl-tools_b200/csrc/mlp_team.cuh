@@ -26,7 +26,7 @@
 // The layers are unrolled: their sizes are then constants in the instructions, not loads at the head of every phase (64-64-64-4 at 64 rows 17.7 -> 16.4 us, 200-200-200-8 at 700 rows 57.6 -> 51.4,
 // 32-32-13 at 32 rows 12.3 -> 11.2).
 // Measured against products whose parts met in shared memory, element-wise passes behind them, 256 threads: 4-256-256-1 at 256 rows 28.7 -> 24.6 us a training step, 33-200-200-7 at 5,003 rows
-// 121 -> 103, PPO epochs of 27-64-64-8 with 2,048 rows 20.3 -> 15.9 us per minibatch. Packed multiply-adds (two per instruction) were slower here: 135 us for the second one, because the pairs
+// 121 -> 103, PPO epochs of 27-64-64-8 with 2,048 rows 20.8 -> 16.7 us per minibatch. Packed multiply-adds (two per instruction) were slower here: 135 us for the second one, because the pairs
 // take twice the registers.
 #pragma once
 #include "common.cuh"
@@ -50,6 +50,7 @@ struct Layer {
     long long poff, aoff;       // offset in the parameter arena (weights, then bias), in the activation arenas (x batch)
     int w, a, p, g, d;          // shared-memory offsets (floats): weight rows [S][P], input rows [R][P]; [R][S]: pre-activations, activation derivatives, d_pre
     int fwd_tiles, fwd_shift, bwd_tiles, bwd_shift;            // 4 x 4 tiles of a product; 2^shift lanes share out its summed index
+    int fwd_parts, bwd_parts;   // ORDERED: among so many of them
     int patch_begin, across;    // gradient patches: first index of this layer, patches along the inputs
     Divisor by_S4, by_I, by_row, by_I4, by_across, by_owner;
 };
@@ -76,6 +77,22 @@ inline int lanes_of_a_tile(int tiles, int K4){
     }
     return best;
 }
+
+// The same where the order of every sum is fixed (ORDERED, ppo_team.cu): the summed index of a tile is dealt out to a number of lanes that is part of the order, as many (a power of two) as
+// give 256 threads a part each, of at least two pieces of a forward and one of a backward product. Up to three lanes without a part come on top where that leaves threads idle: they take some
+// of the tile's rows to the end.
+constexpr int ORDERED_LANES = 256, ORDERED_SCRATCH = ORDERED_LANES * 16;      // the second: floats of add_parts_in_order
+inline int parts(int tiles, int pieces){
+    int s = 0;
+    while(s < 5 && (2 << s) * tiles <= ORDERED_LANES && (2 << s) <= pieces) s++;
+    return s;
+}
+inline int lanes_of_parts(int tiles, int parts){
+    while(parts < 2 && (2 << parts) * tiles <= ORDERED_LANES) parts++;
+    return parts;
+}
+inline int parts_forward(const Net& n, int l){ return parts((n.R / 4) * (n.layer[l].S / 4), (n.layer[l].I / 4 + 1) / 2); }
+inline int parts_backward(const Net& n, int l){ return parts((n.R / 4) * ((n.layer[l].I + 3) / 4), n.layer[l].S / 4); }
 
 // host: a plan is made in three parts, so that a search over team sizes and tiles pays for each of them once: what follows from the team size, what follows from the rows of a tile, and what
 // only the chosen plan needs (32 candidates of 4-256-256-1: 0.5 us, 6.7 with everything made for each of them).
@@ -137,13 +154,18 @@ inline void place(Net& n, int R, bool keep_pre){
     n.rb[1] = off; off += rb;
     n.end = off;
 }
-// What only the kernel reads: tiles, lanes and divisors
-inline void complete(Net& n){
+// What only the kernel reads: tiles, lanes and divisors. `ordered`: sums in the order of parts() and, with the bias column, in as many pieces as a weight row has
+inline void complete(Net& n, bool ordered){
     for(int l = 0; l < n.n_layers; l++){
         Layer& y = n.layer[l];
         const int I4 = (y.I + 3) / 4;
-        y.fwd_tiles = (n.R / 4) * (y.S / 4); y.fwd_shift = lanes_of_a_tile(y.fwd_tiles, y.K4);
-        y.bwd_tiles = (n.R / 4) * I4; y.bwd_shift = l > 0 ? lanes_of_a_tile(y.bwd_tiles, y.S / 4) : 0;
+        y.fwd_tiles = (n.R / 4) * (y.S / 4); y.bwd_tiles = (n.R / 4) * I4;
+        if(ordered){
+            y.K4 = y.I / 4 + 1;
+            y.fwd_parts = 1 << parts_forward(n, l); y.fwd_shift = lanes_of_parts(y.fwd_tiles, parts_forward(n, l));
+            y.bwd_parts = 1 << parts_backward(n, l); y.bwd_shift = lanes_of_parts(y.bwd_tiles, parts_backward(n, l));
+        }
+        else{ y.fwd_shift = lanes_of_a_tile(y.fwd_tiles, y.K4); y.bwd_shift = l > 0 ? lanes_of_a_tile(y.bwd_tiles, y.S / 4) : 0; }
         y.by_S4 = divisor(y.S / 4); y.by_I4 = divisor(I4); y.by_I = divisor(y.I); y.by_row = divisor(y.I / 4); y.by_owner = divisor(l > 0 ? n.layer[l - 1].S : 1); y.by_across = divisor(y.across);
     }
     n.by_quads = divisor(n.quads); n.by_patches = divisor(n.n_patches); n.by_I0 = divisor(n.layer[0].I);
@@ -274,12 +296,64 @@ __device__ __forceinline__ void add_parts(float4 (&v)[4], int shift, int lane){
     if(shift >= 4) add_to(v[0], exchange(v[0], 2));
 }
 
+// The same with the parts added in their order: of up to two parts there is one (lanes without a part hold zeros); four or more meet in shared memory, 64 bytes for each of ORDERED_LANES lanes,
+// which all have a part of one tile then
+__device__ __forceinline__ void add_parts_in_order(float4 (&v)[4], int n_parts, int shift, int lane, int warp, const Share& sh, float* scratch){
+    if(n_parts < 4){ add_parts(v, shift, lane); return; }
+    float4* rows = reinterpret_cast<float4*>(scratch) + 128 * warp;
+#pragma unroll
+    for(int i = 0; i < 4; i++) rows[32 * i + lane] = v[i];
+    __syncwarp();
+    const float4* from = rows + 32 * sh.first + sh.tile;
+    v[0] = from[0];
+#pragma unroll 4
+    for(int p = 1; p < 1 << shift; p++){ const float4 t = from[p << (5 - shift)]; v[0].x += t.x; v[0].y += t.y; v[0].z += t.z; v[0].w += t.w; }
+}
+
+// A lane's part of a 4 x 4 tile of a forward product: the pieces first, first + G, ... of four activation and four weight rows. PAIRS: even and odd summed indices apart, their sums added at the
+// end (packed multiply-adds; the pairs cost 16 more registers).
+template <bool PAIRS>
+__device__ __forceinline__ void tile_products(const float4* a, const float4* w, int P4, int S4, int first, int K4, int G, float4 (&v)[4]){
+    float2 pair[4][PAIRS ? 4 : 1];
+    float acc[4][PAIRS ? 1 : 4];
+#pragma unroll
+    for(int i = 0; i < 4; i++)
+#pragma unroll
+        for(int j = 0; j < 4; j++){ if constexpr(PAIRS) pair[i][j] = make_float2(0.0f, 0.0f); else acc[i][j] = 0.0f; }
+#pragma unroll 1
+    for(int k = first; k < K4; k += G){
+        float4 xv[4], wv[4];
+#pragma unroll
+        for(int i = 0; i < 4; i++) xv[i] = a[i * P4 + k];
+#pragma unroll
+        for(int j = 0; j < 4; j++) wv[j] = w[j * S4 * P4 + k];
+#pragma unroll
+        for(int i = 0; i < 4; i++)
+#pragma unroll
+            for(int j = 0; j < 4; j++){
+                if constexpr(PAIRS){
+                    pair[i][j] = __ffma2_rn(make_float2(xv[i].x, xv[i].y), make_float2(wv[j].x, wv[j].y), pair[i][j]);
+                    pair[i][j] = __ffma2_rn(make_float2(xv[i].z, xv[i].w), make_float2(wv[j].z, wv[j].w), pair[i][j]);
+                }
+                else{
+                    acc[i][j] = fmaf(xv[i].x, wv[j].x, acc[i][j]); acc[i][j] = fmaf(xv[i].y, wv[j].y, acc[i][j]);
+                    acc[i][j] = fmaf(xv[i].z, wv[j].z, acc[i][j]); acc[i][j] = fmaf(xv[i].w, wv[j].w, acc[i][j]);
+                }
+            }
+    }
+#pragma unroll
+    for(int i = 0; i < 4; i++){
+        if constexpr(PAIRS) v[i] = make_float4(pair[i][0].x + pair[i][0].y, pair[i][1].x + pair[i][1].y, pair[i][2].x + pair[i][2].y, pair[i][3].x + pair[i][3].y);
+        else v[i] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    }
+}
+
 // One layer of the forward pass; `a`: where its input rows lie. The values go into the next layer's input rows of the whole team; after the last layer
 // finish(row, first unit, values, derivatives) runs for every row and four units of this CTA. Ends without a barrier.
-template <int C, int L, bool KEEP_PRE, typename FINISH>
-__device__ __forceinline__ void forward_layer(const Net& n, int l, int a_rows, float* smem, int rank, FINISH finish){
+template <int C, int L, bool KEEP_PRE, bool ORDERED, typename FINISH>
+__device__ __forceinline__ void forward_layer(const Net& n, int l, int a_rows, float* smem, int rank, float* scratch, FINISH finish){
     const Layer& y = n.layer[l];
-    const int tid = thread_here(), lane = tid & 31, warp = tid >> 5, S4 = y.S >> 2, P4 = y.P >> 2, shift = y.fwd_shift, G = 1 << shift;
+    const int tid = thread_here(), lane = tid & 31, warp = tid >> 5, S4 = y.S >> 2, P4 = y.P >> 2, shift = y.fwd_shift, G = ORDERED ? y.fwd_parts : 1 << shift;
     const Share sh = share(shift, lane);
 #pragma unroll 1
     for(int t0 = warp << (5 - shift); t0 < y.fwd_tiles; t0 += WARPS << (5 - shift)){
@@ -287,33 +361,13 @@ __device__ __forceinline__ void forward_layer(const Net& n, int l, int a_rows, f
         const bool mine = t0 + sh.tile < y.fwd_tiles;
         const float4* a = reinterpret_cast<const float4*>(smem + a_rows) + rg * 4 * P4;
         const float4* w = reinterpret_cast<const float4*>(smem + y.w) + og * P4;
-        float acc[4][4];
-#pragma unroll
-        for(int i = 0; i < 4; i++)
-#pragma unroll
-            for(int j = 0; j < 4; j++) acc[i][j] = 0.0f;
-#pragma unroll 1
-        for(int k = sh.part; k < y.K4; k += G){
-            float4 xv[4], wv[4];
-#pragma unroll
-            for(int i = 0; i < 4; i++) xv[i] = a[i * P4 + k];
-#pragma unroll
-            for(int j = 0; j < 4; j++) wv[j] = w[j * S4 * P4 + k];
-#pragma unroll
-            for(int i = 0; i < 4; i++)
-#pragma unroll
-                for(int j = 0; j < 4; j++){
-                    acc[i][j] = fmaf(xv[i].x, wv[j].x, acc[i][j]); acc[i][j] = fmaf(xv[i].y, wv[j].y, acc[i][j]);
-                    acc[i][j] = fmaf(xv[i].z, wv[j].z, acc[i][j]); acc[i][j] = fmaf(xv[i].w, wv[j].w, acc[i][j]);
-                }
-        }
         float4 v[4];
-#pragma unroll
-        for(int i = 0; i < 4; i++) v[i] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-        add_parts(v, shift, lane);
+        tile_products<ORDERED>(a, w, P4, S4, sh.part < G ? sh.part : y.K4, y.K4, G, v);
+        if constexpr(ORDERED) add_parts_in_order(v, y.fwd_parts, shift, lane, warp, sh, scratch);
+        else add_parts(v, shift, lane);
         if(!mine) continue;                                              // no barrier or exchange below
         float4 bias = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if((y.I & 3) == 0){                                              // the bias column is not among the pieces summed
+        if(!ORDERED && (y.I & 3) == 0){                                  // the bias column is not among the pieces summed
             const float* b = smem + y.w + og * y.P + y.I;
             bias = make_float4(b[0], b[S4 * y.P], b[2 * S4 * y.P], b[3 * S4 * y.P]);
         }
@@ -375,12 +429,12 @@ __device__ __forceinline__ void store_activations(const Net& n, const float* sme
 
 // Input gradient of layer l > 0 from its d_pre (own units), then d_pre of layer l - 1 (own units): in teams of several CTAs by way of the owners of the inputs, through
 // one of two exchange buffers (`turn` alternates).
-template <int C>
-__device__ __forceinline__ void backward_layer(const Net& n, int l, float* smem, int rank, int turn){
+template <int C, bool ORDERED>
+__device__ __forceinline__ void backward_layer(const Net& n, int l, float* smem, int rank, int turn, float* scratch){
     const Layer& y = n.layer[l];
     const Layer& z = n.layer[l - 1];
     float* rb = smem + n.rb[turn];
-    const int tid = thread_here(), lane = tid & 31, warp = tid >> 5, I4 = (y.I + 3) >> 2, S4 = y.S >> 2, P4 = y.P >> 2, shift = y.bwd_shift, G = 1 << shift;
+    const int tid = thread_here(), lane = tid & 31, warp = tid >> 5, I4 = (y.I + 3) >> 2, S4 = y.S >> 2, P4 = y.P >> 2, shift = y.bwd_shift, G = ORDERED ? y.bwd_parts : 1 << shift;
     const Share sh = share(shift, lane);
     auto below = [&](int at, float4 v){
         const float4 dv = *reinterpret_cast<const float4*>(smem + z.g + at);
@@ -396,7 +450,7 @@ __device__ __forceinline__ void backward_layer(const Net& n, int l, float* smem,
 #pragma unroll
         for(int i = 0; i < 4; i++) v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 1
-        for(int o4 = sh.part; o4 < S4; o4 += G){
+        for(int o4 = sh.part < G ? sh.part : S4; o4 < S4; o4 += G){
             float4 dv[4], wv[4];
 #pragma unroll
             for(int i = 0; i < 4; i++) dv[i] = d[i * S4 + o4];
@@ -409,7 +463,8 @@ __device__ __forceinline__ void backward_layer(const Net& n, int l, float* smem,
                 for(int q = 0; q < 4; q++) v[i] = make_float4(fmaf(e[q], wv[q].x, v[i].x), fmaf(e[q], wv[q].y, v[i].y), fmaf(e[q], wv[q].z, v[i].z), fmaf(e[q], wv[q].w, v[i].w));
             }
         }
-        add_parts(v, shift, lane);
+        if constexpr(ORDERED) add_parts_in_order(v, y.bwd_parts, shift, lane, warp, sh, scratch);
+        else add_parts(v, shift, lane);
         if(!mine || sh.copy != 0) continue;
         const int owner = C == 1 ? 0 : quotient(i4 * 4, y.by_owner), col = i4 * 4 - owner * z.S;
 #pragma unroll 1
@@ -556,28 +611,33 @@ __device__ __forceinline__ float adam_update(float p, float g, float& m, float& 
 }
 
 // All CTAs of the grid share out the parameters: `lanes` threads per quad (a power of two from 4 on) add the teams' sums (thread y of a quad takes teams y, y + lanes, ... ascending,
-// then they are added pairwise: a fixed order), the first four each finish one parameter. Lanes of neighbouring quads lie side by side.
+// then they are added pairwise, neighbours first or, ORDERED, halves first: a fixed order), the first four each finish one parameter. Lanes of neighbouring quads lie side by side.
 struct Owner { int quad, part, step; };
 __device__ __forceinline__ Owner owner(int lanes, int cta, int ctas){
     const int bits = __popc(lanes - 1), per_warp = 32 >> bits, lane = threadIdx.x & 31;
     return Owner{(cta * WARPS + ((int)threadIdx.x >> 5)) * per_warp + (lane & (per_warp - 1)), lane >> (5 - bits), ctas * WARPS * per_warp};
 }
+template <bool ORDERED>
 __device__ __forceinline__ float sum_of_teams(const float4* partial, int u, int quads, int teams, int part, int lanes){
     float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if(u < quads){
         const float4* src = partial + u;
-        for(int t = part; t < teams; t += 8 * lanes){
-            float4 v[8];
+        constexpr int AHEAD = ORDERED ? 10 : 8;                          // loads under way; ten are the 74 teams of half the SMs over eight lanes
+        for(int t = part; t < teams; t += AHEAD * lanes){
+            float4 v[AHEAD];
 #pragma unroll
-            for(int k = 0; k < 8; k++) v[k] = t + k * lanes < teams ? __ldcg(src + (size_t)(t + k * lanes) * quads) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for(int k = 0; k < AHEAD; k++) v[k] = t + k * lanes < teams ? __ldcg(src + (size_t)(t + k * lanes) * quads) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-            for(int k = 0; k < 8; k++){ s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
+            for(int k = 0; k < AHEAD; k++){ s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
         }
     }
-    for(int o = 32 / lanes; o < 32; o <<= 1){
+    auto add = [&](int o){
         s.x += __shfl_xor_sync(0xffffffffu, s.x, o); s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
         s.z += __shfl_xor_sync(0xffffffffu, s.z, o); s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
-    }
+    };
+    const int least = 32 >> __popc(lanes - 1);
+    if(ORDERED) for(int o = 16; o >= least; o >>= 1) add(o);
+    else for(int o = least; o < 32; o <<= 1) add(o);
     return part == 0 ? s.x : part == 1 ? s.y : part == 2 ? s.z : s.w;
 }
 // sink(arena index, gradient, what prefetch(arena index) returned before the sums were loaded)
@@ -589,7 +649,7 @@ __device__ __forceinline__ void reduce_gradients(const Net& n, const float4* par
     for(int u0 = first; u0 < quads; u0 += me.step){
         const int u = u0 + me.quad - first, index = u < quads && me.part < 4 ? arena_index<L>(n, u, me.part) : -1;
         const auto early = prefetch(index);
-        const float g = sum_of_teams(partial, u, quads, teams, me.part, lanes);
+        const float g = sum_of_teams<false>(partial, u, quads, teams, me.part, lanes);
         if(index >= 0) sink(index, g, early);
     }
 }

@@ -5,8 +5,13 @@
 // takes its rows of a minibatch through the network (mlp_team.cuh, teams of one CTA), the row-wise loss gradient of the clipped surrogate or of
 // the value regression in between, writes its gradient sums, and behind a barrier over the network's CTAs every thread adds the sums of the one
 // parameter it owns and steps the optimizer for it, with the moments in registers for the whole epoch. A second barrier publishes the new
-// parameters, in quads of four neighbours of a weight row whose places in shared memory every CTA has a table of. log_std is a quad like the weights. Replaces the
+// parameters, in quads of four neighbours of a weight row whose places in shared memory every CTA has a table of; log_std is quads like the weights. Replaces the
 // per-minibatch body of train (rl/algorithms/ppo/operations_generic.h:159-336), per sample :214-296; Gaussian head random/operations_generic.h:87-121.
+//
+// The order of every sum is fixed (ORDERED in mlp_team.cuh): it follows from the networks and the rows of a minibatch by the rules of parts(), `lanes` below and the two orders of adding, and a
+// change for speed keeps it. The clipped surrogate jumps where a sample's ratio crosses the clipping bound, so a rounding of one sum becomes percents of the actor's first moments once a sample
+// has crossed: with sums in another order an update of 320 minibatches of 27-64-64-8 ended 4e-2 (2-norm, first moments) from this one for some data, 7e-7 for others. Sums in the order that suits
+// the lanes best take 15.9 us per minibatch of it (2,048 rows) and 14.4 of 3-64-64-1 (512 rows, with the loop around it), these 16.7 and 15.3.
 #include "common.cuh"
 #include "grid_barrier.cuh"
 #include "mlp_team.cuh"
@@ -24,6 +29,8 @@ struct PpoNetArgs {
     int ctas, teams, lanes, row_tiles;
     int quads;                               // those of the layers and, behind them, of log_std
     int aux, aux_alt, out;                   // shared memory: columns of a tile (actions [R][S], log-probabilities [R], advantages [R]; targets [R]), distance of the next tile's; outputs [R][S]
+    int std_warp;                            // the first of the warps that add the sums of log_std's quads
+    int scratch;                             // shared memory of add_parts_in_order
     int places, log_std;                     // where the weights of every quad go [quads]; log_std [action dimension rounded up to four]
     int lp, ps, dl;                          // the surrogate's log-probability terms [R][S], (action - mean) / std [R][S], dL / d log-probability [R]
     Divisor by_S;
@@ -97,9 +104,13 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
     if(has_rows) stage(0, cta, false);
     load_weights<L>(n, smem, w.params, 0);
     if(ACTOR && tid < A) smem[w.log_std + tid] = w.params[n.n_params + tid];
-    // the parameter this thread owns: `lanes` threads per quad, one pass over all quads (guaranteed by the host's choice of lanes)
-    const Owner me = owner(w.lanes, cta, w.ctas);
-    const int quads = w.quads, u = me.quad;
+    // the parameter this thread owns: `lanes` threads per quad of the layers, a warp behind them per quad of log_std, one pass over all quads (guaranteed by the host's choice of lanes)
+    Owner me = owner(w.lanes, cta, w.ctas);
+    const int quads = w.quads, std_quad = cta * WARPS + (tid >> 5) - w.std_warp;
+    int lanes = w.lanes;
+    if(me.quad >= n.quads) me.quad = quads;
+    if(ACTOR && std_quad >= 0 && std_quad < quads - n.quads){ me.quad = n.quads + std_quad; me.part = tid & 31; lanes = 32; }
+    const int u = me.quad;
     auto place_of_quad = [&](int q){ return ACTOR && q >= n.quads ? w.log_std + 4 * (q - n.quads) : weights_of_quad<L>(n, q); };
     int* places = reinterpret_cast<int*>(smem + w.places);
     for(int i = tid; i < quads; i += THREADS) places[i] = place_of_quad(i);
@@ -140,7 +151,7 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
             else if(mb + 1 < a.minibatches) stage(mb + 1, cta, !other);
 #pragma unroll
             for(int l = 0; l < L; l++){
-                forward_layer<1, L, false>(n, l, n.layer[l].a + (l == 0 && other ? n.a_alt : 0), smem, 0, [&](int r, int unit, float4 value, float4 derivative){
+                forward_layer<1, L, false, true>(n, l, n.layer[l].a + (l == 0 && other ? n.a_alt : 0), smem, 0, smem + w.scratch, [&](int r, int unit, float4 value, float4 derivative){
                     if constexpr(ACTOR) *reinterpret_cast<float4*>(smem + w.out + r * S + unit) = value;
                     else *reinterpret_cast<float4*>(smem + last.d + r * S + unit) =
                         make_float4(r < rows ? __fmul_rn(__fsub_rn(value.x, aux[r]), value_constant) * derivative.x : 0.0f, 0.0f, 0.0f, 0.0f);       // one output
@@ -196,7 +207,7 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
                 }
             }
 #pragma unroll
-            for(int l = L - 1; l > 0; l--) backward_layer<1>(n, l, smem, 0, 0);
+            for(int l = L - 1; l > 0; l--) backward_layer<1, true>(n, l, smem, 0, 0, smem + w.scratch);
             accumulate_gradients<N, PO, PI>(n, smem, patches, acc, other);
         }
         if(has_rows){
@@ -209,7 +220,7 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
         __syncthreads();
         if(!s_ok) break;
         const float c1 = s_scalars[0][mb & 63], c2 = s_scalars[1][mb & 63];
-        const float g = sum_of_teams(w.partial, adds ? u : quads, quads, w.teams, me.part, w.lanes);
+        const float g = sum_of_teams<true>(w.partial, adds ? u : quads, quads, w.teams, me.part, lanes);
         if(index >= 0){
             // log_std: the entropy bonus of every sample (:262-266); no gradient where it is not learnt
             my_g = !ACTOR || index < n.n_params ? g : a.learn_action_std ? g + (float)a.batch * (-1.0f / (float)a.batch * a.entropy_coefficient) : 0.0f;
@@ -263,13 +274,21 @@ static bool plan_ppo_net(const b200rl_mlp_shape* sh, int batch, int ctas, bool a
         w->places = off; off += (w->quads + 3) / 4 * 4;
         if(actor){ w->log_std = off; off += (A + 3) / 4 * 4; w->lp = off; off += R * S; w->ps = off; off += R * S; w->dl = off; off += R; }
         w->by_S = divisor(S);
+        bool in_parts = false;
+        for(int l = 0; l < n.n_layers; l++) in_parts = in_parts || parts_forward(n, l) > 1 || (l > 0 && parts_backward(n, l) > 1);
+        w->scratch = off; if(in_parts) off += ORDERED_SCRATCH;
         if(sizeof(float) * (size_t)off > PPO_TEAM_SMEM) continue;
         w->net = n; w->ctas = ctas; w->row_tiles = (batch + R - 1) / R; w->teams = w->row_tiles < ctas ? w->row_tiles : ctas;
-        // one parameter per thread, one pass: lanes x quads within the threads of the network's CTAs
-        const int quads = w->quads, threads = ctas * THREADS;
-        if(4ll * quads > threads) return false;
+        // How many threads add a quad's sums is part of their order: as many as give 256 threads of each CTA the pieces of four parameters that there are. One pass over the quads (of patches, whose
+        // edges are quads as well) has to fit all threads
+        int pieces = 0;
+        for(int l = 0; l < n.n_layers; l++) pieces += n.layer[l].S * (n.layer[l].I / 4 + 1);
         w->lanes = 4;
-        while(w->lanes < 32 && 2 * w->lanes <= w->teams && 2ll * w->lanes * quads <= threads) w->lanes *= 2;
+        while(w->lanes < 32 && 2 * w->lanes <= w->teams && 2ll * w->lanes * pieces <= ctas * ORDERED_LANES) w->lanes *= 2;
+        auto warps = [&](){ return (n.quads + 32 / w->lanes - 1) / (32 / w->lanes); };
+        while(w->lanes > 4 && warps() + w->quads - n.quads > ctas * WARPS) w->lanes /= 2;
+        w->std_warp = warps();
+        if(w->std_warp + w->quads - n.quads > ctas * WARPS) return false;
         *smem = sizeof(float) * (size_t)off;
         return true;
     }
@@ -290,7 +309,7 @@ static bool choose_ppo(const b200rl_mlp_shape* actor, const b200rl_mlp_shape* cr
         if(pa == pc) break;
         least = (pa > pc ? pa : pc) - 2;
     }
-    complete(c.actor.net); complete(c.critic.net);
+    complete(c.actor.net, true); complete(c.critic.net, true);
     c.smem = sa > sc ? sa : sc;
     c.bytes = ppo_exchange_bytes(c.actor) + ppo_exchange_bytes(c.critic) + sizeof(float) * 2 * (size_t)minibatches;
     *out = c;

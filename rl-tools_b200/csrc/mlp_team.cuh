@@ -362,7 +362,7 @@ __device__ __forceinline__ void forward_layer(const Net& n, int l, int a_rows, f
         const float4* a = reinterpret_cast<const float4*>(smem + a_rows) + rg * 4 * P4;
         const float4* w = reinterpret_cast<const float4*>(smem + y.w) + og * P4;
         float4 v[4];
-        tile_products<ORDERED>(a, w, P4, S4, sh.part < G ? sh.part : y.K4, y.K4, G, v);
+        tile_products<ORDERED>(a, w, P4, S4, ORDERED && sh.part >= G ? y.K4 : sh.part, y.K4, G, v);
         if constexpr(ORDERED) add_parts_in_order(v, y.fwd_parts, shift, lane, warp, sh, scratch);
         else add_parts(v, shift, lane);
         if(!mine) continue;                                              // no barrier or exchange below
@@ -450,7 +450,7 @@ __device__ __forceinline__ void backward_layer(const Net& n, int l, float* smem,
 #pragma unroll
         for(int i = 0; i < 4; i++) v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 1
-        for(int o4 = sh.part < G ? sh.part : S4; o4 < S4; o4 += G){
+        for(int o4 = ORDERED && sh.part >= G ? S4 : sh.part; o4 < S4; o4 += G){
             float4 dv[4], wv[4];
 #pragma unroll
             for(int i = 0; i < 4; i++) dv[i] = d[i * S4 + o4];

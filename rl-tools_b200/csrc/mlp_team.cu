@@ -31,6 +31,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
     extern __shared__ __align__(16) float smem[];
     __shared__ float s_scalars[2];
     __shared__ int s_ok;
+    __shared__ uint32_t s_age;
     const Net& n = a.net;
     const int tid = threadIdx.x, rank = C == 1 ? 0 : (int)cluster_rank(), t = blockIdx.x / C;
     const Layer& last = n.layer[L - 1];
@@ -64,6 +65,8 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
     __syncthreads();
     stage(t, false);
     load_weights<L>(n, smem, a.params, rank);
+    // the optimizer's age, too, is here before this CTA arrives at the grid barrier: once all have arrived, the first CTA may store the next one
+    if(tid == 0 && a.optimize) copy4_async(reinterpret_cast<float*>(&s_age), reinterpret_cast<const float*>(a.adam_state));
     Patch patches[N];
     Sums<N, PO, PI> acc;
 #pragma unroll
@@ -96,9 +99,8 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
     }
     store_gradients<N, PO, PI>(n, a.partial + (size_t)t * C * n.quads, rank, acc);
     __syncthreads();
-    const uint32_t age = a.optimize ? *reinterpret_cast<volatile uint32_t*>(a.adam_state) : 1u;
     if(tid == 0){ grid_barrier_arrive(a.barrier); s_ok = grid_barrier_wait(a.barrier, gridDim.x); }
-    else if(a.optimize && (tid == 32 || tid == 33)) s_scalars[tid - 32] = adam_bias_correction(tid == 32 ? a.hyper.beta_1 : a.hyper.beta_2, age);
+    else if(a.optimize && (tid == 32 || tid == 33)) s_scalars[tid - 32] = adam_bias_correction(tid == 32 ? a.hyper.beta_1 : a.hyper.beta_2, s_age);
     __syncthreads();
     if(!s_ok){ if(tid == 0) grid_barrier_leave(a.barrier, gridDim.x); return; }
     const float c1 = s_scalars[0], c2 = s_scalars[1];
@@ -114,7 +116,7 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_team_step_kernel(const __grid_
     reduce_gradients<C, L>(n, a.partial, a.teams, blockIdx.x, gridDim.x, a.lanes, prefetch, sink);
     if(blockIdx.x == 0){
         for(int i = n.n_params + tid; i < a.n_total; i += THREADS) sink(i, 0.0f, prefetch(i));      // parameters outside the layers: no gradient from this loss
-        if(tid == 0 && a.optimize){ a.adam_state[0] = age + 1u; a.adam_state[1] = 0u; a.adam_state[2] = __float_as_uint(c1); a.adam_state[3] = __float_as_uint(c2); }
+        if(tid == 0 && a.optimize){ a.adam_state[0] = s_age + 1u; a.adam_state[1] = 0u; a.adam_state[2] = __float_as_uint(c1); a.adam_state[3] = __float_as_uint(c2); }
     }
     if(tid == 0) grid_barrier_leave(a.barrier, gridDim.x);
 }

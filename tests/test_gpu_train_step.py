@@ -142,3 +142,22 @@ def test_the_plan_of_a_step_costs_little(lib, rows, I, dims):
             best = min(best, (time.perf_counter() - begin) / 50)
         return best
     assert least(rows) - least(0) < 2e-6
+
+
+@pytest.mark.parametrize("batch,I,dims", [(256, 4, [256, 256, 1]), (2048, 64, [64, 64, 16]), (700, 64, [320, 320, 16])])
+def test_every_cta_steps_with_the_age_of_its_step(lib, batch, I, dims):
+    """The first steps of an optimizer, whose corrections differ most from one to the next: each equals the optimizer's own kernel on the same gradients, in every parameter."""
+    import torch
+    acts = ["tanh"] * (len(dims) - 1) + ["identity"]
+    net, other = _net(lib, torch, batch, I, dims, acts, 5), _net(lib, torch, batch, I, dims, acts, 5)
+    for n in (net, other):
+        n.m.zero_(); n.v.zero_()
+        n.adam_state[0] = 1
+    x = torch.from_numpy(mg.det_normal(1, batch * I).reshape(batch, I)).cuda()
+    y = torch.from_numpy(mg.det_normal(2, batch * dims[-1]).reshape(batch, dims[-1])).cuda()
+    for step in range(100):
+        net.train_step(x, y, 1.0)
+        other.grads.copy_(net.grads)
+        other.step()
+        for name in ("params", "m", "v", "adam_state"):
+            assert torch.equal(getattr(net, name), getattr(other, name)), (step, name)

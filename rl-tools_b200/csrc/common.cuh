@@ -25,8 +25,8 @@ int cuda_fail(cudaError_t e, const char* where);
 // ---- launches that follow one another closely ------------------------------------------------------------------------------------------------
 // The passes of small networks are chains of dependent kernels of two to six microseconds, of which one is the way from the end of a kernel to the first instruction of the next.
 // A kernel launched by launch_after may start while the kernel before it on its stream still runs (programmatic stream serialization, also inside a captured graph). It opens with
-// after_predecessor(), in front of its first access to memory: every grid before it has then completed and its writes are visible. What it reads goes through opaque(), so that no
-// load through a read-only pointer can be moved in front of that. In the chain of kernels every one that was launched this way waits, so "before" reaches back to the first.
+// after_predecessor(), in front of its first access to memory: every grid before it has then completed and its writes are visible. A pointer that it
+// only reads through (const __restrict__, __ldg) goes through opaque(): such a load could be moved in front of that, others can not (the waits clobber memory). In the chain of kernels every one that was launched this way waits, so "before" reaches back to the first.
 // The wait comes first, then the start of the next kernel: triggered in front of the wait, a chain's kernels are resident several deep, and their blocks share SMs unevenly. us, ordinary
 // launches / trigger first / this: forward and backward of 4-256-256-1, 256 rows 27.9 / 28.1 / 24.9, 100 rows 23.0 / 24.3 / 20.1; evaluate 24-64-64-64-8, 256 rows 6.1 / 6.5 / 5.7.
 __device__ __forceinline__ void after_predecessor(){

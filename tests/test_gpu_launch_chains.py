@@ -70,3 +70,81 @@ def test_a_chain_of_launches_has_the_bits_of_launches_one_by_one(lib, hidden, ba
     for got in results[1:]:
         for a, b in zip(got, results[0]):
             assert torch.equal(a, b)
+
+
+def _digest(torch, tensors):
+    import hashlib
+    h = hashlib.sha256()
+    for t in tensors:
+        h.update(t.detach().contiguous().cpu().numpy().tobytes())
+    return h.hexdigest()
+
+
+def _off_policy(pkg, loops, torch, quadrotor, hidden):
+    """Runner step, replay sampling and SAC update, launch by launch: the environments' kernels, gather_batch, the sampling head, the target values and the min-value gradient."""
+    import numpy as np
+    import os
+    torch.manual_seed(hidden)
+    common = dict(hidden_dim=hidden, replay_capacity=1000, seed=hidden, use_graph=False)
+    if quadrotor:
+        fix = np.load(os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "l2f.npz"))
+        loop = loops.L2fSacLoop(pkg.L2fParameters.make(fix["dynamics"], float(fix["dt"])), fix["mdp"], fix["init"], n_envs=16, batch_size=100, **common)
+    else:
+        loop = loops.PendulumSacLoop(n_envs=3, batch_size=100, n_warmup_steps=50, episode_step_limit=40, **common)
+    for _ in range(130):
+        loop.step()
+    a = loop.agent
+    return [t for n in [a.actor] + a.critics for t in (n.params, n.grads, n.m, n.v)] + [t.params for t in a.critics_target] + [a.log_alpha, loop.states, loop.replay, loop.batch["oa_base"]]
+
+
+def _many_rows(pkg, torch, I, dims, rows):
+    """A training step over two chunks by the tensor-core kernels: padded inputs, chains, gradients, the reduction of their parts."""
+    gen = torch.Generator(device="cuda"); gen.manual_seed(rows)
+    net = pkg.Mlp(I, dims, ["tanh"] * (len(dims) - 1) + ["identity"], rows)
+    net.params.copy_((torch.rand(net.params.shape, device="cuda", generator=gen) - 0.5) * 0.2)
+    x, y = torch.randn(2 * rows, I, device="cuda", generator=gen), torch.randn(2 * rows, dims[-1], device="cuda", generator=gen)
+    for _ in range(5):
+        net.train_step(x, y, 0.5)
+    return [net.params, net.grads, net.m, net.v, net.pre, net.out]
+
+
+def _on_policy(loops, torch, n_envs, batch):
+    """Collect, advantages, shuffled epochs as one call each: row permutation, the statistics of the advantages, the epoch kernel."""
+    torch.manual_seed(batch)
+    loop = loops.PendulumPpoLoop(n_envs=n_envs, steps_per_env=64, batch_size=batch, n_epochs=5, seed=3)
+    for _ in range(3):
+        loop.step()
+    return [t for n in (loop.actor, loop.critic) for t in (n.params, n.grads, n.m, n.v)] + [loop.dataset]
+
+
+def _all_digests():
+    import importlib
+    import json
+    import torch
+    import __graft_entry__ as entry
+    pkg = entry.load_package()
+    loops = importlib.import_module("rl_tools_b200.loops")
+    out = {"pendulum 64": _off_policy(pkg, loops, torch, False, 64), "pendulum 256": _off_policy(pkg, loops, torch, False, 256), "quadrotor": _off_policy(pkg, loops, torch, True, 64),
+           "29-64-64-5": _many_rows(pkg, torch, 29, [64, 64, 5], 16387), "33-200-200-7": _many_rows(pkg, torch, 33, [200, 200, 7], 16390), "ppo": _on_policy(loops, torch, 64, 512)}
+    torch.cuda.synchronize()
+    print(json.dumps({k: _digest(torch, v) for k, v in out.items()}))
+
+
+def test_loops_and_large_steps_have_the_bits_of_launches_one_by_one():
+    """The chains inside native calls: the same program with every launch waited for by the driver (CUDA_LAUNCH_BLOCKING) and without, the second twice."""
+    import json
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+
+    def run(blocking):
+        env = dict(os.environ, CUDA_LAUNCH_BLOCKING="1" if blocking else "0", PYTHONPATH=os.pathsep.join([os.path.dirname(here), here, os.path.join(here, "golden")]))
+        r = subprocess.run([sys.executable, "-c", "import test_gpu_launch_chains as t; t._all_digests()"], env=env, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        return json.loads(r.stdout.splitlines()[-1])
+
+    want = run(True)
+    assert len(want) == 6
+    for _ in range(2):
+        assert run(False) == want

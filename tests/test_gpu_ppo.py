@@ -366,3 +366,32 @@ def test_gae_of_many_environments(lib, orc, torch, N, steps, kernel, pitch):
     call()
     adv, tgt = orc.gae(rewards[:n], values, terminated[:n], truncated[:n], N, steps)
     assert np.array_equal(columns[4][:n].cpu().numpy(), adv) and np.array_equal(columns[5][:n].cpu().numpy(), tgt)
+
+
+@pytest.mark.parametrize("n_rows,columns", [(1, [0, 2]), (4097, [0, 1, 5, 9]), (513, list(range(11)))])
+def test_shuffle_rows_is_the_permutation_and_the_move(lib, torch, n_rows, columns):
+    """Seven calls in a row on two sets of buffers and events, nothing waited for in between: dataset and engine as after shuffle_permutation_host and permute_rows."""
+    rs = np.random.RandomState(n_rows)
+    data = rs.randn(n_rows, 11).astype(np.float32)
+    got, want = torch.from_numpy(data).cuda(), torch.from_numpy(data).cuda()
+    engine, reference = lib.rng_init_host(7), lib.rng_init_host(7)
+    mask, scratch, nbytes = lib.permute_rows_scratch(got, n_rows, columns)
+    host, perm = torch.empty((2, n_rows), dtype=torch.int32, pin_memory=True), torch.empty((2, n_rows), dtype=torch.int32, device="cuda")
+    copies = torch.cuda.Stream()
+    used, sent = [torch.cuda.current_stream().record_event() for _ in range(2)], [copies.record_event() for _ in range(2)]
+
+    def call(k, rows=n_rows, scratch_bytes=nbytes, events=(True, True)):
+        return lib.lib().b200rl_shuffle_rows(got.data_ptr(), got.stride(0), rows, mask, engine.ctypes.data, host[k].data_ptr(), perm[k].data_ptr(), scratch.data_ptr(), scratch_bytes,
+                                             sent[k].cuda_event if events[0] else None, used[k].cuda_event if events[1] else None, copies.cuda_stream, torch.cuda.current_stream().cuda_stream)
+    for epoch in range(7):
+        assert call(epoch & 1) == 0
+    drawn = np.empty(n_rows, np.int32)
+    for _ in range(7):
+        assert lib.shuffle_permutation_host(reference, n_rows, out=drawn.ctypes.data) is None
+        lib.permute_rows(want, n_rows, torch.from_numpy(drawn).cuda(), columns)
+    assert torch.equal(got, want) and np.array_equal(engine, reference)
+    before = engine.copy()
+    for refused in (dict(scratch_bytes=nbytes - 1), dict(rows=-1), dict(events=(False, True)), dict(events=(True, False))):
+        assert call(0, **refused) == 1                                   # B200RL_ERR_INVALID_ARGUMENT, nothing drawn or moved
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and np.array_equal(engine, before)

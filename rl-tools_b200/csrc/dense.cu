@@ -646,7 +646,8 @@ static size_t outputs_before_last(const b200rl_mlp_shape* sh){
 
 // Which training steps take one launch (mlp_team.cu) rather than a launch per pass: those whose chunk of rows has little work. The one launch's time grows with rows x
 // weights from the start, on CUDA cores; the tensor-core kernels take the same time up to a row tile per SM. Measured, one launch against the sequence, us (rows x weights in
-// millions):
+// millions). Lines by work and width do not part all shapes: 300-256-256-10 at 1,024 rows (15 %), 64-256-256-256-16 at 1,024 (106 and 99), 64-320-320-16 at 2,048 (5 %), 17-300-300-300-3 at 256
+// (4 %) take the one launch although the sequence is faster, 64-256-256-16 at 3,072 (5 %) the sequence:
 //   sequence of mlp_chain.cu   64-256-256-16 at 2,048 (176): 78 and 103, at 3,072 (264): 106 and 111, at 4,096 (352): 143 and 113; 33-200-200-7 at 5,003 (240): 100 and 107, at 6,144
 //                              (295): 137 and 108; 33-200-200-200-7 at 2,048 (180): 101 and 122, at 3,072 (270): 140 and 136; 64-256-256-256-16 at 2,048 (310): 176 and 144;
 //                              narrower ones cross earlier: 64-128-128-16 at 8,192 (218): 70 and 74; 64-100-100-100-16 at 8,192 (229): 94 and 88; 64-100-100-16 (147): 50 and 72

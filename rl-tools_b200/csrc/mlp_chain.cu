@@ -624,7 +624,8 @@ __global__ void __launch_bounds__(1024) chain_image_kernel(const __grid_constant
 // ---- host side ---------------------------------------------------------------------------------------------------------------------------
 // Which passes run here: networks of two to eight layers, no wider than 256. A CTA takes 128 rows through all layers in the same time however few CTAs there
 // are (34 us for 64-256-256-256-16, 54 us when everything is kept; 14 and 18 us for 27-64-64-8), while the kernels per layer gain from a smaller batch and
-// start sooner; so the lines lie where the rows fill the SMs or the products are many. Measured, these kernels against the kernels per layer, us (graph of ten
+// start sooner; so the lines lie where the rows fill the SMs or the products are many. The lines for networks of at most 64 columns were drawn with one row tile per SM and still stand where they
+// were: with two, 3-32-32-1 would gain from the chain in the forward pass at 65,536 rows and 10-16-2 in the gradients at 16,384. Measured, these kernels against the kernels per layer, us (graph of ten
 // calls; rows x the network's weights in millions behind the rows):
 //   evaluate            4-256-256-1 at 2,048: 23 and 29; 64-256-16 at 2,048 (42): 17 and 15, at 4,096 (84): 17 and 28; 8-256-4 at 8,192 (25): 15 and 13, at 16,384
 //                       (50): 15 and 20; 64-128-4 at 8,192 (71): 14 and 13, at 16,384 (143): 15 and 17; 3-32-32-1 at 8,192 (9): 11 and 12, at 16,384 (19): 11 and 15

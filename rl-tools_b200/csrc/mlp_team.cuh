@@ -10,7 +10,7 @@
 //     (distributed shared memory), one cluster barrier per layer;
 //   - backward: the input gradient is a sum over the units, i.e. over the team: each CTA forms the partial sums of its own units for all inputs
 //     and stores each part into the CTA that owns that input, which adds the parts in a fixed order;
-//   - parameter gradients: a patch of 4, 8 outputs x 4, 8 inputs per thread, in registers over all row tiles of the launch. The bias is column I of the
+//   - parameter gradients: a patch of 4, 8 outputs x 4, 8 inputs per thread, or up to four of 4 x 4, in registers over all row tiles of the launch. The bias is column I of the
 //     weight row (its input is the constant 1 in column I of the activation rows).
 // A product of a layer is 4 x 4 register tiles with 16-byte shared-memory operands; the summed index of a tile is shared out over 1 ... 16 lanes of ONE warp, which
 // add their parts by shuffles and go on with what follows the product (bias, activation, derivative; derivative of the layer below) on the sums in
@@ -18,7 +18,8 @@
 // Teams write their gradient sums to scratch memory; after a grid-wide barrier all CTAs share out the parameters, add the teams' sums in a fixed
 // order and apply the optimizer step.
 //
-// Bound by shared-memory reads: a 16-byte read takes 4 cycles of an SM for a warp, 2 where all lanes of each half-phase read the same, so a 4 x 4 x 4 step costs 24 cycles of
+// A launch is bound by latency: counters of a PPO epoch of 27-64-64-8 (2,048 rows a minibatch) show 31 % of the issue slots used, the shared-memory pipe at 23 %, the multiply-adds at 16 %, and the
+// warps at barriers for 47 % of their time (those of the CTA between phases and those of the grid). Within a product the reads come before the multiply-adds: a 16-byte read takes 4 cycles of an SM for a warp, 2 where all lanes of each half-phase read the same, so a 4 x 4 x 4 step costs 24 cycles of
 // reads against 16 of multiply-adds; eight lanes in a row share the tile's rows (2 cycles) and read eight weight rows an odd number of 16 bytes apart
 // (4 cycles, no conflicts). Patches of 8 x 8 read 12 cycles for 32 of multiply-adds.
 //
@@ -26,8 +27,8 @@
 // The layers are unrolled: their sizes are then constants in the instructions, not loads at the head of every phase (64-64-64-4 at 64 rows 17.7 -> 16.4 us, 200-200-200-8 at 700 rows 57.6 -> 51.4,
 // 32-32-13 at 32 rows 12.3 -> 11.2).
 // Measured against products whose parts met in shared memory, element-wise passes behind them, 256 threads: 4-256-256-1 at 256 rows 28.7 -> 24.6 us a training step, 33-200-200-7 at 5,003 rows
-// 121 -> 103, PPO epochs of 27-64-64-8 with 2,048 rows 20.8 -> 16.7 us per minibatch. Packed multiply-adds (two per instruction) were slower here: 135 us for the second one, because the pairs
-// take twice the registers.
+// 121 -> 103, PPO epochs of 27-64-64-8 with 2,048 rows 20.8 -> 16.7 us per minibatch. Packed multiply-adds (two per instruction) were slower in the training step:
+// 135 us for the second one, because the pairs take twice the registers; the PPO epoch, whose order of sums has the pairs, holds smaller gradient patches.
 #pragma once
 #include "common.cuh"
 
@@ -489,7 +490,7 @@ __device__ __forceinline__ void backward_layer(const Net& n, int l, float* smem,
     __syncthreads();
 }
 
-// ---- parameter gradients: thread t owns the patch t (and t + THREADS) of the CTA's weight rows ---------------------------------------------
+// ---- parameter gradients: thread t owns the patches t, t + THREADS, ... (up to four) of the CTA's weight rows ------------------------------
 struct Patch { int d, a, pitch, alt; };                 // pitch: of the d_pre rows in the low half, of the input rows in the high half; alt: distance of the other input buffer
 // layer, first output quad and first input quad of a patch; patches ascend over the layers
 template <int L>

@@ -223,7 +223,7 @@ __device__ __forceinline__ void ppo_epoch(const PpoEpochArgs& a, const PpoNetArg
         const float g = sum_of_teams<true>(w.partial, adds ? u : quads, quads, w.teams, me.part, lanes);
         if(index >= 0){
             // log_std: the entropy bonus of every sample (:262-266); no gradient where it is not learnt
-            my_g = !ACTOR || index < n.n_params ? g : a.learn_action_std ? g + (float)a.batch * (-1.0f / (float)a.batch * a.entropy_coefficient) : 0.0f;
+            my_g = !ACTOR || index < n.n_params ? g : a.learn_action_std ? __fadd_rn(g, __fmul_rn((float)a.batch, -1.0f / (float)a.batch * a.entropy_coefficient)) : 0.0f;
             my_p = adam_update(my_p, my_g, my_m, my_v, w.hyper, c1, c2);
         }
         if(adds && me.part < 4) __stcg(w.fresh + 4 * u + me.part, my_p);

@@ -187,10 +187,12 @@ def test_order_of_the_sums_of_a_minibatch(lib, batch, obs, actions, hidden):
     for k in range(per_row.shape[1]):
         for r in range(R):
             s = s + per_row[:, k, r]
-    want_std = _over_teams(s, 32)
+    # the entropy bonus of every sample: a product and a sum, each rounded (at batches that are no power of two the product is not exact)
+    entropy = F(0.01)
+    want_std = _over_teams(s, 32) + F(batch) * (F(-1) / F(batch) * entropy)
 
     dataset = torch.from_numpy(data).cuda()
-    assert ppo._train_epoch(actor, critic, dataset, layout, 1, batch, epsilon_clip=0.2, entropy_coefficient=0.0, advantage_epsilon=1e-8, normalize_advantage=False, learn_action_std=True)
+    assert ppo._train_epoch(actor, critic, dataset, layout, 1, batch, epsilon_clip=0.2, entropy_coefficient=float(entropy), advantage_epsilon=1e-8, normalize_advantage=False, learn_action_std=True)
     assert np.array_equal(critic.grads.cpu().numpy(), want_critic)
     got = actor.grads.cpu().numpy()
     assert np.array_equal(got[:-actions], want_actor)

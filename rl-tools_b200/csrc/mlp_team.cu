@@ -130,9 +130,10 @@ constexpr int TEAM_MAX_ROWS = 8192;          // what was measured; up to there t
 // teams of C CTAs that are resident at once on the current device (clusters do not tile every GPC completely); 0: unknown
 static int team_capacity(int C);
 
-// Team size and rows per tile by an estimate of the launch: a layer of a tile costs its latencies (twice as much where the team exchanges through cluster barriers) and its
-// products, loading the weights and storing and adding the teams' sums cost per float. The constants, in no unit but their own, are fitted to all teams and tiles of 24 shapes (32 ... 256
-// wide, 2 to 4 layers, 32 ... 8,192 rows): 22 choices within 2 % of the fastest, the worst 7 % off (8-64-64-64-4 at 64 rows: 17.7 and 16.6 us).
+// Team size and rows per tile by an estimate of the launch: a layer of a tile costs its latencies (more where the team exchanges through cluster barriers) and its products, loading the weights
+// and storing and adding the teams' sums cost per float, the grid barrier and the sums per CTA. The constants, in no unit but their own, are fitted to all teams and tiles of 110 shapes (16 ... 256
+// wide, 2 to 4 layers, 32 ... 6,000 rows): the choice is 1.3 % from the fastest on average, the worst 9 % off (18-200-200-3 at 563 rows: 24.3 and 22.5 us). Without the cost of a CTA small
+// networks were spread too thin: 12-16-16-3 at 838 rows 12.7 us on 105 CTAs, 12.0 on 42; 5-100-100-2 at 50 rows 15.2 us on 13 CTAs, 13.6 in teams of four.
 // Only plans whose sums fit into scratch_bytes: the scratch of a smaller batch serves a larger one, by its own plan or a better one that fits.
 static bool choose_team(const b200rl_mlp_shape* sh, int rows, size_t scratch_bytes, TeamChoice* out){
     for(int l = 0, I = sh->input_dim; l < sh->n_layers; I = sh->dims[l], l++) if(sh->dims[l] > 512 || I > 512) return false;
@@ -154,8 +155,8 @@ static bool choose_team(const b200rl_mlp_shape* sh, int rows, size_t scratch_byt
             c.row_tiles = (rows + R - 1) / R;
             c.teams = c.row_tiles < max_teams ? c.row_tiles : max_teams;
             if(sizeof(float4) * (size_t)c.teams * C * c.net.quads > scratch_bytes) continue;
-            const double tile = (C == 1 ? 3800.0 : 7700.0) * c.net.n_layers + 0.12 * R * weights;
-            const double cost = 0.15 * weights + tile * ((c.row_tiles + c.teams - 1) / c.teams) + 1.8 * c.net.quads + 0.0016 * C * c.net.quads * c.teams;
+            const double tile = (C == 1 ? 3800.0 : 4700.0) * c.net.n_layers + 0.13 * R * weights;
+            const double cost = 0.15 * weights + tile * ((c.row_tiles + c.teams - 1) / c.teams) + 0.3 * c.net.quads + 0.0013 * C * c.net.quads * c.teams + 45.0 * C * c.teams;
             if(best == 0.0 || cost < best){ best = cost; *out = c; }
         }
     }

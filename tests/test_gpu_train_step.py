@@ -161,3 +161,26 @@ def test_every_cta_steps_with_the_age_of_its_step(lib, batch, I, dims):
         other.step()
         for name in ("params", "m", "v", "adam_state"):
             assert torch.equal(getattr(net, name), getattr(other, name)), (step, name)
+
+
+@pytest.mark.parametrize("batch,I,dims,ctas", [
+    (838, 12, [16, 16, 3], (20, 60)), (508, 5, [16, 16, 14], (20, 60)), (500, 3, [32, 32, 1], (25, 64)),       # a tile of several rows per CTA: fewer CTAs at the barrier
+    (50, 5, [100, 100, 2], (26, 104)), (80, 24, [100, 100, 2], (40, 148)), (700, 5, [100, 100, 100, 2], (100, 148)),      # few rows of wider layers: teams of several CTAs
+    (300, 20, [64, 64, 3], (60, 90))])
+def test_small_steps_are_spread_over_as_many_ctas_as_pay(lib, tmp_path, batch, I, dims, ctas):
+    """The plan's CTAs, whose number the launch shows; and the step by that plan against the separate calls."""
+    import json
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    net = _net(lib, torch, batch, I, dims, ["tanh"] * len(dims), 5)
+    x, y = torch.zeros(batch, I, device="cuda"), torch.zeros(batch, dims[-1], device="cuda")
+    net.train_step(x, y, 1.0)
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        net.train_step(x, y, 1.0)
+        torch.cuda.synchronize()
+    prof.export_chrome_trace(str(tmp_path / "trace.json"))
+    with open(tmp_path / "trace.json") as f:
+        grids = [e["args"]["grid"] for e in json.load(f)["traceEvents"] if e.get("cat") == "kernel" and "mlp_team_step" in e["name"]]
+    assert len(grids) == 1 and ctas[0] <= grids[0][0] <= ctas[1], grids
+    test_train_step_equals_the_separate_calls(lib, batch, 1, I, dims, ["tanh"] * (len(dims) - 1) + ["identity"])

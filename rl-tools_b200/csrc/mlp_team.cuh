@@ -31,6 +31,7 @@
 // 135 us for the second one, because the pairs take twice the registers; the PPO epoch, whose order of sums has the pairs, holds smaller gradient patches.
 #pragma once
 #include "common.cuh"
+#include <algorithm>
 
 namespace b200rl { namespace team {
 
@@ -82,7 +83,7 @@ inline int lanes_of_a_tile(int tiles, int K4){
 // The same where the order of every sum is fixed (ORDERED, ppo_team.cu): the summed index of a tile is dealt out to a number of lanes that is part of the order, as many (a power of two) as
 // give 256 threads a part each, of at least two pieces of a forward and one of a backward product. Up to three lanes without a part come on top where that leaves threads idle: they take some
 // of the tile's rows to the end.
-constexpr int ORDERED_LANES = 256, ORDERED_SCRATCH = ORDERED_LANES * 16;      // the second: floats of add_parts_in_order
+constexpr int ORDERED_LANES = 256;
 inline int parts(int tiles, int pieces){
     int s = 0;
     while(s < 5 && (2 << s) * tiles <= ORDERED_LANES && (2 << s) <= pieces) s++;
@@ -94,6 +95,17 @@ inline int lanes_of_parts(int tiles, int parts){
 }
 inline int parts_forward(const Net& n, int l){ return parts((n.R / 4) * (n.layer[l].S / 4), (n.layer[l].I / 4 + 1) / 2); }
 inline int parts_backward(const Net& n, int l){ return parts((n.R / 4) * ((n.layer[l].I + 3) / 4), n.layer[l].S / 4); }
+// Floats of shared memory that add_parts_in_order takes: 512 for each warp that has tiles of a product in four or more parts
+inline int ordered_scratch(const Net& n){
+    int warps = 0;
+    for(int l = 0; l < n.n_layers; l++){
+        const Layer& y = n.layer[l];
+        const int forward = parts_forward(n, l), backward = l > 0 ? parts_backward(n, l) : 0;
+        if(forward > 1) warps = std::max(warps, (((n.R / 4) * (y.S / 4) << forward) + 31) / 32);
+        if(backward > 1) warps = std::max(warps, (((n.R / 4) * ((y.I + 3) / 4) << backward) + 31) / 32);
+    }
+    return 512 * warps;
+}
 
 // host: a plan is made in three parts, so that a search over team sizes and tiles pays for each of them once: what follows from the team size, what follows from the rows of a tile, and what
 // only the chosen plan needs (32 candidates of 4-256-256-1: 0.5 us, 6.7 with everything made for each of them).
@@ -297,7 +309,7 @@ __device__ __forceinline__ void add_parts(float4 (&v)[4], int shift, int lane){
     if(shift >= 4) add_to(v[0], exchange(v[0], 2));
 }
 
-// The same with the parts added in their order: of up to two parts there is one (lanes without a part hold zeros); four or more meet in shared memory, 64 bytes for each of ORDERED_LANES lanes,
+// The same with the parts added in their order: of up to two parts there is one (lanes without a part hold zeros); four or more meet in shared memory, 64 bytes for each lane,
 // which all have a part of one tile then
 __device__ __forceinline__ void add_parts_in_order(float4 (&v)[4], int n_parts, int shift, int lane, int warp, const Share& sh, float* scratch){
     if(n_parts < 4){ add_parts(v, shift, lane); return; }

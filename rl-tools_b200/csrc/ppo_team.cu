@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(THREADS, 1) ppo_epoch_kernel(const __grid_cons
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------------------------------
-constexpr size_t PPO_TEAM_SMEM = 220 * 1024;
+constexpr size_t PPO_TEAM_SMEM = 220 * 1024, PPO_TEAM_MOST_SMEM = 225 * 1024;      // the second: for the smallest tiles, which nothing smaller can stand in for (1.3 KB more are static)
 
 // rows per tile: one tile per CTA where the batch allows it
 static bool plan_ppo_net(const b200rl_mlp_shape* sh, int batch, int ctas, bool actor, int least, PpoNetArgs* w, size_t* smem){
@@ -274,10 +274,8 @@ static bool plan_ppo_net(const b200rl_mlp_shape* sh, int batch, int ctas, bool a
         w->places = off; off += (w->quads + 3) / 4 * 4;
         if(actor){ w->log_std = off; off += (A + 3) / 4 * 4; w->lp = off; off += R * S; w->ps = off; off += R * S; w->dl = off; off += R; }
         w->by_S = divisor(S);
-        bool in_parts = false;
-        for(int l = 0; l < n.n_layers; l++) in_parts = in_parts || parts_forward(n, l) > 1 || (l > 0 && parts_backward(n, l) > 1);
-        w->scratch = off; if(in_parts) off += ORDERED_SCRATCH;
-        if(sizeof(float) * (size_t)off > PPO_TEAM_SMEM) continue;
+        w->scratch = off; off += ordered_scratch(n);
+        if(sizeof(float) * (size_t)off > (R > 4 ? PPO_TEAM_SMEM : PPO_TEAM_MOST_SMEM)) continue;
         w->net = n; w->ctas = ctas; w->row_tiles = (batch + R - 1) / R; w->teams = w->row_tiles < ctas ? w->row_tiles : ctas;
         // How many threads add a quad's sums is part of their order: as many as give 256 threads of each CTA the pieces of four parameters that there are. One pass over the quads (of patches, whose
         // edges are quads as well) has to fit all threads
@@ -323,7 +321,7 @@ static int launch_ppo_epoch(const PpoEpochArgs& a, size_t smem, cudaStream_t s){
     int rc = current_device(&dev);
     if(rc) return rc;
     if(!configured[dev].load(std::memory_order_acquire)){
-        B200RL_CUDA_TRY(cudaFuncSetAttribute(ppo_epoch_kernel<L, PO, PI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PPO_TEAM_SMEM));
+        B200RL_CUDA_TRY(cudaFuncSetAttribute(ppo_epoch_kernel<L, PO, PI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PPO_TEAM_MOST_SMEM));
         configured[dev].store(true, std::memory_order_release);
     }
     PpoEpochArgs copy = a;

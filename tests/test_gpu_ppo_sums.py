@@ -142,14 +142,14 @@ def _split(net, I, dims):
 
 
 # one tile per team and three; sums in 1 to 16 parts; inputs with the bias in their last piece and in one of its own; patches of each size
-@pytest.mark.parametrize("batch,obs,actions,hidden", [(2048, 27, 8, [64, 64]), (150, 27, 3, [64, 64]), (3001, 8, 1, [32, 33]), (40, 5, 6, [16, 12]), (700, 30, 2, [100, 96]), (260, 3, 4, [64, 64])])
+@pytest.mark.parametrize("batch,obs,actions,hidden", [(2048, 27, 8, [64, 64]), (150, 27, 3, [64, 64]), (3001, 8, 1, [32, 33]), (40, 5, 6, [16, 12]), (700, 30, 2, [100, 96]), (260, 3, 4, [64, 64]), (150, 3000, 3, [4])])
 def test_order_of_the_sums_of_a_minibatch(lib, batch, obs, actions, hidden):
     import torch
     from rl_tools_b200 import ppo
     assert torch.cuda.get_device_properties(0).multi_processor_count == 148
     layout = ppo.DatasetLayout(obs, actions)
     data = mg.det_normal(3, batch * layout.data_dim).reshape(batch, layout.data_dim).astype(F)
-    acts = ["relu", "relu", "identity"]
+    acts = ["relu"] * len(hidden) + ["identity"]
     actor, critic = _net(lib, torch, batch, obs, hidden + [actions], acts, 20, extra=actions), _net(lib, torch, batch, obs, hidden + [1], acts, 30)
     actor.extra("params").fill_(0.0)                                     # standard deviation 1
     ctas = 74
@@ -171,7 +171,7 @@ def test_order_of_the_sums_of_a_minibatch(lib, batch, obs, actions, hidden):
     mean = x
     for l, (W, b) in enumerate(layers[actor]):
         mean = _forward(W, b, mean, R)
-        if l < 2:
+        if l < len(hidden):
             mean = np.maximum(mean, 0)
     ps = data[:, layout.actions] - mean
     terms, log_prob = _log_density(ps), np.zeros(batch, F)

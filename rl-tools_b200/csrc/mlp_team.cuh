@@ -26,7 +26,7 @@
 // Loops over elements stay rolled: a minibatch walks the whole code once, and what does not fit the instruction caches is fetched anew for every one of them.
 // The layers are unrolled: their sizes are then constants in the instructions, not loads at the head of every phase (64-64-64-4 at 64 rows 17.7 -> 16.4 us, 200-200-200-8 at 700 rows 57.6 -> 51.4,
 // 32-32-13 at 32 rows 12.3 -> 11.2).
-// Measured against products whose parts met in shared memory, element-wise passes behind them, 256 threads: 4-256-256-1 at 256 rows 28.7 -> 24.6 us a training step, 33-200-200-7 at 5,003 rows
+// Measured against products whose parts met in shared memory, element-wise passes behind them, 256 threads: 4-256-256-1 at 256 rows 28.7 -> 24.3 us a training step, 33-200-200-7 at 5,003 rows
 // 121 -> 103, PPO epochs of 27-64-64-8 with 2,048 rows 20.8 -> 16.7 us per minibatch. Packed multiply-adds (two per instruction) were slower in the training step:
 // 135 us for the second one, because the pairs take twice the registers; the PPO epoch, whose order of sums has the pairs, holds smaller gradient patches.
 #pragma once

@@ -141,7 +141,7 @@ def test_the_plan_of_a_step_costs_little(lib, rows, I, dims):
                 query(ctypes.byref(shape), batch)
             best = min(best, (time.perf_counter() - begin) / 50)
         return best
-    assert least(rows) - least(0) < 2e-6
+    assert least(rows) - least(0) < 3e-6                                  # between the two, with room for a slower host
 
 
 @pytest.mark.parametrize("batch,I,dims", [(256, 4, [256, 256, 1]), (2048, 64, [64, 64, 16]), (700, 64, [320, 320, 16])])
